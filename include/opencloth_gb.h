@@ -340,7 +340,7 @@ oc_status oc_tune_cache_store(const char* path, const char* key, const oc_launch
  * oc_get_state / oc_get_stats, after which the handle steps on (a cloth whose solve had
  * not ended got no update).  For tests of that path: from the next step on, block
  * `withhold_block` of those launches returns before its first arrival (-1: none), and a
- * wait gives up after `max_polls` polls (0: the default, about half a second).  Nothing
+ * wait gives up after `max_polls` polls (0: the default, about a second).  Nothing
  * waits longer than that bound.  Fails with OC_ERR_UNSUPPORTED when the handle runs no
  * persistent CG. */
 oc_status oc_test_barrier_timeout(oc_solver* s, int32_t withhold_block, uint32_t max_polls);

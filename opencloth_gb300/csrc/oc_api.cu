@@ -18,6 +18,7 @@
 #include <new>
 #include <sstream>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "oc_internal.h"
@@ -73,7 +74,9 @@ struct oc_solver {
     std::vector<BlockInfo> h_blocks;
     int sm_count = 0;
     bool coop = false;
-    int persist_per_sm = 0;
+    // Dynamic shared memory a CTA of k_cg_persist may have (0: not available), and its
+    // co-resident clusters of kPersistMaxCluster and of 2 CTAs.
+    int persist_smem_max = 0, persist_clusters = 0, persist_pairs = 0;
     // Grid cloths' stencil data on the host, to refit the parameter slots when
     // oc_set_spring_params changes Ks or Kd, and each cloth's grid shape as detected
     // ({0, 0}: not a grid).
@@ -88,16 +91,15 @@ struct oc_solver {
     // The CG loop of the streamed REFERENCE cloths as one cooperative launch (k_cg_persist)
     // when there is no COUPLED cloth; otherwise the WHILE loop.
     bool persist = false;
-    int persist_grid = 0;
+    PersistPlan pplan{};  // the streamed REFERENCE cloths' pieces (grid 0: none, or not available)
     // k_assemble_finish runs when a strip-swept cloth is resident or the streamed CG is
     // not the persistent one; otherwise k_cg_persist forms their delta0 itself.
     bool strip_finish = true;
-    unsigned* d_words = nullptr;  // k_cg_persist: one arrival count per cloth
-    int* d_perr = nullptr;        // bit 0: a wait of k_cg_persist gave up
-    // The adjoint solve (every cloth iterates) as one cooperative launch of k_cg_persist
-    // without the update, when the handle has no COUPLED cloth.
+    int* d_perr = nullptr;  // bit 0: a wait of k_cg_persist gave up
+    // The adjoint solve (every cloth iterates) on chip and in one cooperative launch of
+    // k_cg_persist without the update, when the handle has no COUPLED cloth.
+    bool adj_allowed = false;  // not switched off, a device with cooperative launch
     bool adj_persist = false;
-    int adj_persist_grid = 0;
     bool any_provot = false;  // some cloth has OC_PASS_PROVOT: k_provot follows the update
     bool any_passes = false;  // some cloth has a pass after the update
     // Resident buckets run concurrently: forked from the handle's stream onto these.
@@ -183,8 +185,7 @@ oc_status fail_cuda(oc_solver* s, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return fail_cuda(s, e_, #call); \
     } while (0)
 
-// Polls of a cloth's arrival count before a wait of k_cg_persist gives up (about half
-// a second with its 32 ns back-off).
+// Polls of the packets before a wait of k_cg_persist gives up (about a second).
 constexpr uint32_t kDefaultBarrierPolls = 1u << 22;
 
 // A wait of k_cg_persist that gave up (the stream is synchronised).  The error word is
@@ -203,14 +204,6 @@ oc_status check_device_error(oc_solver* s) {
     }
     return OC_OK;
 }
-
-// k_cg_persist over block table a.blocks[0, n): its cloths' arrival counts zeroed, then
-// the cooperative launch.
-cudaError_t persist_cg(oc_solver* s, const StepArgs& a, int32_t n, int grid) {
-    cudaError_t e = cudaMemsetAsync(s->d_words, 0, sizeof(unsigned) * (size_t)s->n_inst, s->stream);
-    return e == cudaSuccess ? launch_cg_persist(a, n, grid, s->d_words, s->d_perr, s->stream) : e;
-}
-
 
 // Whether a grid cloth that may take the strip sweep should: its warps own 28 columns
 // each, so narrow cloths leave lanes idle.  With cfg.strip = 0 every grid cloth stays on
@@ -231,16 +224,6 @@ cudaError_t dalloc(oc_solver* s, T** p, size_t count) {
     if (e == cudaSuccess) s->allocs.push_back(q);
     *p = static_cast<T*>(q);
     return e;
-}
-
-// The persistent CG's words (once per handle).
-oc_status alloc_persist_words(oc_solver* s) {
-    if (s->d_words) return OC_OK;
-    OC_TRY(dalloc(s, &s->d_words, (size_t)s->n_inst));
-    OC_TRY(cudaMemset(s->d_words, 0, sizeof(unsigned) * (size_t)s->n_inst));
-    OC_TRY(dalloc(s, &s->d_perr, 1));
-    OC_TRY(cudaMemset(s->d_perr, 0, sizeof(int)));
-    return OC_OK;
 }
 
 template <class T>
@@ -494,7 +477,7 @@ oc_status step_host_driven(oc_solver* s, float dt, bool per_cloth, KernelTimer* 
         if (s->persist) {
             if (t) OC_TRY(cudaEventRecord(t->ev[0], s->stream));
             sa.persist_d0 = 1;
-            OC_TRY(persist_cg(s, sa, nb, s->persist_grid));
+            OC_TRY(launch_cg_persist(sa, s->pplan, s->stream));
             s->host_launches += 1;
             if (t) {
                 OC_TRY(cudaEventRecord(t->ev[1], s->stream));
@@ -657,8 +640,8 @@ oc_status build_graph(oc_solver* s, float dt) {
         updates.push_back(n_int);
     }
     if (persist) {
-        // The streamed cloths' whole CG loop and update: the memset of their completion
-        // words and the cooperative launch, captured into a child graph.
+        // The streamed cloths' whole CG loop and update: the cooperative launch, captured
+        // into a child graph.
         cudaGraphNode_t n_pc;
         cudaGraph_t pg = nullptr;
         OC_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
@@ -666,7 +649,7 @@ oc_status build_graph(oc_solver* s, float dt) {
         pa.blocks = s->d_streamed_blocks;
         pa.use_cond = 0;
         pa.persist_d0 = 1;
-        cudaError_t le = persist_cg(s, pa, s->n_streamed_blocks, s->persist_grid);
+        cudaError_t le = launch_cg_persist(pa, s->pplan, s->stream);
         cudaError_t ce = cudaStreamEndCapture(s->stream, &pg);
         if (le != cudaSuccess || ce != cudaSuccess) {
             if (pg) cudaGraphDestroy(pg);
@@ -781,22 +764,14 @@ StepArgs gm_args(const oc_solver* s, float dt) {
 
 // The CG alone (no update) of every cloth, from the CG state set up in the planes and
 // the cloths' states: the resident cloths on chip (k_resident unfused, one launch per
-// bucket, beside) and the streamed ones in one cooperative launch of k_cg_persist over
-// the streamed block table.  A handle whose plan has no resident bucket runs every cloth
-// in k_cg_persist.
+// bucket, beside) and the streamed ones in one cooperative launch of k_cg_persist.
 oc_status solve_only(oc_solver* s, const StepArgs& a) {
     StepArgs pa = a;
     pa.cg_only = 1;
-    if (s->buckets.empty()) {
-        OC_TRY(persist_cg(s, pa, s->n_blocks, s->adj_persist_grid));
-        s->host_launches += 1;
-        return OC_OK;
-    }
-    if (oc_status r = launch_resident_all(s, pa, nullptr)) return r;
-    if (s->n_streamed_blocks > 0) {
-        pa.blocks = s->d_streamed_blocks;
-        const int grid = std::min(s->persist_per_sm * s->sm_count, std::max(1, s->n_streamed_blocks));
-        OC_TRY(persist_cg(s, pa, s->n_streamed_blocks, grid));
+    if (!s->buckets.empty())
+        if (oc_status r = launch_resident_all(s, pa, nullptr)) return r;
+    if (s->pplan.grid > 0) {
+        OC_TRY(launch_cg_persist(pa, s->pplan, s->stream));
         s->host_launches += 1;
     }
     return OC_OK;
@@ -961,6 +936,130 @@ void drop_graphs(oc_solver* s) {
     }
 }
 
+// The persistent CG's plan.  At most one CTA per SM, each with at least kPersistThreads
+// vertices where there are that many (a thread then holds one vertex, and fewer CTAs have fewer
+// packets to wait for).  When there are no more cloths than CTAs every cloth gets CTAs of its
+// own, so that a CTA has one piece (PersistPlan::one); otherwise the cloths' vertices, one
+// cloth after another, are cut into one range per CTA.  The CTAs form clusters of
+// kPersistMaxCluster when those, which leave some SMs idle, hold every vertex on chip, else of
+// 2 (see oc_persist.cu for the exchanges' times).  Left without a grid when the device has no
+// cooperative launch or a CTA would hold too many pieces.
+oc_status plan_persist(oc_solver* s) {
+    PersistPlan& P = s->pplan;
+    P.grid = 0;
+    if (!s->coop || s->persist_smem_max <= 0) return OC_OK;
+    std::vector<int32_t> ids;
+    int64_t total = 0;
+    for (int32_t k = 0; k < s->n_inst; ++k)
+        if (!s->resident[(size_t)k]) {
+            ids.push_back(k);
+            total += s->inst_host[(size_t)k].nv;
+        }
+    std::vector<PersistPiece> pieces;
+    std::vector<int32_t> cta_piece;
+    // The cut for clusters of `cluster` CTAs and at most `most` CTAs.
+    auto cut = [&](int32_t cluster, int64_t most) {
+        pieces.clear();
+        cta_piece.assign(1, 0);
+        P.cluster = cluster;
+        P.n_packets = 0;
+        P.one = (int64_t)ids.size() <= most;
+        int64_t want = std::min(most, (total + kPersistThreads - 1) / kPersistThreads);
+        want = std::min(most, (want + cluster - 1) / cluster * cluster);
+        int64_t chunk = ((total + want - 1) / want + 31) / 32 * 32;
+        auto ctas_of = [&](int32_t k) { return (s->inst_host[(size_t)k].nv + chunk - 1) / chunk; };
+        if (P.one)
+            for (;; chunk += 32) {
+                int64_t n = 0;
+                for (int32_t k : ids) n += ctas_of(k);
+                if (n <= most) break;
+            }
+        int32_t open_slots = 0, max_slots = 0;  // of the CTA being filled, of any
+        int64_t open_n = 0;
+        auto close = [&] {
+            cta_piece.push_back((int32_t)pieces.size());
+            open_slots = 0;
+            open_n = 0;
+        };
+        for (int32_t k : ids) {
+            const InstParams& ip = s->inst_host[(size_t)k];
+            const size_t p0 = pieces.size();
+            const int32_t c0 = (int32_t)cta_piece.size() - 1;  // the CTA it starts in
+            const bool behind = (int32_t)p0 > cta_piece.back();
+            int64_t cap = chunk;
+            if (P.one) cap = ((ip.nv + ctas_of(k) - 1) / ctas_of(k) + 31) / 32 * 32;
+            for (int32_t l = 0; l < ip.nv;) {
+                const int32_t n = (int32_t)std::min<int64_t>(cap - open_n, ip.nv - l);
+                PersistPiece pc{};
+                pc.inst = k;
+                pc.head = l == 0;
+                pc.v = ip.v_off + l;
+                pc.n = n;
+                pc.slot0 = open_slots;
+                open_slots += (n + kPersistThreads - 1) / kPersistThreads;
+                pc.slot1 = open_slots;
+                max_slots = std::max(max_slots, open_slots);
+                pieces.push_back(pc);
+                l += n;
+                open_n += n;
+                if (open_n == cap || (P.one && l == ip.nv)) close();
+            }
+            const int32_t c1 = c0 + (int32_t)(pieces.size() - p0) - 1;  // the CTA it ends in
+            const int32_t n_cl = c1 / cluster - c0 / cluster + 1;
+            for (int32_t c = c0; c <= c1; ++c) {
+                PersistPiece& pc = pieces[p0 + (size_t)(c - c0)];
+                const int32_t first = std::max(c0, c / cluster * cluster);
+                pc.rank0 = first % cluster;
+                pc.ranks = std::min(c1, c / cluster * cluster + cluster - 1) - first + 1;
+                pc.tail = first == c0 && behind;
+                pc.clusters = n_cl;
+                pc.k = c / cluster - c0 / cluster;
+                pc.packet = P.n_packets;
+                pc.full = c0 % cluster == 0 && c1 % cluster == cluster - 1;
+            }
+            if (n_cl > 1) P.n_packets += n_cl * cluster;
+        }
+        if (open_n > 0) close();
+        // A last cluster's CTAs beyond the vertices take part with no piece (an empty one when
+        // every CTA has one).
+        while (((int64_t)cta_piece.size() - 1) % cluster != 0) {
+            if (P.one) pieces.push_back(PersistPiece{});
+            close();
+        }
+        P.max_pieces = 0;
+        for (size_t b = 0; b + 1 < cta_piece.size(); ++b)
+            P.max_pieces = std::max(P.max_pieces, cta_piece[b + 1] - cta_piece[b]);
+        P.max_slots = max_slots;
+        persist_layout(&P, s->persist_smem_max);
+    };
+    if (s->persist_clusters > 0) cut(kPersistMaxCluster, (int64_t)kPersistMaxCluster * s->persist_clusters);
+    if (s->persist_clusters <= 0 || !P.on_chip) {
+        const int all = std::max(1, s->sm_count);
+        cut(2 * s->persist_pairs >= all ? 2 : 1, all);
+    }
+    if (P.smem > (size_t)s->persist_smem_max) return OC_OK;
+    auto put = [&](auto** p, const auto& v) {
+        auto* q = const_cast<std::remove_const_t<std::remove_pointer_t<std::remove_reference_t<decltype(*p)>>>*>(*p);
+        const cudaError_t e = reupload(s, &q, v);
+        *p = q;
+        return e;
+    };
+    OC_TRY(put(&P.pieces, pieces));
+    OC_TRY(put(&P.cta_piece, cta_piece));
+    dfree(s, &P.packets);
+    OC_TRY(dalloc(s, &P.packets, 2 * (size_t)P.n_packets));
+    OC_TRY(cudaMemset(P.packets, 0, std::max<size_t>(1, 2 * (size_t)P.n_packets) * sizeof(ulonglong2)));
+    if (!P.ctl) {
+        OC_TRY(dalloc(s, &P.ctl, 1));
+        OC_TRY(cudaMemset(P.ctl, 0, sizeof(PersistCtl)));
+        OC_TRY(dalloc(s, &s->d_perr, 1));
+        OC_TRY(cudaMemset(s->d_perr, 0, sizeof(int)));
+        P.err = s->d_perr;
+    }
+    P.grid = (int32_t)cta_piece.size() - 1;
+    return OC_OK;
+}
+
 // The launch plan from the handle's cloths and its launch configuration: which cloths run
 // resident (one cluster per cloth, the whole step on chip) and which streamed, resident
 // cloths grouped by launch shape into buckets, the assembly tables (record gather,
@@ -1063,14 +1162,11 @@ oc_status plan_execution(oc_solver* s) {
         any_coupled |= s->inst_host[(size_t)k].coupled != 0;
         any_streamed |= !s->resident[(size_t)k] && !s->inst_host[(size_t)k].coupled;
     }
-    s->persist = false;
-    const int pgrid = std::min(s->persist_per_sm * s->sm_count, std::max(1, s->n_streamed_blocks));
-    if (cfg.persist && s->coop && s->persist_per_sm > 0 && any_streamed && !any_coupled &&
-        (int64_t)s->n_streamed_blocks <= (int64_t)persist_max_entries_per_block() * pgrid) {
-        s->persist = true;
-        s->persist_grid = pgrid;
-        if (oc_status r = alloc_persist_words(s)) return r;
-    }
+    s->pplan.grid = 0;
+    if (any_streamed && !any_coupled)
+        if (oc_status r = plan_persist(s)) return r;
+    s->persist = cfg.persist && s->pplan.grid > 0;
+    s->adj_persist = s->adj_allowed && s->persist_smem_max > 0 && !any_coupled && (!any_streamed || s->pplan.grid > 0);
     s->strip_finish = false;
     for (int32_t k = 0; k < s->n_inst; ++k)
         if (s->inst_host[(size_t)k].strip && (s->resident[(size_t)k] || !s->persist)) s->strip_finish = true;
@@ -1346,8 +1442,7 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
         a.r[k] = planes + (9 + k) * stride;
         a.d[k] = planes + (12 + k) * stride;
     }
-    OC_CREATE_TRY(dalloc(s, &a.partials, 2 * P.blocks.size()));
-    a.partials_b = a.partials + P.blocks.size();
+    OC_CREATE_TRY(dalloc(s, &a.partials, P.blocks.size()));
     InstParams* inst = nullptr;
     OC_CREATE_TRY(upload(s, &inst, P.inst));
     a.inst = inst;
@@ -1442,25 +1537,10 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
         int coop = 0;
         OC_CREATE_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
         s->coop = coop != 0;
-        s->persist_per_sm = s->executor != OC_EXEC_PLAIN ? persist_blocks_per_sm() : 0;
+        if (s->coop && s->executor != OC_EXEC_PLAIN) OC_CREATE_TRY(prepare_persist(s->device, &s->persist_smem_max, &s->persist_clusters, &s->persist_pairs));
+        s->adj_allowed = !(pe && std::atoi(pe) == 0) && s->coop;
         s->h_blocks = P.blocks;
         if (oc_status r = plan_execution(s)) return bail(r);
-    }
-    {
-        const char* pe = std::getenv("OC_PERSIST");
-        const bool allowed = !(pe && std::atoi(pe) == 0) && s->executor != OC_EXEC_PLAIN;
-        const int per_sm = allowed ? s->persist_per_sm : 0;
-        const int n_sm = s->sm_count;
-        const int coop = s->coop ? 1 : 0;
-        // The adjoint solve runs every cloth's CG over the full block table: one
-        // cooperative launch without the update, any number of cloths.
-        const int adj_grid = std::min(per_sm * n_sm, std::max(1, s->n_blocks));
-        if (allowed && coop && per_sm > 0 && !P.any_coupled &&
-            (int64_t)s->n_blocks <= (int64_t)persist_max_entries_per_block() * adj_grid) {
-            s->adj_persist = true;
-            s->adj_persist_grid = adj_grid;
-            if (oc_status r = alloc_persist_words(s)) return bail(r);
-        }
     }
     OC_CREATE_TRY(dalloc(s, &a.unconverged, 1));
     OC_CREATE_TRY(dalloc(s, &a.grid_ticket, 1));
@@ -2104,6 +2184,9 @@ oc_status tape_begin(oc_solver* s, float dt, int32_t n, int32_t checkpoint_every
     OC_TRY(cudaStreamSynchronize(s->stream));
     auto& T = s->tape;
     T.valid = false;
+    if (T.mode == OC_TAPE_DISPLACEMENT && !s->adj_persist)
+        return fail(s, OC_ERR_UNSUPPORTED, "oc_tape_forward: the displacement mode needs the cooperative CG, which the "
+                                           "launch configuration set since does not allow");
     int32_t every = checkpoint_every;
     if (every == 0) every = std::max(1, (int32_t)std::ceil(std::sqrt((double)n)));
     every = std::min(every, n);

@@ -94,7 +94,6 @@ struct StepArgs {
     float* r[3];
     float* d[3];
     double* partials;        // one per streamed block
-    double* partials_b;      // a second set (the persistent CG's phases of odd parity)
     const InstParams* inst;
     InstState* state;
     const BlockInfo* blocks;
@@ -245,17 +244,59 @@ enum KernelKind { K_ASSEMBLE = 0, K_CG_DIR = 1, K_CG_UPDATE = 2, K_INTEGRATE = 3
                   K_ASSEMBLE_GRID = 11, K_CG_PERSIST = 12, K_ASSEMBLE_STRIP = 13, K_ASSEMBLE_FINISH = 14,
                   K_COUNT = 15 };
 
-// The whole CG loop of the cloths of block table a.blocks[0, n_entries) in one
-// cooperative launch of `grid` blocks (oc_kernels.cu), any number of cloths; a block
-// owns at most persist_max_entries_per_block() entries.  words: one arrival count per
-// cloth of the handle, indexed by cloth, zeroed before each launch.  The per-block
-// partials are double buffered (StepArgs::partials, partials_b).  err: bit 0 set if a
-// wait gave up.
-int persist_max_entries_per_block();
-int persist_blocks_per_sm();
 cudaError_t launch_test_cr_arith(unsigned long long* counts, uint64_t n_pairs, uint64_t seed, cudaStream_t stream);
-cudaError_t launch_cg_persist(const StepArgs& a, int32_t n_entries, int grid, unsigned* words, int* err,
-                              cudaStream_t stream);
+// The persistent CG (k_cg_persist, oc_persist.cu): the whole CG loop and the update of the
+// streamed REFERENCE cloths in one cooperative launch.  A piece is the part of one cloth that
+// lies in one CTA's range of the concatenated streamed vertices; its slots are runs of up to
+// kPersistThreads of its vertices.
+constexpr int kPersistThreads = 256;
+constexpr int kPersistMaxCluster = 16;
+constexpr int kPersistPieceBytes = 336;  // shared memory of one piece's scalars
+struct PersistPiece {
+    int32_t inst;
+    int32_t n;             // vertices v ... v + n - 1
+    int64_t v;             // first vertex (global index)
+    int32_t slot0, slot1;  // its slots of kPersistThreads vertices, counted from its CTA's first
+    int32_t head;          // 1: the cloth's first piece
+    // The cloth's CTAs in this CTA's cluster: ranks rank0 ... rank0 + ranks - 1; tail 1 when
+    // the cloth starts in CTA rank0 behind another cloth (it is that CTA's last piece, not
+    // its first).
+    int32_t rank0, ranks, tail;
+    // The clusters the cloth lies in, this one's place among them, and the first of their
+    // packets (the cluster size x clusters of them).
+    int32_t clusters, k, packet;
+    int32_t full;          // 1: every CTA of those clusters has a piece of the cloth
+};
+struct PersistCtl {
+    uint32_t base;  // tags up to base have been used by earlier launches
+    uint32_t used;  // tags that the running launch uses (so far)
+    uint32_t left;  // CTAs of the running launch that have left it
+};
+struct PersistPlan {
+    const PersistPiece* pieces;
+    const int32_t* cta_piece;  // grid + 1: each CTA's first piece
+    ulonglong2* packets;       // two sets, by the phase's parity
+    PersistCtl* ctl;
+    int* err;                  // bit 0: a wait gave up
+    int32_t grid, cluster;     // CTAs, CTAs per cluster
+    int32_t n_packets;         // of one set
+    int32_t one;               // 1: pieces[b] is CTA b's only piece (n = 0: none)
+    int32_t max_pieces, max_slots;  // of one CTA
+    int32_t smem_slots;        // slots of a CTA held in shared memory
+    int32_t x_slots;           // slots of a CTA whose x is in shared memory
+    int32_t on_chip;           // 1: no slot left in the planes
+    size_t smem;               // dynamic shared memory
+};
+__host__ __device__ constexpr size_t persist_state_bytes(int max_pieces) {
+    return ((size_t)max_pieces * kPersistPieceBytes + 127) / 128 * 128;
+}
+// What a plan with max_pieces and max_slots keeps in registers and shared memory (smem may
+// come out above max_smem when the pieces' scalars alone do not fit).
+void persist_layout(PersistPlan* plan, int max_smem);
+// Function attributes; the dynamic shared memory one CTA may have, and how many clusters of
+// kPersistMaxCluster and of 2 CTAs are co-resident with all of it (0: none).
+cudaError_t prepare_persist(int device, int* max_smem, int* max_clusters, int* max_pairs);
+cudaError_t launch_cg_persist(const StepArgs& a, const PersistPlan& plan, cudaStream_t stream);
 
 // Interaction kernels (oc_interact.cu).
 cudaError_t launch_pick(const float4* X, int64_t v0, int64_t nv, const float pt[3], double radius, int32_t* out,

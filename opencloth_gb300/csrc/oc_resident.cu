@@ -74,36 +74,6 @@ __device__ Acc cluster_sum(Acc part, int C, Acc (*slots)[kResidentMaxCluster], i
     return v;
 }
 
-// The CG's scalar arithmetic on the pairs, with no FP64 (one FP64 division costs a
-// resident CTA about a tenth of its time on this GPU).  norm: the pair's value as
-// hi + lo with hi = fl(hi + lo) (TwoSum).  div: the quotient of two normalised pairs,
-// rounded to float: q0 = fl(a.hi / b.hi), the exact remainder a - q0 b (an FMA for the
-// head product, Sterbenz for the subtraction), then q0 + remainder / b.hi rounded once;
-// it is the correctly rounded quotient unless the exact one lies within about 2^-46 of a
-// rounding boundary.  gt: a > b for normalised pairs.
-__device__ __forceinline__ Acc pair_norm(Acc a) {
-    const float s = a.s + a.c;
-    const float bp = s - a.s;
-    return make_acc(s, (a.s - (s - bp)) + (a.c - bp));
-}
-
-__device__ __forceinline__ float pair_div(Acc a, Acc b) {
-    const float q0 = __fdiv_rn(a.s, b.s);
-    const float ph = __fmul_rn(q0, b.s);
-    const float pl = __fmaf_rn(q0, b.s, -ph);
-    const float r = (((a.s - ph) - pl) + a.c) - __fmul_rn(q0, b.c);
-    return __fadd_rn(q0, __fdiv_rn(r, b.s));
-}
-
-__device__ __forceinline__ bool pair_gt(Acc a, Acc b) { return a.s > b.s || (a.s == b.s && a.c > b.c); }
-
-__device__ __forceinline__ bool pair_finite(Acc a) { return isfinite(a.s) && isfinite(a.c); }
-
-__device__ __forceinline__ Acc pair_from(double x) {
-    const float h = (float)x;
-    return make_acc(h, (float)(x - (double)h));
-}
-
 // Resident CTAs per SM the register budget is set for: 128-thread CTAs hold up to 512
 // vertices, 256-thread CTAs 256 to 1024, 512-thread CTAs 2048 (shared memory holds only
 // A, 24 bytes per vertex; x, r and d are in registers).
