@@ -102,16 +102,10 @@ __device__ float3 chunk_gather(const StepArgs& a, const InstParams& ip, int64_t 
             const float4 Xs = sm.X[self], Vs = sm.V[self];
             float3 f = make_float3(0.f, 0.f, 0.f);
             if (Vs.w == 0.0f) {  // pinned vertices take no spring force (IMP:730-733)
-                const bool as_p2 = rec.x < 0;
+                // evaluated with the vertex as p1 and added, whichever end it is (add_spring_forces)
                 const int32_t o = rec.x & 0x7fffffff;
                 const float4 Xo = __ldg(a.X + o), Vo = __ldg(a.V + o);
-                const float rest = __int_as_float(rec.y), ks = __int_as_float(rec.z), kd = __int_as_float(rec.w);
-                if (as_p2) {  // F[p2] -= f, IMP:733
-                    f = spring_force(Xo, Xs, Vo, Vs, rest, ks, kd);
-                    f = make_float3(-f.x, -f.y, -f.z);
-                } else {  // F[p1] += f, IMP:731
-                    f = spring_force(Xs, Xo, Vs, Vo, rest, ks, kd);
-                }
+                f = spring_force(Xs, Xo, Vs, Vo, __int_as_float(rec.y), __int_as_float(rec.z), __int_as_float(rec.w));
             }
             sm.fx[k - rb] = f.x;
             sm.fy[k - rb] = f.y;
@@ -198,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_assemble_grid(const StepArgs
         const float4 Xg = __ldg(a.X + g), Vg = __ldg(a.V + g);
         const int2 ends = __ldg(a.own_ends + g);
         prefetch_own(a, g, ends);  // into L1 while the forces are gathered
-        const float3 F = B == 1 ? stencil_gather(a, ip, g, Xg, Vg) : stencil_gather_ahead<B>(a, ip, g, Xg, Vg);
+        const float3 F = stencil_gather<B>(a, ip, g, Xg, Vg);
         acc_add(part, assemble_vertex(a, g, Xg, Vg, F, load_own_at(a, g, ends)));
     }
     finish<K_ASSEMBLE>(a, bi.gblk, bi.inst, true, part);
@@ -760,29 +754,7 @@ __global__ void __launch_bounds__(kThreads) k_integrate(const StepArgs a) {
 // value.  Pin flags come from a separate byte array: V is written here.
 __device__ __forceinline__ void provot_incidence(const StepArgs& a, float ratio, const float4 Xg, bool pin_self,
                                                  int32_t o, bool is_p2, float rest, float4& Vg) {
-    const float4 Xo = __ldg(a.X + o);
-    const float4 p1 = is_p2 ? Xo : Xg, p2 = is_p2 ? Xg : Xo;
-    const float dx = p1.x - p2.x, dy = p1.y - p2.y, dz = p1.z - p2.z;
-    const float sqr = dx * dx + dy * dy + dz * dz;
-    float dist = sqrtf(sqr);
-    const float lim = rest * ratio;
-    if (!(dist > lim)) return;
-    dist = dist - lim;
-    dist = dist / 2.0f;
-    const float inv = 1.0f / sqrtf(sqr);
-    const float cx = (dx * inv) * dist, cy = (dy * inv) * dist, cz = (dz * inv) * dist;
-    const bool pin_o = __ldg(a.pinflag + o) != 0;
-    if (!is_p2) {
-        if (!pin_self) {  // p1 moves unless pinned
-            Vg.x = Vg.x - cx;
-            Vg.y = Vg.y - cy;
-            Vg.z = Vg.z - cz;
-        }
-    } else if (pin_o || !pin_self) {  // p2 moves when p1 is pinned or p2 is free
-        Vg.x = Vg.x + cx;
-        Vg.y = Vg.y + cy;
-        Vg.z = Vg.z + cz;
-    }
+    provot_pair(a, ratio, Xg, __ldg(a.X + o), pin_self, o, is_p2, rest, Vg);
 }
 
 __global__ void __launch_bounds__(kThreads) k_provot(const StepArgs a) {

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(T, resident_min_blocks<T>()) k_resident(const 
             const float4 Xg = a.X[g], Vg = a.V[g];
             const OwnSpring os = load_own<false>(a, g);
             const float3 F =
-                ip.grid_cols > 0 ? stencil_gather<false>(a, ip, g, Xg, Vg) : thread_gather<1, false>(a, ip, g, Xg, Vg);
+                ip.grid_cols > 0 ? stencil_gather<1, false>(a, ip, g, Xg, Vg) : thread_gather<1, false>(a, ip, g, Xg, Vg);
             const VertexSystem sys = vertex_system(a.dt, Xg, Vg, F, os);
             const CgInit c = cg_init(sys, a.x[0][g], a.x[1][g], a.x[2][g], Vg.w != 0.0f);
 #pragma unroll
