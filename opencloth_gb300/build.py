@@ -34,7 +34,7 @@ NVCC_FLAGS = ARCH + [
 GRADIENT_FLAGS = ["--fmad=true", "-prec-div=false", "-prec-sqrt=false"]
 GRADIENT_SOURCES = {"oc_adjoint.cu"}
 SOURCES = ["oc_kernels.cu", "oc_resident.cu", "oc_adjoint.cu", "oc_api.cu", "oc_topology.cpp", "oc_noalloc.cu",
-           "oc_coupled.cu", "oc_interact.cu", "oc_bsr.cu", "oc_persist.cu"]
+           "oc_coupled.cu", "oc_interact.cu", "oc_bsr.cu", "oc_persist.cu", "oc_sim.cu"]
 
 
 def _nvcc() -> str:

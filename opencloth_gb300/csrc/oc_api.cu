@@ -47,6 +47,16 @@ struct oc_solver {
     };
     std::vector<Bucket> buckets;
     std::vector<uint8_t> resident;  // per instance
+    // A handle whose cloths are all resident and few enough to run side by side steps them in
+    // k_sim, any number of steps in one launch per group of cloths of one launch shape (empty:
+    // the step graph).
+    struct SimGroup {
+        SimLaunch launch;
+        int n;
+        int32_t* d_ids;
+    };
+    std::vector<SimGroup> sim;
+    int sim_smem_max = 0;
     // OC_RESIDENT_FUSED=1: resident cloths assemble inside the resident kernel (no
     // k_assemble pass over them).  Off by default: on 4096 cloths of 64 to 16,384 vertices
     // the fused step measured 4.97 ms against 4.37 ms for the separate passes (the
@@ -200,7 +210,7 @@ oc_status check_device_error(oc_solver* s) {
         OC_TRY(cudaMemset(s->d_perr, 0, sizeof(int)));
         OC_TRY(cudaMemset(s->args.state, 0, sizeof(InstState) * (size_t)s->n_inst));
         return fail(s, OC_ERR_DEVICE_TIMEOUT,
-                    "k_cg_persist: a wait gave up (cloths whose solve had not ended were not updated)");
+                    "a wait between CTAs gave up (cloths whose solve had not ended were not updated)");
     }
     return OC_OK;
 }
@@ -936,6 +946,91 @@ void drop_graphs(oc_solver* s) {
     }
 }
 
+// Streams beside the handle's own for `want` concurrent launches (at most 8).
+oc_status ensure_aux(oc_solver* s, size_t want) {
+    if (!s->fork_ev) OC_TRY(cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming));
+    while (s->aux.size() < std::min<size_t>(want, 8)) {
+        cudaStream_t x = nullptr;
+        cudaEvent_t e = nullptr;
+        OC_TRY(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+        s->aux.push_back(x);
+        OC_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        s->aux_done.push_back(e);
+    }
+    return OC_OK;
+}
+
+// The word in which k_cg_persist and k_sim report a wait that gave up (once per handle).
+oc_status alloc_error_word(oc_solver* s) {
+    if (s->d_perr) return OC_OK;
+    OC_TRY(dalloc(s, &s->d_perr, 1));
+    OC_TRY(cudaMemset(s->d_perr, 0, sizeof(int)));
+    return OC_OK;
+}
+
+// k_sim's plan: every cloth of the handle resident, each on the fewest CTAs of 256, 512 or 1024
+// vertices that make a cluster of kSimMaxCluster at most, and all of these CTAs together no more
+// than the SMs: then a step is bound by latencies, which k_sim shortens; with more cloths it is
+// bound by instructions, and the assembly's and the resident CG's own launches keep more warps in
+// flight.
+oc_status plan_sim(oc_solver* s) {
+    for (auto& g : s->sim) dfree(s, &g.d_ids);
+    s->sim.clear();
+    if (s->sim_smem_max <= 0 || s->resident_fused || s->any_coupled) return OC_OK;
+    for (uint8_t r : s->resident)
+        if (!r) return OC_OK;
+    struct Shape {
+        SimLaunch launch{};
+        std::vector<int32_t> ids;
+    };
+    const int sizes[3][2] = {{256, 1}, {512, 1}, {512, 2}};
+    std::map<std::pair<int, int>, Shape> shapes;
+    for (int first = 0;; ++first) {
+        if (first == 3) return OC_OK;
+        int64_t total = 0;
+        shapes.clear();
+        for (int32_t k = 0; k < s->n_inst; ++k) {
+            const InstParams& ip = s->inst_host[(size_t)k];
+            int i = first, c = 0;
+            for (; i < 3; ++i) {
+                const int cap = sizes[i][0] * sizes[i][1];
+                c = (ip.nv + cap - 1) / cap;
+                if (c <= kSimMaxCluster) break;
+            }
+            if (i == 3) return OC_OK;
+            total += c;
+            const int chunk = (ip.nv + c - 1) / c;
+            Shape& sh = shapes[{i, c}];
+            SimLaunch& L = sh.launch;
+            L.cluster = c;
+            L.threads = sizes[i][0];
+            L.vpt = sizes[i][1];
+            L.window = std::max(L.window, std::min(ip.nv, chunk + 4 * std::max(0, ip.grid_cols)));
+            if (ip.grid_cols > 0) {
+                const int32_t* st = s->h_st_data.data() + ip.st_off;
+                L.entries = std::max(L.entries, st[kStencilClasses] - kStencilClasses - 1);
+                if (ip.st_rest)
+                    for (int q = 0; q < kStencilClasses; ++q) L.rest = std::max(L.rest, st[q + 1] - st[q]);
+            }
+            sh.ids.push_back(k);
+        }
+        if (total <= s->sm_count) break;
+    }
+    for (const auto& kv : shapes)
+        if (sim_smem_bytes(kv.second.launch) > (size_t)s->sim_smem_max) return OC_OK;
+    if (oc_status r = alloc_error_word(s)) return r;
+    for (const auto& kv : shapes) {
+        oc_solver::SimGroup g{};
+        g.launch = kv.second.launch;
+        g.launch.err = s->d_perr;
+        g.n = (int)kv.second.ids.size();
+        OC_TRY(upload(s, &g.d_ids, kv.second.ids));
+        g.launch.inst_ids = g.d_ids;
+        s->sim.push_back(g);
+    }
+    return ensure_aux(s, s->sim.size());
+}
+
 // The persistent CG's plan.  At most one CTA per SM, each with at least kPersistThreads
 // vertices where there are that many (a thread then holds one vertex, and fewer CTAs have fewer
 // packets to wait for).  When there are no more cloths than CTAs every cloth gets CTAs of its
@@ -1052,10 +1147,9 @@ oc_status plan_persist(oc_solver* s) {
     if (!P.ctl) {
         OC_TRY(dalloc(s, &P.ctl, 1));
         OC_TRY(cudaMemset(P.ctl, 0, sizeof(PersistCtl)));
-        OC_TRY(dalloc(s, &s->d_perr, 1));
-        OC_TRY(cudaMemset(s->d_perr, 0, sizeof(int)));
-        P.err = s->d_perr;
     }
+    if (oc_status r = alloc_error_word(s)) return r;
+    P.err = s->d_perr;
     P.grid = (int32_t)cta_piece.size() - 1;
     return OC_OK;
 }
@@ -1144,16 +1238,7 @@ oc_status plan_execution(oc_solver* s) {
                       cudaMemcpyHostToDevice));
     if (!s->buckets.empty()) {
         OC_TRY(prepare_resident());
-        const size_t naux = std::min<size_t>(s->buckets.size(), 8);
-        if (!s->fork_ev) OC_TRY(cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming));
-        while (s->aux.size() < naux) {
-            cudaStream_t x = nullptr;
-            cudaEvent_t e = nullptr;
-            OC_TRY(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
-            s->aux.push_back(x);
-            OC_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            s->aux_done.push_back(e);
-        }
+        if (oc_status r = ensure_aux(s, s->buckets.size())) return r;
     }
     // Persistent CG for the streamed REFERENCE cloths, any number of them: no COUPLED
     // cloth, a cooperative launch fits, and the configuration allows it.
@@ -1167,6 +1252,7 @@ oc_status plan_execution(oc_solver* s) {
         if (oc_status r = plan_persist(s)) return r;
     s->persist = cfg.persist && s->pplan.grid > 0;
     s->adj_persist = s->adj_allowed && s->persist_smem_max > 0 && !any_coupled && (!any_streamed || s->pplan.grid > 0);
+    if (oc_status r = plan_sim(s)) return r;
     s->strip_finish = false;
     for (int32_t k = 0; k < s->n_inst; ++k)
         if (s->inst_host[(size_t)k].strip && (s->resident[(size_t)k] || !s->persist)) s->strip_finish = true;
@@ -1538,6 +1624,7 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
         OC_CREATE_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
         s->coop = coop != 0;
         if (s->coop && s->executor != OC_EXEC_PLAIN) OC_CREATE_TRY(prepare_persist(s->device, &s->persist_smem_max, &s->persist_clusters, &s->persist_pairs));
+        if (s->executor != OC_EXEC_PLAIN) OC_CREATE_TRY(prepare_sim(s->device, &s->sim_smem_max));
         s->adj_allowed = !(pe && std::atoi(pe) == 0) && s->coop;
         s->h_blocks = P.blocks;
         if (oc_status r = plan_execution(s)) return bail(r);
@@ -1668,6 +1755,42 @@ oc_status oc_step_host(oc_solver* s, float dt, int32_t n_steps, float* X, float*
     return check_device_error(s);
 }
 
+namespace {
+
+// n_steps steps of a handle whose cloths run in k_sim: one launch per group (on streams of
+// their own, forked from the handle's and joined back, when there are several), at most
+// kSimSteps steps each, so that a launch ends within some milliseconds.
+constexpr int32_t kSimSteps = 512;
+
+oc_status step_sim(oc_solver* s, float dt, int32_t n_steps) {
+    StepArgs a = s->args;
+    a.dt = dt;
+    const size_t n = s->sim.size(), used = std::min(n, s->aux.size());
+    const bool fork = n > 1;
+    if (n_steps <= 0) return OC_OK;
+    if (fork) {
+        OC_TRY(cudaEventRecord(s->fork_ev, s->stream));
+        for (size_t i = 0; i < used; ++i) OC_TRY(cudaStreamWaitEvent(s->aux[i], s->fork_ev, 0));
+    }
+    for (size_t i = 0; i < n; ++i) {
+        const auto& g = s->sim[i];
+        SimLaunch L = g.launch;
+        for (int32_t done = 0; done < n_steps; done += L.n_steps) {
+            L.n_steps = std::min(n_steps - done, kSimSteps);
+            OC_TRY(launch_sim(a, L, g.n, fork ? s->aux[i % used] : s->stream));
+            s->host_launches += 1;
+        }
+    }
+    if (fork)
+        for (size_t i = 0; i < used; ++i) {
+            OC_TRY(cudaEventRecord(s->aux_done[i], s->aux[i]));
+            OC_TRY(cudaStreamWaitEvent(s->stream, s->aux_done[i], 0));
+        }
+    return OC_OK;
+}
+
+}  // namespace
+
 oc_status oc_step(oc_solver* s, float dt, int32_t n_steps) {
     if (!valid_solver(s) || n_steps < 0 || !std::isfinite(dt)) return OC_ERR_INVALID_ARGUMENT;
     OC_TRY(cudaSetDevice(s->device));
@@ -1685,6 +1808,7 @@ oc_status oc_step(oc_solver* s, float dt, int32_t n_steps) {
         }
         return OC_OK;
     }
+    if (!s->sim.empty()) return step_sim(s, dt, n_steps);
     if (!s->exec || s->graph_dt != dt) {
         oc_status st = build_graph(s, dt);
         if (st != OC_OK) return st;

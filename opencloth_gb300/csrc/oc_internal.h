@@ -336,6 +336,23 @@ cudaError_t prepare_resident();  // function attributes (once per device)
 cudaError_t launch_resident(const StepArgs& a, const ResidentLaunch& L, int threads, int n_clusters,
                             cudaStream_t stream);
 
+// Whole steps of small REFERENCE cloths (k_sim, oc_sim.cu): n_steps of them in one launch, one
+// cluster of CTAs per cloth, vpt vertices per thread.
+constexpr int kSimMaxCluster = 16;
+struct SimLaunch {
+    const int32_t* inst_ids;  // the cloth of each cluster
+    int32_t cluster;
+    int32_t threads, vpt;     // 256 x 1, 512 x 1 or 512 x 2
+    // The largest of the launch's cloths: vertices of a CTA's window, entries of a stencil, and
+    // incidences of a vertex whose rest lengths are read one by one.
+    int32_t window, entries, rest;
+    int32_t n_steps;
+    int* err;                 // bit 0: a wait gave up
+};
+size_t sim_smem_bytes(const SimLaunch& L);
+cudaError_t prepare_sim(int device, int* max_smem);
+cudaError_t launch_sim(const StepArgs& a, const SimLaunch& L, int n_clusters, cudaStream_t stream);
+
 cudaError_t launch_state_in(const StepArgs& a, const float* X3, const float* V3, const float* dV3, int64_t nv,
                             int32_t* err, cudaStream_t stream);
 cudaError_t launch_state_out(const StepArgs& a, float* X3, float* V3, float* dV3, int64_t nv, cudaStream_t stream);
