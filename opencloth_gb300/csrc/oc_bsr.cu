@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "oc_device.cuh"
+#include "oc_exchange.cuh"
 #include "oc_internal.h"
 
 namespace oc {
@@ -331,72 +332,57 @@ __global__ void __launch_bounds__(kThreads) k_bsr_update(const BsrArgs a) {
 }
 
 // Dynamic shared memory of the resident CG: each row's new direction r + d4 p (a 16-byte
-// record the neighbours gather; x passes through it during init); the system's blocks
-// without padding: two float4 planes, component 8 and an 8-bit local column (a resident
-// system has at most 256 rows); each warp's offset of each slot (ints, `stride` of them
-// per warp: the longest row's block count).
-__host__ __device__ constexpr size_t resident_vec_bytes(int threads) { return 16 * (size_t)threads; }
+// record the neighbours gather; x passes through it during init); the blocks of the free rows
+// without padding, as two float4 planes and one of {component 8, 16 x local column} (a resident
+// system has at most 256 rows), with 32 more entries that a slot's idle lanes may read; and each
+// warp's offset of each slot (`stride` of them per warp, a multiple of kResSlots).
+__host__ __device__ constexpr int64_t resident_entries(int64_t nnzb) { return (nnzb + 32 + 7) / 8 * 8; }
 __host__ __device__ constexpr size_t resident_smem_bytes(int threads, int64_t nnzb, int stride) {
-    return resident_vec_bytes(threads) + ((size_t)nnzb * 37 + 15) / 16 * 16 + 4 * (size_t)(threads / 32) * stride;
+    return 16 * (size_t)threads + 40 * (size_t)resident_entries(nnzb) + 4 * (size_t)(threads / 32) * stride;
 }
 constexpr int kResSlots = 4;    // slots of a row multiplied together in the resident loop
 constexpr int kResMaxDeg = 64;  // blocks of a resident system's longest row (bounds the offset table)
 
-// The first half of block_sum_acc: each warp's pair, reduced by the same shuffle tree,
-// is stored in wacc[warp] (read after a barrier).
-__device__ __forceinline__ void warp_partial(Acc v, Acc* wacc) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        Acc u;
-        u.s = __shfl_down_sync(0xffffffffu, v.s, o);
-        u.c = __shfl_down_sync(0xffffffffu, v.c, o);
-        v = acc_merge(v, u);
-    }
-    if ((threadIdx.x & 31) == 0) wacc[threadIdx.x >> 5] = v;
+// |v| < tiny (tiny >= 0) for a normalised pair.
+__device__ __forceinline__ bool pair_below(Acc v, float tiny) {
+    const float s = fabsf(v.s), c = v.s < 0.0f ? -v.c : v.c;
+    return s < tiny || (s == tiny && c < 0.0f);
 }
 
-// The second half, by warp 0 (every lane calls it; the result is valid in lane 0): lane i
-// turns warp i's pair into s + c in FP64, then block_sum_acc's shuffle tree over at most 8
-// warp values.  The tree's first two levels add zeros (lanes 8-31), which leaves each value
-// unchanged (a warp value is never -0: its pair starts at +0), so its result is
-// ((w0 + w4) + (w2 + w6)) + ((w1 + w5) + (w3 + w7)), formed here by three shuffle levels:
-// the same bits, with one FP64 warp instruction per conversion or level rather than one
-// per warp and a serial sum in one thread.
-__device__ __forceinline__ double sum_warp_pairs(const Acc* wacc, int nw) {
-    const int lane = threadIdx.x & 31;
-    double v = lane < nw ? (double)wacc[lane].s + (double)wacc[lane].c : 0.0;
-    v += __shfl_down_sync(0xffffffffu, v, 4);
-    v += __shfl_down_sync(0xffffffffu, v, 2);
-    v += __shfl_down_sync(0xffffffffu, v, 1);
-    return v;
-}
-
-// The whole solve of one small system in one CTA: the system's blocks are read once
+// The whole solve of one small system in one CTA: the blocks of its free rows are read once
 // from the caller's CSR into shared memory (the pack), then init and every iteration
-// run on chip with the streamed kernels' arithmetic.  Thread t owns internal row
-// row0 + t, as in the system's only block of the streamed path, and the dot products
-// go through the same block sums, so the results are the streamed path's bits.
+// run on chip with the streamed kernels' FP32 arithmetic.  Thread t owns internal row
+// row0 + t; a resident system's rows are ordered by decreasing block count, fixed rows last.
 //
-// Shared-memory layout of the blocks (jagged diagonals): a system's rows are sorted by
-// decreasing block count, so in each warp the lanes whose row has more than j blocks
-// are lanes 0 .. cnt_j - 1.  Slot j of the warp's rows is stored as those cnt_j entries,
-// after the warp's slots 0 .. j-1; cnt_j is a ballot over the warp.
-// map[e] places the caller's block e: its internal local row (bits 0-7), its slot in the
-// row (bits 8-15) and its internal local column (bits 16-23), so the pack reads the
-// caller's blocks in order, coalesced.
-__global__ void __launch_bounds__(kThreads) k_bsr_resident(const BsrArgs a, const int32_t* ids, int64_t nnzb_max,
+// Shared-memory layout of the blocks (jagged diagonals): in each warp the lanes whose row has more
+// than j blocks are lanes 0 .. cnt_j - 1, and slot j of the warp's rows is stored as those cnt_j
+// entries, after the warp's slots 0 .. j-1; s_pre holds the slots' offsets, padded to the warp's
+// next multiple of kResSlots.  map[e] places the caller's block e: its entry (bits 0-15; 0xffff: a
+// fixed row's, not kept) and its internal local column (bits 16-23), so the pack reads the caller's
+// blocks in order, coalesced.
+//
+// What bounds it is shared memory (40 bytes a block and the 16-byte direction it meets, whose
+// gather takes about 8 wavefronts where 4 would do without conflicts) and instructions, then the
+// latency of two reductions an iteration.  So a slot is three loads from the same offset, its
+// gather and eighteen FP32 operations; fixed rows hold no slot; and the sums run in float pairs (48
+// bits, as the cloth solvers'), every warp forming the totals and the quotients itself, with three
+// barriers an iteration.  Before, a slot was 45 instructions and the scalars FP64 sums and
+// divisions in one warp while the others waited at five barriers.  Measured on 1,024 bodies of the
+// demo's 176 rows, 20 iterations: 238 -> 181 us (the pack is 8 to 11 us of each CTA's 60, an
+// iteration 5,500 cycles with three CTAs an SM and 4,000 alone).  Rows in the caller's order, whose
+// gathers have half the wavefronts, need nearly twice the slots (109 against 56) and took 243.
+__global__ void __launch_bounds__(kThreads, 3) k_bsr_resident(const BsrArgs a, const int32_t* ids, int64_t nnzb_max,
                                                            const uint32_t* map, int stride) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ float s_d3, s_d4;
     __shared__ int s_wcount[kThreads / 32];
-    __shared__ Acc s_w0[kThreads / 32], s_w1[kThreads / 32], s_w2[kThreads / 32];
-    static_assert(kThreads / 32 <= 8, "sum_warp_pairs takes at most 8 warps");
+    __shared__ Acc s_w0[8], s_w1[8], s_w2[8];
+    static_assert(kThreads / 32 <= 8, "the totals take at most 8 warps");
+    const int64_t entries = resident_entries(nnzb_max);
     float4* s_n4 = reinterpret_cast<float4*>(smem);
     float4* s_b0 = s_n4 + blockDim.x;
-    float4* s_b1 = s_b0 + nnzb_max;
-    float* s_b8 = reinterpret_cast<float*>(s_b1 + nnzb_max);
-    uint8_t* s_col = reinterpret_cast<uint8_t*>(s_b8 + nnzb_max);
-    int* s_pre = reinterpret_cast<int*>(smem + resident_smem_bytes(blockDim.x, nnzb_max, 0));
+    float4* s_b1 = s_b0 + entries;
+    float2* s_b2 = reinterpret_cast<float2*>(s_b1 + entries);
+    int* s_pre = reinterpret_cast<int*>(s_b2 + entries);
     constexpr unsigned kFull = 0xffffffffu;
 
     const int k = ids[blockIdx.x];
@@ -404,81 +390,89 @@ __global__ void __launch_bounds__(kThreads) k_bsr_resident(const BsrArgs a, cons
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const bool valid = t < sp.n_rows;
     const int64_t g = sp.row0 + t;
-    bool fx = true;
-    int n = 0;
+    bool act = false;
+    int n = 0;  // blocks of a free row
     float x0 = 0.0f, x1 = 0.0f, x2 = 0.0f;
     if (valid) {
-        fx = a.fixed[g] != 0;
-        n = a.deg[g];
+        act = a.fixed[g] == 0;
+        if (act) n = a.deg[g];
+        x0 = a.x[0][g];
+        x1 = a.x[1][g];
+        x2 = a.x[2][g];
     }
     const int width = __reduce_max_sync(kFull, n);
     const int wsum = __reduce_add_sync(kFull, n);
     if (lane == 0) s_wcount[w] = wsum;
-    __syncthreads();
-    int base = 0;
-    for (int u = 0; u < w; ++u) base += s_wcount[u];
-    {  // each warp's slot offsets, then k_bsr_pack into shared memory
-        int pre = base;
-        for (int j = 0; j < width; ++j) {
-            const int cnt = __popc(__ballot_sync(kFull, n > j));
-            if (lane == 0) s_pre[w * stride + j] = pre;
-            pre += cnt;
-        }
-        __syncthreads();
+    if (t < 8) s_w0[t] = s_w1[t] = s_w2[t] = acc_zero();
+    s_n4[t] = make_float4(x0, x1, x2, 0.0f);  // x, for init's gathers
+    {  // k_bsr_pack into shared memory
         const int64_t e1 = a.row_ptr[sp.row0 + sp.n_rows];
 #pragma unroll 4
         for (int64_t e = a.row_ptr[sp.row0] + t; e < e1; e += blockDim.x) {
             const uint32_t mp = __ldg(map + e);
-            const int i = mp & 255, j = (mp >> 8) & 255;
+            const int pos = mp & 0xffff;
+            if (pos == 0xffff) continue;
             const float* m = a.cblk + 9 * (size_t)e;
-            const int pos = s_pre[(i >> 5) * stride + j] + (i & 31);
             s_b0[pos] = make_float4(m[0], m[1], m[2], m[3]);
             s_b1[pos] = make_float4(m[4], m[5], m[6], m[7]);
-            s_b8[pos] = m[8];
-            s_col[pos] = (uint8_t)(mp >> 16);
+            s_b2[pos] = make_float2(m[8], __int_as_float((int)(mp >> 16) * 16));
         }
     }
-    if (valid) {
-        x0 = a.x[0][g];
-        x1 = a.x[1][g];
-        x2 = a.x[2][g];
-        s_n4[t] = make_float4(x0, x1, x2, 0.0f);  // x, for init's gathers
-    }
     __syncthreads();
+    {  // each warp's slot offsets
+        int pre = 0;
+        for (int u = 0; u < w; ++u) pre += s_wcount[u];
+        for (int j = 0; j < stride; ++j) {
+            const int cnt = __popc(__ballot_sync(kFull, n > j));
+            if (lane == 0) s_pre[w * stride + j] = pre;
+            pre += cnt;
+        }
+        __syncwarp();
+    }
+    // Slots j ... j + 3 of every row times the directions (or x) in s_n4: the products of the lane's
+    // row, of which the first n - j count (an idle lane's are of some other entry's block).
+    const char* const n4 = reinterpret_cast<const char*>(s_n4);
+    const int* const pre = s_pre + w * stride;
+    auto products = [&](int j, float (&o)[kResSlots][3]) {
+        const int4 off = *reinterpret_cast<const int4*>(pre + j);
+        const int pos[kResSlots] = {off.x + lane, off.y + lane, off.z + lane, off.w + lane};
+#pragma unroll
+        for (int u = 0; u < kResSlots; ++u) {
+            const float4 b0 = s_b0[pos[u]], b1 = s_b1[pos[u]];
+            const float2 b2 = s_b2[pos[u]];
+            const int at = j + u < n ? __float_as_int(b2.y) : 0;
+            const float4 nc = *reinterpret_cast<const float4*>(n4 + at);
+            const float m[9] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w, b2.x};
+            block_mv(m, nc.x, nc.y, nc.z, o[u][0], o[u][1], o[u][2]);
+        }
+    };
     // k_bsr_init: r = b - A V, p = r.
-    const bool act = valid && !fx;
     float r0 = 0.0f, r1 = 0.0f, r2 = 0.0f;
     if (act) {
         r0 = a.b[3 * g];
         r1 = a.b[3 * g + 1];
         r2 = a.b[3 * g + 2];
     }
-    {
-        int pre = base;
-        for (int j = 0; j < width; ++j) {
-            const int cnt = __popc(__ballot_sync(kFull, n > j));
-            if (act && j < n) {
-                const int pos = pre + lane;
-                const float4 u = s_b0[pos], v = s_b1[pos];
-                const float m[9] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w, s_b8[pos]};
-                const float4 xc = s_n4[s_col[pos]];
-                float o0, o1, o2;
-                block_mv(m, xc.x, xc.y, xc.z, o0, o1, o2);
-                r0 = r0 - o0;
-                r1 = r1 - o1;
-                r2 = r2 - o2;
+    for (int j = 0; j < width; j += kResSlots) {
+        float o[kResSlots][3];
+        products(j, o);
+#pragma unroll
+        for (int u = 0; u < kResSlots; ++u)
+            if (j + u < n) {
+                r0 = r0 - o[u][0];
+                r1 = r1 - o[u][1];
+                r2 = r2 - o[u][2];
             }
-            pre += cnt;
-        }
     }
     float p0 = r0, p1 = r1, p2 = r2;
-    double d = 0.0, d1 = 0.0, d2 = 0.0;
+    Acc d = acc_zero(), d1 = acc_zero(), d2 = acc_zero();
     float d3 = 0.0f, d4 = 0.0f;
-    const double tiny = (double)sp.tiny;
-    const int nw = (int)(blockDim.x >> 5);
-    // Five barriers an iteration: after the directions, the products (d2), d3, the
-    // update (d1) and d4; the last also orders this iteration's reads of the directions
-    // before the next iteration writes them.
+    // The total of the warps' pairs, in every lane (every eight lanes read all eight).
+    auto total = [&](const Acc* wacc) { return pair_norm(lanes_sum<4>(wacc[lane & 7])); };
+    __syncthreads();  // init's reads of x are done
+    // Three barriers an iteration: after the directions, the products (d2) and the update (d1);
+    // the last two also order this iteration's reads of the directions before the next one's
+    // writes.
     for (int it = 0; it < sp.imax; ++it) {
         const bool first = it == 0;
         // The new direction of every row, fixed rows included (r = p = 0 there), by the
@@ -489,64 +483,38 @@ __global__ void __launch_bounds__(kThreads) k_bsr_resident(const BsrArgs a, cons
             n1 = r1 + n1 * d4;
             n2 = r2 + n2 * d4;
         }
-        if (first) __syncthreads();  // init's reads of x are done (later: the barrier after d4)
-        if (valid) s_n4[t] = make_float4(n0, n1, n2, 0.0f);
+        s_n4[t] = make_float4(n0, n1, n2, 0.0f);
         __syncthreads();
-        // k_bsr_spmv
-        Acc pd = acc_zero(), pd2 = acc_zero();
+        // k_bsr_spmv: four slots' loads and products are issued together, their sums run in slot
+        // order.
         float q0 = 0.0f, q1 = 0.0f, q2 = 0.0f;
-        // Four slots at a time: their loads and products are independent, so they are
-        // issued together (a slot past the row's end reads entry 0, which every system
-        // with blocks has, and is not added); the sums still run in slot order.
-        int pre = base;
         for (int j = 0; j < width; j += kResSlots) {
-            int pos[kResSlots];
-            bool ok[kResSlots];
-#pragma unroll
-            for (int u = 0; u < kResSlots; ++u) {
-                const int cnt = __popc(__ballot_sync(kFull, n > j + u));
-                ok[u] = act && j + u < n;
-                pos[u] = ok[u] ? pre + lane : 0;
-                pre += cnt;
-            }
             float o[kResSlots][3];
+            products(j, o);
 #pragma unroll
-            for (int u = 0; u < kResSlots; ++u) {
-                const float4 b0 = s_b0[pos[u]], b1 = s_b1[pos[u]];
-                const float m[9] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w, s_b8[pos[u]]};
-                const float4 nc = s_n4[s_col[pos[u]]];
-                block_mv(m, nc.x, nc.y, nc.z, o[u][0], o[u][1], o[u][2]);
-            }
-#pragma unroll
-            for (int u = 0; u < kResSlots; ++u) {
-                if (ok[u]) {
+            for (int u = 0; u < kResSlots; ++u)
+                if (j + u < n) {
                     q0 = q0 + o[u][0];
                     q1 = q1 + o[u][1];
                     q2 = q2 + o[u][2];
                 }
-            }
         }
+        Acc pd = acc_zero(), pd2 = acc_zero();
         if (act) {
             acc_add(pd, r0 * r0 + r1 * r1 + r2 * r2);
             acc_add(pd2, n0 * q0 + n1 * q1 + n2 * q2);
         }
         // d = r.r is the previous update's d1: the same terms in the same order.
-        if (first) warp_partial(pd, s_w0);
-        warp_partial(pd2, s_w1);
-        __syncthreads();
-        if (w == 0) {  // bsr_scalars<0>, in thread 0
-            const double t0 = first ? sum_warp_pairs(s_w0, nw) : d1;
-            const double t1 = sum_warp_pairs(s_w1, nw);
-            if (t == 0) {
-                d = t0;
-                d2 = t1;
-                double dd2 = d2;
-                if (fabs(dd2) < tiny) dd2 = tiny;  // FEM:885-886
-                s_d3 = (float)(t0 / dd2);
-            }
+        if (first) {
+            pd = lanes_sum<16>(pd);
+            if (lane == 0) s_w0[w] = pd;
         }
-        __syncthreads();  // d3, and every row's reads of r and p are done
-        d3 = s_d3;
+        pd2 = lanes_sum<16>(pd2);
+        if (lane == 0) s_w1[w] = pd2;
+        __syncthreads();
+        d = first ? total(s_w0) : d1;
+        d2 = total(s_w1);
+        d3 = quotient(d, pair_below(d2, sp.tiny) ? make_acc(sp.tiny, 0.0f) : d2);  // FEM:885-886
         // k_bsr_update
         Acc pd1 = acc_zero();
         if (act) {
@@ -561,22 +529,14 @@ __global__ void __launch_bounds__(kThreads) k_bsr_resident(const BsrArgs a, cons
             p2 = n2;
             acc_add(pd1, r0 * r0 + r1 * r1 + r2 * r2);
         }
-        warp_partial(pd1, s_w2);
+        pd1 = lanes_sum<16>(pd1);
+        if (lane == 0) s_w2[w] = pd1;
         __syncthreads();
-        if (w == 0) {  // bsr_scalars<1>, in thread 0
-            const double t2 = sum_warp_pairs(s_w2, nw);
-            if (t == 0) {
-                d1 = t2;
-                double dd = d;
-                if (fabs(dd) < tiny) dd = tiny;  // FEM:908-909
-                s_d4 = (float)(t2 / dd);
-            }
-        }
-        __syncthreads();
-        d4 = s_d4;
+        d1 = total(s_w2);
+        d4 = quotient(d1, pair_below(d, sp.tiny) ? make_acc(sp.tiny, 0.0f) : d);  // FEM:908-909
     }
     if (valid) {
-        if (!fx) {
+        if (act) {
             a.x[0][g] = x0;
             a.x[1][g] = x1;
             a.x[2][g] = x2;
@@ -586,9 +546,9 @@ __global__ void __launch_bounds__(kThreads) k_bsr_resident(const BsrArgs a, cons
     }
     if (t == 0) {
         BsrState& st = a.state[k];
-        st.d = d;
-        st.d1 = d1;
-        st.d2 = d2;
+        st.d = (double)d.s + (double)d.c;
+        st.d1 = (double)d1.s + (double)d1.c;
+        st.d2 = (double)d2.s + (double)d2.c;
         st.d3 = d3;
         st.d4 = d4;
         st.iter = sp.imax;
@@ -702,7 +662,7 @@ struct oc_bsr_solver {
     int32_t n_res = 0;
     int32_t* d_res_ids = nullptr;
     int32_t res_threads = 0;
-    int64_t res_nnzb_max = 0;  // blocks of the largest resident system
+    int64_t res_nnzb_max = 0;  // blocks in the free rows of the largest resident system
     int32_t res_stride = 0;    // blocks of the longest row of a resident system
     uint32_t* d_res_map = nullptr;
     size_t res_smem = 0;
@@ -935,10 +895,22 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
             order[r] = r;
         }
         auto degree = [&](int32_t r) { return d.row_ptr[r + 1] - d.row_ptr[r]; };
+        // A system of one block of rows whose blocks fit in shared memory runs resident.
+        int32_t maxdeg = 0;
+        for (int32_t r = 0; r < d.n_rows; ++r) maxdeg = std::max(maxdeg, degree(r));
+        const bool fits = d.n_rows <= kThreads && maxdeg <= kResMaxDeg &&
+                          resident_smem_bytes(kThreads, d.nnzb, kResMaxDeg) <= smem_cap && d.nnzb < 0xffff;
+        if (o.executor == OC_EXEC_RESIDENT && !fits) {
+            bsr_fail(s, OC_ERR_UNSUPPORTED, who_of(k) + "too large for the resident executor");
+            return bail(OC_ERR_UNSUPPORTED);
+        }
+        // (k_bsr_resident keeps no blocks of fixed rows: there they come last.)
+        const bool resident = fits && o.executor != OC_EXEC_STREAMED && o.executor != OC_EXEC_PLAIN;
+        auto weight = [&](int32_t r) { return resident && fixed[r0 + r] ? 0 : degree(r); };
         for (int32_t w0 = 0; w0 < d.n_rows; w0 += kSortWindow) {
             const int32_t w1 = std::min(d.n_rows, w0 + kSortWindow);
             std::stable_sort(order.begin() + w0, order.begin() + w1,
-                             [&](int32_t x, int32_t y) { return degree(x) > degree(y); });
+                             [&](int32_t x, int32_t y) { return weight(x) > weight(y); });
         }
         for (int32_t i = 0; i < d.n_rows; ++i) {
             const int32_t u = order[i];
@@ -947,28 +919,21 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
             deg_int[r0 + i] = degree(u);
             fixed_int[r0 + i] = fixed[r0 + u];
         }
-        for (int32_t i = 0; i < d.n_rows; i += 32) {
+        for (int32_t i = 0; i < d.n_rows && !resident; i += 32) {
             int32_t w = 0;
             for (int32_t l = i; l < std::min(d.n_rows, i + 32); ++l) w = std::max(w, deg_int[r0 + l]);
             slice_ptr.push_back(slots);
             width.push_back(w);
             slots += w;
         }
-        // A system of one block of rows whose blocks fit in shared memory runs resident.
-        int32_t maxdeg = 0;
-        for (int32_t r = 0; r < d.n_rows; ++r) maxdeg = std::max(maxdeg, degree(r));
-        const bool fits = d.n_rows <= kThreads && maxdeg <= kResMaxDeg &&
-                          resident_smem_bytes(kThreads, d.nnzb, kResMaxDeg) <= smem_cap;
-        if (o.executor == OC_EXEC_RESIDENT && !fits) {
-            bsr_fail(s, OC_ERR_UNSUPPORTED, who_of(k) + "too large for the resident executor");
-            return bail(OC_ERR_UNSUPPORTED);
-        }
-        if (fits && o.executor != OC_EXEC_STREAMED && o.executor != OC_EXEC_PLAIN) {
+        if (resident) {
             sp.blk0 = 0;
             sp.nblk = 0;
             res_ids.push_back(k);
-            s->res_nnzb_max = std::max<int64_t>(s->res_nnzb_max, d.nnzb);
-            s->res_stride = std::max(s->res_stride, std::max(maxdeg, 1));
+            int64_t kept = 0;
+            for (int32_t r = 0; r < d.n_rows; ++r) kept += weight(r);
+            s->res_nnzb_max = std::max(s->res_nnzb_max, kept);
+            s->res_stride = std::max(s->res_stride, (maxdeg / kResSlots + 1) * kResSlots);
             s->res_threads = std::max(s->res_threads, (d.n_rows + 31) / 32 * 32);
             s->res_rows += d.n_rows;
             s->res_nnzb += d.nnzb;
@@ -991,6 +956,7 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
     s->n_slots = slots;
     std::vector<int32_t> scol((size_t)slots * 32, -1);
     for (int32_t k = 0; k < n_systems; ++k) {
+        if (sys[k].nblk == 0) continue;  // resident: no slices
         const oc_bsr_desc& d = descs[k];
         const int64_t r0 = s->row_off[k];
         for (int32_t r = 0; r < d.n_rows; ++r) {
@@ -1075,15 +1041,31 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
     if (s->n_res > 0) {
         BSR_CREATE_TRY(bsr_upload(s, &s->d_res_ids, res_ids));
         s->res_smem = resident_smem_bytes(s->res_threads, s->res_nnzb_max, s->res_stride);
-        // Where each caller block goes: internal local row, slot, internal local column.
-        std::vector<uint32_t> map((size_t)std::max<int64_t>(nnzb, 1), 0u);
+        // Where each block of a free row goes, warp by warp and slot by slot in lane order, and its
+        // internal local column.
+        std::vector<uint32_t> map((size_t)std::max<int64_t>(nnzb, 1), 0xffffu);
         for (int32_t k : res_ids) {
             const oc_bsr_desc& d = descs[k];
             const int64_t r0 = s->row_off[k], e0 = s->nnz_off[k];
-            for (int32_t r = 0; r < d.n_rows; ++r)
-                for (int32_t e = d.row_ptr[r]; e < d.row_ptr[r + 1]; ++e)
-                    map[(size_t)(e0 + e)] = (uint32_t)(perm[r0 + r] - r0) | (uint32_t)(e - d.row_ptr[r]) << 8 |
-                                            (uint32_t)(perm[r0 + d.col[e]] - r0) << 16;
+            uint32_t pos = 0;  // the warp's first entry
+            for (int32_t w0 = 0; w0 < d.n_rows; w0 += 32) {
+                const int32_t w1 = std::min(d.n_rows, w0 + 32);
+                uint32_t pre[kResMaxDeg + 1];  // its slots' first entries: lanes in order of their counts
+                int32_t end = w1;
+                pre[0] = pos;
+                for (int32_t j = 0; j < kResMaxDeg; ++j) {
+                    while (end > w0 && (fixed_int[r0 + end - 1] || deg_int[r0 + end - 1] <= j)) --end;
+                    pre[j + 1] = pre[j] + (uint32_t)(end - w0);
+                }
+                pos = pre[kResMaxDeg];
+                for (int32_t i = w0; i < w1 && !fixed_int[r0 + i]; ++i) {
+                    const int32_t r = (int32_t)(iperm[r0 + i] - r0);
+                    const int32_t* col = d.col + d.row_ptr[r];
+                    uint32_t* out = map.data() + e0 + d.row_ptr[r];
+                    for (int32_t j = 0; j < deg_int[r0 + i]; ++j)
+                        out[j] = (pre[j] + (uint32_t)(i - w0)) | (uint32_t)(perm[r0 + col[j]] - r0) << 16;
+                }
+            }
         }
         BSR_CREATE_TRY(bsr_upload(s, &s->d_res_map, map));
         BSR_CREATE_TRY(cudaFuncSetAttribute(k_bsr_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
