@@ -8,14 +8,16 @@
 // and cut into slices of 32 rows (one warp) stored slot-major (sliced ELL with sorting):
 // slot j of lane l of slice s holds the j-th block of that row as two float4 and a
 // {component 8, column} pair, so every load of a warp is coalesced; the columns are a
-// static table built at create time, and each solve first packs the caller's CSR blocks.
+// static table built at create time, and oc_bsr_set_system packs the caller's CSR blocks.
 // Each lane sums its own row's products in slot order (the reference's order).
 //
-//   k_bsr_pack    CSR blocks -> sliced planes
+//   k_bsr_pack    CSR blocks -> sliced planes (when the caller sets them)
 //   k_bsr_init    r = b - A V, p = r               (FEM:841-859)
 //   k_bsr_spmv    p = r + d4 p (not in the first pass, FEM:913-917, rebuilt for the
 //                 neighbours from their r and p); q = A p; d = r.r, d2 = p.q  (FEM:865-883)
 //   k_bsr_update  d3 = d / d2; V += d3 p; r -= d3 q; d1 = r.r  (FEM:885-901), d4 = d1 / d
+//   k_bsr_persist  init and all iterations of the streamed systems in one cooperative launch, when
+//                 there are no more of them than SMs (else a WHILE loop of spmv and update)
 //   k_bsr_resident  all of the above for a system of up to 256 rows whose blocks fit in
 //                 shared memory, in one CTA: the blocks are read once, the iterations run
 //                 on chip, with the streamed kernels' bits (the default executor's choice)
@@ -118,6 +120,13 @@ __device__ __forceinline__ int32_t load_block(const BsrArgs& a, int64_t pos, flo
     m[4] = v.x; m[5] = v.y; m[6] = v.z; m[7] = v.w;
     m[8] = w.x;
     return __float_as_int(w.y);
+}
+
+// The next slot of the row requested into L1 while this one's neighbours are gathered.
+__device__ __forceinline__ void prefetch_block(const BsrArgs& a, int64_t pos) {
+    prefetch_l1(a.sb0 + pos);
+    prefetch_l1(a.sb1 + pos);
+    prefetch_l1(a.sb2 + pos);
 }
 
 __global__ void __launch_bounds__(kThreads) k_bsr_pack(const BsrArgs a) {
@@ -557,6 +566,297 @@ __global__ void __launch_bounds__(kThreads, 3) k_bsr_resident(const BsrArgs a, c
     }
 }
 
+// ---- the whole solve of the streamed systems in one cooperative launch -------------------------
+// The WHILE loop's iteration is two launches with a last-block epilogue each, whose gaps cost a
+// fifth of it, and its update pass streams 109 bytes a row through memory.  Here a system has
+// CTAs of its own (at most one per SM, 1024 threads), each with a contiguous range of its rows; a
+// thread's first kOwnRows rows keep x, r, p and q in registers, so the update writes only the
+// 16-byte r and p records the neighbours gather.  An iteration is the matrix-vector pass of
+// k_bsr_spmv, an exchange (d2), the update, and an exchange (d1) that also publishes the records:
+// every CTA sends its partial sum to all CTAs of its system as one packet in L2 (oc_exchange.cuh)
+// and sums the packets itself in the same order.  Before the packet of an update goes out, the
+// CTA's stores are fenced, and after the packets have come in, a fence drops what its L1 holds of
+// the records: one thread's fences, ordered with the others by the CTA's barriers.
+// The waits are bounded like those of the cloths' persistent CG (oc_persist.cu).
+// Measured on the 128 x 40 x 40 mesh (217k rows, 2.66 M blocks, 20 iterations): 1,088 us for the
+// loop before, now 571, 28 us an iteration for 108 MB of blocks (16 us at the copy rate) and two
+// exchanges of about 2.5 us.  Requesting a row's next slot into L1 while this one's neighbours are
+// gathered is 80 us of it (two slots ahead 587, four 609; into L2 648; in k_bsr_spmv, at twice the
+// threads, it costs 5 us a pass); plain instead of evict-first block loads 730; two rows in
+// registers 675, 512 threads with three rows 681.
+constexpr int kBT = 1024;
+constexpr int kBW = kBT / 32;
+constexpr int kOwnRows = 1;
+
+struct BsrPiece {
+    int32_t sys;
+    int32_t n;        // rows g0 ... g0 + n - 1 (n = 0: none)
+    int64_t g0;
+    int32_t idx, np;  // this CTA among its system's np CTAs
+    int32_t packet;   // the system's first packet
+    int32_t pad_;
+};
+
+struct BsrPlan {
+    const BsrPiece* pieces;  // one per CTA
+    ulonglong2* packets;     // two sets of n_packets, by the exchange's parity
+    PersistCtl* ctl;
+    int* err;
+    int32_t grid, n_packets;
+    uint32_t polls;
+};
+
+// q of row g: the products of its blocks with the directions (first: p alone; else r + d4 p), in
+// slot order.
+__device__ __forceinline__ void row_product(const BsrArgs& a, const BsrParams& sp, int64_t g, bool first, float d4,
+                                            float& q0, float& q1, float& q2) {
+    q0 = q1 = q2 = 0.0f;
+    const int n = a.deg[g];
+    const int64_t base = slot_pos(a, sp, g, 0);
+    for (int j = 0; j < n; ++j) {
+        if (j + 1 < n) prefetch_block(a, base + 32 * (int64_t)(j + 1));
+        float m[9];
+        const int32_t c = load_block(a, base + 32 * (int64_t)j, m);
+        const float4 pc = a.p4[c];
+        float v0 = pc.x, v1 = pc.y, v2 = pc.z;
+        if (!first) {
+            const float4 rc = a.r4[c];
+            v0 = rc.x + v0 * d4;
+            v1 = rc.y + v1 * d4;
+            v2 = rc.z + v2 * d4;
+        }
+        float o0, o1, o2;
+        block_mv(m, v0, v1, v2, o0, o1, o2);
+        q0 = q0 + o0;
+        q1 = q1 + o1;
+        q2 = q2 + o2;
+    }
+}
+
+__global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const BsrPlan P) {
+    __shared__ Acc s_w[kBW];
+    __shared__ float s_scal;
+    __shared__ int s_ok;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const BsrPiece pc = P.pieces[blockIdx.x];
+    const uint32_t base = *(volatile uint32_t*)&P.ctl->base;
+    if (tid == 0) s_ok = 1;
+    uint32_t tag = base;
+    StepArgs lim{};
+    lim.barrier_polls = P.polls;
+    // The sum of p over the system, in every lane of warp 0; publish: the CTA's stores before this
+    // are visible to the others' loads after their receive.
+    auto exchange = [&](Acc p, bool publish, Acc& total) -> bool {
+        ++tag;
+        p = lanes_sum<16>(p);
+        if (lane == 0) s_w[w] = p;
+        __syncthreads();
+        bool ok = true;
+        if (w == 0) {
+            total = lanes_sum<16>(s_w[lane]);
+            ulonglong2* const packets = P.packets + (size_t)(tag & 1) * P.n_packets + pc.packet;
+            if (pc.np > 1) {
+                if (lane == 0) {
+                    if (publish) __threadfence();
+                    put_global(packets + pc.idx, total, tag);
+                }
+                Acc sum = acc_zero();
+                for (int k0 = 0; k0 < pc.np && ok; k0 += 5 * 32) {
+                    Acc y[5];
+                    unsigned want = 0;
+#pragma unroll
+                    for (int u = 0; u < 5; ++u) {
+                        y[u] = acc_zero();
+                        if (k0 + u * 32 + lane < pc.np) want |= 1u << u;
+                    }
+                    ok = poll<5>(want, lim, P.err,
+                                 [&](int u) { return get_global(packets + k0 + u * 32 + lane, tag, y[u]); });
+                    sum = acc_merge(sum, acc_merge(acc_merge(acc_merge(y[0], y[1]), acc_merge(y[2], y[3])), y[4]));
+                }
+                total = lanes_sum<16>(sum);
+                if (publish && lane == 0) __threadfence();
+                __syncwarp();
+            }
+            total = pair_norm(total);
+        }
+        return ok;
+    };
+    auto settle = [&](bool ok, float scal) {  // by warp 0, then the barrier that hands it out
+        if (w == 0 && lane == 0) {
+            s_scal = scal;
+            if (!ok) {
+                s_ok = 0;
+                atomicOr(P.err, 1);
+            }
+        }
+        __syncthreads();
+    };
+    Acc d = acc_zero(), d1 = acc_zero(), d2 = acc_zero();
+    float d3 = 0.0f, d4 = 0.0f;
+    if (pc.n > 0) {
+        const BsrParams& sp = a.sys[pc.sys];
+        const float tiny = sp.tiny;
+        const int rows = (pc.n + kBT - 1) / kBT;
+        float x[kOwnRows][3], r[kOwnRows][3], p[kOwnRows][3], q[kOwnRows][3];
+        bool own[kOwnRows];
+        // r = b - A V, p = r.
+        Acc part = acc_zero();
+        auto residual = [&](int64_t g, float (&rr)[3]) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) rr[k] = a.b[3 * g + k];
+            const int n = a.deg[g];
+            const int64_t at = slot_pos(a, sp, g, 0);
+            for (int j = 0; j < n; ++j) {
+                if (j + 1 < n) prefetch_block(a, at + 32 * (int64_t)(j + 1));
+                float m[9], o0, o1, o2;
+                const int32_t c = load_block(a, at + 32 * (int64_t)j, m);
+                block_mv(m, a.x[0][c], a.x[1][c], a.x[2][c], o0, o1, o2);
+                rr[0] = rr[0] - o0;
+                rr[1] = rr[1] - o1;
+                rr[2] = rr[2] - o2;
+            }
+        };
+#pragma unroll
+        for (int u = 0; u < kOwnRows; ++u) {
+            const int64_t g = pc.g0 + u * kBT + tid;
+            const bool in = u * kBT + tid < pc.n;
+            own[u] = in && !a.fixed[g];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) x[u][k] = r[u][k] = p[u][k] = q[u][k] = 0.0f;
+            if (own[u]) {
+                residual(g, r[u]);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    p[u][k] = r[u][k];
+                    x[u][k] = a.x[k][g];
+                }
+                acc_add(part, r[u][0] * r[u][0] + r[u][1] * r[u][1] + r[u][2] * r[u][2]);
+            }
+            if (in) {
+                a.r4[g] = make_float4(r[u][0], r[u][1], r[u][2], 0.0f);
+                a.p4[g] = make_float4(r[u][0], r[u][1], r[u][2], 0.0f);
+            }
+        }
+        for (int u = kOwnRows; u < rows; ++u) {
+            const int64_t g = pc.g0 + (int64_t)u * kBT + tid;
+            if (u * kBT + tid >= pc.n) break;
+            float rr[3] = {0.0f, 0.0f, 0.0f};
+            if (!a.fixed[g]) {
+                residual(g, rr);
+                acc_add(part, rr[0] * rr[0] + rr[1] * rr[1] + rr[2] * rr[2]);
+            }
+            a.r4[g] = make_float4(rr[0], rr[1], rr[2], 0.0f);
+            a.p4[g] = make_float4(rr[0], rr[1], rr[2], 0.0f);
+        }
+        if (sp.imax > 0) {
+            const bool ok = exchange(part, true, d);
+            settle(ok, 0.0f);
+        }
+        for (int it = 0; it < sp.imax && s_ok; ++it) {
+            const bool first = it == 0;
+            // The new directions of the thread's rows and their products.
+            part = acc_zero();
+#pragma unroll
+            for (int u = 0; u < kOwnRows; ++u) {
+                if (!own[u]) continue;
+                if (!first) {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) p[u][k] = r[u][k] + p[u][k] * d4;
+                }
+                row_product(a, sp, pc.g0 + u * kBT + tid, first, d4, q[u][0], q[u][1], q[u][2]);
+                acc_add(part, p[u][0] * q[u][0] + p[u][1] * q[u][1] + p[u][2] * q[u][2]);
+            }
+            for (int u = kOwnRows; u < rows; ++u) {
+                const int64_t g = pc.g0 + (int64_t)u * kBT + tid;
+                if (u * kBT + tid >= pc.n) break;
+                if (a.fixed[g]) continue;
+                const float4 pg = a.p4[g], rg = a.r4[g];
+                float n0 = pg.x, n1 = pg.y, n2 = pg.z;
+                if (!first) {
+                    n0 = rg.x + n0 * d4;
+                    n1 = rg.y + n1 * d4;
+                    n2 = rg.z + n2 * d4;
+                }
+                float q0, q1, q2;
+                row_product(a, sp, g, first, d4, q0, q1, q2);
+                a.q[0][g] = q0;
+                a.q[1][g] = q1;
+                a.q[2][g] = q2;
+                acc_add(part, n0 * q0 + n1 * q1 + n2 * q2);
+            }
+            bool ok = exchange(part, false, d2);
+            settle(ok, w == 0 ? quotient(d, pair_below(d2, tiny) ? make_acc(tiny, 0.0f) : d2) : 0.0f);  // FEM:885-886
+            if (!s_ok) break;
+            d3 = s_scal;
+            // V += p d3, r -= q d3 (FEM:895-896); the records for the neighbours.
+            part = acc_zero();
+#pragma unroll
+            for (int u = 0; u < kOwnRows; ++u) {
+                if (!own[u]) continue;
+                const int64_t g = pc.g0 + u * kBT + tid;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    x[u][k] = x[u][k] + p[u][k] * d3;
+                    r[u][k] = r[u][k] - q[u][k] * d3;
+                }
+                a.r4[g] = make_float4(r[u][0], r[u][1], r[u][2], 0.0f);
+                a.p4[g] = make_float4(p[u][0], p[u][1], p[u][2], 0.0f);
+                acc_add(part, r[u][0] * r[u][0] + r[u][1] * r[u][1] + r[u][2] * r[u][2]);
+            }
+            for (int u = kOwnRows; u < rows; ++u) {
+                const int64_t g = pc.g0 + (int64_t)u * kBT + tid;
+                if (u * kBT + tid >= pc.n) break;
+                if (a.fixed[g]) continue;
+                const float4 rg = a.r4[g], pg = a.p4[g];
+                const float ro[3] = {rg.x, rg.y, rg.z}, po[3] = {pg.x, pg.y, pg.z};
+                float rn[3], pn[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    pn[k] = first ? po[k] : ro[k] + po[k] * d4;
+                    a.x[k][g] = a.x[k][g] + pn[k] * d3;
+                    rn[k] = ro[k] - a.q[k][g] * d3;
+                }
+                a.r4[g] = make_float4(rn[0], rn[1], rn[2], 0.0f);
+                a.p4[g] = make_float4(pn[0], pn[1], pn[2], 0.0f);
+                acc_add(part, rn[0] * rn[0] + rn[1] * rn[1] + rn[2] * rn[2]);
+            }
+            ok = exchange(part, true, d1);
+            settle(ok, w == 0 ? quotient(d1, pair_below(d, tiny) ? make_acc(tiny, 0.0f) : d) : 0.0f);  // FEM:908-909
+            d4 = s_scal;
+            if (it + 1 < sp.imax) d = d1;
+        }
+        if (s_ok) {
+#pragma unroll
+            for (int u = 0; u < kOwnRows; ++u)
+                if (own[u]) {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) a.x[k][pc.g0 + u * kBT + tid] = x[u][k];
+                }
+            if (pc.idx == 0 && tid == 0) {
+                BsrState& st = a.state[pc.sys];
+                st.d = (double)d.s + (double)d.c;
+                st.d1 = (double)d1.s + (double)d1.c;
+                st.d2 = (double)d2.s + (double)d2.c;
+                st.d3 = d3;
+                st.d4 = d4;
+                st.iter = sp.imax;
+                st.active = 0;
+                st.ticket = 0;
+            }
+        }
+    }
+    if (tid == 0) {
+        // The last CTA to leave moves the tags past those of this launch.
+        atomicMax(&P.ctl->used, tag - base + 1);
+        __threadfence();
+        if (atomicAdd(&P.ctl->left, 1u) == gridDim.x - 1) {
+            P.ctl->base = base + *(volatile uint32_t*)&P.ctl->used;
+            P.ctl->used = 0;
+            P.ctl->left = 0;
+        }
+    }
+}
+
 // Host arrays arrive in the caller's order in staging buffers.  k_bsr_check flags a
 // non-finite block or b in a free row, or a non-finite x (FEM:392-393 puts FLT_MAX in
 // fixed rows); nothing is committed unless the flag stays clear.
@@ -642,7 +942,7 @@ struct oc_bsr_solver {
     std::vector<void*> allocs;
     uint8_t* d_fixed = nullptr;
     int32_t* d_row_ptr = nullptr;
-    float* d_cblk = nullptr;  // the caller's CSR blocks (packed at each solve)
+    float* d_cblk = nullptr;  // the caller's CSR blocks (oc_bsr_set_system packs the streamed systems')
     float* d_b = nullptr;
     // set_system's staging (caller order) and the tables its kernels use
     float* d_stage_blk = nullptr;
@@ -666,6 +966,7 @@ struct oc_bsr_solver {
     int32_t res_stride = 0;    // blocks of the longest row of a resident system
     uint32_t* d_res_map = nullptr;
     size_t res_smem = 0;
+    BsrPlan plan{};     // k_bsr_persist over the streamed systems (grid 0: the WHILE loop)
     int64_t st_rows = 0, st_nnzb = 0, res_rows = 0, res_nnzb = 0;  // streamed / resident sizes
     std::string err;
 };
@@ -728,6 +1029,82 @@ void launch_resident(const oc_bsr_solver* s, const BsrArgs& a) {
                                                                         s->d_res_map, s->res_stride);
 }
 
+cudaError_t launch_bsr_persist(const oc_bsr_solver* s) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)s->plan.grid);
+    cfg.blockDim = dim3(kBT);
+    cfg.stream = s->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_bsr_persist, s->args, s->plan);
+}
+
+// k_bsr_persist's plan: every streamed system on CTAs of its own, in proportion to its rows and
+// with at least kBsrMinRows each (a CTA of few rows has idle warps, but its rows' chains of
+// dependent loads run side by side), where there are no more systems than SMs.
+constexpr int64_t kBsrMinRows = 256;
+
+oc_status plan_bsr_persist(oc_bsr_solver* s, const std::vector<BsrParams>& sys) {
+    int sms = 0, coop = 0;
+    BSR_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+    BSR_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
+    std::vector<int32_t> ids;
+    for (int32_t k = 0; k < s->n_sys; ++k)
+        if (sys[k].nblk > 0) ids.push_back(k);
+    if (!coop || ids.empty() || (int)ids.size() > sms || std::getenv("OC_BSR_VARIANT")) return OC_OK;
+    int64_t chunk = std::max<int64_t>(kBsrMinRows, ((s->st_rows + sms - 1) / sms + 31) / 32 * 32);
+    for (;; chunk += 32) {
+        int64_t n = 0;
+        for (int32_t k : ids) n += (sys[k].n_rows + chunk - 1) / chunk;
+        if (n <= sms) break;
+    }
+    std::vector<BsrPiece> pieces;
+    int32_t packets = 0;
+    for (int32_t k : ids) {
+        const int64_t n = sys[k].n_rows, c = (n + chunk - 1) / chunk, each = ((n + c - 1) / c + 31) / 32 * 32;
+        const size_t p0 = pieces.size();
+        for (int64_t r = 0; r < n; r += each) {
+            BsrPiece pc{};
+            pc.sys = k;
+            pc.g0 = sys[k].row0 + r;
+            pc.n = (int32_t)std::min(each, n - r);
+            pc.idx = (int32_t)(pieces.size() - p0);
+            pc.packet = packets;
+            pieces.push_back(pc);
+        }
+        for (size_t i = p0; i < pieces.size(); ++i) pieces[i].np = (int32_t)(pieces.size() - p0);
+        packets += (int32_t)(pieces.size() - p0);
+    }
+    BsrPlan& P = s->plan;
+    BsrPiece* d = nullptr;
+    BSR_TRY(bsr_upload(s, &d, pieces));
+    P.pieces = d;
+    const size_t n_words = 2 * (size_t)packets + 2;  // the packets, the tags' state, the error word
+    static_assert(sizeof(PersistCtl) <= sizeof(ulonglong2), "the tags' state in one packet's place");
+    BSR_TRY(bsr_alloc(s, &P.packets, n_words));
+    BSR_TRY(cudaMemset(P.packets, 0, n_words * sizeof(ulonglong2)));
+    P.ctl = reinterpret_cast<PersistCtl*>(P.packets + 2 * (size_t)packets);
+    P.err = reinterpret_cast<int*>(P.packets + 2 * (size_t)packets + 1);
+    P.n_packets = packets;
+    P.polls = 1u << 22;
+    P.grid = (int32_t)pieces.size();
+    return OC_OK;
+}
+
+// Synchronises the stream; a wait of k_bsr_persist that gave up is reported, once.
+oc_status bsr_finish(oc_bsr_solver* s) {
+    *s->h_flag = 0;
+    if (s->plan.err)
+        BSR_TRY(cudaMemcpyAsync(s->h_flag, s->plan.err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    BSR_TRY(cudaStreamSynchronize(s->stream));
+    if (*s->h_flag == 0) return OC_OK;
+    BSR_TRY(cudaMemset(s->plan.err, 0, sizeof(int)));
+    return bsr_fail(s, OC_ERR_DEVICE_TIMEOUT, "k_bsr_persist: a wait gave up (the solution is not complete)");
+}
+
 oc_status bsr_build_graph(oc_bsr_solver* s) {
     cudaGraph_t g = nullptr;
     BSR_TRY(cudaGraphCreate(&g, 0));
@@ -744,7 +1121,7 @@ oc_status bsr_build_graph(oc_bsr_solver* s) {
         p.kernelParams = params;
         return p;
     };
-    cudaGraphNode_t n_reset, n_pack, n_init, n_loop, n_spmv, n_upd, n_res;
+    cudaGraphNode_t n_reset, n_init, n_loop, n_spmv, n_upd, n_res;
     if (s->n_res > 0) {  // independent of the streamed systems' nodes
         const int32_t* ids = s->d_res_ids;
         int64_t nnzb_max = s->res_nnzb_max;
@@ -777,10 +1154,8 @@ oc_status bsr_build_graph(oc_bsr_solver* s) {
     mp.height = 1;
     mp.pitch = sizeof(int32_t);
     BSR_TRY(cudaGraphAddMemsetNode(&n_reset, g, nullptr, 0, &mp));
-    cudaKernelNodeParams p = kp(k_bsr_pack);
-    BSR_TRY(cudaGraphAddKernelNode(&n_pack, g, &n_reset, 1, &p));
-    p = kp(k_bsr_init);
-    BSR_TRY(cudaGraphAddKernelNode(&n_init, g, &n_pack, 1, &p));
+    cudaKernelNodeParams p = kp(k_bsr_init);
+    BSR_TRY(cudaGraphAddKernelNode(&n_init, g, &n_reset, 1, &p));
     cudaGraphNodeParams cp{};
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = handle;
@@ -906,11 +1281,13 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
         }
         // (k_bsr_resident keeps no blocks of fixed rows: there they come last.)
         const bool resident = fits && o.executor != OC_EXEC_STREAMED && o.executor != OC_EXEC_PLAIN;
-        auto weight = [&](int32_t r) { return resident && fixed[r0 + r] ? 0 : degree(r); };
+        std::vector<int32_t> weight(d.n_rows);
+        for (int32_t r = 0; r < d.n_rows; ++r) weight[r] = resident && fixed[r0 + r] ? 0 : degree(r);
+        const int32_t* wt = weight.data();
         for (int32_t w0 = 0; w0 < d.n_rows; w0 += kSortWindow) {
             const int32_t w1 = std::min(d.n_rows, w0 + kSortWindow);
             std::stable_sort(order.begin() + w0, order.begin() + w1,
-                             [&](int32_t x, int32_t y) { return weight(x) > weight(y); });
+                             [wt](int32_t x, int32_t y) { return wt[x] > wt[y]; });
         }
         for (int32_t i = 0; i < d.n_rows; ++i) {
             const int32_t u = order[i];
@@ -931,7 +1308,7 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
             sp.nblk = 0;
             res_ids.push_back(k);
             int64_t kept = 0;
-            for (int32_t r = 0; r < d.n_rows; ++r) kept += weight(r);
+            for (int32_t r = 0; r < d.n_rows; ++r) kept += weight[r];
             s->res_nnzb_max = std::max(s->res_nnzb_max, kept);
             s->res_stride = std::max(s->res_stride, (maxdeg / kResSlots + 1) * kResSlots);
             s->res_threads = std::max(s->res_threads, (d.n_rows + 31) / 32 * 32);
@@ -1071,6 +1448,10 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
         BSR_CREATE_TRY(cudaFuncSetAttribute(k_bsr_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)s->res_smem));
     }
+    if (oc_status st = plan_bsr_persist(s, sys)) return bail(st);
+    BSR_CREATE_TRY(cudaDeviceSynchronize());
+    launch(k_bsr_pack, a, s->n_blocks, s->stream);  // the columns; oc_bsr_set_system packs the blocks
+    BSR_CREATE_TRY(cudaGetLastError());
     BSR_CREATE_TRY(cudaDeviceSynchronize());
 #undef BSR_CREATE_TRY
     *out = s;
@@ -1125,6 +1506,11 @@ oc_status oc_bsr_set_system(oc_bsr_solver* s, const float* blocks, const float* 
     if (blocks)
         BSR_TRY(cudaMemcpyAsync(s->d_cblk, s->d_stage_blk, sizeof(float) * 9 * s->nnzb, cudaMemcpyDeviceToDevice,
                                 s->stream));
+    if (blocks && s->n_blocks > 0) {  // the streamed systems' sliced planes
+        launch(k_bsr_pack, s->args, s->n_blocks, s->stream);
+        BSR_TRY(cudaGetLastError());
+        s->launches += 1;
+    }
     if (b || x) {
         k_bsr_commit<<<grid, kThreads, 0, s->stream>>>(s->args, s->d_b, b ? s->d_stage_b : nullptr,
                                                        x ? s->d_stage_x : nullptr, s->d_perm, rows);
@@ -1136,13 +1522,22 @@ oc_status oc_bsr_set_system(oc_bsr_solver* s, const float* blocks, const float* 
 oc_status oc_bsr_solve(oc_bsr_solver* s) {
     if (!bsr_valid(s)) return OC_ERR_INVALID_ARGUMENT;
     BSR_TRY(cudaSetDevice(s->device));
+    if (s->use_graph && s->plan.grid > 0) {
+        if (s->n_res > 0) {
+            launch_resident(s, s->args);
+            BSR_TRY(cudaGetLastError());
+        }
+        BSR_TRY(launch_bsr_persist(s));
+        s->launches += 1 + (s->n_res > 0 ? 1 : 0);
+        return OC_OK;
+    }
     if (s->use_graph) {
         if (!s->exec) {
             oc_status st = bsr_build_graph(s);
             if (st != OC_OK) return st;
         }
         BSR_TRY(cudaGraphLaunch(s->exec, s->stream));
-        s->launches += (s->n_blocks > 0 ? 2 : 0) + (s->n_res > 0 ? 1 : 0);
+        s->launches += (s->n_blocks > 0 ? 1 : 0) + (s->n_res > 0 ? 1 : 0);
         return OC_OK;
     }
     BsrArgs a = s->args;
@@ -1154,10 +1549,9 @@ oc_status oc_bsr_solve(oc_bsr_solver* s) {
     }
     if (s->n_blocks == 0) return OC_OK;
     BSR_TRY(cudaMemsetAsync(a.unfinished, 0, sizeof(int32_t), s->stream));
-    launch(k_bsr_pack, a, s->n_blocks, s->stream);
     launch(k_bsr_init, a, s->n_blocks, s->stream);
     BSR_TRY(cudaGetLastError());
-    s->launches += 2;
+    s->launches += 1;
     int32_t* h = nullptr;
     BSR_TRY(cudaMallocHost(&h, sizeof(int32_t)));
     for (;;) {
@@ -1267,8 +1661,7 @@ oc_status oc_bsr_get_solution(oc_bsr_solver* s, float* x, float* residual) {
     if (x) BSR_TRY(cudaMemcpyAsync(x, dx, sizeof(float) * 3 * rows, cudaMemcpyDeviceToHost, s->stream));
     if (residual)
         BSR_TRY(cudaMemcpyAsync(residual, dr, sizeof(float) * 3 * rows, cudaMemcpyDeviceToHost, s->stream));
-    BSR_TRY(cudaStreamSynchronize(s->stream));
-    return OC_OK;
+    return bsr_finish(s);
 }
 
 oc_status oc_bsr_get_launch_count(oc_bsr_solver* s, int64_t* kernels_launched) {
@@ -1283,8 +1676,7 @@ oc_status oc_bsr_get_launch_count(oc_bsr_solver* s, int64_t* kernels_launched) {
 
 oc_status oc_bsr_synchronize(oc_bsr_solver* s) {
     if (!bsr_valid(s)) return OC_ERR_INVALID_ARGUMENT;
-    BSR_TRY(cudaStreamSynchronize(s->stream));
-    return OC_OK;
+    return bsr_finish(s);
 }
 
 }  // extern "C"
