@@ -384,7 +384,7 @@ def _cg_roofline(prof: dict, peak: float) -> dict:
     """The SpMV-bound CG kernels the step actually launched (persistent, block-resident,
     direction/update or the COUPLED pair), their algorithmic bytes over their summed
     CUDA-event durations."""
-    cg = ["k_cg_persist", "k_resident", "k_cg_dir", "k_cg_update", "k_cpl_dir", "k_cpl_update"]
+    cg = ["k_cg_persist", "k_resident", "k_cg_dir", "k_cg_update", "k_cpl_persist", "k_cpl_dir", "k_cpl_update"]
     pair = [k for k in cg if k in prof and prof[k]["launches"] > 0]
     if not pair:
         return None

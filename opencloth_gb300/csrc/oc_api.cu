@@ -101,6 +101,9 @@ struct oc_solver {
     // The CG loop of the streamed REFERENCE cloths as one cooperative launch (k_cg_persist)
     // when there is no COUPLED cloth; otherwise the WHILE loop.
     bool persist = false;
+    bool cpl_persist = false;  // k_cpl_persist runs the COUPLED cloths
+    CplPlan cplan{};           // their pieces (grid 0: none, or not available)
+    int cpl_rows_max = 0;
     PersistPlan pplan{};  // the streamed REFERENCE cloths' pieces (grid 0: none, or not available)
     // k_assemble_finish runs when a strip-swept cloth is resident or the streamed CG is
     // not the persistent one; otherwise k_cg_persist forms their delta0 itself.
@@ -329,6 +332,10 @@ void account_step_bytes(const oc_solver* s, KernelTimer* t) {
             const double it = (double)st.iter;
             double dirs = it > 0 ? 37.0 * nv + 53.0 * nv * (it - 1.0) + 48.0 * ns * it : 0.0;
             if (st.flags & OC_FLAG_BREAKDOWN) dirs += (it > 0 ? 53.0 : 37.0) * nv + 48.0 * ns;
+            if (s->cpl_persist) {  // k_cpl_persist: the same passes and the update in one launch
+                t->bytes[K_CPL_PERSIST] += dirs + (it > 0 ? 132.0 * nv + 148.0 * nv * (it - 1.0) : 0.0) + 76.0 * nv;
+                continue;
+            }
             t->bytes[K_CPL_DIR] += dirs;
             t->bytes[K_CPL_UPDATE] += it > 0 ? 132.0 * nv + 148.0 * nv * (it - 1.0) : 0.0;
             t->bytes[K_INTEGRATE] += 76.0 * nv;
@@ -484,18 +491,20 @@ oc_status step_host_driven(oc_solver* s, float dt, bool per_cloth, KernelTimer* 
         }
         if ((st = launch_resident_all(s, a, t)) != OC_OK) return st;
         const int nb = s->n_streamed_blocks, nc = s->n_cpl_blocks;
-        if (s->persist) {
+        if (s->persist || s->cpl_persist) {  // (not both: k_cpl_persist wants every other cloth resident)
+            const KernelKind k = s->persist ? K_CG_PERSIST : K_CPL_PERSIST;
             if (t) OC_TRY(cudaEventRecord(t->ev[0], s->stream));
             sa.persist_d0 = 1;
-            OC_TRY(launch_cg_persist(sa, s->pplan, s->stream));
+            OC_TRY(s->persist ? launch_cg_persist(sa, s->pplan, s->stream)
+                              : launch_cpl_persist(ca, s->cplan, s->stream));
             s->host_launches += 1;
             if (t) {
                 OC_TRY(cudaEventRecord(t->ev[1], s->stream));
                 OC_TRY(cudaEventSynchronize(t->ev[1]));
                 float ms = 0.0f;
                 OC_TRY(cudaEventElapsedTime(&ms, t->ev[0], t->ev[1]));
-                t->ms[K_CG_PERSIST] += ms;
-                t->launches[K_CG_PERSIST] += 1;
+                t->ms[k] += ms;
+                t->launches[k] += 1;
             }
         } else if (nb > 0 || nc > 0) {
             for (;;) {
@@ -543,7 +552,8 @@ oc_status build_graph(oc_solver* s, float dt) {
     s->graph = g;
     const bool persist = s->persist;
     const bool streamed = s->n_streamed_blocks > 0 && !persist, coupled = s->n_cpl_blocks > 0;
-    const bool loop = streamed || coupled;
+    const bool cpl_persist = s->cpl_persist;
+    const bool loop = streamed || (coupled && !cpl_persist);
     // The WHILE loop's handle exists only when there are streamed cloths (a handle that
     // no conditional node uses makes the graph fail to instantiate).
     cudaGraphConditionalHandle handle = 0;
@@ -641,7 +651,7 @@ oc_status build_graph(oc_solver* s, float dt) {
             OC_TRY(add_body(K_CG_DIR, T_STR));
             OC_TRY(add_body(K_CG_UPDATE, T_STR));
         }
-        if (coupled) {
+        if (coupled) {  // (no k_cpl_persist beside streamed cloths)
             OC_TRY(add_body(K_CPL_DIR, T_CPL));
             OC_TRY(add_body(K_CPL_UPDATE, T_CPL));
         }
@@ -649,9 +659,9 @@ oc_status build_graph(oc_solver* s, float dt) {
         OC_TRY(cudaGraphAddKernelNode(&n_int, g, &n_loop, 1, &kp));
         updates.push_back(n_int);
     }
-    if (persist) {
-        // The streamed cloths' whole CG loop and update: the cooperative launch, captured
-        // into a child graph.
+    if (persist || cpl_persist) {
+        // The streamed (or the COUPLED) cloths' whole CG loop and update: the cooperative launch,
+        // captured into a child graph.
         cudaGraphNode_t n_pc;
         cudaGraph_t pg = nullptr;
         OC_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
@@ -659,11 +669,12 @@ oc_status build_graph(oc_solver* s, float dt) {
         pa.blocks = s->d_streamed_blocks;
         pa.use_cond = 0;
         pa.persist_d0 = 1;
-        cudaError_t le = launch_cg_persist(pa, s->pplan, s->stream);
+        cudaError_t le = persist ? launch_cg_persist(pa, s->pplan, s->stream)
+                                 : launch_cpl_persist(ca, s->cplan, s->stream);
         cudaError_t ce = cudaStreamEndCapture(s->stream, &pg);
         if (le != cudaSuccess || ce != cudaSuccess) {
             if (pg) cudaGraphDestroy(pg);
-            return fail_cuda(s, le != cudaSuccess ? le : ce, "capture of k_cg_persist");
+            return fail_cuda(s, le != cudaSuccess ? le : ce, persist ? "capture of k_cg_persist" : "capture of k_cpl_persist");
         }
         cudaError_t e = cudaGraphAddChildGraphNode(&n_pc, g, &n_last, 1, pg);
         cudaGraphDestroy(pg);
@@ -1154,6 +1165,69 @@ oc_status plan_persist(oc_solver* s) {
     return OC_OK;
 }
 
+// k_cpl_persist's plan: every COUPLED cloth on CTAs of its own, in proportion to its vertices and
+// with at least kCplMinRows each, where there are no more such cloths than SMs.  Streamed
+// REFERENCE cloths beside them keep the WHILE loop of both (two cooperative launches of one CTA
+// per SM would run one behind the other).
+constexpr int64_t kCplMinRows = 256;
+
+oc_status plan_coupled(oc_solver* s) {
+    CplPlan& P = s->cplan;
+    P.grid = 0;
+    if (!s->coop || s->cpl_rows_max <= 0) return OC_OK;
+    int64_t total = 0;
+    int32_t cloths = 0;
+    for (const InstParams& ip : s->inst_host)
+        if (ip.coupled) {
+            total += ip.nv;
+            ++cloths;
+        }
+    if (cloths == 0 || cloths > s->sm_count || s->n_streamed_blocks > 0) return OC_OK;
+    int64_t chunk = std::max<int64_t>(kCplMinRows, ((total + s->sm_count - 1) / s->sm_count + 31) / 32 * 32);
+    for (;; chunk += 32) {
+        int64_t n = 0;
+        for (const InstParams& ip : s->inst_host)
+            if (ip.coupled) n += (ip.nv + chunk - 1) / chunk;
+        if (n <= s->sm_count) break;
+    }
+    std::vector<CplPiece> pieces;
+    P.n_packets = 0;
+    int64_t most = 0;
+    for (int32_t k = 0; k < s->n_inst; ++k) {
+        const InstParams& ip = s->inst_host[(size_t)k];
+        if (!ip.coupled) continue;
+        const int64_t c = (ip.nv + chunk - 1) / chunk, each = ((ip.nv + c - 1) / c + 31) / 32 * 32;
+        const size_t p0 = pieces.size();
+        for (int64_t l = 0; l < ip.nv; l += each) {
+            CplPiece pc{};
+            pc.v = ip.v_off + l;
+            pc.n = (int32_t)std::min<int64_t>(each, ip.nv - l);
+            pc.inst = k;
+            pc.idx = (int32_t)(pieces.size() - p0);
+            pc.packet = P.n_packets;
+            pieces.push_back(pc);
+        }
+        for (size_t i = p0; i < pieces.size(); ++i) pieces[i].np = (int32_t)(pieces.size() - p0);
+        P.n_packets += (int32_t)(pieces.size() - p0);
+        most = std::max(most, each);
+    }
+    P.smem_rows = (int32_t)std::min<int64_t>(most, s->cpl_rows_max);
+    CplPiece* d = const_cast<CplPiece*>(P.pieces);
+    OC_TRY(reupload(s, &d, pieces));
+    P.pieces = d;
+    dfree(s, &P.packets);
+    OC_TRY(dalloc(s, &P.packets, 2 * (size_t)P.n_packets));
+    OC_TRY(cudaMemset(P.packets, 0, 2 * (size_t)P.n_packets * sizeof(ulonglong2)));
+    if (!P.ctl) {
+        OC_TRY(dalloc(s, &P.ctl, 1));
+        OC_TRY(cudaMemset(P.ctl, 0, sizeof(PersistCtl)));
+    }
+    if (oc_status r = alloc_error_word(s)) return r;
+    P.err = s->d_perr;
+    P.grid = (int32_t)pieces.size();
+    return OC_OK;
+}
+
 // The launch plan from the handle's cloths and its launch configuration: which cloths run
 // resident (one cluster per cloth, the whole step on chip) and which streamed, resident
 // cloths grouped by launch shape into buckets, the assembly tables (record gather,
@@ -1251,6 +1325,9 @@ oc_status plan_execution(oc_solver* s) {
     if (any_streamed && !any_coupled)
         if (oc_status r = plan_persist(s)) return r;
     s->persist = cfg.persist && s->pplan.grid > 0;
+    if (any_coupled)
+        if (oc_status r = plan_coupled(s)) return r;
+    s->cpl_persist = cfg.persist && s->cplan.grid > 0;
     s->adj_persist = s->adj_allowed && s->persist_smem_max > 0 && !any_coupled && (!any_streamed || s->pplan.grid > 0);
     if (oc_status r = plan_sim(s)) return r;
     s->strip_finish = false;
@@ -1542,7 +1619,7 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
     s->any_coupled = P.any_coupled;
     if (P.any_coupled) {
         // Slot-major per-incidence layout: slices of 32 vertices, each as wide as its
-        // largest degree (padding slots hold the vertex itself and are never read).
+        // largest degree (padding slots are neither written nor read).
         const int64_t n_slices = (P.nv + 31) / 32;
         std::vector<int64_t> slice((size_t)n_slices + 1, 0);
         for (int64_t sl = 0; sl < n_slices; ++sl) {
@@ -1552,21 +1629,11 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
             slice[(size_t)sl + 1] = slice[(size_t)sl] + 32 * (int64_t)width;
         }
         const size_t slots = std::max<size_t>((size_t)slice[(size_t)n_slices], 1);
-        std::vector<int32_t> other(slots, 0);
-        for (int64_t g = 0; g < P.nv; ++g) {
-            const int64_t base = slice[(size_t)(g >> 5)] + (g & 31);
-            const int32_t deg = P.rowptr[g + 1] - P.rowptr[g];
-            for (int32_t e = 0; e < deg; ++e) other[(size_t)(base + 32 * e)] = P.inc[P.rowptr[g] + e].x & 0x7fffffff;
-        }
         int64_t* d_slice = nullptr;
         OC_CREATE_TRY(upload(s, &d_slice, slice));
         a.cpl_slice = d_slice;
-        int32_t* d_other = nullptr;
-        OC_CREATE_TRY(upload(s, &d_other, other));
-        a.cpl_o = d_other;
-        float* cplanes = nullptr;
-        OC_CREATE_TRY(dalloc(s, &cplanes, 5 * slots));
-        for (int k = 0; k < 5; ++k) a.cpl_c[k] = cplanes + (size_t)k * slots;
+        OC_CREATE_TRY(dalloc(s, &a.cpl_nb, slots));
+        OC_CREATE_TRY(dalloc(s, &a.cpl_go, slots));
         float* vplanes = nullptr;
         OC_CREATE_TRY(dalloc(s, &vplanes, 4 * stride));
         OC_CREATE_TRY(cudaMemset(vplanes, 0, 4 * stride * sizeof(float)));
@@ -1623,6 +1690,7 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
         int coop = 0;
         OC_CREATE_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
         s->coop = coop != 0;
+        if (s->coop && s->executor != OC_EXEC_PLAIN && s->any_coupled) OC_CREATE_TRY(prepare_coupled(s->device, &s->cpl_rows_max));
         if (s->coop && s->executor != OC_EXEC_PLAIN) OC_CREATE_TRY(prepare_persist(s->device, &s->persist_smem_max, &s->persist_clusters, &s->persist_pairs));
         if (s->executor != OC_EXEC_PLAIN) OC_CREATE_TRY(prepare_sim(s->device, &s->sim_smem_max));
         s->adj_allowed = !(pe && std::atoi(pe) == 0) && s->coop;
@@ -1819,7 +1887,7 @@ oc_status oc_step(oc_solver* s, float dt, int32_t n_steps) {
     // the device (loop_count).
     const int64_t per_step = (s->n_asm_blocks > 0 ? 1 : 0) + (s->n_grid_blocks > 0 ? 1 : 0) +
                              (s->args.n_strip_work > 0 ? (s->strip_finish ? 2 : 1) : 0) + (s->n_cpl_blocks > 0 ? 1 : 0) +
-                             (s->persist ? 1 : (s->n_upd_blocks > 0 ? 1 : 0)) + (int64_t)s->buckets.size() +
+                             (s->persist || s->n_upd_blocks > 0 ? 1 : 0) + (int64_t)s->buckets.size() +
                              (s->any_provot ? 1 : 0);
     s->host_launches += per_step * (int64_t)n_steps;
     return OC_OK;
@@ -2028,7 +2096,7 @@ oc_status oc_profile_steps(oc_solver* s, float dt, int32_t n_steps, int32_t max_
     if (st != OC_OK) return st;
     const KernelKind kinds[] = {K_ASSEMBLE, K_ASSEMBLE_GRID, K_ASSEMBLE_STRIP, K_ASSEMBLE_FINISH, K_CG_DIR,
                                 K_CG_UPDATE, K_INTEGRATE, K_CG_PERSIST, K_RESIDENT, K_PROVOT,
-                                K_CPL_ASSEMBLE, K_CPL_DIR, K_CPL_UPDATE};
+                                K_CPL_ASSEMBLE, K_CPL_DIR, K_CPL_UPDATE, K_CPL_PERSIST};
     int32_t n = 0;
     for (KernelKind k : kinds) {
         if (n >= max_kernels) break;
@@ -2036,6 +2104,8 @@ oc_status oc_profile_steps(oc_solver* s, float dt, int32_t n_steps, int32_t max_
         if ((k == K_CPL_ASSEMBLE || k == K_CPL_DIR || k == K_CPL_UPDATE) && !s->any_coupled) continue;
         if (k == K_ASSEMBLE_GRID && s->n_grid_blocks == 0) continue;
         if (k == K_CG_PERSIST && !s->persist) continue;
+        if (k == K_CPL_PERSIST && !s->cpl_persist) continue;
+        if ((k == K_CPL_DIR || k == K_CPL_UPDATE || k == K_INTEGRATE) && s->cpl_persist) continue;
         if ((k == K_CG_DIR || k == K_CG_UPDATE || k == K_INTEGRATE) && s->persist) continue;
         if ((k == K_ASSEMBLE_STRIP || k == K_ASSEMBLE_FINISH) && s->args.n_strip_work == 0) continue;
         if (k == K_ASSEMBLE_FINISH && !s->strip_finish) continue;
@@ -2828,7 +2898,7 @@ oc_status oc_autotune(oc_solver* s, float dt, const char* cache_path, int32_t fl
 
 oc_status oc_test_barrier_timeout(oc_solver* s, int32_t withhold_block, uint32_t max_polls) {
     if (!valid_solver(s) || withhold_block < -1) return OC_ERR_INVALID_ARGUMENT;
-    if (!s->persist && !s->adj_persist) return fail(s, OC_ERR_UNSUPPORTED, "the handle runs no persistent CG");
+    if (!s->persist && !s->cpl_persist && !s->adj_persist) return fail(s, OC_ERR_UNSUPPORTED, "the handle runs no persistent CG");
     OC_TRY(cudaSetDevice(s->device));
     OC_TRY(cudaStreamSynchronize(s->stream));
     s->args.withhold_block = withhold_block;

@@ -648,38 +648,8 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
     // are visible to the others' loads after their receive.
     auto exchange = [&](Acc p, bool publish, Acc& total) -> bool {
         ++tag;
-        p = lanes_sum<16>(p);
-        if (lane == 0) s_w[w] = p;
-        __syncthreads();
-        bool ok = true;
-        if (w == 0) {
-            total = lanes_sum<16>(s_w[lane]);
-            ulonglong2* const packets = P.packets + (size_t)(tag & 1) * P.n_packets + pc.packet;
-            if (pc.np > 1) {
-                if (lane == 0) {
-                    if (publish) __threadfence();
-                    put_global(packets + pc.idx, total, tag);
-                }
-                Acc sum = acc_zero();
-                for (int k0 = 0; k0 < pc.np && ok; k0 += 5 * 32) {
-                    Acc y[5];
-                    unsigned want = 0;
-#pragma unroll
-                    for (int u = 0; u < 5; ++u) {
-                        y[u] = acc_zero();
-                        if (k0 + u * 32 + lane < pc.np) want |= 1u << u;
-                    }
-                    ok = poll<5>(want, lim, P.err,
-                                 [&](int u) { return get_global(packets + k0 + u * 32 + lane, tag, y[u]); });
-                    sum = acc_merge(sum, acc_merge(acc_merge(acc_merge(y[0], y[1]), acc_merge(y[2], y[3])), y[4]));
-                }
-                total = lanes_sum<16>(sum);
-                if (publish && lane == 0) __threadfence();
-                __syncwarp();
-            }
-            total = pair_norm(total);
-        }
-        return ok;
+        return pull_sum<kBW>(p, P.packets + (size_t)(tag & 1) * P.n_packets + pc.packet, pc.idx, pc.np, tag, publish,
+                             lim, P.err, s_w, total);
     };
     auto settle = [&](bool ok, float scal) {  // by warp 0, then the barrier that hands it out
         if (w == 0 && lane == 0) {
@@ -845,16 +815,7 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
             }
         }
     }
-    if (tid == 0) {
-        // The last CTA to leave moves the tags past those of this launch.
-        atomicMax(&P.ctl->used, tag - base + 1);
-        __threadfence();
-        if (atomicAdd(&P.ctl->left, 1u) == gridDim.x - 1) {
-            P.ctl->base = base + *(volatile uint32_t*)&P.ctl->used;
-            P.ctl->used = 0;
-            P.ctl->left = 0;
-        }
-    }
+    if (tid == 0) leave_tags(P.ctl, base, tag - base + 1);
 }
 
 // Host arrays arrive in the caller's order in staging buffers.  k_bsr_check flags a

@@ -1,4 +1,5 @@
-// What the kernels that run whole CG loops share (oc_persist.cu, oc_sim.cu): the packets by
+// What the kernels that run whole CG loops share (oc_persist.cu, oc_sim.cu, oc_bsr.cu,
+// oc_coupled.cu): the packets by
 // which CTAs exchange partial sums, the bounded polls that wait for them, the quotient of the
 // scalar rule, and the two passes of one vertex.
 //
@@ -9,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "oc_device.cuh"
+#include "oc_internal.h"
 
 namespace oc {
 namespace {
@@ -84,6 +86,57 @@ __device__ __forceinline__ bool poll(unsigned want, const StepArgs& a, const int
         ++spins;
         if (spins > a.barrier_polls || ((spins & 63u) == 0 && __any_sync(0xffffffffu, load_relaxed(err) != 0)))
             return false;
+    }
+}
+
+// The sum of `part` over the threads of `np` CTAs without clusters, in every lane of warp 0 (in
+// the others `total` is not set): the CTA's own sum goes out as packet `idx` of `packets`, and
+// warp 0 reads all of them.  With `publish`, what the CTA's threads stored before is visible to
+// the other CTAs' loads after the barrier that the caller puts behind.  False (in warp 0) when a
+// wait gave up.  Every thread of the CTA, of WARPS <= 32 warps, calls it.
+template <int WARPS>
+__device__ __forceinline__ bool pull_sum(Acc part, ulonglong2* packets, int idx, int np, uint32_t tag, bool publish,
+                                         const StepArgs& a, const int* err, Acc* warp_sums, Acc& total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    part = lanes_sum<16>(part);
+    if (lane == 0) warp_sums[w] = part;
+    __syncthreads();
+    if (w != 0) return true;
+    bool ok = true;
+    total = lanes_sum<16>(lane < WARPS ? warp_sums[lane] : acc_zero());
+    if (np > 1) {
+        if (lane == 0) {
+            if (publish) __threadfence();
+            put_global(packets + idx, total, tag);
+        }
+        Acc sum = acc_zero();
+        for (int k0 = 0; k0 < np && ok; k0 += 5 * 32) {
+            Acc y[5];
+            unsigned want = 0;
+#pragma unroll
+            for (int u = 0; u < 5; ++u) {
+                y[u] = acc_zero();
+                if (k0 + u * 32 + lane < np) want |= 1u << u;
+            }
+            ok = poll<5>(want, a, err, [&](int u) { return get_global(packets + k0 + u * 32 + lane, tag, y[u]); });
+            sum = acc_merge(sum, acc_merge(acc_merge(acc_merge(y[0], y[1]), acc_merge(y[2], y[3])), y[4]));
+        }
+        total = lanes_sum<16>(sum);
+        if (publish && lane == 0) __threadfence();
+        __syncwarp();
+    }
+    total = pair_norm(total);
+    return ok;
+}
+
+// By one thread of a CTA that leaves: the last one moves the tags past those of this launch.
+__device__ __forceinline__ void leave_tags(PersistCtl* ctl, uint32_t base, uint32_t used) {
+    atomicMax(&ctl->used, used);
+    __threadfence();
+    if (atomicAdd(&ctl->left, 1u) == gridDim.x - 1) {
+        ctl->base = base + *(volatile uint32_t*)&ctl->used;
+        ctl->used = 0;
+        ctl->left = 0;
     }
 }
 

@@ -158,8 +158,8 @@ struct StepArgs {
     // incidence e of vertex g sits at cpl_slice[g >> 5] + 32 e + (g & 31), so a warp's
     // accesses to one slot are contiguous.
     const int64_t* cpl_slice;
-    const int32_t* cpl_o;
-    float* cpl_c[5];         // n0, n1, n2, beta, gamma
+    float4* cpl_nb;          // n0, n1, n2, beta
+    float2* cpl_go;          // gamma, the neighbour (an int32_t)
     float* cpl_m;
     float4* cpl_z;           // z = P^-1 r, 16-byte records (w unused): a neighbour's z and d are
     float4* cpl_d;           // two vector loads in k_cpl_dir
@@ -242,7 +242,7 @@ __host__ __device__ inline int stencil_class_1d(int32_t i, int32_t n) {
 enum KernelKind { K_ASSEMBLE = 0, K_CG_DIR = 1, K_CG_UPDATE = 2, K_INTEGRATE = 3, K_FORCES = 4, K_RESIDENT = 5,
                   K_PROVOT = 6, K_ELLIPSOID = 7, K_CPL_ASSEMBLE = 8, K_CPL_DIR = 9, K_CPL_UPDATE = 10,
                   K_ASSEMBLE_GRID = 11, K_CG_PERSIST = 12, K_ASSEMBLE_STRIP = 13, K_ASSEMBLE_FINISH = 14,
-                  K_COUNT = 15 };
+                  K_CPL_PERSIST = 15, K_COUNT = 16 };
 
 cudaError_t launch_test_cr_arith(unsigned long long* counts, uint64_t n_pairs, uint64_t seed, cudaStream_t stream);
 // The persistent CG (k_cg_persist, oc_persist.cu): the whole CG loop and the update of the
@@ -310,6 +310,27 @@ cudaError_t launch_set_pins(float4* V, uint8_t* pinflag, int64_t v0, int64_t nv,
 // COUPLED kernels (oc_coupled.cu).
 const void* coupled_fn(KernelKind k);
 cudaError_t launch_coupled(KernelKind k, const StepArgs& a, int nblocks, cudaStream_t stream);
+// The whole CG loop and the update of the COUPLED cloths in one cooperative launch
+// (k_cpl_persist): one CTA per SM at most, each with one contiguous piece of one cloth.
+constexpr int kCplThreads = 1024;
+constexpr int kCplRowFloats = 19;  // on-chip state of a vertex
+struct CplPiece {
+    int64_t v;        // vertices v ... v + n - 1
+    int32_t n, inst;
+    int32_t idx, np;  // this CTA among its cloth's np CTAs
+    int32_t packet;   // the cloth's first packet
+    int32_t pad_;
+};
+struct CplPlan {
+    const CplPiece* pieces;  // one per CTA
+    ulonglong2* packets;     // two sets of n_packets, by the exchange's parity
+    PersistCtl* ctl;
+    int* err;                // bit 0: a wait gave up
+    int32_t grid, n_packets;
+    int32_t smem_rows;       // vertices of a CTA (a multiple of 32) whose state is in shared memory
+};
+cudaError_t prepare_coupled(int device, int* max_rows);  // the most that smem_rows may be
+cudaError_t launch_cpl_persist(const StepArgs& a, const CplPlan& plan, cudaStream_t stream);
 
 const char* kernel_name(KernelKind k);
 const void* kernel_fn(KernelKind k, const StepArgs& a);  // the variant a selects

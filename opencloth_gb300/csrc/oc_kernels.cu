@@ -995,6 +995,7 @@ const char* kernel_name(KernelKind k) {
         case K_ASSEMBLE_FINISH: return "k_assemble_finish";
         case K_CPL_DIR: return "k_cpl_dir";
         case K_CPL_UPDATE: return "k_cpl_update";
+        case K_CPL_PERSIST: return "k_cpl_persist";
         default: return "?";
     }
 }

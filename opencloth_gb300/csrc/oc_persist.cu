@@ -492,16 +492,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
         if (!s_ok) break;
     }
     if (CS > 1) cluster_arrive();
-    if (tid == 0) {
-        // The last CTA to leave moves the tags past those of this launch.
-        atomicMax(&P.ctl->used, q + 2);
-        __threadfence();
-        if (atomicAdd(&P.ctl->left, 1u) == gridDim.x - 1) {
-            P.ctl->base = base + *(volatile uint32_t*)&P.ctl->used;
-            P.ctl->used = 0;
-            P.ctl->left = 0;
-        }
-    }
+    if (tid == 0) leave_tags(P.ctl, base, q + 2);
     if (s_ok) {
         // The cloths' scalars for the host, by each cloth's first piece.
         for (int j = tid; j < np; j += kPT) {
@@ -865,14 +856,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
     }
     if (CS > 1) cluster_arrive();
     if (tid == 0) {
-        // The last CTA to leave moves the tags past those of this launch.
-        atomicMax(&P.ctl->used, q + 2);
-        __threadfence();
-        if (atomicAdd(&P.ctl->left, 1u) == gridDim.x - 1) {
-            P.ctl->base = base + *(volatile uint32_t*)&P.ctl->used;
-            P.ctl->used = 0;
-            P.ctl->left = 0;
-        }
+        leave_tags(P.ctl, base, q + 2);
         if (s_ok && pc.head && n > 0) {
             InstState& is = a.state[pc.inst];
             is.delta0 = d0;
