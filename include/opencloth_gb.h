@@ -280,7 +280,7 @@ oc_status oc_tape_displacement(oc_solver* s, float* u);
 
 /* ---- launch configuration and its autotuner ------------------------------------------ */
 /* How a handle launches its step: which cloths run resident and in what CTA shape, whether
- * the resident kernel also assembles, whether up to 16 streamed cloths run their CG as one
+ * the resident kernel also assembles, whether the streamed cloths run their CG as one
  * cooperative launch, the force-gather variant, and the strip sweep of grid cloths.  None
  * of these changes the method; the resident kernel's reductions follow its CTA shape, so
  * results of different resident shapes can differ in the last bits (each shape is
@@ -292,7 +292,8 @@ typedef struct oc_launch_config {
     int32_t resident_fused;        /* 1: resident cloths assemble inside the resident kernel */
     int32_t persist;               /* 1: the CG of the streamed cloths as one cooperative launch */
     int32_t gather_variant;        /* incidence-record force gather: 0 block-cooperative, 1..6 per vertex */
-    int32_t strip;                 /* 1: grid cloths in the reference's spring order take the strip sweep */
+    int32_t strip;                 /* 1: grid cloths in the reference's spring order take the strip sweep (by default
+                                      where a handle's cloths all suit it and have 175,000 vertices together) */
     int32_t strip_rows;            /* rows per strip band (1 ... 64); 0: chosen from the work size */
     int32_t strip_variant;         /* strip CTAs per SM the registers are capped for: 2 or 3 */
 } oc_launch_config;

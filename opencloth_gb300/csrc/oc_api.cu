@@ -228,6 +228,29 @@ bool strip_wanted(const oc_launch_config& cfg, const InstParams& ip) {
     return cols >= 20 && 2 * cols >= 32 * strips;  // at least half the lanes own a vertex
 }
 
+// Whether a handle's grid cloths take the strip sweep where the environment leaves it open: every
+// cloth does, with at least three quarters of its lanes on a vertex of their own (a second
+// assembly kernel for the others runs behind it with a tail of its own: 24 cloths of 100 to 250 a
+// side 83 us against 63 for k_assemble_grid alone; 512 of 8 to 128, 195 against 187), and there are
+// vertices enough for its warps, of which an SM holds 16.  Measured, us of k_assemble_grid and of
+// the sweep (with k_assemble_finish where the cloths are resident):
+// 257 x 257 12.4 / 14.4, 385 x 385 16.7 / 17.6, 420 x 420 22.1 / 17.5, 513 x 513 25.1 / 20.5,
+// 700 x 700 41.4 / 30.1, 1025 x 1025 73.8 / 56.7, 2000 x 2000 265 / 204; 12 of 120 x 120 20.3 /
+// 20.3, 24 of them 30.9 / 26.5, 64 of 100 x 100 60 / 46, 256 of 55 x 55 73 / 54.
+constexpr int64_t kStripMinVertices = 175000;
+bool strip_default(const std::vector<InstParams>& inst) {
+    oc_launch_config on{};
+    on.strip = 1;
+    int64_t n = 0;
+    for (const InstParams& ip : inst) {
+        if (ip.coupled) continue;
+        const int32_t strips = (ip.grid_cols + kStripOwned - 1) / kStripOwned;
+        if (!strip_wanted(on, ip) || 4 * ip.grid_cols < 3 * 32 * strips) return false;
+        n += ip.nv;
+    }
+    return n >= kStripMinVertices;
+}
+
 int strip_blocks(int32_t n_work) { return (n_work + kStripThreads / 32 - 1) / (kStripThreads / 32); }
 
 template <class T>
@@ -1673,11 +1696,8 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
         c.persist = (pe && std::atoi(pe) == 0) ? 0 : 1;
         const char* gv = std::getenv("OC_GATHER_VARIANT");
         c.gather_variant = gv ? std::atoi(gv) : 6;
-        // The strip sweep is off by default: on GB300 it measured level with the stencil
-        // gather on the 1M-vertex cloth (its delta0 reduction costs what its single spring
-        // evaluations save) and slower on the 4096-cloth batch; the autotuner tries it.
         const char* se = std::getenv("OC_STRIP");
-        c.strip = (se && std::atoi(se) != 0) ? 1 : 0;
+        c.strip = se ? (std::atoi(se) != 0 ? 1 : 0) : (strip_default(P.inst) ? 1 : 0);
         const char* sr = std::getenv("OC_STRIP_ROWS");
         c.strip_rows = sr ? std::max(0, std::atoi(sr)) : 0;
         const char* sv = std::getenv("OC_STRIP_VARIANT");
