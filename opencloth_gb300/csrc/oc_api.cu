@@ -416,7 +416,7 @@ oc_status launch_resident_all(oc_solver* s, const StepArgs& a, KernelTimer* t) {
         for (size_t i = 0; i < s->aux.size(); ++i) OC_TRY(cudaStreamWaitEvent(s->aux[i], s->fork_ev, 0));
         for (size_t i = 0; i < s->buckets.size(); ++i) {
             const auto& b = s->buckets[i];
-            ResidentLaunch L{b.d_ids, b.cluster, b.vcta, (s->resident_fused && !a.cg_only) ? 1 : 0};
+            ResidentLaunch L{b.d_ids, b.cluster, b.vcta, (s->resident_fused && !a.cg_only) ? 1 : 0, s->d_perr};
             OC_TRY(launch_resident(a, L, b.threads, b.n, s->aux[i % s->aux.size()]));
             s->host_launches += 1;
         }
@@ -428,7 +428,7 @@ oc_status launch_resident_all(oc_solver* s, const StepArgs& a, KernelTimer* t) {
     }
     for (const auto& b : s->buckets) {
         if (t) OC_TRY(cudaEventRecord(t->ev[0], s->stream));
-        ResidentLaunch L{b.d_ids, b.cluster, b.vcta, (s->resident_fused && !a.cg_only) ? 1 : 0};
+        ResidentLaunch L{b.d_ids, b.cluster, b.vcta, (s->resident_fused && !a.cg_only) ? 1 : 0, s->d_perr};
         OC_TRY(launch_resident(a, L, b.threads, b.n, s->stream));
         s->host_launches += 1;
         if (t) {
@@ -994,7 +994,7 @@ oc_status ensure_aux(oc_solver* s, size_t want) {
     return OC_OK;
 }
 
-// The word in which k_cg_persist and k_sim report a wait that gave up (once per handle).
+// The word in which k_cg_persist, k_cpl_persist, k_resident and k_sim report a wait that gave up (once per handle).
 oc_status alloc_error_word(oc_solver* s) {
     if (s->d_perr) return OC_OK;
     OC_TRY(dalloc(s, &s->d_perr, 1));
@@ -1335,6 +1335,7 @@ oc_status plan_execution(oc_solver* s) {
                       cudaMemcpyHostToDevice));
     if (!s->buckets.empty()) {
         OC_TRY(prepare_resident());
+        if (oc_status r = alloc_error_word(s)) return r;
         if (oc_status r = ensure_aux(s, s->buckets.size())) return r;
     }
     // Persistent CG for the streamed REFERENCE cloths, any number of them: no COUPLED

@@ -348,6 +348,7 @@ struct ResidentLaunch {
     int32_t cluster;
     int32_t vcta;
     int32_t fused;  // 1: the kernel assembles its cloth's system itself (no k_assemble pass)
+    int* err;       // bit 0: a wait gave up
 };
 constexpr int kResidentMaxVcta = 2048;
 constexpr int kResidentVpt = 4;  // vertices per thread of the resident kernel: vcta <= 4 x threads
