@@ -95,6 +95,8 @@ struct oc_solver {
     std::vector<int2> grid_shape;
     BlockInfo* d_cpl_blocks = nullptr;
     int32_t n_cpl_blocks = 0;
+    std::vector<std::array<uint16_t, 6>> kind_slots;  // see PackedHost
+    KernelKind grid_kind = K_ASSEMBLE_GRID;  // the kernel of d_grid_blocks: K_ASSEMBLE_KINDS when all its cloths allow it
     BlockInfo* d_upd_blocks = nullptr;
     int32_t n_upd_blocks = 0;
     bool any_coupled = false;
@@ -218,6 +220,8 @@ oc_status check_device_error(oc_solver* s) {
     return OC_OK;
 }
 
+constexpr int kResidentDefaultVcta = 1024;  // vertices of a resident CTA
+
 // Whether a grid cloth that may take the strip sweep should: its warps own 28 columns
 // each, so narrow cloths leave lanes idle.  With cfg.strip = 0 every grid cloth stays on
 // k_assemble_grid (both give the same bits).
@@ -333,7 +337,7 @@ void account_step_bytes(const oc_solver* s, KernelTimer* t) {
             // planes by anchor.
             t->bytes[K_ASSEMBLE_STRIP] += 116.0 * nv + (s->inst_host[k].st_rest ? 24.0 * nv : 0.0);
         } else if (!fused && s->inst_host[k].grid_cols > 0)  // no incidence records, no row pointer
-            t->bytes[K_ASSEMBLE_GRID] +=              // unless rest lengths are per incidence
+            t->bytes[s->executor == OC_EXEC_PLAIN ? K_ASSEMBLE_GRID : s->grid_kind] +=              // unless rest lengths are per incidence
                 116.0 * nv + (s->inst_host[k].st_rest ? 4.0 * nv + 8.0 * ns : 0.0);
         else if (!fused)
             t->bytes[K_ASSEMBLE] += 120.0 * nv + 32.0 * ns;
@@ -497,7 +501,7 @@ oc_status step_host_driven(oc_solver* s, float dt, bool per_cloth, KernelTimer* 
             s->host_launches += 1;
         }
         if (s->n_grid_blocks > 0) {
-            if ((st = launch_timed(s, K_ASSEMBLE_GRID, ga, s->n_grid_blocks, t)) != OC_OK) return st;
+            if ((st = launch_timed(s, s->grid_kind, ga, s->n_grid_blocks, t)) != OC_OK) return st;
             s->host_launches += 1;
         }
         if (s->args.n_strip_work > 0) {
@@ -631,7 +635,7 @@ oc_status build_graph(oc_solver* s, float dt) {
     }
     if (s->n_grid_blocks > 0) {  // serialised after k_assemble: both end in the same counters
         cudaGraphNode_t prev = n_asm;
-        kp = kparams(K_ASSEMBLE_GRID, T_GRID);
+        kp = kparams(s->grid_kind, T_GRID);
         OC_TRY(cudaGraphAddKernelNode(&n_asm, g, &prev, 1, &kp));
     }
     if (s->args.n_strip_work > 0) {  // the strip sweep, then its cloths' delta0 totals
@@ -740,7 +744,6 @@ oc_status build_graph(oc_solver* s, float dt) {
 // Launch shape of a resident cloth: up to 1024 vertices one CTA (vertex capacity the
 // next power of two, at least 128); beyond, clusters of CTAs of 1024 vertices each, up
 // to max_vertices and kResidentMaxCluster CTAs.
-constexpr int kResidentDefaultVcta = 1024;
 
 // The per-CTA vertex capacity and thread count come from the launch configuration
 // (resident_vcta, resident_threads).
@@ -1268,6 +1271,7 @@ oc_status plan_execution(oc_solver* s) {
     s->buckets.clear();
     std::vector<BlockInfo> streamed, asm_ref, cpl, upd, grid;
     std::map<std::tuple<int, int, int>, std::vector<int32_t>> groups;
+    s->grid_kind = K_ASSEMBLE_KINDS;
     for (int32_t k = 0; k < s->n_inst; ++k) {
         InstParams& ip = s->inst_host[(size_t)k];
         const bool cpl_k = ip.coupled != 0;
@@ -1294,6 +1298,7 @@ oc_status plan_execution(oc_solver* s) {
             if (!ip.strip) {  // a cloth on the strip sweep is in no block table of the assembly
                 auto& tab = ip.grid_cols > 0 ? grid : asm_ref;
                 tab.insert(tab.end(), kb, kb + ip.nblk);
+                if (ip.grid_cols > 0 && (!ip.kinds || ip.grid_cols > kKindsMaxCols)) s->grid_kind = K_ASSEMBLE_GRID;
             }
         }
         if (want) {
@@ -1420,6 +1425,9 @@ oc_status refit_stencils(oc_solver* s) {
                     slots_changed = true;
                 }
             }
+        const int32_t was = ip.kinds;
+        set_kinds(&ip, s->kind_slots[(size_t)k], s->h_st_param.data() + ip.st_par);
+        moved = moved || ip.kinds != was;
         const int32_t cols = fits ? shape.x : 0;
         if (cols != ip.grid_cols) {
             ip.grid_cols = cols;
@@ -1507,6 +1515,10 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
             want = (want + 31) / 32 * 32;
             vpb = (int)std::min<int64_t>(std::max<int64_t>(want, 256), vpb);
         }
+        // Many small cloths: each ends in a part of a block, so no size fills whole waves, and
+        // shorter blocks leave a shorter tail (512 cloths of 8 to 128 a side: k_assemble_kinds 190
+        // us with 2,048 vertices, 179 with 1,024, 181 with 512).
+        if (total <= (int64_t)n_instances * kResidentMaxCluster * kResidentDefaultVcta) vpb = std::min(vpb, 1024);
     }
     const int vpt = (vpb + kernel_block_threads() - 1) / kernel_block_threads();
     PackedHost P;
@@ -1716,6 +1728,7 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
         if (s->executor != OC_EXEC_PLAIN) OC_CREATE_TRY(prepare_sim(s->device, &s->sim_smem_max));
         s->adj_allowed = !(pe && std::atoi(pe) == 0) && s->coop;
         s->h_blocks = P.blocks;
+        s->kind_slots = P.kind_slots;
         if (oc_status r = plan_execution(s)) return bail(r);
     }
     OC_CREATE_TRY(dalloc(s, &a.unconverged, 1));
@@ -2115,7 +2128,7 @@ oc_status oc_profile_steps(oc_solver* s, float dt, int32_t n_steps, int32_t max_
     cudaEventDestroy(t.ev[0]);
     cudaEventDestroy(t.ev[1]);
     if (st != OC_OK) return st;
-    const KernelKind kinds[] = {K_ASSEMBLE, K_ASSEMBLE_GRID, K_ASSEMBLE_STRIP, K_ASSEMBLE_FINISH, K_CG_DIR,
+    const KernelKind kinds[] = {K_ASSEMBLE, K_ASSEMBLE_GRID, K_ASSEMBLE_KINDS, K_ASSEMBLE_STRIP, K_ASSEMBLE_FINISH, K_CG_DIR,
                                 K_CG_UPDATE, K_INTEGRATE, K_CG_PERSIST, K_RESIDENT, K_PROVOT,
                                 K_CPL_ASSEMBLE, K_CPL_DIR, K_CPL_UPDATE, K_CPL_PERSIST};
     int32_t n = 0;
@@ -2123,7 +2136,9 @@ oc_status oc_profile_steps(oc_solver* s, float dt, int32_t n_steps, int32_t max_
         if (n >= max_kernels) break;
         if (k == K_PROVOT && !s->any_provot) continue;
         if ((k == K_CPL_ASSEMBLE || k == K_CPL_DIR || k == K_CPL_UPDATE) && !s->any_coupled) continue;
-        if (k == K_ASSEMBLE_GRID && s->n_grid_blocks == 0) continue;
+        if ((k == K_ASSEMBLE_GRID || k == K_ASSEMBLE_KINDS) &&
+            (s->n_grid_blocks == 0 || k != (s->executor == OC_EXEC_PLAIN ? K_ASSEMBLE_GRID : s->grid_kind)))
+            continue;
         if (k == K_CG_PERSIST && !s->persist) continue;
         if (k == K_CPL_PERSIST && !s->cpl_persist) continue;
         if ((k == K_CPL_DIR || k == K_CPL_UPDATE || k == K_INTEGRATE) && s->cpl_persist) continue;

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -43,6 +44,12 @@ struct InstParams {
     int32_t strip_w0;
     int32_t strip_nw;
     int64_t strip_rest;
+    // kinds 1: strip_ok, and the springs of a kind share their Ks and Kd in the whole cloth: those of
+    // slot kind_slots (4 bits a kind as in strip_slot).  Their rest lengths: planes as strip_rest's at
+    // kind_rest, or -1 when the slot holds them.
+    int32_t kinds;
+    uint32_t kind_slots;
+    int64_t kind_rest;
     float provot_ratio;     // IMP:808
     float ellipsoid[16];    // object -> world, column-major (IMP:583-585)
     float ellipsoid_inv[16];
@@ -77,6 +84,7 @@ struct StripWork {
     int32_t c0;
     int32_t r0, r1;
 };
+constexpr int kKindsMaxCols = 128;  // columns of a cloth that k_assemble_kinds takes
 constexpr int kStripOwned = 28;    // owned columns per warp
 constexpr int kStripThreads = 256;  // 8 warps per CTA
 
@@ -242,7 +250,7 @@ __host__ __device__ inline int stencil_class_1d(int32_t i, int32_t n) {
 enum KernelKind { K_ASSEMBLE = 0, K_CG_DIR = 1, K_CG_UPDATE = 2, K_INTEGRATE = 3, K_FORCES = 4, K_RESIDENT = 5,
                   K_PROVOT = 6, K_ELLIPSOID = 7, K_CPL_ASSEMBLE = 8, K_CPL_DIR = 9, K_CPL_UPDATE = 10,
                   K_ASSEMBLE_GRID = 11, K_CG_PERSIST = 12, K_ASSEMBLE_STRIP = 13, K_ASSEMBLE_FINISH = 14,
-                  K_CPL_PERSIST = 15, K_COUNT = 16 };
+                  K_CPL_PERSIST = 15, K_ASSEMBLE_KINDS = 16, K_COUNT = 17 };
 
 cudaError_t launch_test_cr_arith(unsigned long long* counts, uint64_t n_pairs, uint64_t seed, cudaStream_t stream);
 // The persistent CG (k_cg_persist, oc_persist.cu): the whole CG loop and the update of the
@@ -401,6 +409,7 @@ struct PackedHost {
     std::vector<int32_t> st_data;                     // stencils of the grid cloths (see StepArgs)
     std::vector<float4> st_param;
     bool any_st_rest = false;                         // a grid cloth reads rest lengths per incidence
+    std::vector<std::array<uint16_t, 6>> kind_slots;  // a cloth's slots by spring kind, as bits (strip_ok)
     std::vector<uint32_t> strip_slot;                 // strip sweep tables (see InstParams)
     std::vector<float> strip_rest;
     bool any_provot = false;                          // some cloth has OC_PASS_PROVOT
@@ -413,5 +422,7 @@ oc_status pack_instances(const oc_cloth_desc* descs, int32_t n, int32_t vertices
 // parameter slot per spring kind and anchor class (InstParams::strip_ok) and builds their
 // slot words and, where the rest lengths vary, their rest planes.
 void build_strip_tables(PackedHost* P);
+// InstParams::kinds and kind_slots from the slots of each kind and the cloth's parameter slots.
+void set_kinds(InstParams* ip, const std::array<uint16_t, 6>& masks, const float4* par);
 
 }  // namespace oc

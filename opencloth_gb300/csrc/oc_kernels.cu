@@ -6,6 +6,8 @@
 //                the assembly of A_i, b_i, P_i (IMP:781-786) and the CG set-up
 //                r = b - A x, d = P^-1 r, delta0 = r.(P r) (IMP:310-318).
 //   k_assemble_grid  the same for grid cloths, with the neighbours from a stencil
+//   k_assemble_kinds  the same for narrow ones in the reference's spring order, from a window of
+//                the states in shared memory
 //   k_cg_dir     [d = r + beta d]; alpha = delta_new / d.(A d)    (IMP:320-321, 327)
 //   k_cg_update  x += alpha d; r -= alpha A d; delta_new = r.r     (IMP:322-326)
 //   (k_cg_persist, oc_persist.cu: the two passes above and the update in one launch)
@@ -194,6 +196,81 @@ __global__ void __launch_bounds__(kThreads, MINB) k_assemble_grid(const StepArgs
         prefetch_own(a, g, ends);  // into L1 while the forces are gathered
         const float3 F = stencil_gather<B>(a, ip, g, Xg, Vg);
         acc_add(part, assemble_vertex(a, g, Xg, Vg, F, load_own_at(a, g, ends)));
+    }
+    finish<K_ASSEMBLE>(a, bi.gblk, bi.inst, true, part);
+}
+
+// Assembly of grid cloths in the reference's spring order whose springs of a kind share their
+// parameters (InstParams::kinds), of up to kKindsMaxCols columns: as k_assemble_grid, with the
+// states of a chunk of vertices and two rows to both sides copied to shared memory first (a
+// contiguous range), the twelve incidences spelled out (kind_gather) and the lines of the rest
+// lengths, x and spring i's records requested meanwhile.  Bound by instructions, 1,545 a vertex
+// against 1,772, 750 of them FP32, at 0.65 a cycle and scheduler.  Measured on 512 cloths of 8 to
+// 128 a side (3.06 M vertices): 220 -> 179 us.  The twelve incidences without the window 212;
+// without the requests 212, without spring i's ends from the window 189; 2,048 vertices a block
+// instead of 1,024 190; five CTAs an SM 219, three 214.  A window of 2,048 vertices for up to 384
+// columns leaves three CTAs an SM (220), and it copies more rows than it assembles: 385 x 385 17
+// -> 21 us; so wider cloths stay on k_assemble_grid.
+constexpr int kKindsChunk = 512;
+
+constexpr int kKindsCap = kKindsChunk + 4 * kKindsMaxCols;  // vertices of a window
+
+__global__ void __launch_bounds__(kThreads, 4) k_assemble_kinds(const StepArgs a) {
+    __shared__ __align__(16) float4 win[2 * kKindsCap];  // X, then V
+    __shared__ float4 par[6];
+    const int blk = blockIdx.x + a.blk_base;
+    const BlockInfo bi = a.blocks[blk];
+    const InstParams& ip = a.inst[bi.inst];
+    const int halo = 2 * ip.grid_cols;
+    const int64_t v0 = ip.v_off, v1 = ip.v_off + ip.nv;
+    if (threadIdx.x < 6) par[threadIdx.x] = __ldg(a.st_param + ip.st_par + (ip.kind_slots >> (4 * threadIdx.x) & 15u));
+    Acc part = acc_zero();
+    for (int64_t base = bi.v_begin; base < bi.v_end; base += kKindsChunk) {
+        const int64_t w0 = base - halo;  // win[0]'s vertex
+        const int64_t lo = max(w0, v0), hi = min(min(base + kKindsChunk, bi.v_end) + halo, v1);
+        __syncthreads();  // the last chunk has been read
+        for (int64_t v = lo + threadIdx.x; v < hi; v += kThreads) {
+            copy_async16(win + (v - w0), a.X + v);
+            copy_async16(win + kKindsCap + (v - w0), a.V + v);
+        }
+        int2 ends[kKindsChunk / kThreads];
+#pragma unroll
+        for (int u = 0; u < kKindsChunk / kThreads; ++u) {
+            const int64_t g = base + u * kThreads + threadIdx.x;
+            ends[u] = g < bi.v_end ? __ldg(a.own_ends + g) : make_int2(-1, -1);
+            if (g < bi.v_end) {
+                prefetch_l1(a.own_par + g);
+                if (ip.kind_rest >= 0) {
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) prefetch_l1(a.strip_rest + ip.kind_rest + (int64_t)k * ip.nv + (g - v0));
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) prefetch_l1(a.x[k] + g);
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+#pragma unroll 1
+        for (int u = 0; u < kKindsChunk / kThreads; ++u) {
+            const int64_t g = base + u * kThreads + threadIdx.x;
+            if (g >= bi.v_end) break;
+            const float4* const X = win + halo + u * kThreads + threadIdx.x;
+            const float3 F = kind_gather(a, ip, g, X, X + kKindsCap, par);
+            // Spring i's ends lie in the window for all but tall cloths' last rows.
+            const int2 e = u == 0 ? ends[0] : ends[1];
+            OwnSpring os;
+            if (e.x >= lo && e.x < hi && e.y >= lo && e.y < hi) {
+                os.ends = e;
+                os.par = __ldg(a.own_par + g);
+                os.E1 = win[e.x - w0];
+                os.E2 = win[e.y - w0];
+                os.W1 = win[kKindsCap + (e.x - w0)];
+                os.W2 = win[kKindsCap + (e.y - w0)];
+            } else {
+                os = load_own_at(a, g, e);
+            }
+            acc_add(part, assemble_vertex(a, g, *X, X[kKindsCap], F, os));
+        }
     }
     finish<K_ASSEMBLE>(a, bi.gblk, bi.inst, true, part);
 }
@@ -990,6 +1067,7 @@ const char* kernel_name(KernelKind k) {
         case K_ELLIPSOID: return "k_ellipsoid";
         case K_CPL_ASSEMBLE: return "k_cpl_assemble";
         case K_ASSEMBLE_GRID: return "k_assemble_grid";
+        case K_ASSEMBLE_KINDS: return "k_assemble_kinds";
         case K_CG_PERSIST: return "k_cg_persist";
         case K_ASSEMBLE_STRIP: return "k_assemble_strip";
         case K_ASSEMBLE_FINISH: return "k_assemble_finish";
@@ -1013,6 +1091,7 @@ const void* kernel_fn(KernelKind k, const StepArgs& a) {
         case K_CPL_DIR:
         case K_CPL_UPDATE: return coupled_fn(k);
         case K_ASSEMBLE_GRID: return (const void*)grid_asm_fn();
+        case K_ASSEMBLE_KINDS: return (const void*)k_assemble_kinds;
         case K_ASSEMBLE_STRIP: return strip_fn(a.strip_variant);
         case K_ASSEMBLE_FINISH: return (const void*)k_assemble_finish;
         default: return nullptr;
@@ -1078,6 +1157,7 @@ cudaError_t launch_kernel(KernelKind k, const StepArgs& a, int nblocks, cudaStre
         case K_CPL_DIR:
         case K_CPL_UPDATE: return launch_coupled(k, a, nblocks, stream);
         case K_ASSEMBLE_GRID: grid_asm_fn()<<<nblocks, kThreads, 0, stream>>>(a); break;
+        case K_ASSEMBLE_KINDS: k_assemble_kinds<<<nblocks, kThreads, 0, stream>>>(a); break;
         case K_ASSEMBLE_STRIP:
             reinterpret_cast<void (*)(StepArgs)>(const_cast<void*>(strip_fn(a.strip_variant)))
                 <<<nblocks, kStripThreads, 0, stream>>>(a);

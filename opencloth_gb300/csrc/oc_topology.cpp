@@ -383,13 +383,30 @@ int strip_entries(int32_t r, int32_t c, int32_t rows, int32_t cols, StripEntry* 
 
 }  // namespace
 
+void set_kinds(InstParams* ip, const std::array<uint16_t, 6>& masks, const float4* par) {
+    ip->kinds = ip->strip_ok;
+    ip->kind_slots = 0;
+    for (int kind = 0; kind < 6; ++kind) {
+        int first = -1;
+        for (int q = 0; q < kStencilSlots; ++q) {
+            if (!(masks[kind] >> q & 1)) continue;
+            if (first < 0) first = q;
+            if (std::memcmp(&par[q].y, &par[first].y, 2 * sizeof(float)) != 0) ip->kinds = 0;
+        }
+        ip->kind_slots |= (uint32_t)std::max(first, 0) << (4 * kind);
+    }
+}
+
 void build_strip_tables(PackedHost* Pp) {
     PackedHost& P = *Pp;
     P.strip_slot.clear();
     P.strip_rest.clear();
+    P.kind_slots.assign((size_t)P.n_inst, std::array<uint16_t, 6>{});
     for (int32_t k = 0; k < P.n_inst; ++k) {
         InstParams& ip = P.inst[k];
-        ip.strip = ip.strip_ok = 0;
+        ip.strip = ip.strip_ok = ip.kinds = 0;
+        ip.kind_slots = 0;
+        ip.kind_rest = -1;
         ip.strip_slot = -1;
         ip.strip_rest = -1;
         if (ip.grid_cols <= 0 || ip.coupled) continue;
@@ -444,11 +461,30 @@ void build_strip_tables(PackedHost* Pp) {
             for (int kind = 0; kind < 6; ++kind) w |= (uint32_t)(std::max(slot[kind][cl], 0) & 15) << (4 * kind);
             P.strip_slot.push_back(w);
         }
+        std::array<uint16_t, 6>& masks = P.kind_slots[(size_t)k];
+        bool several = false;  // a kind with several slots: equal but for the rest lengths, if ip.kinds
+        for (int kind = 0; kind < 6; ++kind) {
+            for (int x : slot[kind])
+                if (x >= 0) masks[kind] |= (uint16_t)(1u << x);
+            several = several || (masks[kind] & (masks[kind] - 1));
+        }
+        set_kinds(&ip, masks, P.st_param.data() + ip.st_par);
         if (ip.st_rest) {
             ip.strip_rest = (int64_t)P.strip_rest.size();
             const size_t base = P.strip_rest.size();
             P.strip_rest.resize(base + rest_bits.size());
             std::memcpy(P.strip_rest.data() + base, rest_bits.data(), rest_bits.size() * sizeof(float));
+            ip.kind_rest = ip.strip_rest;
+        } else if (several && ip.kinds && cols <= kKindsMaxCols) {
+            // (The sweep takes these rest lengths from the slots.)
+            ip.kind_rest = (int64_t)P.strip_rest.size();
+            P.strip_rest.resize(P.strip_rest.size() + 6 * (size_t)nvk, 0.0f);
+            const float4* par = P.st_param.data() + ip.st_par;
+            for (int kind = 0; kind < 6; ++kind)
+                for (int32_t l = 0; l < nvk; ++l) {
+                    const int sl = slot[kind][stencil_class_1d(l / cols, rows) * 6 + stencil_class_1d(l % cols, cols)];
+                    if (sl >= 0) P.strip_rest[(size_t)ip.kind_rest + (size_t)kind * nvk + l] = par[sl].x;
+                }
         }
     }
 }
