@@ -25,6 +25,7 @@ namespace oc {
 namespace {
 
 constexpr int kAdjThreads = 256;
+constexpr int kAdjChunk = 128;  // vertices, and threads, of a CTA of k_adj_vertex and k_adj_springs
 
 __device__ __forceinline__ float dot3f(float ax, float ay, float az, float bx, float by, float bz) {
     return ax * bx + ay * by + az * bz;
@@ -162,106 +163,81 @@ __device__ __forceinline__ void spring_jac_adj(const Geo& Gm, const float4 v1, c
 // Per vertex i: lambda -> g_F = h lambda, the terms of A_i and b_i: g_J = h^2 lambda (V +
 // dV)^T, g_Jv = h lambda dV^T, g_V += h^2 J lambda + damping g_F, g_ext += g_F; spring
 // i's Jacobian adjoint goes to the vertex's own-spring slots and to Ks_i, Kd_i.
-// Variants (AdjArgs::vertex_variant): VPT vertices per thread with every load of a stage
-// in flight together (the vertex's own entries, then spring i's ends and old gradient
-// entries, then the arithmetic), and CTAs per SM the register budget is set for.  The
-// default, one vertex and three CTAs, measured 0.08 ms faster per reverse step on 12 M
-// vertices than two vertices and two CTAs.
-template <int VPT, int MINB>
-__global__ void __launch_bounds__(kAdjThreads, MINB) k_adj_vertex(const StepArgs a, const AdjArgs j) {
-    const int blk = blockIdx.x + a.blk_base;
-    const BlockInfo bi = a.blocks[blk];
+// One vertex a thread with every load of a stage in flight together (the vertex's own entries, then
+// spring i's ends and old gradient entries, then the arithmetic).  A CTA takes kAdjChunk of a block's
+// vertices: measured, 24 cloths (231k vertices), 15.9 -> 10.6 us; a CTA of 256 threads for a whole
+// block of 384 vertices leaves half its threads idle in a second pass.  Eight CTAs an SM; six 10.9,
+// five 13.6.
+__global__ void __launch_bounds__(kAdjChunk, 8) k_adj_vertex(const StepArgs a, const AdjArgs j) {
+    const BlockInfo bi = a.blocks[blockIdx.x + a.blk_base];
     const InstParams& ip = a.inst[bi.inst];
     const float h = a.dt;
-    const int64_t T = blockDim.x;
-    for (int64_t base = bi.v_begin + threadIdx.x; base < bi.v_end; base += VPT * T) {
-        float4 Vg[VPT];
-        float lam[VPT][3], dv[VPT][3], gv[VPT][3];
-        OwnSpring os[VPT];
-        int32_t sid[VPT];
-        float gk_old[VPT], gd_old[VPT];
-        bool ok[VPT];
+    const int64_t g = bi.v_begin + (int64_t)blockIdx.y * kAdjChunk + threadIdx.x;
+    if (g >= bi.v_end) return;
+    const float4 Vg = a.V[g];
+    float lam[3], dv[3], gv[3];
 #pragma unroll
-        for (int u = 0; u < VPT; ++u) {
-            const int64_t g = base + u * T;
-            ok[u] = g < bi.v_end;
-            const int64_t q = ok[u] ? g : base;
-            Vg[u] = a.V[q];
+    for (int k = 0; k < 3; ++k) {
+        lam[k] = a.x[k][g];
+        dv[k] = j.dV[k][g];
+        gv[k] = j.gV[k][g];
+    }
+    OwnSpring os;
+    os.ends = __ldg(a.own_ends + g);
+    const int32_t sid = __ldg(j.own_sid + g);
+    const bool pinned = Vg.w != 0.0f, own = os.ends.x >= 0 && !pinned;
+    float gk_old = 0.0f, gd_old = 0.0f;
+    if (own) {
+        os.par = __ldg(a.own_par + g);
+        os.E1 = __ldg(a.X + os.ends.x);
+        os.E2 = __ldg(a.X + os.ends.y);
+        os.W1 = __ldg(a.V + os.ends.x);
+        os.W2 = __ldg(a.V + os.ends.y);
+        gk_old = j.gKs[sid];
+        gd_old = j.gKd[sid];
+    }
+    const float v[3] = {Vg.x, Vg.y, Vg.z};
+    float gF[3];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                lam[u][k] = a.x[k][q];
-                dv[u][k] = j.dV[k][q];
-                gv[u][k] = j.gV[k][q];
+    for (int k = 0; k < 3; ++k) gF[k] = pinned ? 0.0f : h * lam[k];
+    float gdP[3] = {0.f, 0.f, 0.f}, gdVs[3] = {0.f, 0.f, 0.f};
+    if (own) {
+        const Geo geo = spring_geo(a, os.ends.x, os.ends.y, os.E1, os.E2, os.par.x, a.gm_own, g);
+        SpringEval e;
+        spring_eval(geo, os.W1, os.W2, e);
+        float J[6], Jv[6];
+        jac_element(e, os.par.y, os.par.z, 0, 0, J[0], Jv[0]);
+        jac_element(e, os.par.y, os.par.z, 0, 1, J[1], Jv[1]);
+        jac_element(e, os.par.y, os.par.z, 0, 2, J[2], Jv[2]);
+        jac_element(e, os.par.y, os.par.z, 1, 1, J[3], Jv[3]);
+        jac_element(e, os.par.y, os.par.z, 1, 2, J[4], Jv[4]);
+        jac_element(e, os.par.y, os.par.z, 2, 2, J[5], Jv[5]);
+        float jl0, jl1, jl2;
+        matvec(J, lam[0], lam[1], lam[2], jl0, jl1, jl2);
+        gv[0] += h * h * jl0;
+        gv[1] += h * h * jl1;
+        gv[2] += h * h * jl2;
+        float G[3][3], H[3][3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                G[r][c] = h * h * lam[r] * (v[c] + dv[c]);
+                H[r][c] = h * lam[r] * dv[c];
             }
-            os[u].ends = __ldg(a.own_ends + q);
-            sid[u] = __ldg(j.own_sid + q);
-            if (!ok[u]) os[u].ends.x = -1;
-        }
+        float gks, gkd;
+        spring_jac_adj(geo, os.W1, os.W2, os.par.y, os.par.z, G, H, gdP, gdVs, gks, gkd);
+        j.gKs[sid] = gk_old + gks;
+        j.gKd[sid] = gd_old + gkd;
+    }
 #pragma unroll
-        for (int u = 0; u < VPT; ++u) {
-            os[u].par = make_float4(0.f, 0.f, 0.f, 0.f);
-            os[u].E1 = os[u].E2 = os[u].W1 = os[u].W2 = make_float4(0.f, 0.f, 0.f, 0.f);
-            gk_old[u] = gd_old[u] = 0.0f;
-            if (os[u].ends.x >= 0 && Vg[u].w == 0.0f) {
-                const int64_t g = base + u * T;
-                os[u].par = __ldg(a.own_par + g);
-                os[u].E1 = __ldg(a.X + os[u].ends.x);
-                os[u].E2 = __ldg(a.X + os[u].ends.y);
-                os[u].W1 = __ldg(a.V + os[u].ends.x);
-                os[u].W2 = __ldg(a.V + os[u].ends.y);
-                gk_old[u] = j.gKs[sid[u]];
-                gd_old[u] = j.gKd[sid[u]];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < VPT; ++u) {
-            if (!ok[u]) continue;
-            const int64_t g = base + u * T;
-            const bool pinned = Vg[u].w != 0.0f;
-            const float v[3] = {Vg[u].x, Vg[u].y, Vg[u].z};
-            float gF[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) gF[k] = pinned ? 0.0f : h * lam[u][k];
-            float gdP[3] = {0.f, 0.f, 0.f}, gdVs[3] = {0.f, 0.f, 0.f};
-            if (os[u].ends.x >= 0 && !pinned) {
-                const Geo geo = spring_geo(a, os[u].ends.x, os[u].ends.y, os[u].E1, os[u].E2, os[u].par.x, a.gm_own, g);
-                SpringEval e;
-                spring_eval(geo, os[u].W1, os[u].W2, e);
-                float J[6], Jv[6];
-                jac_element(e, os[u].par.y, os[u].par.z, 0, 0, J[0], Jv[0]);
-                jac_element(e, os[u].par.y, os[u].par.z, 0, 1, J[1], Jv[1]);
-                jac_element(e, os[u].par.y, os[u].par.z, 0, 2, J[2], Jv[2]);
-                jac_element(e, os[u].par.y, os[u].par.z, 1, 1, J[3], Jv[3]);
-                jac_element(e, os[u].par.y, os[u].par.z, 1, 2, J[4], Jv[4]);
-                jac_element(e, os[u].par.y, os[u].par.z, 2, 2, J[5], Jv[5]);
-                float jl0, jl1, jl2;
-                matvec(J, lam[u][0], lam[u][1], lam[u][2], jl0, jl1, jl2);
-                gv[u][0] += h * h * jl0;
-                gv[u][1] += h * h * jl1;
-                gv[u][2] += h * h * jl2;
-                float G[3][3], H[3][3];
-#pragma unroll
-                for (int r = 0; r < 3; ++r)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        G[r][c] = h * h * lam[u][r] * (v[c] + dv[u][c]);
-                        H[r][c] = h * lam[u][r] * dv[u][c];
-                    }
-                float gks, gkd;
-                spring_jac_adj(geo, os[u].W1, os[u].W2, os[u].par.y, os[u].par.z, G, H, gdP, gdVs, gks, gkd);
-                j.gKs[sid[u]] = gk_old[u] + gks;
-                j.gKd[sid[u]] = gd_old[u] + gkd;
-            }
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                gv[u][k] += ip.damping * gF[k];
-                j.gV[k][g] = gv[u][k];
-                j.gF[k][g] = gF[k];
-                j.gOwn[k][g] = gdP[k];
-                j.gOwn[3 + k][g] = gdVs[k];
-                if (!pinned) j.gExt[k][g] += gF[k];
-            }
-        }
+    for (int k = 0; k < 3; ++k) {
+        gv[k] += ip.damping * gF[k];
+        j.gV[k][g] = gv[k];
+        j.gF[k][g] = gF[k];
+        j.gOwn[k][g] = gdP[k];
+        j.gOwn[3 + k][g] = gdVs[k];
+        if (!pinned) j.gExt[k][g] += gF[k];
     }
 }
 
@@ -281,9 +257,9 @@ struct AdjInc {
     float rest, ks, kd;
 };
 
-template <bool STENCIL, int kAdjAhead>
+template <bool STENCIL, bool STAGED, int kAdjAhead>
 __device__ __forceinline__ void adj_springs_vertex(const StepArgs& a, const AdjArgs& j, const InstParams& ip,
-                                                   int64_t g) {
+                                                   int64_t g, const int4* s_rec, const int32_t* s_sid, int32_t kA) {
     const float4* __restrict__ X = a.X;
     const float4* __restrict__ V = a.V;
     const float* __restrict__ gF0 = j.gF[0];
@@ -294,6 +270,8 @@ __device__ __forceinline__ void adj_springs_vertex(const StepArgs& a, const AdjA
     float gx[3] = {j.gX[0][g], j.gX[1][g], j.gX[2][g]};
     float gv[3] = {j.gV[0][g], j.gV[1][g], j.gV[2][g]};
     const int32_t k0 = __ldg(a.rowptr + g), k1 = __ldg(a.rowptr + g + 1);
+    const int32_t o0 = __ldg(j.own_rowptr + g), o1 = __ldg(j.own_rowptr + g + 1);
+    prefetch_l1(j.own_ent + o0);
     const int32_t* st = nullptr;
     const float4* par = nullptr;
     int32_t ebase = 0;
@@ -320,11 +298,11 @@ __device__ __forceinline__ void adj_springs_vertex(const StepArgs& a, const AdjA
                 in[u] = AdjInc{(int32_t)(g + (int64_t)di * cols + dj), (v & 64) != 0,
                                ip.st_rest ? __ldg(a.rest_inc + k) : p.x, p.y, p.z};
             } else {
-                const int4 rec = __ldg(a.inc + k);
+                const int4 rec = STAGED ? s_rec[k - kA] : __ldg(a.inc + k);
                 in[u] = AdjInc{rec.x & 0x7fffffff, rec.x < 0, __int_as_float(rec.y), __int_as_float(rec.z),
                                __int_as_float(rec.w)};
             }
-            sid[u] = (k < k1 && !in[u].p2) ? __ldg(j.inc_sid + k) : 0;
+            sid[u] = (k < k1 && !in[u].p2) ? (STAGED ? s_sid[k - kA] : __ldg(j.inc_sid + k)) : 0;
         }
         float4 Xo[kAdjAhead], Vo[kAdjAhead];
         float gFo[kAdjAhead][3], gk_old[kAdjAhead], gd_old[kAdjAhead];
@@ -369,7 +347,6 @@ __device__ __forceinline__ void adj_springs_vertex(const StepArgs& a, const AdjA
             }
         }
     }
-    const int32_t o0 = __ldg(j.own_rowptr + g), o1 = __ldg(j.own_rowptr + g + 1);
     for (int32_t k = o0; k < o1; ++k) {
         const int32_t e = __ldg(j.own_ent + k);
         const int32_t i = e & 0x7fffffff;
@@ -387,20 +364,50 @@ __device__ __forceinline__ void adj_springs_vertex(const StepArgs& a, const AdjA
     }
 }
 
-// Variants (AdjArgs::springs_variant): incidences in flight per batch and CTAs per SM
-// the register budget is set for.  The default, two incidences and three CTAs (80
-// registers), measured 0.3 ms faster per reverse step on 12M vertices than four and two.
-template <int AHEAD, int MINB>
-__global__ void __launch_bounds__(kAdjThreads, MINB) k_adj_springs(const StepArgs a, const AdjArgs j) {
-    const int blk = blockIdx.x + a.blk_base;
-    const BlockInfo bi = a.blocks[blk];
+// The chunk's incidence records (contiguous) and spring ids are copied to shared memory first
+// (STAGE): read from memory by their threads they are 192 bytes apart, a line each, and the
+// neighbours' loads wait for them.  T threads, a vertex each; AHEAD incidences in flight; grid.y CTAs
+// take the chunks of a block of the table in turn (the grid's x-neighbours, which run together, are
+// then a block apart: with adjacent chunks the same kernel took 67 us instead of 50).
+// Measured, 24 cloths (231k vertices, a record a spring), us: 89 with <2, 256, 3, false> over whole
+// blocks, 67 with <4, 128, 4, false> over chunks, 50 with <4, 128, 4, true>; two incidences and six
+// CTAs an SM 78, three and four 62, six and three 59; 64 threads 56; four and three 57 (the copies
+// and the gathered states share an SM's L1).  700 x 700 stencil 133 -> 101, 257 x 257 31 -> 22.
+constexpr int kSpringStage = 13;  // records of a vertex that the copies have room for, on average
+
+template <int AHEAD, int T, int MINB, bool STAGE>
+__global__ void __launch_bounds__(T, MINB) k_adj_springs(const StepArgs a, const AdjArgs j) {
+    __shared__ int4 s_rec[STAGE ? T * kSpringStage : 1];
+    __shared__ int32_t s_sid[STAGE ? T * kSpringStage : 1];
+    const BlockInfo bi = a.blocks[blockIdx.x + a.blk_base];
     const InstParams& ip = a.inst[bi.inst];
-    if (ip.grid_cols > 0) {
-        for (int64_t g = bi.v_begin + threadIdx.x; g < bi.v_end; g += blockDim.x)
-            adj_springs_vertex<true, AHEAD>(a, j, ip, g);
-    } else {
-        for (int64_t g = bi.v_begin + threadIdx.x; g < bi.v_end; g += blockDim.x)
-            adj_springs_vertex<false, AHEAD>(a, j, ip, g);
+    const bool stencil = ip.grid_cols > 0;
+    for (int64_t base = bi.v_begin + (int64_t)blockIdx.y * T; base < bi.v_end; base += (int64_t)gridDim.y * T) {
+        const int64_t g = base + threadIdx.x, end = min(base + T, bi.v_end);
+        int32_t kA = 0;
+        bool staged = false;
+        if constexpr (STAGE) {
+            kA = __ldg(a.rowptr + base);
+            const int32_t n = __ldg(a.rowptr + end) - kA;
+            staged = n <= T * kSpringStage;
+            __syncthreads();  // the last copies have been read
+            if (staged) {
+                for (int i = threadIdx.x; i < n; i += T) {
+                    if (!stencil) copy_async16(s_rec + i, a.inc + kA + i);
+                    copy_async4(s_sid + i, j.inc_sid + kA + i);
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+            }
+            __syncthreads();
+        }
+        if (g >= end) continue;
+        if (stencil) {
+            if (staged) adj_springs_vertex<true, true, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
+            else adj_springs_vertex<true, false, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
+        } else {
+            if (staged) adj_springs_vertex<false, true, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
+            else adj_springs_vertex<false, false, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
+        }
     }
 }
 
@@ -610,24 +617,20 @@ __global__ void k_set_spring_params(const StepArgs a, const AdjArgs j, const flo
 
 }  // namespace
 
-cudaError_t launch_adjoint(int which, const StepArgs& a, const AdjArgs& j, int nblocks, cudaStream_t stream) {
+cudaError_t launch_adjoint(int which, const StepArgs& a, const AdjArgs& j, int nblocks, int vpb, bool stencil,
+                           cudaStream_t stream) {
     if (nblocks <= 0) return cudaSuccess;
+    const int parts = (vpb + kAdjChunk - 1) / kAdjChunk;
     switch (which) {
         case 0: k_gm_seed_own<<<nblocks, kAdjThreads, 0, stream>>>(a, j); break;
-        case 1:
-            switch (j.vertex_variant) {
-                case 1: k_adj_vertex<2, 2><<<nblocks, kAdjThreads, 0, stream>>>(a, j); break;
-                case 2: k_adj_vertex<2, 3><<<nblocks, kAdjThreads, 0, stream>>>(a, j); break;
-                default: k_adj_vertex<1, 3><<<nblocks, kAdjThreads, 0, stream>>>(a, j); break;
-            }
-            break;
+        case 1: k_adj_vertex<<<dim3(nblocks, parts), kAdjChunk, 0, stream>>>(a, j); break;
         case 2:
-            switch (j.springs_variant) {
-                case 1: k_adj_springs<4, 2><<<nblocks, kAdjThreads, 0, stream>>>(a, j); break;
-                case 2: k_adj_springs<2, 2><<<nblocks, kAdjThreads, 0, stream>>>(a, j); break;
-                case 3: k_adj_springs<1, 4><<<nblocks, kAdjThreads, 0, stream>>>(a, j); break;
-                default: k_adj_springs<2, 3><<<nblocks, kAdjThreads, 0, stream>>>(a, j); break;
-            }
+            // Large handles of stencil cloths alone read no records to copy, and their whole blocks
+            // make waves enough: 2 M vertices 327 us against 366, 4 M 624 against 741.
+            if (stencil && (int64_t)nblocks * vpb >= 1500000)
+                k_adj_springs<2, kAdjThreads, 3, false><<<nblocks, kAdjThreads, 0, stream>>>(a, j);
+            else
+                k_adj_springs<4, kAdjChunk, 4, true><<<dim3(nblocks, std::min(parts, 3)), kAdjChunk, 0, stream>>>(a, j);
             break;
         default: return cudaErrorInvalidValue;
     }

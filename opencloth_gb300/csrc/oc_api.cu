@@ -1629,8 +1629,6 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
         s->adj.own_sid = own_sid;
         s->adj.own_rowptr = own_rowptr;
         s->adj.own_ent = own_ent;
-        if (const char* e = std::getenv("OC_ADJ_SPRINGS_VARIANT")) s->adj.springs_variant = std::atoi(e);
-        if (const char* e = std::getenv("OC_ADJ_VERTEX_VARIANT")) s->adj.vertex_variant = std::atoi(e);
     }
     float* planes = nullptr;
     OC_CREATE_TRY(dalloc(s, &planes, 15 * stride));
@@ -2570,6 +2568,8 @@ oc_status oc_tape_backward(oc_solver* s, const float* dL_dX, const float* dL_dV,
     a.blk_base = 0;
     a.use_cond = 0;
     a.all_streamed = 1;
+    bool stencil = true;
+    for (const InstParams& ip : s->inst_host) stencil = stencil && ip.grid_cols > 0;
     // One reverse step on the state b.X, b.V with the step's dV at dv (three planes): the
     // system's diagonal blocks rebuilt from spring i as the step formed them, the adjoint
     // seed, lambda = A^-1 g_dV, then the vertex and spring terms.
@@ -2577,7 +2577,7 @@ oc_status oc_tape_backward(oc_solver* s, const float* dL_dX, const float* dL_dV,
         AdjArgs jj = j;
         for (int k = 0; k < 3; ++k) jj.dV[k] = dv + k * st;
         if (gm) {
-            OC_TRY(launch_adjoint(0, b, jj, s->n_blocks, s->stream));
+            OC_TRY(launch_adjoint(0, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->stream));
         } else if (s->adj_persist) {
             OC_TRY(launch_adj_seed_own(b, jj, s->n_blocks, s->stream));
         }
@@ -2596,8 +2596,8 @@ oc_status oc_tape_backward(oc_solver* s, const float* dL_dX, const float* dL_dV,
             OC_TRY(cudaGraphExecKernelNodeSetParams(T.exec, T.n_seed, &kp));
             OC_TRY(cudaGraphLaunch(T.exec, s->stream));
         }
-        OC_TRY(launch_adjoint(1, b, jj, s->n_blocks, s->stream));
-        OC_TRY(launch_adjoint(2, b, jj, s->n_blocks, s->stream));
+        OC_TRY(launch_adjoint(1, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->stream));
+        OC_TRY(launch_adjoint(2, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->stream));
         return OC_OK;
     };
     if (T.replay) {

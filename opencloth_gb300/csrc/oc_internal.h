@@ -188,14 +188,13 @@ struct AdjArgs {
     const int32_t* own_sid;  // vertex i -> id of spring i, or -1
     const int32_t* own_rowptr;  // vertex -> vertices whose spring touches it
     const int32_t* own_ent;     // that vertex | (1 << 31 when the vertex is the spring's p2)
-    int32_t springs_variant;    // k_adj_springs' launch variant (OC_ADJ_SPRINGS_VARIANT; 0 default)
-    int32_t vertex_variant;     // k_adj_vertex's launch variant (OC_ADJ_VERTEX_VARIANT; 0 default)
 };
 
 // Adjoint kernels (oc_adjoint.cu) over the blocks a.blocks[blk_base, blk_base + nblocks):
 //   0 the displacement mode's seed (spring i's blocks rebuilt, adj_seed_vertex);
 //   1 the vertex terms (k_adj_vertex); 2 the spring terms (k_adj_springs).
-cudaError_t launch_adjoint(int which, const StepArgs& a, const AdjArgs& j, int nblocks, cudaStream_t stream);
+cudaError_t launch_adjoint(int which, const StepArgs& a, const AdjArgs& j, int nblocks, int vpb, bool stencil,
+                           cudaStream_t stream);  // vpb: vertices of a block at most; stencil: every cloth has one
 
 // The replay tape of one cloth (oc_tape_forward).  The forward keeps the solution dV of
 // every step; the cloth's state (X then V, nv float4 each) is kept every `every` steps

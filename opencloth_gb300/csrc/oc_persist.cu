@@ -81,10 +81,6 @@ struct PieceState {
 };
 static_assert(sizeof(PieceState) == kPersistPieceBytes, "persist_state_bytes");
 
-__device__ __forceinline__ void copy_async4(float* dst, const float* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-
 // The update (IMP:790-797) of a piece's slots [b, e), four vertices of a thread in flight; x out
 // of shared memory where it was kept there.
 __device__ __forceinline__ void persist_update(const StepArgs& a, const InstParams& ip, int64_t v, int n, int b, int e,
