@@ -286,7 +286,8 @@ oc_status oc_tape_displacement(oc_solver* s, float* u);
  * results of different resident shapes can differ in the last bits (each shape is
  * deterministic).  No counterpart in the reference (its step has one serial code path). */
 typedef struct oc_launch_config {
-    int32_t resident_max_vertices; /* OC_EXEC_AUTO: cloths up to this many vertices run resident; 0: none */
+    int32_t resident_max_vertices; /* OC_EXEC_AUTO: cloths up to this many vertices run resident (beside larger ones
+                                      of a handle of few cloths they may join those in one launch); 0: none */
     int32_t resident_vcta;         /* vertices per resident CTA: 256, 512, 1024 or 2048 */
     int32_t resident_threads;      /* threads per resident CTA: 128, 256 or 512, with vcta <= 4 x threads */
     int32_t resident_fused;        /* 1: resident cloths assemble inside the resident kernel */

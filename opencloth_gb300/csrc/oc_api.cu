@@ -1254,6 +1254,45 @@ oc_status plan_coupled(oc_solver* s) {
     return OC_OK;
 }
 
+// Whether the cloths small enough for the resident kernel stream too, because others of the handle
+// do: k_cg_persist and the resident launches run one behind the other (its CTAs need whole SMs), so
+// where every cloth can have CTAs of its own in one k_cg_persist launch and these come out about as
+// large as if the vertices were cut evenly, that is the faster step.  Measured, us a step (and of a
+// taped step forward and back), resident and streamed: a 200 x 200 cloth with 5 of 120 x 120 47 / 33
+// (246 / 218), with 50 of 64 x 64 56 / 49 (355 / 344), with 50 of 20 x 20 31 / 31 (178 / 168); 24
+// cloths of 16 to 192 a side 82 / 65; 1000 x 1000 with 5 of 30 x 30 147 / 134.  Cut unevenly: the
+// same with 50 of 30 x 30 156 / 175, 200 x 200 with 100 of 20 x 20 32 / 39; many cloths: 200 x 200
+// with 140 of 64 x 64 88 / 105, with 100 of 120 x 120 195 / 251.
+constexpr int32_t kJoinMaxCloths = 64;
+
+bool all_stream(const oc_solver* s) {
+    const oc_launch_config& c = s->cfg;
+    if (s->executor != OC_EXEC_AUTO || !c.persist || c.resident_fused || !s->coop || s->persist_smem_max <= 0 ||
+        s->n_inst > kJoinMaxCloths)
+        return false;
+    int64_t total = 0, small = 0;
+    for (const InstParams& ip : s->inst_host) {
+        if (ip.coupled) return false;
+        total += ip.nv;
+        int threads = 0, cluster = 0, vcta = 0;
+        if (resident_shape(ip.nv, c.resident_max_vertices, c.resident_vcta, c.resident_threads, &threads, &cluster, &vcta))
+            small += ip.nv;
+    }
+    if (small == 0 || small == total) return false;
+    const int64_t most = total <= (int64_t)kPersistMaxCluster * s->persist_clusters * 16 * kPersistThreads
+                             ? (int64_t)kPersistMaxCluster * s->persist_clusters
+                             : std::max(1, s->sm_count);  // (clusters hold about that many on chip)
+    const int64_t even = (total + most - 1) / most;
+    if (s->n_inst > most) return false;
+    int64_t chunk = even, n = 0;
+    for (;; chunk += 32) {
+        n = 0;
+        for (const InstParams& ip : s->inst_host) n += (ip.nv + chunk - 1) / chunk;
+        if (n <= most) break;
+    }
+    return 5 * chunk <= 7 * even || chunk <= even + kPersistThreads;
+}
+
 // The launch plan from the handle's cloths and its launch configuration: which cloths run
 // resident (one cluster per cloth, the whole step on chip) and which streamed, resident
 // cloths grouped by launch shape into buckets, the assembly tables (record gather,
@@ -1272,6 +1311,7 @@ oc_status plan_execution(oc_solver* s) {
     std::vector<BlockInfo> streamed, asm_ref, cpl, upd, grid;
     std::map<std::tuple<int, int, int>, std::vector<int32_t>> groups;
     s->grid_kind = K_ASSEMBLE_KINDS;
+    const bool join = all_stream(s);
     for (int32_t k = 0; k < s->n_inst; ++k) {
         InstParams& ip = s->inst_host[(size_t)k];
         const bool cpl_k = ip.coupled != 0;
@@ -1279,7 +1319,7 @@ oc_status plan_execution(oc_solver* s) {
             return fail(s, OC_ERR_UNSUPPORTED,
                         "instance " + std::to_string(k) + " is COUPLED: the resident executor runs REFERENCE cloths");
         int threads = 0, cluster = 0, vcta = 0;
-        const bool want = !cpl_k && (s->executor == OC_EXEC_RESIDENT || s->executor == OC_EXEC_AUTO) &&
+        const bool want = !cpl_k && !join && (s->executor == OC_EXEC_RESIDENT || s->executor == OC_EXEC_AUTO) &&
                           resident_shape(ip.nv, max_res, cfg.resident_vcta, cfg.resident_threads, &threads, &cluster,
                                          &vcta);
         if (s->executor == OC_EXEC_RESIDENT && !want)
