@@ -618,7 +618,7 @@ __global__ void k_set_spring_params(const StepArgs a, const AdjArgs j, const flo
 }  // namespace
 
 cudaError_t launch_adjoint(int which, const StepArgs& a, const AdjArgs& j, int nblocks, int vpb, bool stencil,
-                           cudaStream_t stream) {
+                           int sms, cudaStream_t stream) {
     if (nblocks <= 0) return cudaSuccess;
     const int parts = (vpb + kAdjChunk - 1) / kAdjChunk;
     switch (which) {
@@ -626,8 +626,11 @@ cudaError_t launch_adjoint(int which, const StepArgs& a, const AdjArgs& j, int n
         case 1: k_adj_vertex<<<dim3(nblocks, parts), kAdjChunk, 0, stream>>>(a, j); break;
         case 2:
             // Large handles of stencil cloths alone read no records to copy, and their whole blocks
-            // make waves enough: 2 M vertices 327 us against 366, 4 M 624 against 741.
-            if (stencil && (int64_t)nblocks * vpb >= 1500000)
+            // make waves enough: 2 M vertices 327 us against 366, 4 M 624 against 741.  Nor does the
+            // displacement mode, with more arithmetic a spring, take chunks that just miss one wave
+            // where whole blocks make it: 24 of 64 x 64 25 us against 34.
+            if (stencil && ((int64_t)nblocks * vpb >= 1500000 ||
+                            (a.gm && nblocks * parts > 4 * sms && nblocks <= 3 * sms)))
                 k_adj_springs<2, kAdjThreads, 3, false><<<nblocks, kAdjThreads, 0, stream>>>(a, j);
             else
                 k_adj_springs<4, kAdjChunk, 4, true><<<dim3(nblocks, std::min(parts, 3)), kAdjChunk, 0, stream>>>(a, j);

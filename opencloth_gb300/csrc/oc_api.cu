@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <array>
 #include <map>
+#include <set>
 #include <tuple>
 #include <cmath>
 #include <cstdio>
@@ -106,6 +107,10 @@ struct oc_solver {
     bool cpl_persist = false;  // k_cpl_persist runs the COUPLED cloths
     CplPlan cplan{};           // their pieces (grid 0: none, or not available)
     int cpl_rows_max = 0;
+    // The adjoint's and the displacement mode's solves in one launch over every cloth (grid 0: the
+    // resident cloths by k_resident, the others by pplan); made when a tape begins.
+    PersistPlan aplan{};
+    bool aplan_made = false;
     PersistPlan pplan{};  // the streamed REFERENCE cloths' pieces (grid 0: none, or not available)
     // k_assemble_finish runs when a strip-swept cloth is resident or the streamed CG is
     // not the persistent one; otherwise k_cg_persist forms their delta0 itself.
@@ -810,11 +815,17 @@ StepArgs gm_args(const oc_solver* s, float dt) {
 }
 
 // The CG alone (no update) of every cloth, from the CG state set up in the planes and
-// the cloths' states: the resident cloths on chip (k_resident unfused, one launch per
-// bucket, beside) and the streamed ones in one cooperative launch of k_cg_persist.
+// the cloths' states: in one cooperative launch of k_cg_persist where plan_adjoint made one, else the
+// resident cloths on chip (k_resident unfused, one launch per bucket, beside) and the streamed ones in
+// k_cg_persist.
 oc_status solve_only(oc_solver* s, const StepArgs& a) {
     StepArgs pa = a;
     pa.cg_only = 1;
+    if (s->aplan.grid > 0) {
+        OC_TRY(launch_cg_persist(pa, s->aplan, s->stream));
+        s->host_launches += 1;
+        return OC_OK;
+    }
     if (!s->buckets.empty())
         if (oc_status r = launch_resident_all(s, pa, nullptr)) return r;
     if (s->pplan.grid > 0) {
@@ -1006,8 +1017,10 @@ oc_status alloc_error_word(oc_solver* s) {
 }
 
 // k_sim's plan: every cloth of the handle resident, each on the fewest CTAs of 256, 512 or 1024
-// vertices that make a cluster of kSimMaxCluster at most, and all of these CTAs together no more
-// than the SMs: then a step is bound by latencies, which k_sim shortens; with more cloths it is
+// vertices that make a cluster of kSimMaxCluster at most, all of these CTAs together no more than the
+// SMs, and the small and the large clusters each no more than are co-resident (a cluster of 16 takes a
+// GPC, so 7 run at once: 8 cloths of 64 x 64 on 256-vertex CTAs took 21 us a step in two turns against
+// 12 for 4 of them, and 14 on 512-vertex ones): then a step is bound by latencies, which k_sim shortens; with more cloths it is
 // bound by instructions, and the assembly's and the resident CG's own launches keep more warps in
 // flight.
 oc_status plan_sim(oc_solver* s) {
@@ -1051,7 +1064,20 @@ oc_status plan_sim(oc_solver* s) {
             }
             sh.ids.push_back(k);
         }
-        if (total <= s->sm_count) break;
+        if (total > s->sm_count) continue;
+        double turns[2] = {0.0, 0.0};  // of the clusters of two to four CTAs, of the larger ones
+        for (const auto& kv : shapes) {
+            const SimLaunch& L = kv.second.launch;
+            if (sim_smem_bytes(L) > (size_t)s->sim_smem_max) return OC_OK;
+            if (L.cluster == 1) continue;
+            int n = 0;
+            if (sim_max_clusters(L, &n) != cudaSuccess || n < 1) {
+                cudaGetLastError();
+                return OC_OK;
+            }
+            turns[L.cluster > 4] += (double)kv.second.ids.size() / n;
+        }
+        if (turns[0] <= 1.0 && turns[1] <= 1.0) break;
     }
     for (const auto& kv : shapes)
         if (sim_smem_bytes(kv.second.launch) > (size_t)s->sim_smem_max) return OC_OK;
@@ -1076,17 +1102,12 @@ oc_status plan_sim(oc_solver* s) {
 // kPersistMaxCluster when those, which leave some SMs idle, hold every vertex on chip, else of
 // 2 (see oc_persist.cu for the exchanges' times).  Left without a grid when the device has no
 // cooperative launch or a CTA would hold too many pieces.
-oc_status plan_persist(oc_solver* s) {
-    PersistPlan& P = s->pplan;
+oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_t>& ids) {
+    PersistPlan& P = *plan;
     P.grid = 0;
     if (!s->coop || s->persist_smem_max <= 0) return OC_OK;
-    std::vector<int32_t> ids;
     int64_t total = 0;
-    for (int32_t k = 0; k < s->n_inst; ++k)
-        if (!s->resident[(size_t)k]) {
-            ids.push_back(k);
-            total += s->inst_host[(size_t)k].nv;
-        }
+    for (int32_t k : ids) total += s->inst_host[(size_t)k].nv;
     std::vector<PersistPiece> pieces;
     std::vector<int32_t> cta_piece;
     // The cut for clusters of `cluster` CTAs and at most `most` CTAs.
@@ -1254,43 +1275,65 @@ oc_status plan_coupled(oc_solver* s) {
     return OC_OK;
 }
 
-// Whether the cloths small enough for the resident kernel stream too, because others of the handle
-// do: k_cg_persist and the resident launches run one behind the other (its CTAs need whole SMs), so
-// where every cloth can have CTAs of its own in one k_cg_persist launch and these come out about as
-// large as if the vertices were cut evenly, that is the faster step.  Measured, us a step (and of a
-// taped step forward and back), resident and streamed: a 200 x 200 cloth with 5 of 120 x 120 47 / 33
-// (246 / 218), with 50 of 64 x 64 56 / 49 (355 / 344), with 50 of 20 x 20 31 / 31 (178 / 168); 24
-// cloths of 16 to 192 a side 82 / 65; 1000 x 1000 with 5 of 30 x 30 147 / 134.  Cut unevenly: the
-// same with 50 of 30 x 30 156 / 175, 200 x 200 with 100 of 20 x 20 32 / 39; many cloths: 200 x 200
-// with 140 of 64 x 64 88 / 105, with 100 of 120 x 120 195 / 251.
+// Whether one k_cg_persist launch can run every cloth of the handle without cutting them unevenly:
+// few cloths, each with CTAs of its own that come out about as large as if the vertices were cut
+// evenly.
 constexpr int32_t kJoinMaxCloths = 64;
 
-bool all_stream(const oc_solver* s) {
-    const oc_launch_config& c = s->cfg;
-    if (s->executor != OC_EXEC_AUTO || !c.persist || c.resident_fused || !s->coop || s->persist_smem_max <= 0 ||
-        s->n_inst > kJoinMaxCloths)
-        return false;
-    int64_t total = 0, small = 0;
+bool may_join(const oc_solver* s) {
+    if (!s->cfg.persist || !s->coop || s->persist_smem_max <= 0 || s->n_inst > kJoinMaxCloths) return false;
+    int64_t total = 0;
     for (const InstParams& ip : s->inst_host) {
         if (ip.coupled) return false;
         total += ip.nv;
-        int threads = 0, cluster = 0, vcta = 0;
-        if (resident_shape(ip.nv, c.resident_max_vertices, c.resident_vcta, c.resident_threads, &threads, &cluster, &vcta))
-            small += ip.nv;
     }
-    if (small == 0 || small == total) return false;
     const int64_t most = total <= (int64_t)kPersistMaxCluster * s->persist_clusters * 16 * kPersistThreads
                              ? (int64_t)kPersistMaxCluster * s->persist_clusters
                              : std::max(1, s->sm_count);  // (clusters hold about that many on chip)
     const int64_t even = (total + most - 1) / most;
     if (s->n_inst > most) return false;
-    int64_t chunk = even, n = 0;
+    int64_t chunk = even;
     for (;; chunk += 32) {
-        n = 0;
+        int64_t n = 0;
         for (const InstParams& ip : s->inst_host) n += (ip.nv + chunk - 1) / chunk;
         if (n <= most) break;
     }
     return 5 * chunk <= 7 * even || chunk <= even + kPersistThreads;
+}
+
+// Whether the cloths small enough for the resident kernel stream too.  (a) Others of the handle do:
+// k_cg_persist and the resident launches run one behind the other (its CTAs need whole SMs).  (b)
+// None does, but they take kJoinBuckets resident launches or more, and k_sim does not run them.
+// Measured, us a step (and of four taped steps forward and back), resident and streamed: (a) a 200 x
+// 200 cloth with 5 of 120 x 120 47 / 33 (983 / 871), with 50 of 20 x 20 31 / 31 (712 / 671); 24 cloths
+// of 16 to 192 a side 82 / 65; 1000 x 1000 with 5 of 30 x 30 147 / 134, with 50 (cut unevenly) 156 /
+// 175; 200 x 200 with 100 of 20 x 20 (unevenly) 32 / 39, with 140 of 64 x 64 (many) 88 / 105.  (b) 36 of
+// 16 to 128 a side (12 launches) 50 / 37, 64 of them (13) 66 / 61, 48 of 16 to 96 (8) 41 / 37; of one
+// size (one launch) 24 of 90 x 90 44 / 49, 16 of 128 x 128 47 / 51.
+constexpr size_t kJoinBuckets = 5;
+
+oc_status all_stream(oc_solver* s, bool* join) {
+    const oc_launch_config& c = s->cfg;
+    *join = false;
+    if (s->executor != OC_EXEC_AUTO || c.resident_fused || !may_join(s)) return OC_OK;
+    int32_t small = 0;
+    std::set<std::tuple<int, int, int>> shapes;
+    for (const InstParams& ip : s->inst_host) {
+        int threads = 0, cluster = 0, vcta = 0;
+        if (!resident_shape(ip.nv, c.resident_max_vertices, c.resident_vcta, c.resident_threads, &threads, &cluster, &vcta))
+            continue;
+        ++small;
+        shapes.insert(std::make_tuple(threads, cluster, vcta));
+    }
+    if (small == 0 || small < s->n_inst) {
+        *join = small > 0;
+        return OC_OK;
+    }
+    if (shapes.size() < kJoinBuckets) return OC_OK;
+    s->resident.assign((size_t)s->n_inst, 1);
+    if (oc_status r = plan_sim(s)) return r;
+    *join = s->sim.empty();
+    return OC_OK;
 }
 
 // The launch plan from the handle's cloths and its launch configuration: which cloths run
@@ -1305,13 +1348,14 @@ oc_status plan_execution(oc_solver* s) {
     a.strip_variant = cfg.strip_variant;
     s->resident_fused = cfg.resident_fused != 0;
     const int max_res = cfg.resident_max_vertices;
+    bool join = false;
+    if (oc_status r = all_stream(s, &join)) return r;
     s->resident.assign((size_t)s->n_inst, 0);
     for (oc_solver::Bucket& b : s->buckets) dfree(s, &b.d_ids);
     s->buckets.clear();
     std::vector<BlockInfo> streamed, asm_ref, cpl, upd, grid;
     std::map<std::tuple<int, int, int>, std::vector<int32_t>> groups;
     s->grid_kind = K_ASSEMBLE_KINDS;
-    const bool join = all_stream(s);
     for (int32_t k = 0; k < s->n_inst; ++k) {
         InstParams& ip = s->inst_host[(size_t)k];
         const bool cpl_k = ip.coupled != 0;
@@ -1390,9 +1434,13 @@ oc_status plan_execution(oc_solver* s) {
         any_coupled |= s->inst_host[(size_t)k].coupled != 0;
         any_streamed |= !s->resident[(size_t)k] && !s->inst_host[(size_t)k].coupled;
     }
-    s->pplan.grid = 0;
+    s->pplan.grid = s->aplan.grid = 0;
+    s->aplan_made = false;
+    std::vector<int32_t> streamed_ids;
+    for (int32_t k = 0; k < s->n_inst; ++k)
+        if (!s->resident[(size_t)k]) streamed_ids.push_back(k);
     if (any_streamed && !any_coupled)
-        if (oc_status r = plan_persist(s)) return r;
+        if (oc_status r = plan_persist(s, &s->pplan, streamed_ids)) return r;
     s->persist = cfg.persist && s->pplan.grid > 0;
     if (any_coupled)
         if (oc_status r = plan_coupled(s)) return r;
@@ -1929,6 +1977,23 @@ oc_status step_sim(oc_solver* s, float dt, int32_t n_steps) {
     return OC_OK;
 }
 
+// One step of k_sim's launches as a graph.
+oc_status build_sim_graph(oc_solver* s, float dt) {
+    drop_graphs(s);
+    cudaGraph_t g = nullptr;
+    OC_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    const int64_t launches = s->host_launches;
+    const oc_status st = step_sim(s, dt, 1);
+    s->host_launches = launches;
+    const cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+    s->graph = g;
+    if (st != OC_OK) return st;
+    if (e != cudaSuccess) return fail_cuda(s, e, "capture of k_sim");
+    OC_TRY(cudaGraphInstantiate(&s->exec, g, 0));
+    s->graph_dt = dt;
+    return OC_OK;
+}
+
 }  // namespace
 
 oc_status oc_step(oc_solver* s, float dt, int32_t n_steps) {
@@ -1948,7 +2013,18 @@ oc_status oc_step(oc_solver* s, float dt, int32_t n_steps) {
         }
         return OC_OK;
     }
-    if (!s->sim.empty()) return step_sim(s, dt, n_steps);
+    if (!s->sim.empty()) {
+        // One step of several launches goes as a graph: the launches and the events that fork and join
+        // them are more host time than the step (12 cloths of 16 to 96 a side, 10 launches).
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (n_steps == 1 && s->sim.size() > 1) OC_TRY(cudaStreamIsCapturing(s->stream, &cap));
+        if (n_steps != 1 || s->sim.size() == 1 || cap != cudaStreamCaptureStatusNone) return step_sim(s, dt, n_steps);
+        if (!s->exec || s->graph_dt != dt)
+            if (oc_status st = build_sim_graph(s, dt)) return st;
+        OC_TRY(cudaGraphLaunch(s->exec, s->stream));
+        s->host_launches += (int64_t)s->sim.size();
+        return OC_OK;
+    }
     if (!s->exec || s->graph_dt != dt) {
         oc_status st = build_graph(s, dt);
         if (st != OC_OK) return st;
@@ -2433,6 +2509,22 @@ oc_status taped_forward(oc_solver* s, float dt) {
     return OC_OK;
 }
 
+// The plan of solve_only's one launch: where it can run every cloth (may_join) and the resident
+// launches are several (three or more) or one cluster's.  Measured, us of four steps forward and
+// back, start's resident launches and the one launch: 24 cloths of 16 to 96 a side 789 / 725, 18 of 16
+// to 128 907 / 856; in the displacement mode, where every solve goes this way, one 64 x 64 cloth 585 /
+// 565, but 24 of them (one launch either way) 904 / 935 and 8 of them 646 / 674.
+oc_status plan_adjoint(oc_solver* s) {
+    if (s->aplan_made) return OC_OK;
+    s->aplan_made = true;
+    s->aplan.grid = 0;
+    if (s->buckets.empty() || !s->adj_persist || !may_join(s)) return OC_OK;
+    if (s->buckets.size() < 3 && (s->n_inst > 1 || s->inst_host[0].nv <= kResidentDefaultVcta)) return OC_OK;
+    std::vector<int32_t> ids((size_t)s->n_inst);
+    for (int32_t k = 0; k < s->n_inst; ++k) ids[(size_t)k] = k;
+    return plan_persist(s, &s->aplan, ids);
+}
+
 // Chooses the tape and its intervals, allocates it and runs the taped forward.
 //   every_in != null: the replay tape with those per-cloth intervals.
 //   otherwise: every cloth at the interval `checkpoint_every` (0: ceil(sqrt(n)), which
@@ -2455,6 +2547,7 @@ oc_status tape_begin(oc_solver* s, float dt, int32_t n, int32_t checkpoint_every
     if (T.mode == OC_TAPE_DISPLACEMENT && !s->adj_persist)
         return fail(s, OC_ERR_UNSUPPORTED, "oc_tape_forward: the displacement mode needs the cooperative CG, which the "
                                            "launch configuration set since does not allow");
+    if (oc_status r = plan_adjoint(s)) return r;
     int32_t every = checkpoint_every;
     if (every == 0) every = std::max(1, (int32_t)std::ceil(std::sqrt((double)n)));
     every = std::min(every, n);
@@ -2617,7 +2710,7 @@ oc_status oc_tape_backward(oc_solver* s, const float* dL_dX, const float* dL_dV,
         AdjArgs jj = j;
         for (int k = 0; k < 3; ++k) jj.dV[k] = dv + k * st;
         if (gm) {
-            OC_TRY(launch_adjoint(0, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->stream));
+            OC_TRY(launch_adjoint(0, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->sm_count, s->stream));
         } else if (s->adj_persist) {
             OC_TRY(launch_adj_seed_own(b, jj, s->n_blocks, s->stream));
         }
@@ -2636,8 +2729,8 @@ oc_status oc_tape_backward(oc_solver* s, const float* dL_dX, const float* dL_dV,
             OC_TRY(cudaGraphExecKernelNodeSetParams(T.exec, T.n_seed, &kp));
             OC_TRY(cudaGraphLaunch(T.exec, s->stream));
         }
-        OC_TRY(launch_adjoint(1, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->stream));
-        OC_TRY(launch_adjoint(2, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->stream));
+        OC_TRY(launch_adjoint(1, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->sm_count, s->stream));
+        OC_TRY(launch_adjoint(2, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->sm_count, s->stream));
         return OC_OK;
     };
     if (T.replay) {

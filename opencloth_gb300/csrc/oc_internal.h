@@ -194,7 +194,7 @@ struct AdjArgs {
 //   0 the displacement mode's seed (spring i's blocks rebuilt, adj_seed_vertex);
 //   1 the vertex terms (k_adj_vertex); 2 the spring terms (k_adj_springs).
 cudaError_t launch_adjoint(int which, const StepArgs& a, const AdjArgs& j, int nblocks, int vpb, bool stencil,
-                           cudaStream_t stream);  // vpb: vertices of a block at most; stencil: every cloth has one
+                           int sms, cudaStream_t stream);  // vpb: vertices of a block at most; stencil: every cloth has one
 
 // The replay tape of one cloth (oc_tape_forward).  The forward keeps the solution dV of
 // every step; the cloth's state (X then V, nv float4 each) is kept every `every` steps
@@ -380,6 +380,7 @@ struct SimLaunch {
 };
 size_t sim_smem_bytes(const SimLaunch& L);
 cudaError_t prepare_sim(int device, int* max_smem);
+cudaError_t sim_max_clusters(const SimLaunch& L, int* n);  // co-resident clusters of a launch's shape
 cudaError_t launch_sim(const StepArgs& a, const SimLaunch& L, int n_clusters, cudaStream_t stream);
 
 cudaError_t launch_state_in(const StepArgs& a, const float* X3, const float* V3, const float* dV3, int64_t nv,

@@ -537,6 +537,21 @@ cudaError_t prepare_sim(int device, int* max_smem) {
     return e;
 }
 
+cudaError_t sim_max_clusters(const SimLaunch& L, int* n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)L.cluster);
+    cfg.blockDim = dim3((unsigned)L.threads);
+    cfg.dynamicSmemBytes = sim_smem_bytes(L);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)L.cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaOccupancyMaxActiveClusters(n, sim_fn(L.threads, L.vpt), &cfg);
+}
+
 cudaError_t launch_sim(const StepArgs& a, const SimLaunch& L, int n_clusters, cudaStream_t stream) {
     if (n_clusters <= 0) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
