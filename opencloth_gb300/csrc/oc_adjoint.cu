@@ -257,7 +257,7 @@ struct AdjInc {
     float rest, ks, kd;
 };
 
-template <bool STENCIL, bool STAGED, int kAdjAhead>
+template <bool STENCIL, bool STAGED, bool GM, int kAdjAhead>
 __device__ __forceinline__ void adj_springs_vertex(const StepArgs& a, const AdjArgs& j, const InstParams& ip,
                                                    int64_t g, const int4* s_rec, const int32_t* s_sid, int32_t kA) {
     const float4* __restrict__ X = a.X;
@@ -266,6 +266,7 @@ __device__ __forceinline__ void adj_springs_vertex(const StepArgs& a, const AdjA
     const float* __restrict__ gF1 = j.gF[1];
     const float* __restrict__ gF2 = j.gF[2];
     const float4 Xg = __ldg(X + g), Vg = __ldg(V + g);
+    const float4 Bg = GM ? __ldg(a.Xbase + g) : Xg;
     const float gFg[3] = {__ldg(gF0 + g), __ldg(gF1 + g), __ldg(gF2 + g)};
     float gx[3] = {j.gX[0][g], j.gX[1][g], j.gX[2][g]};
     float gv[3] = {j.gV[0][g], j.gV[1][g], j.gV[2][g]};
@@ -304,13 +305,18 @@ __device__ __forceinline__ void adj_springs_vertex(const StepArgs& a, const AdjA
             }
             sid[u] = (k < k1 && !in[u].p2) ? (STAGED ? s_sid[k - kA] : __ldg(j.inc_sid + k)) : 0;
         }
-        float4 Xo[kAdjAhead], Vo[kAdjAhead];
+        float4 Xo[kAdjAhead], Vo[kAdjAhead], Bo[GM ? kAdjAhead : 1];
+        float2 Ko[GM ? kAdjAhead : 1];  // displacement mode: the other end's base and the constants
         float gFo[kAdjAhead][3], gk_old[kAdjAhead], gd_old[kAdjAhead];
 #pragma unroll
         for (int u = 0; u < kAdjAhead; ++u) {
             const int32_t o = in[u].o;
             Xo[u] = __ldg(X + o);
             Vo[u] = __ldg(V + o);
+            if constexpr (GM) {
+                Bo[u] = __ldg(a.Xbase + o);
+                Ko[u] = __ldg(a.gm_inc + min(kb + u, k1 - 1));
+            }
             gFo[u][0] = __ldg(gF0 + o);
             gFo[u][1] = __ldg(gF1 + o);
             gFo[u][2] = __ldg(gF2 + o);
@@ -328,13 +334,17 @@ __device__ __forceinline__ void adj_springs_vertex(const StepArgs& a, const AdjA
 #pragma unroll
             for (int c = 0; c < 3; ++c) gf[c] = as_p2 ? gFo[u][c] - gFg[c] : gFg[c] - gFo[u][c];
             float gdP[3], gdV[3], gks, gkd;
-            const int32_t o = in[u].o;
-            if (as_p2)
-                spring_force_adj(spring_geo(a, o, (int32_t)g, Xo[u], Xg, in[u].rest, a.gm_inc, kb + u), Vo[u], Vg,
-                                 in[u].ks, in[u].kd, gf, gdP, gdV, gks, gkd);
-            else
-                spring_force_adj(spring_geo(a, (int32_t)g, o, Xg, Xo[u], in[u].rest, a.gm_inc, kb + u), Vg, Vo[u],
-                                 in[u].ks, in[u].kd, gf, gdP, gdV, gks, gkd);
+            if (as_p2) {
+                Geo geo;
+                if constexpr (GM) geo = geo_disp(Bo[u], Bg, Xo[u], Xg, Ko[u]);
+                else geo = geo_plain(Xo[u], Xg, in[u].rest);
+                spring_force_adj(geo, Vo[u], Vg, in[u].ks, in[u].kd, gf, gdP, gdV, gks, gkd);
+            } else {
+                Geo geo;
+                if constexpr (GM) geo = geo_disp(Bg, Bo[u], Xg, Xo[u], Ko[u]);
+                else geo = geo_plain(Xg, Xo[u], in[u].rest);
+                spring_force_adj(geo, Vg, Vo[u], in[u].ks, in[u].kd, gf, gdP, gdV, gks, gkd);
+            }
             const float sgn = as_p2 ? -1.0f : 1.0f;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
@@ -372,10 +382,12 @@ __device__ __forceinline__ void adj_springs_vertex(const StepArgs& a, const AdjA
 // Measured, 24 cloths (231k vertices, a record a spring), us: 89 with <2, 256, 3, false> over whole
 // blocks, 67 with <4, 128, 4, false> over chunks, 50 with <4, 128, 4, true>; two incidences and six
 // CTAs an SM 78, three and four 62, six and three 59; 64 threads 56; four and three 57 (the copies
-// and the gathered states share an SM's L1).  700 x 700 stencil 133 -> 101, 257 x 257 31 -> 22.
+// and the gathered states share an SM's L1).  700 x 700 stencil 133 -> 101.  GM: the displacement
+// mode, whose bases and constants are loaded with the neighbour's state: 257 x 257 32 -> 18, 600 x 600
+// 139 -> 84 (loaded at their use 257 x 257 22; three incidences 28, four at three CTAs 24).
 constexpr int kSpringStage = 13;  // records of a vertex that the copies have room for, on average
 
-template <int AHEAD, int T, int MINB, bool STAGE>
+template <int AHEAD, int T, int MINB, bool STAGE, bool GM>
 __global__ void __launch_bounds__(T, MINB) k_adj_springs(const StepArgs a, const AdjArgs j) {
     __shared__ int4 s_rec[STAGE ? T * kSpringStage : 1];
     __shared__ int32_t s_sid[STAGE ? T * kSpringStage : 1];
@@ -402,11 +414,11 @@ __global__ void __launch_bounds__(T, MINB) k_adj_springs(const StepArgs a, const
         }
         if (g >= end) continue;
         if (stencil) {
-            if (staged) adj_springs_vertex<true, true, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
-            else adj_springs_vertex<true, false, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
+            if (staged) adj_springs_vertex<true, true, GM, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
+            else adj_springs_vertex<true, false, GM, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
         } else {
-            if (staged) adj_springs_vertex<false, true, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
-            else adj_springs_vertex<false, false, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
+            if (staged) adj_springs_vertex<false, true, GM, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
+            else adj_springs_vertex<false, false, GM, AHEAD>(a, j, ip, g, s_rec, s_sid, kA);
         }
     }
 }
@@ -431,22 +443,35 @@ __device__ __forceinline__ float2 spring_consts(const float4 b1, const float4 b2
     return make_float2((float)(L0 - (double)rest), (float)L0);
 }
 
+// Threads of a vertex in k_gm_consts: its incidences are a root in FP64 each.  100 x 100 28 -> 15 us;
+// four threads 16, and 257 x 257 55 against 50.
+constexpr int kGmLanes = 2;
+
 // 4: the spring constants from Xbase, and u = 0 (mass kept in w).
 __global__ void k_gm_consts(const StepArgs a, int64_t nv) {
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < nv; g += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t n = nv * kGmLanes, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += step) {
+        const int64_t g = t / kGmLanes;
+        const int q = (int)(t % kGmLanes);
         const float4 bg = __ldg(a.Xbase + g);
         const int32_t k0 = __ldg(a.rowptr + g), k1 = __ldg(a.rowptr + g + 1);
-        for (int32_t k = k0; k < k1; ++k) {
-            const int4 rec = __ldg(a.inc + k);
-            const float4 bo = __ldg(a.Xbase + (rec.x & 0x7fffffff));
-            const float rest = __int_as_float(rec.y);
-            const_cast<float2*>(a.gm_inc)[k] = rec.x < 0 ? spring_consts(bo, bg, rest) : spring_consts(bg, bo, rest);
+        for (int32_t k = k0 + q; k <= k1; k += kGmLanes) {  // the incidences, then spring i
+            int2 e;
+            float rest;
+            if (k < k1) {
+                const int4 rec = __ldg(a.inc + k);
+                const int32_t o = rec.x & 0x7fffffff;
+                e = rec.x < 0 ? make_int2(o, (int)g) : make_int2((int)g, o);
+                rest = __int_as_float(rec.y);
+            } else {
+                e = __ldg(a.own_ends + g);
+                rest = __ldg(a.own_par + g).x;
+            }
+            float2 c = make_float2(0.f, 0.f);
+            if (e.x >= 0) c = spring_consts(__ldg(a.Xbase + e.x), __ldg(a.Xbase + e.y), rest);
+            const_cast<float2*>(k < k1 ? a.gm_inc + k : a.gm_own + g)[0] = c;
         }
-        const int2 e = __ldg(a.own_ends + g);
-        float2 own = make_float2(0.f, 0.f);
-        if (e.x >= 0) own = spring_consts(__ldg(a.Xbase + e.x), __ldg(a.Xbase + e.y), __ldg(a.own_par + g).x);
-        const_cast<float2*>(a.gm_own)[g] = own;
-        a.X[g] = make_float4(0.f, 0.f, 0.f, bg.w);
+        if (q == 0) a.X[g] = make_float4(0.f, 0.f, 0.f, bg.w);
     }
 }
 
@@ -494,7 +519,12 @@ __device__ __forceinline__ void gm_own_blocks(const StepArgs& a, int64_t g, floa
     }
 }
 
-__global__ void __launch_bounds__(kAdjThreads) k_gm_assemble(const StepArgs a) {
+// Bound by the latency of an incidence's record, its neighbour and that one's state: two incidences in
+// flight at four CTAs an SM, 100 x 100 14.9 -> 12.1 us, 600 x 600 60 -> 54 (four in flight 11.6 and
+// 62, at three CTAs 12.8 and 82).
+constexpr int kGmAhead = 2;
+
+__global__ void __launch_bounds__(kAdjThreads, 4) k_gm_assemble(const StepArgs a) {
     const int blk = blockIdx.x + a.blk_base;
     const BlockInfo bi = a.blocks[blk];
     const InstParams& ip = a.inst[bi.inst];
@@ -520,23 +550,38 @@ __global__ void __launch_bounds__(kAdjThreads) k_gm_assemble(const StepArgs a) {
                 Fz += e.z;
             }
             const int32_t k0 = __ldg(a.rowptr + g), k1 = __ldg(a.rowptr + g + 1);
-            for (int32_t k = k0; k < k1; ++k) {
-                const int4 rec = __ldg(a.inc + k);
-                const int32_t o = rec.x & 0x7fffffff;
-                const float4 Uo = a.X[o], Vo = a.V[o];
-                const float ks = __int_as_float(rec.z), kd = __int_as_float(rec.w);
-                if (rec.x < 0) {  // F[p2] -= f
-                    const float3 f =
-                        spring_force_geo(spring_geo(a, o, (int32_t)g, Uo, Ug, 0.0f, a.gm_inc, k), Vo, Vg, ks, kd);
-                    Fx -= f.x;
-                    Fy -= f.y;
-                    Fz -= f.z;
-                } else {  // F[p1] += f
-                    const float3 f =
-                        spring_force_geo(spring_geo(a, (int32_t)g, o, Ug, Uo, 0.0f, a.gm_inc, k), Vg, Vo, ks, kd);
-                    Fx += f.x;
-                    Fy += f.y;
-                    Fz += f.z;
+            const float4 Bg = __ldg(a.Xbase + g);
+            for (int32_t kb = k0; kb < k1; kb += kGmAhead) {
+                int4 rec[kGmAhead];
+                float4 Uo[kGmAhead], Vo[kGmAhead], Bo[kGmAhead];
+                float2 Ko[kGmAhead];
+#pragma unroll
+                for (int u = 0; u < kGmAhead; ++u) {
+                    rec[u] = __ldg(a.inc + min(kb + u, k1 - 1));
+                    Ko[u] = __ldg(a.gm_inc + min(kb + u, k1 - 1));
+                }
+#pragma unroll
+                for (int u = 0; u < kGmAhead; ++u) {
+                    const int32_t o = rec[u].x & 0x7fffffff;
+                    Uo[u] = a.X[o];
+                    Vo[u] = a.V[o];
+                    Bo[u] = __ldg(a.Xbase + o);
+                }
+#pragma unroll
+                for (int u = 0; u < kGmAhead; ++u) {
+                    if (kb + u >= k1) break;
+                    const float ks = __int_as_float(rec[u].z), kd = __int_as_float(rec[u].w);
+                    if (rec[u].x < 0) {  // F[p2] -= f
+                        const float3 f = spring_force_geo(geo_disp(Bo[u], Bg, Uo[u], Ug, Ko[u]), Vo[u], Vg, ks, kd);
+                        Fx -= f.x;
+                        Fy -= f.y;
+                        Fz -= f.z;
+                    } else {  // F[p1] += f
+                        const float3 f = spring_force_geo(geo_disp(Bg, Bo[u], Ug, Uo[u], Ko[u]), Vg, Vo[u], ks, kd);
+                        Fx += f.x;
+                        Fy += f.y;
+                        Fz += f.z;
+                    }
                 }
             }
         }
@@ -618,7 +663,7 @@ __global__ void k_set_spring_params(const StepArgs a, const AdjArgs j, const flo
 }  // namespace
 
 cudaError_t launch_adjoint(int which, const StepArgs& a, const AdjArgs& j, int nblocks, int vpb, bool stencil,
-                           int sms, cudaStream_t stream) {
+                           cudaStream_t stream) {
     if (nblocks <= 0) return cudaSuccess;
     const int parts = (vpb + kAdjChunk - 1) / kAdjChunk;
     switch (which) {
@@ -626,14 +671,15 @@ cudaError_t launch_adjoint(int which, const StepArgs& a, const AdjArgs& j, int n
         case 1: k_adj_vertex<<<dim3(nblocks, parts), kAdjChunk, 0, stream>>>(a, j); break;
         case 2:
             // Large handles of stencil cloths alone read no records to copy, and their whole blocks
-            // make waves enough: 2 M vertices 327 us against 366, 4 M 624 against 741.  Nor does the
-            // displacement mode, with more arithmetic a spring, take chunks that just miss one wave
-            // where whole blocks make it: 24 of 64 x 64 25 us against 34.
-            if (stencil && ((int64_t)nblocks * vpb >= 1500000 ||
-                            (a.gm && nblocks * parts > 4 * sms && nblocks <= 3 * sms)))
-                k_adj_springs<2, kAdjThreads, 3, false><<<nblocks, kAdjThreads, 0, stream>>>(a, j);
-            else
-                k_adj_springs<4, kAdjChunk, 4, true><<<dim3(nblocks, std::min(parts, 3)), kAdjChunk, 0, stream>>>(a, j);
+            // make waves enough: 2 M vertices 327 us against 366, 4 M 624 against 741.
+            if (stencil && (int64_t)nblocks * vpb >= 1500000) {
+                if (a.gm) k_adj_springs<2, kAdjThreads, 2, false, true><<<nblocks, kAdjThreads, 0, stream>>>(a, j);
+                else k_adj_springs<2, kAdjThreads, 3, false, false><<<nblocks, kAdjThreads, 0, stream>>>(a, j);
+            } else {
+                const dim3 grid(nblocks, std::min(parts, 3));
+                if (a.gm) k_adj_springs<4, kAdjChunk, 4, true, true><<<grid, kAdjChunk, 0, stream>>>(a, j);
+                else k_adj_springs<4, kAdjChunk, 4, true, false><<<grid, kAdjChunk, 0, stream>>>(a, j);
+            }
             break;
         default: return cudaErrorInvalidValue;
     }
@@ -649,7 +695,10 @@ cudaError_t launch_gm(int which, const StepArgs& a, int n, cudaStream_t stream) 
         case 1: if (n > 0) k_gm_assemble<<<n, kAdjThreads, 0, stream>>>(a); break;
         case 2: if (n > 0) k_gm_update<<<n, kAdjThreads, 0, stream>>>(a); break;
         case 3: k_gm_leave<<<gs, kAdjThreads, 0, stream>>>(a, nv); break;
-        case 4: k_gm_consts<<<gs, kAdjThreads, 0, stream>>>(a, nv); break;
+        case 4:
+            k_gm_consts<<<(int)std::max<int64_t>(1, std::min<int64_t>((nv * kGmLanes + kAdjThreads - 1) / kAdjThreads, 152 * 8)),
+                          kAdjThreads, 0, stream>>>(a, nv);
+            break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

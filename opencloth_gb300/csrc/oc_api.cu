@@ -2710,7 +2710,7 @@ oc_status oc_tape_backward(oc_solver* s, const float* dL_dX, const float* dL_dV,
         AdjArgs jj = j;
         for (int k = 0; k < 3; ++k) jj.dV[k] = dv + k * st;
         if (gm) {
-            OC_TRY(launch_adjoint(0, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->sm_count, s->stream));
+            OC_TRY(launch_adjoint(0, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->stream));
         } else if (s->adj_persist) {
             OC_TRY(launch_adj_seed_own(b, jj, s->n_blocks, s->stream));
         }
@@ -2729,8 +2729,8 @@ oc_status oc_tape_backward(oc_solver* s, const float* dL_dX, const float* dL_dV,
             OC_TRY(cudaGraphExecKernelNodeSetParams(T.exec, T.n_seed, &kp));
             OC_TRY(cudaGraphLaunch(T.exec, s->stream));
         }
-        OC_TRY(launch_adjoint(1, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->sm_count, s->stream));
-        OC_TRY(launch_adjoint(2, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->sm_count, s->stream));
+        OC_TRY(launch_adjoint(1, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->stream));
+        OC_TRY(launch_adjoint(2, b, jj, s->n_blocks, s->vertices_per_block, stencil, s->stream));
         return OC_OK;
     };
     if (T.replay) {

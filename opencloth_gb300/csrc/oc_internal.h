@@ -194,7 +194,7 @@ struct AdjArgs {
 //   0 the displacement mode's seed (spring i's blocks rebuilt, adj_seed_vertex);
 //   1 the vertex terms (k_adj_vertex); 2 the spring terms (k_adj_springs).
 cudaError_t launch_adjoint(int which, const StepArgs& a, const AdjArgs& j, int nblocks, int vpb, bool stencil,
-                           int sms, cudaStream_t stream);  // vpb: vertices of a block at most; stencil: every cloth has one
+                           cudaStream_t stream);  // vpb: vertices of a block at most; stencil: every cloth has one
 
 // The replay tape of one cloth (oc_tape_forward).  The forward keeps the solution dV of
 // every step; the cloth's state (X then V, nv float4 each) is kept every `every` steps
