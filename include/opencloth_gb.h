@@ -143,9 +143,10 @@ oc_status oc_get_vertex_offsets(const oc_solver* s, int64_t* offsets /* n_instan
 
 /* State = X, V and the CG warm start dV (IMP:361, reused as the initial guess at
  * IMP:788).  Host pointers; any may be NULL to leave that array unchanged/unread.
- * Synchronous with respect to the handle's stream.  oc_set_state stages the arrays and
- * checks them on the device first: a NaN or Inf fails with OC_ERR_NON_FINITE and leaves
- * the state unchanged. */
+ * The arrays are the caller's again on return; oc_get_state waits for the handle's stream.
+ * oc_set_state stages the arrays and checks them first (on the device, or on the host for
+ * a handle of up to 16,384 vertices, which it does not wait for): a NaN or Inf fails with
+ * OC_ERR_NON_FINITE and leaves the state unchanged. */
 oc_status oc_set_state(oc_solver* s, const float* X, const float* V, const float* dV);
 oc_status oc_get_state(oc_solver* s, float* X, float* V, float* dV);
 /* Same with device pointers (packed float triples); enqueued on the handle's stream,

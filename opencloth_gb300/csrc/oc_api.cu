@@ -180,6 +180,13 @@ struct oc_solver {
     float graph_dt = 0.0f;
     int64_t host_launches = 0;  // k_assemble, k_integrate, k_resident, k_provot launches enqueued
     unsigned long long* h_loop = nullptr;
+    // Small handles (kSmallState): the host's side of oc_set_state and oc_get_state, pinned, and the
+    // event behind the last copy out of it.
+    float* h_small = nullptr;
+    int32_t* h_perr = nullptr;
+    cudaEvent_t small_ev = nullptr;
+    bool small_busy = false;
+    void* h_block = nullptr;  // the pinned block of all h_ pointers
     std::string err;
 };
 
@@ -188,6 +195,15 @@ namespace {
 // Floats between the staging planes of X, V and dV (three floats per vertex, rounded up
 // to 64 so that every plane is 256-byte aligned for the float4 check of k_state_check4).
 size_t stage_stride(int64_t nv) { return (3 * (size_t)nv + 63) / 64 * 64; }
+
+// Handles of up to this many vertices check the caller's arrays on the host and move them through
+// pinned memory of their own, one copy each way, with one wait a frame instead of four (after the
+// device's check, after the commit, behind each pageable copy out, for the error word).  Measured, us
+// of a frame of ImplicitCloth (state in, a step, state out) 21 x 21 114 -> 65, 48 x 48 139 -> 92, 100 x
+// 100 286 -> 220, 126 x 126 344 / 330, 150 x 150 423 / 405; of oc_step_host on pinned arrays 60 x 60
+// 103 -> 75, 110 x 110 125 -> 112, 126 x 126 130 / 125, but 160 x 160 140 / 159 and 220 x 220 174 / 263:
+// the host's check and copies.
+constexpr int64_t kSmallState = 16384;
 
 oc_status fail(oc_solver* s, oc_status code, const std::string& msg) {
     if (s) s->err = msg;
@@ -212,10 +228,16 @@ constexpr uint32_t kDefaultBarrierPolls = 1u << 22;
 // cleared once reported and the cloths' CG state (which the abandoned launch left part
 // updated) is zeroed: every step's assembly sets it up again, and the next launch starts
 // from zeroed arrival counts, so the handle steps on.
+oc_status report_device_error(oc_solver* s, int h);
+
 oc_status check_device_error(oc_solver* s) {
     if (!s->d_perr) return OC_OK;
     int h = 0;
     OC_TRY(cudaMemcpy(&h, s->d_perr, sizeof(int), cudaMemcpyDeviceToHost));
+    return report_device_error(s, h);
+}
+
+oc_status report_device_error(oc_solver* s, int h) {
     if (h != 0) {
         OC_TRY(cudaMemset(s->d_perr, 0, sizeof(int)));
         OC_TRY(cudaMemset(s->args.state, 0, sizeof(InstState) * (size_t)s->n_inst));
@@ -304,9 +326,8 @@ void release(oc_solver* s) {
     if (s->graph) cudaGraphDestroy(s->graph);
     for (void* p : s->allocs) cudaFree(p);
     s->allocs.clear();
-    if (s->h_state) cudaFreeHost(s->h_state);
-    if (s->h_scalar) cudaFreeHost(s->h_scalar);
-    if (s->h_loop) cudaFreeHost(s->h_loop);
+    if (s->h_block) cudaFreeHost(s->h_block);
+    if (s->small_ev) cudaEventDestroy(s->small_ev);
     if (s->tape.exec) cudaGraphExecDestroy(s->tape.exec);
     if (s->tape.graph) cudaGraphDestroy(s->tape.graph);
     for (cudaStream_t x : s->aux) cudaStreamDestroy(x);
@@ -1821,13 +1842,24 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
     OC_CREATE_TRY(dalloc(s, &a.grid_ticket, 1));
     OC_CREATE_TRY(dalloc(s, &a.loop_count, 1));
     OC_CREATE_TRY(cudaMemset(a.loop_count, 0, sizeof(unsigned long long)));
-    OC_CREATE_TRY(cudaMallocHost(&s->h_loop, sizeof(unsigned long long)));
     OC_CREATE_TRY(cudaMemset(a.unconverged, 0, sizeof(int32_t)));
     OC_CREATE_TRY(cudaMemset(a.grid_ticket, 0, sizeof(uint32_t)));
     OC_CREATE_TRY(dalloc(s, &s->stage, 3 * stage_stride(P.nv)));
     OC_CREATE_TRY(dalloc(s, &s->d_err, 1));
-    OC_CREATE_TRY(cudaMallocHost(&s->h_state, sizeof(InstState) * P.n_inst));
-    OC_CREATE_TRY(cudaMallocHost(&s->h_scalar, sizeof(int32_t)));
+    {
+        const size_t state = (sizeof(InstState) * P.n_inst + 63) / 64 * 64;
+        const size_t small = P.nv <= kSmallState ? 3 * stage_stride(P.nv) * sizeof(float) : 0;
+        OC_CREATE_TRY(cudaMallocHost(&s->h_block, 256 + state + small));
+        char* const b = static_cast<char*>(s->h_block);
+        s->h_scalar = reinterpret_cast<int32_t*>(b);
+        s->h_loop = reinterpret_cast<unsigned long long*>(b + 64);
+        s->h_perr = reinterpret_cast<int32_t*>(b + 128);
+        s->h_state = reinterpret_cast<InstState*>(b + 256);
+        if (small > 0) {
+            s->h_small = reinterpret_cast<float*>(b + 256 + state);
+            OC_CREATE_TRY(cudaEventCreateWithFlags(&s->small_ev, cudaEventDisableTiming));
+        }
+    }
     a.vpt = vpt;
     a.barrier_polls = kDefaultBarrierPolls;
     a.withhold_block = -1;
@@ -1898,11 +1930,78 @@ oc_status stage_checked(oc_solver* s, const float* X, const float* V, const floa
     return OC_OK;
 }
 
+bool all_finite(const float* p, size_t n) {
+    uint32_t bad = 0;
+    for (size_t i = 0; i < n; ++i) {
+        uint32_t b;
+        std::memcpy(&b, p + i, 4);
+        bad |= (b & 0x7f800000u) == 0x7f800000u;
+    }
+    return bad == 0;
+}
+
+// oc_set_state of a small handle.  Nothing here waits for the device but a copy out of h_small that
+// is still under way.
+oc_status set_state_small(oc_solver* s, const float* X, const float* V, const float* dV, const char* who) {
+    const size_t n3 = 3 * (size_t)s->nv, ps = stage_stride(s->nv);
+    const float* const in[3] = {X, V, dV};
+    for (const float* p : in)
+        if (p && !all_finite(p, n3))
+            return fail(s, OC_ERR_NON_FINITE, std::string(who) + ": non-finite value in the input state (nothing changed)");
+    if (s->small_busy) OC_TRY(cudaEventSynchronize(s->small_ev));
+    s->small_busy = false;
+    float* dev[3] = {nullptr, nullptr, nullptr};
+    for (int k = 0; k < 3; ++k)
+        if (in[k]) {
+            std::memcpy(s->h_small + k * ps, in[k], n3 * sizeof(float));
+            dev[k] = s->stage + k * ps;
+        }
+    for (int k = 0; k < 3; ++k) {  // neighbouring arrays in one copy
+        if (!in[k]) continue;
+        int e = k;
+        while (e < 2 && in[e + 1]) ++e;
+        OC_TRY(cudaMemcpyAsync(dev[k], s->h_small + k * ps, ((size_t)(e - k) * ps + n3) * sizeof(float),
+                               cudaMemcpyHostToDevice, s->stream));
+        k = e;
+    }
+    OC_TRY(cudaEventRecord(s->small_ev, s->stream));
+    s->small_busy = true;
+    OC_TRY(cudaMemsetAsync(s->d_err, 0, sizeof(int32_t), s->stream));
+    OC_TRY(launch_state_in(s->args, dev[0], dev[1], dev[2], s->nv, s->d_err, s->stream));
+    return OC_OK;
+}
+
+// oc_get_state of a small handle: one copy, one wait.
+oc_status get_state_small(oc_solver* s, float* X, float* V, float* dV) {
+    const size_t n3 = 3 * (size_t)s->nv, ps = stage_stride(s->nv);
+    float* const out[3] = {X, V, dV};
+    float* dev[3] = {nullptr, nullptr, nullptr};
+    int first = 3, last = -1;
+    for (int k = 0; k < 3; ++k)
+        if (out[k]) {
+            dev[k] = s->stage + k * ps;
+            first = std::min(first, k);
+            last = k;
+        }
+    OC_TRY(launch_state_out(s->args, dev[0], dev[1], dev[2], s->nv, s->stream));
+    if (last >= 0)
+        OC_TRY(cudaMemcpyAsync(s->h_small + first * ps, s->stage + first * ps, ((size_t)(last - first) * ps + n3) * sizeof(float),
+                               cudaMemcpyDeviceToHost, s->stream));
+    *s->h_perr = 0;
+    if (s->d_perr) OC_TRY(cudaMemcpyAsync(s->h_perr, s->d_perr, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    OC_TRY(cudaStreamSynchronize(s->stream));
+    s->small_busy = false;
+    for (int k = 0; k < 3; ++k)
+        if (out[k]) std::memcpy(out[k], s->h_small + k * ps, n3 * sizeof(float));
+    return report_device_error(s, *s->h_perr);
+}
+
 }  // namespace
 
 oc_status oc_set_state(oc_solver* s, const float* X, const float* V, const float* dV) {
     if (!valid_solver(s)) return OC_ERR_INVALID_ARGUMENT;
     OC_TRY(cudaSetDevice(s->device));
+    if (s->h_small) return set_state_small(s, X, V, dV, "oc_set_state");
     float *sx, *sv, *sd;
     if (oc_status st = stage_checked(s, X, V, dV, &sx, &sv, &sd, "oc_set_state")) return st;
     OC_TRY(launch_state_in(s->args, sx, sv, sd, s->nv, s->d_err, s->stream));
@@ -1913,6 +2012,7 @@ oc_status oc_set_state(oc_solver* s, const float* X, const float* V, const float
 oc_status oc_get_state(oc_solver* s, float* X, float* V, float* dV) {
     if (!valid_solver(s)) return OC_ERR_INVALID_ARGUMENT;
     OC_TRY(cudaSetDevice(s->device));
+    if (s->h_small) return get_state_small(s, X, V, dV);
     const size_t n3 = 3 * (size_t)s->nv;
     const size_t ps = stage_stride(s->nv);
     float* sx = X ? s->stage : nullptr;
@@ -1929,6 +2029,12 @@ oc_status oc_get_state(oc_solver* s, float* X, float* V, float* dV) {
 oc_status oc_step_host(oc_solver* s, float dt, int32_t n_steps, float* X, float* V) {
     if (!valid_solver(s) || n_steps < 0 || !std::isfinite(dt)) return OC_ERR_INVALID_ARGUMENT;
     OC_TRY(cudaSetDevice(s->device));
+    if (s->h_small) {
+        if (X || V)
+            if (oc_status st = set_state_small(s, X, V, nullptr, "oc_step_host")) return st;
+        if (oc_status st = oc_step(s, dt, n_steps)) return st;
+        return get_state_small(s, X, V, nullptr);
+    }
     const size_t n3 = 3 * (size_t)s->nv;
     // The input is staged and checked before anything is committed: a NaN or Inf leaves
     // the device state and the caller's arrays as they were.
