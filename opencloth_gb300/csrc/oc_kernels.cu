@@ -963,6 +963,48 @@ __global__ void k_state_out(const StepArgs a, float* X3, float* V3, float* dV3, 
     }
 }
 
+// k_state_out for 16-byte aligned arrays: a CTA turns 256 vertices' components into triples in
+// shared memory and stores them as float4 (three stores 12 bytes apart write each sector three
+// times): 3.06 M vertices 52.6 -> 36.5 us, 80 bytes a vertex at the copy rate.  (The same way in is no
+// faster: k_state_in moves 112 bytes a vertex at that rate already.)
+__global__ void __launch_bounds__(kThreads) k_state_out4(const StepArgs a, float* X3, float* V3, float* dV3, int64_t nv) {
+    __shared__ __align__(16) float tri[3][3 * kThreads];
+    const int t = threadIdx.x;
+    for (int64_t base = blockIdx.x * (int64_t)kThreads; base < nv; base += (int64_t)gridDim.x * kThreads) {
+        const int64_t g = base + t;
+        const int n = (int)min((int64_t)kThreads, nv - base);
+        if (t < n) {
+            if (X3) {
+                const float4 v = a.X[g];
+                tri[0][3 * t] = v.x;
+                tri[0][3 * t + 1] = v.y;
+                tri[0][3 * t + 2] = v.z;
+            }
+            if (V3) {
+                const float4 v = a.V[g];
+                tri[1][3 * t] = v.x;
+                tri[1][3 * t + 1] = v.y;
+                tri[1][3 * t + 2] = v.z;
+            }
+            if (dV3) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) tri[2][3 * t + k] = a.x[k][g];
+            }
+        }
+        __syncthreads();
+        float* const out[3] = {X3, V3, dV3};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            if (!out[q]) continue;
+            float* const p = out[q] + 3 * base;
+            for (int i = t; i < 3 * n / 4; i += kThreads)
+                reinterpret_cast<float4*>(p)[i] = reinterpret_cast<const float4*>(tri[q])[i];
+            for (int i = 3 * n / 4 * 4 + t; i < 3 * n; i += kThreads) p[i] = tri[q][i];
+        }
+        __syncthreads();
+    }
+}
+
 // k_state_check for 16-byte aligned arrays: float4 loads, the same finiteness test.
 __device__ __forceinline__ bool finite4(const float4 v) {
     return isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w);
@@ -1133,7 +1175,10 @@ cudaError_t launch_state_check(const float* X3, const float* V3, const float* dV
 }
 
 cudaError_t launch_state_out(const StepArgs& a, float* X3, float* V3, float* dV3, int64_t nv, cudaStream_t stream) {
-    k_state_out<<<state_blocks(nv), kThreads, 0, stream>>>(a, X3, V3, dV3, nv);
+    if (aligned16(X3) && aligned16(V3) && aligned16(dV3))
+        k_state_out4<<<state_blocks(nv), kThreads, 0, stream>>>(a, X3, V3, dV3, nv);
+    else
+        k_state_out<<<state_blocks(nv), kThreads, 0, stream>>>(a, X3, V3, dV3, nv);
     return cudaGetLastError();
 }
 

@@ -63,3 +63,27 @@ def test_step_host(shape):
         for x, y in zip(s.get_state(), t.get_state()):
             assert np.array_equal(x, y)
         assert np.array_equal(b, t.get_state()[1])
+
+
+@pytest.mark.parametrize("n", [9, 255, 256, 257, 1023, 40000])
+@pytest.mark.parametrize("offset", [0, 1, 4])
+def test_state_out_to_device_arrays(n, offset):
+    """k_state_out4 (16-byte aligned arrays) and k_state_out, in whole blocks and remainders, with
+    nothing written beyond the arrays."""
+    torch = pytest.importorskip("torch")
+    _, sp = grid_cloth(3, 3)
+    rng = np.random.default_rng(n)
+    A = [rng.normal(0, 1, (n, 3)).astype(np.float32) for _ in range(3)]
+    with ClothSolver(ClothDesc(n_vertices=n, springs=sp)) as s:
+        s.set_state(*A)
+        for given in ((0, 1, 2), (0,), (1, 2), (2,)):
+            out = [torch.full((3 * n + 16,), 7.0, device="cuda") for _ in range(3)]
+            torch.cuda.synchronize()
+            s.get_state_device(*(out[k].data_ptr() + 4 * offset if k in given else 0 for k in range(3)))
+            s.synchronize()
+            for k in range(3):
+                o = out[k].cpu().numpy()
+                want = np.full(3 * n + 16, 7.0, np.float32)
+                if k in given:
+                    want[offset:offset + 3 * n] = A[k].ravel()
+                assert np.array_equal(o, want)
