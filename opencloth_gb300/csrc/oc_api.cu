@@ -644,41 +644,38 @@ oc_status build_graph(oc_solver* s, float dt) {
         return kp;
     };
 
-    cudaGraphNode_t n_reset, n_asm;
-    cudaMemsetParams mp{};
-    mp.dst = a.unconverged;
-    mp.value = 0;
-    mp.elementSize = sizeof(int32_t);
-    mp.width = 1;
-    mp.height = 1;
-    mp.pitch = sizeof(int32_t);
-    OC_TRY(cudaGraphAddMemsetNode(&n_reset, g, nullptr, 0, &mp));
+    // The WHILE loop's counter of cloths that still iterate, which the assemblies raise: set to zero
+    // first (nothing reads it where there is no loop; the memset and the wait for it are 2 us a step).
+    std::vector<cudaGraphNode_t> reset, prev;  // what the next node waits for
+    if (loop) {
+        cudaGraphNode_t n;
+        cudaMemsetParams mp{};
+        mp.dst = a.unconverged;
+        mp.value = 0;
+        mp.elementSize = sizeof(int32_t);
+        mp.width = 1;
+        mp.height = 1;
+        mp.pitch = sizeof(int32_t);
+        OC_TRY(cudaGraphAddMemsetNode(&n, g, nullptr, 0, &mp));
+        reset = prev = {n};
+    }
     cudaKernelNodeParams kp{};
-    n_asm = n_reset;
-    if (s->n_asm_blocks > 0) {
-        kp = kparams(K_ASSEMBLE, T_ASM);
-        OC_TRY(cudaGraphAddKernelNode(&n_asm, g, &n_reset, 1, &kp));
-    }
-    if (s->n_grid_blocks > 0) {  // serialised after k_assemble: both end in the same counters
-        cudaGraphNode_t prev = n_asm;
-        kp = kparams(s->grid_kind, T_GRID);
-        OC_TRY(cudaGraphAddKernelNode(&n_asm, g, &prev, 1, &kp));
-    }
+    // The assemblies one after the other: they end in the same counters.
+    auto add = [&](KernelKind k, Table tab) -> cudaError_t {
+        cudaGraphNode_t n;
+        kp = kparams(k, tab);
+        const cudaError_t e = cudaGraphAddKernelNode(&n, g, prev.data(), prev.size(), &kp);
+        prev = {n};
+        return e;
+    };
+    if (s->n_asm_blocks > 0) OC_TRY(add(K_ASSEMBLE, T_ASM));
+    if (s->n_grid_blocks > 0) OC_TRY(add(s->grid_kind, T_GRID));
     if (s->args.n_strip_work > 0) {  // the strip sweep, then its cloths' delta0 totals
-        cudaGraphNode_t prev = n_asm;
-        kp = kparams(K_ASSEMBLE_STRIP, T_STRIP);
-        OC_TRY(cudaGraphAddKernelNode(&n_asm, g, &prev, 1, &kp));
-        if (s->strip_finish) {
-            prev = n_asm;
-            kp = kparams(K_ASSEMBLE_FINISH, T_SFIN);
-            OC_TRY(cudaGraphAddKernelNode(&n_asm, g, &prev, 1, &kp));
-        }
+        OC_TRY(add(K_ASSEMBLE_STRIP, T_STRIP));
+        if (s->strip_finish) OC_TRY(add(K_ASSEMBLE_FINISH, T_SFIN));
     }
-    cudaGraphNode_t n_last = n_asm;  // the loop waits for every assembly
-    if (coupled) {
-        kp = kparams(K_CPL_ASSEMBLE, T_CPL);
-        OC_TRY(cudaGraphAddKernelNode(&n_last, g, &n_asm, 1, &kp));
-    }
+    const std::vector<cudaGraphNode_t> assembled = prev;
+    if (coupled) OC_TRY(add(K_CPL_ASSEMBLE, T_CPL));  // the loop waits for every assembly
     std::vector<cudaGraphNode_t> updates;  // the nodes that write X and V
 
     if (loop) {
@@ -688,16 +685,16 @@ oc_status build_graph(oc_solver* s, float dt) {
         cp.conditional.handle = handle;
         cp.conditional.type = cudaGraphCondTypeWhile;
         cp.conditional.size = 1;
-        OC_TRY(cudaGraphAddNode(&n_loop, g, &n_last, nullptr, 1, &cp));
+        OC_TRY(cudaGraphAddNode(&n_loop, g, prev.data(), nullptr, prev.size(), &cp));
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         // Body: the REFERENCE pair, then the COUPLED pair; the last update kernel's last
         // block sets the condition from the counter both loops decrement.
-        cudaGraphNode_t prev = nullptr;
+        cudaGraphNode_t last = nullptr;
         auto add_body = [&](KernelKind k, Table tab) -> cudaError_t {
             cudaKernelNodeParams bp = kparams(k, tab);
             cudaGraphNode_t n;
-            cudaError_t e = cudaGraphAddKernelNode(&n, body, prev ? &prev : nullptr, prev ? 1 : 0, &bp);
-            prev = n;
+            cudaError_t e = cudaGraphAddKernelNode(&n, body, last ? &last : nullptr, last ? 1 : 0, &bp);
+            last = n;
             return e;
         };
         if (streamed) {
@@ -729,7 +726,7 @@ oc_status build_graph(oc_solver* s, float dt) {
             if (pg) cudaGraphDestroy(pg);
             return fail_cuda(s, le != cudaSuccess ? le : ce, persist ? "capture of k_cg_persist" : "capture of k_cpl_persist");
         }
-        cudaError_t e = cudaGraphAddChildGraphNode(&n_pc, g, &n_last, 1, pg);
+        cudaError_t e = cudaGraphAddChildGraphNode(&n_pc, g, prev.data(), prev.size(), pg);
         cudaGraphDestroy(pg);
         if (e != cudaSuccess) return fail_cuda(s, e, "cudaGraphAddChildGraphNode");
         updates.push_back(n_pc);
@@ -752,7 +749,8 @@ oc_status build_graph(oc_solver* s, float dt) {
         }
         if (ce != cudaSuccess) return fail_cuda(s, ce, "cudaStreamEndCapture");
         cudaGraphNode_t n_res;
-        cudaError_t e = cudaGraphAddChildGraphNode(&n_res, g, s->resident_fused ? &n_reset : &n_asm, 1, rg);
+        const std::vector<cudaGraphNode_t>& after = s->resident_fused ? reset : assembled;
+        cudaError_t e = cudaGraphAddChildGraphNode(&n_res, g, after.data(), after.size(), rg);
         cudaGraphDestroy(rg);
         if (e != cudaSuccess) return fail_cuda(s, e, "cudaGraphAddChildGraphNode");
         updates.push_back(n_res);
