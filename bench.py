@@ -675,9 +675,9 @@ def measure_fem(name: str, seed: int, local: int, solves: int) -> dict:
     prof = s.profile(2)
     peaks_path = ROOT / "MEASURED_PEAKS.json"
     peak = float(json.loads(peaks_path.read_text())["hbm_gbs"]) if peaks_path.exists() else 6800.0
-    # The dominant kernel: the streamed matrix-vector pass, or the resident CG when every
+    # The dominant kernel: the streamed systems' one launch (or their matrix-vector pass), or the resident CG when every
     # system runs on chip (the demo's 176-row bodies).
-    kname = max(("k_bsr_spmv", "k_bsr_resident"), key=lambda k: prof.get(k, {"ms_total": 0.0})["ms_total"])
+    kname = max(("k_bsr_persist", "k_bsr_spmv", "k_bsr_resident"), key=lambda k: prof.get(k, {"ms_total": 0.0})["ms_total"])
     dom = prof[kname]
     achieved = dom["bytes"] / (dom["ms_total"] / 1e3) / 1e9 if dom["ms_total"] > 0 else 0.0
     roof = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak, "unit": "GB/s",

@@ -914,6 +914,7 @@ struct oc_bsr_solver {
     int32_t* d_perm = nullptr;
     int* d_flag = nullptr;
     int* h_flag = nullptr;
+    double persist_bytes = 0.0;  // algorithmic bytes of k_bsr_persist
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int64_t launches = 0;
@@ -1024,7 +1025,10 @@ oc_status plan_bsr_persist(oc_bsr_solver* s, const std::vector<BsrParams>& sys) 
     }
     std::vector<BsrPiece> pieces;
     int32_t packets = 0;
+    s->persist_bytes = 0.0;
     for (int32_t k : ids) {
+        const double rows = (double)sys[k].n_rows, blocks = (double)(s->nnz_off[k + 1] - s->nnz_off[k]);
+        s->persist_bytes += 40.0 * blocks + 61.0 * rows + sys[k].imax * (40.0 * blocks + 162.0 * rows);
         const int64_t n = sys[k].n_rows, c = (n + chunk - 1) / chunk, each = ((n + c - 1) / c + 31) / 32 * 32;
         const size_t p0 = pieces.size();
         for (int64_t r = 0; r < n; r += each) {
@@ -1548,12 +1552,14 @@ oc_status oc_bsr_profile(oc_bsr_solver* s, int32_t n_solves, int32_t max_kernels
     // and out, r and p out): its iterations stay on chip.
     const double nb = (double)s->st_nnzb, nr = (double)s->st_rows;
     const double rb = (double)s->res_nnzb, rr = (double)s->res_rows;
-    constexpr int K = 5;
-    const char* kname[K] = {"k_bsr_pack", "k_bsr_init", "k_bsr_spmv", "k_bsr_update", "k_bsr_resident"};
+    // k_bsr_persist: its systems' init and passes.
+    constexpr int K = 6;
+    const char* kname[K] = {"k_bsr_pack", "k_bsr_init", "k_bsr_spmv", "k_bsr_update", "k_bsr_resident", "k_bsr_persist"};
+    const bool persist = s->use_graph && s->plan.grid > 0;
     const double kbytes[K] = {72.0 * nb + 8.0 * nr, 40.0 * nb + 61.0 * nr, 40.0 * nb + 53.0 * nr, 109.0 * nr,
-                              40.0 * rb + 85.0 * rr};
-    double ms[K] = {0, 0, 0, 0, 0};
-    int64_t cnt[K] = {0, 0, 0, 0, 0};
+                              40.0 * rb + 85.0 * rr, s->persist_bytes};
+    double ms[K] = {0, 0, 0, 0, 0, 0};
+    int64_t cnt[K] = {0, 0, 0, 0, 0, 0};
     cudaEvent_t e0, e1;
     BSR_TRY(cudaEventCreate(&e0));
     BSR_TRY(cudaEventCreate(&e1));
@@ -1566,8 +1572,10 @@ oc_status oc_bsr_profile(oc_bsr_solver* s, int32_t n_solves, int32_t max_kernels
         cudaError_t x = cudaEventRecord(e0, s->stream);
         if (k < 4)
             launch(kfn[k], a, s->n_blocks, s->stream);
-        else
+        else if (k == 4)
             launch_resident(s, a);
+        else if (x == cudaSuccess)
+            x = launch_bsr_persist(s);
         if (x == cudaSuccess) x = cudaGetLastError();
         if (x == cudaSuccess) x = cudaEventRecord(e1, s->stream);
         if (x == cudaSuccess) x = cudaEventSynchronize(e1);
@@ -1582,6 +1590,10 @@ oc_status oc_bsr_profile(oc_bsr_solver* s, int32_t n_solves, int32_t max_kernels
         if (s->n_blocks == 0) continue;
         if (e == cudaSuccess) e = cudaMemsetAsync(a.unfinished, 0, sizeof(int32_t), s->stream);
         if (e == cudaSuccess) e = timed(0);
+        if (persist) {
+            if (e == cudaSuccess) e = timed(5);
+            continue;
+        }
         if (e == cudaSuccess) e = timed(1);
         for (;;) {
             if (e == cudaSuccess) e = cudaMemcpyAsync(h, a.unfinished, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream);
