@@ -65,6 +65,16 @@ constexpr int kFullSlots = 7;  // the largest piece held in registers with x, X 
 constexpr int kSlotFloats = 12;  // A, r, d of a slot in shared memory
 constexpr int kMaxCluster = kPersistMaxCluster;
 
+// Whether the launch has the plan's clusters: without them a packet would go to a CTA that does not
+// exist, which is a fault, so a launch that lost them (a tool's own replay) sets the error word instead.
+__device__ __forceinline__ bool clusters_as_planned(const PersistPlan& P) {
+    uint32_t n;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+    if (n == (uint32_t)P.cluster) return true;
+    if (threadIdx.x == 0) atomicOr(P.err, 1);
+    return false;
+}
+
 // Shared memory of a piece: its warps' packets by parity (a piece that shares no cluster with
 // another CTA), and the scalars of its cloth.
 struct PieceState {
@@ -127,6 +137,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
     __shared__ __align__(16) ulonglong2 s_box[2][2][kMaxCluster * kWarps];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int CS = P.cluster, rank = (int)blockIdx.x % CS;
+    if (!clusters_as_planned(P)) return;
     const int pc0 = P.cta_piece[blockIdx.x], np = P.cta_piece[blockIdx.x + 1] - pc0;
     const PersistPiece* __restrict__ pieces = P.pieces + pc0;
     PieceState* const st = reinterpret_cast<PieceState*>(smem_raw);
@@ -527,6 +538,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
     __shared__ __align__(16) ulonglong2 s_box[2][kMaxCluster * kWarps];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int CS = P.cluster, rank = (int)blockIdx.x % CS;
+    if (!clusters_as_planned(P)) return;
     const PersistPiece pc = P.pieces[blockIdx.x];
     const uint32_t base = *(volatile uint32_t*)&P.ctl->base;
     float* const sm = reinterpret_cast<float*>(smem_raw) + tid;
