@@ -1075,7 +1075,7 @@ oc_status plan_sim(oc_solver* s) {
             L.cluster = c;
             L.threads = sizes[i][0];
             L.vpt = sizes[i][1];
-            L.window = std::max(L.window, std::min(ip.nv, chunk + 4 * std::max(0, ip.grid_cols)));
+            L.window = std::max(L.window, std::min(ip.nv, chunk + (ip.grid_cols > 0 ? 2 * ip.st_reach : 0)));
             if (ip.grid_cols > 0) {
                 const int32_t* st = s->h_st_data.data() + ip.st_off;
                 L.entries = std::max(L.entries, st[kStencilClasses] - kStencilClasses - 1);

@@ -31,6 +31,8 @@ struct InstParams {
     int32_t st_off;     // its class table and entries in StepArgs::st_data
     int32_t st_par;     // its first parameter slot in StepArgs::st_param
     int32_t st_rest;    // 1: rest lengths vary; read them per incidence from StepArgs::rest_inc
+    int32_t st_reach;   // the farthest neighbour of its stencil: |di cols + dj| at most (2 cols + 2 where a
+                        // spring goes two rows and two columns)
     // The strip sweep (k_assemble_strip), for grid cloths whose incidences follow the
     // reference's spring order: strip_slot is the cloth's first word in StepArgs::strip_slot
     // (36 words, one per anchor position class, six 4-bit parameter slots each: H, bR, V,

@@ -5,8 +5,8 @@
 // One cluster of up to 16 CTAs of 256 threads per cloth; a thread owns VPT vertices.  Every
 // vertex's system and CG state live in registers (with VPT > 1 they pass through shared memory
 // between the assembly's loop and the CG's), the warm start across steps too, and the CTA's
-// window of positions and velocities (its own vertices and, of a grid cloth, the 2 cols vertices
-// on either side that its stencils reach) in shared memory: a step reads global memory only for
+// window of positions and velocities (its own vertices and, of a grid cloth, those on either side
+// that its stencil reaches: 2 cols in the reference's order) in shared memory: a step reads global memory only for
 // the window's halo, which the neighbouring CTAs wrote at the end of the step before, and for the
 // springs' constants, which stay in L1.  Neighbours outside the window (a general mesh on more
 // than one CTA) are read through L2.
@@ -61,7 +61,8 @@ __device__ __forceinline__ void window_at(const StepArgs& a, const InstParams& i
 }
 
 // A grid cloth's stencil in shared memory: the first entry of each class, and per entry the
-// neighbour's offset, the side (sign bit set: the vertex is the spring's p2) and the parameters.
+// neighbour's offset, the side and the parameters.  The window's halo is the stencil's own reach, so
+// its neighbours are indexed without a test.
 struct Stencil {
     const int32_t* first;  // kStencilClasses + 1
     const float4* entry;   // {offset << 1 | is_p2, rest, ks, kd}
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
     const InstParams& ip = a.inst[inst];
     const int nv = ip.nv, chunk = (nv + C - 1) / C;
     const int lb = rank * chunk, n = max(0, min(nv, lb + chunk) - lb);
-    const int halo = ip.grid_cols > 0 ? 2 * ip.grid_cols : 0;
+    const int halo = ip.grid_cols > 0 ? ip.st_reach : 0;
     const int wlo = max(0, lb - halo), whi = n > 0 ? min(nv, lb + n + halo) : wlo;
     float4* const wX = reinterpret_cast<float4*>(smem_raw);
     float4* const wV = wX + L.window;

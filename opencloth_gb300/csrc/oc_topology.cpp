@@ -3,6 +3,7 @@
 // incidence (CSR) ordered by spring id.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <limits>
 
@@ -237,7 +238,7 @@ oc_status pack_instances(const oc_cloth_desc* descs, int32_t n, int32_t vpb, Pac
         InstParams& ip = P.inst[k];
         ip.grid_cols = ip.grid_rows = 0;
         ip.st_off = ip.st_par = -1;
-        ip.st_rest = 0;
+        ip.st_rest = ip.st_reach = 0;
         const int64_t vo = P.v_off[k];
         const int32_t nvk = ip.nv;
         if (nvk < 9) continue;
@@ -315,6 +316,9 @@ oc_status pack_instances(const oc_cloth_desc* descs, int32_t n, int32_t vpb, Pac
         }
         P.st_data.push_back(pos);
         for (int cl = 0; cl < kStencilClasses; ++cl) P.st_data.insert(P.st_data.end(), tmpl[cl].begin(), tmpl[cl].end());
+        for (const std::vector<int32_t>& entries : tmpl)
+            for (int32_t v : entries)
+                ip.st_reach = std::max(ip.st_reach, std::abs(((v & 7) - 2) * cols + (((v >> 3) & 7) - 2)));
         ip.st_par = (int32_t)P.st_param.size();
         for (int q = 0; q < kStencilSlots; ++q) {
             float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
