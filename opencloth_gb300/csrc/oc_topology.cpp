@@ -466,24 +466,29 @@ void build_strip_tables(PackedHost* Pp) {
             P.strip_slot.push_back(w);
         }
         std::array<uint16_t, 6>& masks = P.kind_slots[(size_t)k];
-        bool several = false;  // a kind with several slots: equal but for the rest lengths, if ip.kinds
+        const float4* par = P.st_param.data() + ip.st_par;
+        bool rests = false;  // a kind whose slots differ in their rest lengths
         for (int kind = 0; kind < 6; ++kind) {
-            for (int x : slot[kind])
-                if (x >= 0) masks[kind] |= (uint16_t)(1u << x);
-            several = several || (masks[kind] & (masks[kind] - 1));
+            int first = -1;
+            for (int x : slot[kind]) {
+                if (x < 0) continue;
+                masks[kind] |= (uint16_t)(1u << x);
+                if (first < 0) first = x;
+                rests = rests || std::memcmp(&par[x].x, &par[first].x, sizeof(float)) != 0;
+            }
         }
-        set_kinds(&ip, masks, P.st_param.data() + ip.st_par);
+        set_kinds(&ip, masks, par);
         if (ip.st_rest) {
             ip.strip_rest = (int64_t)P.strip_rest.size();
             const size_t base = P.strip_rest.size();
             P.strip_rest.resize(base + rest_bits.size());
             std::memcpy(P.strip_rest.data() + base, rest_bits.data(), rest_bits.size() * sizeof(float));
             ip.kind_rest = ip.strip_rest;
-        } else if (several && ip.kinds && cols <= kKindsMaxCols) {
-            // (The sweep takes these rest lengths from the slots.)
+        } else if (rests && cols <= kKindsMaxCols) {
+            // (The sweep takes these rest lengths from the slots.)  Whether or not the cloth is of
+            // kinds now: new Ks and Kd may make it so, the rest lengths stay.
             ip.kind_rest = (int64_t)P.strip_rest.size();
             P.strip_rest.resize(P.strip_rest.size() + 6 * (size_t)nvk, 0.0f);
-            const float4* par = P.st_param.data() + ip.st_par;
             for (int kind = 0; kind < 6; ++kind)
                 for (int32_t l = 0; l < nvk; ++l) {
                     const int sl = slot[kind][stencil_class_1d(l / cols, rows) * 6 + stencil_class_1d(l % cols, cols)];
