@@ -347,6 +347,9 @@ oc_status oc_tune_cache_store(const char* path, const char* key, const oc_launch
  * waits longer than that bound.  Fails with OC_ERR_UNSUPPORTED when the handle runs no
  * persistent CG. */
 oc_status oc_test_barrier_timeout(oc_solver* s, int32_t withhold_block, uint32_t max_polls);
+/* For tests of a handle's age: the tags of the packets by which its CG launches exchange sums run on
+ * from launch to launch in 32 bits; the next ones continue after `last`. */
+oc_status oc_test_packet_tags(oc_solver* s, uint32_t last);
 
 /* No counterpart in the reference.  For tests: the step computes spring lengths, their
  * reciprocals, the quotients of ComputeForces / CalcForceDerivatives (IMP:720-727) and the

@@ -1221,11 +1221,9 @@ oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_
     OC_TRY(put(&P.cta_piece, cta_piece));
     dfree(s, &P.packets);
     OC_TRY(dalloc(s, &P.packets, 2 * (size_t)P.n_packets));
-    OC_TRY(cudaMemset(P.packets, 0, std::max<size_t>(1, 2 * (size_t)P.n_packets) * sizeof(ulonglong2)));
-    if (!P.ctl) {
-        OC_TRY(dalloc(s, &P.ctl, 1));
-        OC_TRY(cudaMemset(P.ctl, 0, sizeof(PersistCtl)));
-    }
+    OC_TRY(cudaMemsetAsync(P.packets, 0, std::max<size_t>(1, 2 * (size_t)P.n_packets) * sizeof(ulonglong2), s->stream));
+    if (!P.ctl) OC_TRY(dalloc(s, &P.ctl, 1));
+    OC_TRY(cudaMemsetAsync(P.ctl, 0, sizeof(PersistCtl), s->stream));  // cleared packets have the tag 0, the next launch's begin at 1
     if (oc_status r = alloc_error_word(s)) return r;
     P.err = s->d_perr;
     P.grid = (int32_t)cta_piece.size() - 1;
@@ -1284,11 +1282,9 @@ oc_status plan_coupled(oc_solver* s) {
     P.pieces = d;
     dfree(s, &P.packets);
     OC_TRY(dalloc(s, &P.packets, 2 * (size_t)P.n_packets));
-    OC_TRY(cudaMemset(P.packets, 0, 2 * (size_t)P.n_packets * sizeof(ulonglong2)));
-    if (!P.ctl) {
-        OC_TRY(dalloc(s, &P.ctl, 1));
-        OC_TRY(cudaMemset(P.ctl, 0, sizeof(PersistCtl)));
-    }
+    OC_TRY(cudaMemsetAsync(P.packets, 0, 2 * (size_t)P.n_packets * sizeof(ulonglong2), s->stream));
+    if (!P.ctl) OC_TRY(dalloc(s, &P.ctl, 1));
+    OC_TRY(cudaMemsetAsync(P.ctl, 0, sizeof(PersistCtl), s->stream));  // (as in plan_persist)
     if (oc_status r = alloc_error_word(s)) return r;
     P.err = s->d_perr;
     P.grid = (int32_t)pieces.size();
@@ -3168,6 +3164,16 @@ oc_status oc_autotune(oc_solver* s, float dt, const char* cache_path, int32_t fl
     if (chosen) *chosen = best;
     if (ms_per_step) *ms_per_step = t_best;
     return cleanup(st);
+}
+
+oc_status oc_test_packet_tags(oc_solver* s, uint32_t last) {
+    if (!valid_solver(s)) return OC_ERR_INVALID_ARGUMENT;
+    OC_TRY(cudaSetDevice(s->device));
+    OC_TRY(cudaStreamSynchronize(s->stream));
+    for (PersistCtl* c : {s->pplan.ctl, s->aplan.ctl, s->cplan.ctl})
+        if (c) OC_TRY(cudaMemcpyAsync(&c->base, &last, sizeof(last), cudaMemcpyHostToDevice, s->stream));
+    OC_TRY(cudaStreamSynchronize(s->stream));
+    return OC_OK;
 }
 
 oc_status oc_test_barrier_timeout(oc_solver* s, int32_t withhold_block, uint32_t max_polls) {

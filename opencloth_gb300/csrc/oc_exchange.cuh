@@ -25,6 +25,12 @@ __device__ __forceinline__ unsigned long long word_of(float v, uint32_t tag) {
     return (unsigned long long)tag << 32 | __float_as_uint(v);
 }
 
+// What a box holds before its first packet in a launch whose tags are base + 1, base + 2, ...
+__device__ __forceinline__ ulonglong2 empty_packet(uint32_t base) {
+    const unsigned long long w = word_of(0.0f, base);
+    return make_ulonglong2(w, w);
+}
+
 __device__ __forceinline__ void put_global(ulonglong2* p, Acc v, uint32_t tag) {
     asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(word_of(v.s, tag)), "l"(word_of(v.c, tag))
                  : "memory");

@@ -28,7 +28,9 @@
 // Packets are double buffered by the phase's parity: a CTA writes phase q + 1's only after it
 // has read all of phase q's, which its cloths' CTAs write after reading all of phase q - 1's.
 // Tags run on from launch to launch (PersistCtl::base; the last CTA to leave moves it past the
-// tags that were used), so nothing has to be cleared between launches.
+// tags that were used), so the packets in memory are never cleared between launches.  They wrap after
+// 2^32, some hours of stepping: a launch's own boxes therefore start with the tag `base`, the one
+// that none of its phases has, and not with a fixed one.
 //
 // Measured (time of the launch, a wave of arrival counts over memory-resident planes before):
 // 257 x 257 cloth, 4 iterations, 51 -> 20 us; 120,000-vertex mesh, 22 iterations, 317 -> 92 us;
@@ -147,13 +149,14 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
     const uint32_t base = *(volatile uint32_t*)&P.ctl->base;
 
     if (tid == 0) s_ok = 1;
-    for (int i = tid; i < 2 * 2 * kMaxCluster * kWarps; i += kPT) (&s_box[0][0][0])[i] = make_ulonglong2(0, 0);
+    const ulonglong2 none = empty_packet(base);
+    for (int i = tid; i < 2 * 2 * kMaxCluster * kWarps; i += kPT) (&s_box[0][0][0])[i] = none;
     for (int j = tid; j < np; j += kPT) {
         const InstState& is = a.state[pieces[j].inst];
         const InstParams& ip = a.inst[pieces[j].inst];
         const double d0 = __ldcg(&is.delta0);
 #pragma unroll
-        for (int i = 0; i < kWarps; ++i) st[j].box[0][i] = st[j].box[1][i] = make_ulonglong2(0, 0);
+        for (int i = 0; i < kWarps; ++i) st[j].box[0][i] = st[j].box[1][i] = none;
         st[j].d0 = d0;
         st[j].dn = pair_from(__ldcg(&is.delta_new));
         st[j].thresh = pair_from((double)ip.eps2 * d0);
@@ -549,7 +552,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
     const bool upd = !a.cg_only;
 
     if (tid == 0) s_ok = 1;
-    for (int i = tid; i < 2 * kMaxCluster * kWarps; i += kPT) (&s_box[0][0])[i] = make_ulonglong2(0, 0);
+    for (int i = tid; i < 2 * kMaxCluster * kWarps; i += kPT) (&s_box[0][0])[i] = empty_packet(base);
     if (CS > 1) cluster_arrive();
     float A[KR][6], r[KR][3], d[KR][3];
     float x[FULL ? KR : 1][3];
