@@ -335,17 +335,16 @@ oc_status oc_tune_key_of(const oc_solver* s, char* key, int32_t key_size);
 oc_status oc_tune_cache_lookup(const char* path, const char* key, oc_launch_config* cfg, int32_t* found);
 oc_status oc_tune_cache_store(const char* path, const char* key, const oc_launch_config* cfg, double ms_per_step);
 
-/* ---- testing aid: the bounded waits of the persistent CG -------------------------- */
-/* The persistent CG (one cooperative launch per step for the streamed cloths, and for
- * the adjoint solves) waits, before each pass over a cloth's vertices, for that cloth's
- * previous pass to complete on every block; each wait gives up after a bounded number of
- * polls and the step then fails with OC_ERR_DEVICE_TIMEOUT at the next oc_synchronize /
- * oc_get_state / oc_get_stats, after which the handle steps on (a cloth whose solve had
- * not ended got no update).  For tests of that path: from the next step on, block
- * `withhold_block` of those launches returns before its first arrival (-1: none), and a
- * wait gives up after `max_polls` polls (0: the default, about a second).  Nothing
- * waits longer than that bound.  Fails with OC_ERR_UNSUPPORTED when the handle runs no
- * persistent CG. */
+/* ---- testing aid: the bounded waits ------------------------------------------------- */
+/* The CTAs of a CG launch (k_cg_persist, k_cpl_persist, k_sim) wait for one another's partial sums.
+ * Each wait gives up after a bounded number of polls, or when another wait of the handle has given
+ * up; the step then fails with OC_ERR_DEVICE_TIMEOUT at the next oc_synchronize / oc_get_state /
+ * oc_get_stats, after which the handle steps on.  A cloth whose solve had not ended on any of its CTAs
+ * got no update; the state of the others may be that of different steps and has to be set again.
+ * For tests of that path: from the next step on, block `withhold_block` of those launches sends no
+ * sums (-1: none), and a wait gives up after `max_polls` polls (0: the default, about a second for
+ * sums that travel through memory, a tenth of one within a cluster).  Nothing waits longer than
+ * that bound.  Fails with OC_ERR_UNSUPPORTED when the handle runs no such kernel. */
 oc_status oc_test_barrier_timeout(oc_solver* s, int32_t withhold_block, uint32_t max_polls);
 /* For tests of a handle's age: the tags of the packets by which its CG launches exchange sums run on
  * from launch to launch in 32 bits; the next ones continue after `last`. */

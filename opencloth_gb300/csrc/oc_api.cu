@@ -222,13 +222,14 @@ oc_status fail_cuda(oc_solver* s, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return fail_cuda(s, e_, #call); \
     } while (0)
 
-// Polls of the packets before a wait of k_cg_persist gives up (about a second).
+// Polls of the packets before a wait gives up: about a second for packets in memory, a tenth of one
+// for packets in shared memory.
 constexpr uint32_t kDefaultBarrierPolls = 1u << 22;
 
-// A wait of k_cg_persist that gave up (the stream is synchronised).  The error word is
+// A wait that gave up (the stream is synchronised).  The error word is
 // cleared once reported and the cloths' CG state (which the abandoned launch left part
-// updated) is zeroed: every step's assembly sets it up again, and the next launch starts
-// from zeroed arrival counts, so the handle steps on.
+// updated) is zeroed: every step's assembly sets it up again, and the next launch's packets have
+// tags of their own, so the handle steps on.
 oc_status report_device_error(oc_solver* s, int h);
 
 oc_status check_device_error(oc_solver* s) {
@@ -3178,7 +3179,7 @@ oc_status oc_test_packet_tags(oc_solver* s, uint32_t last) {
 
 oc_status oc_test_barrier_timeout(oc_solver* s, int32_t withhold_block, uint32_t max_polls) {
     if (!valid_solver(s) || withhold_block < -1) return OC_ERR_INVALID_ARGUMENT;
-    if (!s->persist && !s->cpl_persist && !s->adj_persist) return fail(s, OC_ERR_UNSUPPORTED, "the handle runs no persistent CG");
+    if (!s->d_perr) return fail(s, OC_ERR_UNSUPPORTED, "the handle runs no kernel whose CTAs wait for one another");
     OC_TRY(cudaSetDevice(s->device));
     OC_TRY(cudaStreamSynchronize(s->stream));
     s->args.withhold_block = withhold_block;

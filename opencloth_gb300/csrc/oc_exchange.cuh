@@ -60,6 +60,14 @@ __device__ __forceinline__ void put_cluster(ulonglong2* p, int rank, Acc v, uint
                  : "memory");
 }
 
+// 1 into the word of CTA `rank` of the cluster at this CTA's address p.
+__device__ __forceinline__ void flag_cluster(int* p, int rank) {
+    asm volatile("{ .reg .b32 a; mapa.shared::cluster.u32 a, %0, %1;\n\t"
+                 "st.relaxed.cluster.shared::cluster.b32 [a], %2; }" ::"r"(smem_addr(p)),
+                 "r"(rank), "r"(1)
+                 : "memory");
+}
+
 __device__ __forceinline__ bool get_cluster(const ulonglong2* p, uint32_t tag, Acc& v) {
     unsigned long long s, c;
     asm volatile("ld.relaxed.cluster.shared::cta.v2.b64 {%0, %1}, [%2];" : "=l"(s), "=l"(c) : "r"(smem_addr(p)) : "memory");

@@ -149,8 +149,12 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
     constexpr int kDirect = 32 / kSW;
     __shared__ __align__(16) ulonglong2 s_box[2][2][32], s_cbox[2][2][kSimMaxCluster];
     __shared__ float s_scal;
-    __shared__ int s_run, s_ok;
+    // Whether the CG goes on, by the parity of the exchange that decided it: warp 0 may give up in the
+    // next one while another warp has yet to read this one's.
+    __shared__ int s_run[2], s_ok;
+    __shared__ int s_gone[2];  // a CTA of the cluster gave up, by the parity of the barriers inside the steps
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const bool hold = (int)blockIdx.x == a.withhold_block;  // (a testing aid: its packets are not sent)
     const int C = L.cluster, rank = (int)blockIdx.x % C;
     const int inst = L.inst_ids[blockIdx.x / C];
     const InstParams& ip = a.inst[inst];
@@ -168,7 +172,10 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
     const Stencil sten{s_first, s_ent};
     const int64_t vo = ip.v_off;
 
-    if (tid == 0) s_ok = 1;
+    if (tid == 0) {
+        s_ok = 1;
+        s_gone[0] = s_gone[1] = 0;
+    }
     if (tid < 2 * 2 * 32) (&s_box[0][0][0])[tid] = make_ulonglong2(0, 0);
     if (tid < 2 * 2 * kSimMaxCluster) (&s_cbox[0][0][0])[tid] = make_ulonglong2(0, 0);
     if (C > 1) cluster_arrive();  // every CTA's boxes are clear before a packet is sent
@@ -231,6 +238,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
     // CTA's first.
     auto send = [&](Acc p, int value) {
         p = lanes_sum<16>(p);
+        if (hold) return;
         if (C > kDirect || C == 1) {
             if (lane == 0) put_local(&s_box[tag & 1][value][w], p, tag);
         } else if (lane < C) {
@@ -245,6 +253,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
             p = acc_merge(p, u);
             p2 = acc_merge(p2, u2);
         }
+        if (hold) return;
         if (C > kDirect || C == 1) {
             if (lane < 2) put_local(&s_box[tag & 1][lane][w], lane == 0 ? p : p2, tag);
         } else if (lane < C) {
@@ -259,11 +268,11 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
         bool ok = poll<1>(mine ? 1u : 0u, a, L.err, [&](int) { return get_cluster(box, tag, t); });
         if (!mine) t = acc_zero();
         total = lanes_sum<16>(t);
-        if (C > kDirect) {
-            if (lane < C) put_cluster(&s_cbox[tag & 1][value][rank], lane, total, tag);
+        if (C > kDirect && ok) {
+            if (lane < C && !hold) put_cluster(&s_cbox[tag & 1][value][rank], lane, total, tag);
             t = acc_zero();
             const ulonglong2* cbox = &s_cbox[tag & 1][value][lane % kSimMaxCluster];
-            ok = poll<1>(lane < C ? 1u : 0u, a, L.err, [&](int) { return get_cluster(cbox, tag, t); }) && ok;
+            ok = poll<1>(lane < C ? 1u : 0u, a, L.err, [&](int) { return get_cluster(cbox, tag, t); });
             if (lane >= C) t = acc_zero();
             total = lanes_sum<16>(t);
         }
@@ -273,10 +282,9 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
     auto decide = [&](bool ok, bool run, float scal) {  // by warp 0, for the CTA
         if (lane == 0) {
             s_scal = scal;
-            s_run = run ? 1 : 0;
+            s_run[tag & 1] = run && ok ? 1 : 0;
             if (!ok) {
                 s_ok = 0;
-                s_run = 0;
                 atomicOr(L.err, 1);
             }
         }
@@ -294,6 +302,21 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
         }
         decide(ok, run, scal);
     };
+
+    // The cluster's barrier inside a step: true when no CTA's wait has given up.  One whose has takes the
+    // barrier like the others, having told them first, and all of them leave behind the same barrier: a
+    // CTA that left alone would be missing at the others' next barrier, and their packets would go to
+    // shared memory that is no longer its own.  Two flags, as a CTA may be one barrier ahead of
+    // another that has not read its flag yet, but not two.
+    unsigned met = 0;
+    auto together = [&]() -> bool {
+        int* const gone = &s_gone[met++ & 1];
+        if (!s_ok && tid < C) flag_cluster(gone, tid);
+        cluster_arrive();
+        cluster_wait();
+        return *(volatile int*)gone == 0;
+    };
+    bool all_ok = true;
 
     __syncthreads();
     if (C > 1) cluster_wait();
@@ -388,7 +411,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
                 decide(ok, false, 0.0f);
         }
         __syncthreads();
-        while (s_run) {
+        while (s_run[tag & 1]) {
             // x += alpha d; r -= alpha A d; r.r, IMP:322-325.
             const float alpha = s_scal;
             Acc part = acc_zero();
@@ -418,7 +441,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
                 decide(ok, run, beta);
             }
             __syncthreads();
-            if (!s_run) break;
+            if (!s_run[tag & 1]) break;
             // d = r + beta d; d.(A d), IMP:320-321, 327.
             const float beta = s_scal;
             part = acc_zero();
@@ -433,14 +456,17 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
             }
             __syncthreads();
         }
-        if (!s_ok) break;
+        // A wait that gave up: no update; the CTAs of a cluster go on to their next barrier.
+        const bool ok = s_ok != 0;
+        all_ok = ok;
+        if (!ok && C == 1) break;
         // The update (IMP:790-797) and the ellipsoid; the window's own part, and, for the other
         // CTAs and at the end, global memory.
         const bool last = step + 1 == L.n_steps;
         const bool prov = (ip.passes & OC_PASS_PROVOT) != 0;
 #pragma unroll
         for (int u = 0; u < VPT; ++u)
-            if (own[u]) {
+            if (own[u] && ok) {
                 const int j = tid + u * kST, i = lb + j - wlo;
                 float4 X = wX[i], V = wV[i];
                 update_vertex(ip, a.dt, x[u][0], x[u][1], x[u][2], X, V);
@@ -458,8 +484,8 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
             }
         if (prov) {
             if (C > 1) {
-                cluster_arrive();
-                cluster_wait();
+                all_ok = together();
+                if (!all_ok) break;
                 for (int i = wlo + tid; i < whi; i += kST)
                     if (i < lb || i >= lb + n) wX[i - wlo] = __ldcg(a.X + vo + i);
             }
@@ -477,8 +503,8 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
         }
         if (!last) {
             if (C > 1) {  // the neighbouring CTAs' new state into the halo
-                cluster_arrive();
-                cluster_wait();
+                all_ok = together();
+                if (!all_ok) break;
                 for (int i = wlo + tid; i < whi; i += kST)
                     if (i < lb || i >= lb + n) {
                         if (!prov) wX[i - wlo] = __ldcg(a.X + vo + i);
@@ -488,7 +514,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
             __syncthreads();
         }
     }
-    if (rank == 0 && tid == 0 && s_ok) {
+    if (rank == 0 && tid == 0 && all_ok) {
         InstState& st = a.state[inst];
         st.delta0 = (double)dn0.s + (double)dn0.c;
         st.delta_new = (double)dn.s + (double)dn.c;
