@@ -42,7 +42,9 @@
 // after a.barrier_polls polls or when another CTA has given up: it sets bit 0 of *err and the
 // CTA leaves without its update.  The CTA a.withhold_block (a testing aid; normally -1) leaves
 // before its first packets, so the waits on its cloths run out.  The CTAs of a cluster leave
-// together, so no packet meets the shared memory of a CTA that has gone.
+// together, so no packet meets the shared memory of a CTA that has gone.  Whether a wait has given
+// up is kept by the phase's parity, like the scalars: the warp that gives up in one phase need not wait
+// for the others, which may have yet to read what the phase before decided.
 //
 // Compiled with --fmad=false; the dot terms are FP32, summed in error-free pairs at every
 // level (about 48 bits, as the resident kernel's), in a fixed order; alpha and beta are the
@@ -133,7 +135,7 @@ __device__ __forceinline__ void persist_update(const StepArgs& a, const InstPara
 
 __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const PersistPlan P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_ok;
+    __shared__ int s_ok[2];  // 0: a wait gave up in the phase before the one of that parity
     // Packets of the warps of the cluster's CTAs, for the CTA's first and last piece (no other
     // piece has vertices in another CTA): by parity, piece, and sender's rank and warp.
     __shared__ __align__(16) ulonglong2 s_box[2][2][kMaxCluster * kWarps];
@@ -148,7 +150,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
     const int s_end = kRegSlots + P.smem_slots;                       // slots from here on stay in the planes
     const uint32_t base = *(volatile uint32_t*)&P.ctl->base;
 
-    if (tid == 0) s_ok = 1;
+    if (tid < 2) s_ok[tid] = 1;
     const ulonglong2 none = empty_packet(base);
     for (int i = tid; i < 2 * 2 * kMaxCluster * kWarps; i += kPT) (&s_box[0][0][0])[i] = none;
     for (int j = tid; j < np; j += kPT) {
@@ -241,6 +243,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
     asm volatile("cp.async.wait_all;" ::: "memory");  // a thread reads back only its own copies
     __syncthreads();
     if (CS > 1) cluster_wait();
+    bool whole = true;  // no wait of this CTA has given up
     unsigned q = 0;
     for (;; ++q) {
         const int cur = q & 1, nxt = cur ^ 1;
@@ -250,8 +253,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
         for (int j = 0; j < np; ++j) any |= st[j].run[cur];
         if (!any) break;
         if ((int)blockIdx.x == a.withhold_block) {
-            if (tid == 0) s_ok = 0;
-            __syncthreads();
+            whole = false;
             break;
         }
         // The pass of every running piece; each warp sends its partial to the cloth's CTAs of
@@ -496,14 +498,15 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
         }
         if (!ok && lane == 0) {
             atomicOr(P.err, 1);
-            s_ok = 0;
+            s_ok[nxt] = 0;
         }
         __syncthreads();
-        if (!s_ok) break;
+        whole = s_ok[nxt] != 0;
+        if (!whole) break;
     }
     if (CS > 1) cluster_arrive();
     if (tid == 0) leave_tags(P.ctl, base, q + 2);
-    if (s_ok) {
+    if (whole) {
         // The cloths' scalars for the host, by each cloth's first piece.
         for (int j = tid; j < np; j += kPT) {
             if (!pieces[j].head) continue;
@@ -535,7 +538,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
 template <int KR, bool FULL>
 __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, const PersistPlan P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_ok;
+    __shared__ int s_ok[2];
     __shared__ float s_scal[2];
     __shared__ int s_run[2];
     __shared__ __align__(16) ulonglong2 s_box[2][kMaxCluster * kWarps];
@@ -551,7 +554,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
     const int64_t v = pc.v + tid;
     const bool upd = !a.cg_only;
 
-    if (tid == 0) s_ok = 1;
+    if (tid < 2) s_ok[tid] = 1;
     for (int i = tid; i < 2 * kMaxCluster * kWarps; i += kPT) (&s_box[0][0])[i] = empty_packet(base);
     if (CS > 1) cluster_arrive();
     float A[KR][6], r[KR][3], d[KR][3];
@@ -640,6 +643,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
         const int from = (u * 32 + lane) / kWarps;
         if (from >= pc.rank0 && from < pc.rank0 + pc.ranks) want_box |= 1u << u;
     }
+    bool whole = true;  // no wait of this CTA has given up
     unsigned q = 0;
     for (;; ++q) {
         const int cur = q & 1, nxt = cur ^ 1;
@@ -647,8 +651,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
         const uint32_t tag = base + q + 1;
         if (!s_run[cur]) break;
         if ((int)blockIdx.x == a.withhold_block) {
-            if (tid == 0) s_ok = 0;
-            __syncthreads();
+            whole = false;
             break;
         }
         const float scal = s_scal[cur];
@@ -858,17 +861,18 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
                 s_run[nxt] = run ? 1 : 0;
                 if (!ok) {
                     atomicOr(P.err, 1);
-                    s_ok = 0;
+                    s_ok[nxt] = 0;
                 }
             }
         }
         __syncthreads();
-        if (!s_ok) break;
+        whole = s_ok[nxt] != 0;
+        if (!whole) break;
     }
     if (CS > 1) cluster_arrive();
     if (tid == 0) {
         leave_tags(P.ctl, base, q + 2);
-        if (s_ok && pc.head && n > 0) {
+        if (whole && pc.head && n > 0) {
             InstState& is = a.state[pc.inst];
             is.delta0 = d0;
             is.delta_new = (double)dn.s + (double)dn.c;
@@ -881,7 +885,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
             is.ticket = 0;
         }
     }
-    if (s_ok && n > 0) {
+    if (whole && n > 0) {
         const InstParams& ip = a.inst[pc.inst];
         if constexpr (FULL) {
 #pragma unroll

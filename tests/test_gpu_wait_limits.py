@@ -52,3 +52,12 @@ def test_whole_steps_in_one_launch(shapes, passes, block, polls, steps):
 
 def test_one_cta():
     check([grid(15, 16, 1)], 3, 0, 1000)
+
+
+@pytest.mark.parametrize("polls", [50, 3000])
+@pytest.mark.parametrize("block", [0, 1])
+@pytest.mark.parametrize("shapes", [[(30, 30)], [(200, 190)], [(300, 280), (120, 90), (60, 60)],
+                                    [(6 + k % 25, 7 + k % 23) for k in range(330)]],
+                         ids=["a cluster", "clusters", "several", "pieces"])
+def test_persistent_cg(shapes, block, polls):
+    check([grid(c, r, k) for k, (c, r) in enumerate(shapes)], 2, block, polls, executor="streamed")
