@@ -336,7 +336,7 @@ oc_status oc_tune_cache_lookup(const char* path, const char* key, oc_launch_conf
 oc_status oc_tune_cache_store(const char* path, const char* key, const oc_launch_config* cfg, double ms_per_step);
 
 /* ---- testing aid: the bounded waits ------------------------------------------------- */
-/* The CTAs of a CG launch (k_cg_persist, k_cpl_persist, k_sim) wait for one another's partial sums.
+/* The CTAs of a CG launch (k_cg_persist, k_cpl_persist, k_sim, k_resident) wait for one another's partial sums.
  * Each wait gives up after a bounded number of polls, or when another wait of the handle has given
  * up; the step then fails with OC_ERR_DEVICE_TIMEOUT at the next oc_synchronize / oc_get_state /
  * oc_get_stats, after which the handle steps on.  A cloth whose solve had not ended on any of its CTAs
@@ -432,6 +432,9 @@ oc_status oc_bsr_get_launch_count(oc_bsr_solver* s, int64_t* kernels_launched);
 oc_status oc_bsr_profile(oc_bsr_solver* s, int32_t n_solves, int32_t max_kernels, char* names, double* ms_total,
                          int64_t* launches, double* algorithmic_bytes, int32_t* n_kernels);
 oc_status oc_bsr_synchronize(oc_bsr_solver* s);
+/* oc_test_barrier_timeout for the solves that follow: a wait that ran out is reported as
+ * OC_ERR_DEVICE_TIMEOUT by oc_bsr_get_solution and oc_bsr_synchronize, once. */
+oc_status oc_bsr_test_barrier_timeout(oc_bsr_solver* s, int32_t withhold_block, uint32_t max_polls);
 
 /* ---- reference topology builder (IMP:497-565) ------------------------------------ */
 /* Host only (no device work): validate the descriptors as oc_create does and report, per

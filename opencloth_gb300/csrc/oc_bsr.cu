@@ -603,7 +603,8 @@ struct BsrPlan {
     PersistCtl* ctl;
     int* err;
     int32_t grid, n_packets;
-    uint32_t polls;
+    uint32_t polls;    // of the packets before a wait gives up
+    int32_t withhold;  // a CTA that takes no part (-1: none; a testing aid)
 };
 
 // q of row g: the products of its blocks with the directions (first: p alone; else r + d4 p), in
@@ -663,7 +664,7 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
     };
     Acc d = acc_zero(), d1 = acc_zero(), d2 = acc_zero();
     float d3 = 0.0f, d4 = 0.0f;
-    if (pc.n > 0) {
+    if (pc.n > 0 && (int)blockIdx.x != P.withhold) {
         const BsrParams& sp = a.sys[pc.sys];
         const float tiny = sp.tiny;
         const int rows = (pc.n + kBT - 1) / kBT;
@@ -1008,6 +1009,7 @@ cudaError_t launch_bsr_persist(const oc_bsr_solver* s) {
 // with at least kBsrMinRows each (a CTA of few rows has idle warps, but its rows' chains of
 // dependent loads run side by side), where there are no more systems than SMs.
 constexpr int64_t kBsrMinRows = 256;
+constexpr uint32_t kBsrPolls = 1u << 22;  // about a second
 
 oc_status plan_bsr_persist(oc_bsr_solver* s, const std::vector<BsrParams>& sys) {
     int sms = 0, coop = 0;
@@ -1054,7 +1056,8 @@ oc_status plan_bsr_persist(oc_bsr_solver* s, const std::vector<BsrParams>& sys) 
     P.ctl = reinterpret_cast<PersistCtl*>(P.packets + 2 * (size_t)packets);
     P.err = reinterpret_cast<int*>(P.packets + 2 * (size_t)packets + 1);
     P.n_packets = packets;
-    P.polls = 1u << 22;
+    P.polls = kBsrPolls;
+    P.withhold = -1;
     P.grid = (int32_t)pieces.size();
     return OC_OK;
 }
@@ -1644,6 +1647,14 @@ oc_status oc_bsr_get_launch_count(oc_bsr_solver* s, int64_t* kernels_launched) {
                             s->stream));
     BSR_TRY(cudaStreamSynchronize(s->stream));
     *kernels_launched = s->launches + 2 * (int64_t)*s->h_loop;
+    return OC_OK;
+}
+
+oc_status oc_bsr_test_barrier_timeout(oc_bsr_solver* s, int32_t withhold_block, uint32_t max_polls) {
+    if (!bsr_valid(s) || withhold_block < -1) return OC_ERR_INVALID_ARGUMENT;
+    if (s->plan.grid == 0) return bsr_fail(s, OC_ERR_UNSUPPORTED, "the handle's solves have no CTAs that wait for one another");
+    s->plan.withhold = withhold_block;
+    s->plan.polls = max_polls > 0 ? max_polls : kBsrPolls;
     return OC_OK;
 }
 

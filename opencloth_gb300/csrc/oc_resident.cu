@@ -60,7 +60,7 @@ __device__ __forceinline__ bool cluster_sum(Acc part, int C, int rank, SumBuffer
     total = lanes_sum<W / 2>(b.warps[cur][lane & (W - 1)]);
     if (C > 1) {
         ulonglong2* const box = b.box[cur];
-        if (lane < C) put_cluster(box + rank, lane, total, tag);
+        if (lane < C && (int)blockIdx.x != a.withhold_block) put_cluster(box + rank, lane, total, tag);
         Acc v = acc_zero();
         ok = poll<1>(lane < C ? 1u : 0u, a, err, [&](int) { return get_cluster(box + lane, tag, v); });
         total = lanes_sum<kResidentMaxCluster / 2>(v);

@@ -6,6 +6,8 @@ import pytest
 
 from opencloth_gb300 import PASS_PROVOT, ClothSolver, OcError
 from opencloth_gb300 import _native as N
+from opencloth_gb300.fem import BsrSolver
+from test_gpu_fem_resident import system
 from test_gpu_sim import grid, same_bits
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +63,36 @@ def test_one_cta():
                          ids=["a cluster", "clusters", "several", "pieces"])
 def test_persistent_cg(shapes, block, polls):
     check([grid(c, r, k) for k, (c, r) in enumerate(shapes)], 2, block, polls, executor="streamed")
+
+
+@pytest.mark.parametrize("polls", [50, 3000])
+@pytest.mark.parametrize("count", [1, 40])
+def test_resident_cg(count, polls):
+    """k_resident: a handle without graphs, and more cloths of several CTAs than k_sim takes."""
+    parts = [grid(120, 100, 1)] + [grid(70 + k % 3, 60, k) for k in range(count - 1)]
+    check(parts, 1, 1, polls, **({"use_graph": False} if count == 1 else {}))
+
+
+@pytest.mark.parametrize("polls", [50, 3000])
+@pytest.mark.parametrize("block", [0, 1])
+@pytest.mark.parametrize("sizes", [[3000], [2000, 40, 1500]])
+def test_fem_solve(sizes, block, polls):
+    systems = [system(n, n, 9, i_max=7) for n in sizes]
+    arrays = [np.concatenate([g[k] for g in systems]) for k in ("blocks", "b", "V")]
+    lib = N.load()
+    with BsrSolver(systems, executor=1) as s:
+        s.set_system(*arrays)
+        s.solve()
+        want = s.solution()
+        assert lib.oc_bsr_test_barrier_timeout(s._h, block, polls) == 0
+        s.set_system(*arrays)
+        s.solve()
+        with pytest.raises(OcError) as e:
+            s.synchronize()
+        assert e.value.status == 8
+        s.synchronize()  # (reported once)
+        assert lib.oc_bsr_test_barrier_timeout(s._h, -1, 0) == 0
+        for _ in range(2):
+            s.set_system(*arrays)
+            s.solve()
+            assert all(np.array_equal(a, b) for a, b in zip(s.solution(), want))
