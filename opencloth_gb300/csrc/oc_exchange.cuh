@@ -136,7 +136,7 @@ __device__ __forceinline__ bool pull_sum(Acc part, ulonglong2* packets, int idx,
             sum = acc_merge(sum, acc_merge(acc_merge(acc_merge(y[0], y[1]), acc_merge(y[2], y[3])), y[4]));
         }
         total = lanes_sum<16>(sum);
-        if (publish && lane == 0) __threadfence();
+        if (publish) __threadfence();  // by every lane that has read packets, before the caller's barrier
         __syncwarp();
     }
     total = pair_norm(total);
