@@ -149,12 +149,9 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
     constexpr int kDirect = 32 / kSW;
     __shared__ __align__(16) ulonglong2 s_box[2][2][32], s_cbox[2][2][kSimMaxCluster];
     __shared__ float s_scal;
-    // Whether the CG goes on, by the parity of the exchange that decided it: warp 0 may give up in the
-    // next one while another warp has yet to read this one's.
-    __shared__ int s_run[2], s_ok;
+    __shared__ int s_run, s_ok;
     __shared__ int s_gone[2];  // a CTA of the cluster gave up, by the parity of the barriers inside the steps
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const bool hold = (int)blockIdx.x == a.withhold_block;  // (a testing aid: its packets are not sent)
     const int C = L.cluster, rank = (int)blockIdx.x % C;
     const int inst = L.inst_ids[blockIdx.x / C];
     const InstParams& ip = a.inst[inst];
@@ -238,7 +235,6 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
     // CTA's first.
     auto send = [&](Acc p, int value) {
         p = lanes_sum<16>(p);
-        if (hold) return;
         if (C > kDirect || C == 1) {
             if (lane == 0) put_local(&s_box[tag & 1][value][w], p, tag);
         } else if (lane < C) {
@@ -253,7 +249,6 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
             p = acc_merge(p, u);
             p2 = acc_merge(p2, u2);
         }
-        if (hold) return;
         if (C > kDirect || C == 1) {
             if (lane < 2) put_local(&s_box[tag & 1][lane][w], lane == 0 ? p : p2, tag);
         } else if (lane < C) {
@@ -266,10 +261,18 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
         Acc t = acc_zero();
         const ulonglong2* box = &s_box[tag & 1][value][lane];
         bool ok = poll<1>(mine ? 1u : 0u, a, L.err, [&](int) { return get_cluster(box, tag, t); });
+        if (!ok) {
+            // Nothing of this exchange may be decided before the CTA's other warps, which have read the
+            // last one's decision when they send, have sent (they wait for nothing on the way).
+            const int from = C > kDirect ? 0 : rank * kSW;
+            const bool theirs = lane >= from && lane < from + kSW;
+            for (unsigned i = 0; i < 1u << 22; ++i)
+                if (__all_sync(0xffffffffu, !theirs || get_cluster(box, tag, t))) break;
+        }
         if (!mine) t = acc_zero();
         total = lanes_sum<16>(t);
         if (C > kDirect && ok) {
-            if (lane < C && !hold) put_cluster(&s_cbox[tag & 1][value][rank], lane, total, tag);
+            if (lane < C) put_cluster(&s_cbox[tag & 1][value][rank], lane, total, tag);
             t = acc_zero();
             const ulonglong2* cbox = &s_cbox[tag & 1][value][lane % kSimMaxCluster];
             ok = poll<1>(lane < C ? 1u : 0u, a, L.err, [&](int) { return get_cluster(cbox, tag, t); });
@@ -282,7 +285,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
     auto decide = [&](bool ok, bool run, float scal) {  // by warp 0, for the CTA
         if (lane == 0) {
             s_scal = scal;
-            s_run[tag & 1] = run && ok ? 1 : 0;
+            s_run = run && ok ? 1 : 0;
             if (!ok) {
                 s_ok = 0;
                 atomicOr(L.err, 1);
@@ -320,7 +323,15 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
 
     __syncthreads();
     if (C > 1) cluster_wait();
-    for (int32_t step = 0; step < L.n_steps; ++step) {
+    int32_t n_steps = L.n_steps;
+    if ((int)blockIdx.x == a.withhold_block) {  // (a testing aid) sends no packets, meets the others at their first barrier
+        if (tid == 0) s_ok = 0;
+        __syncthreads();
+        if (C > 1 && (n_steps > 1 || (ip.passes & OC_PASS_PROVOT))) together();
+        all_ok = false;
+        n_steps = 0;
+    }
+    for (int32_t step = 0; step < n_steps; ++step) {
         // The assembly of the CTA's vertices, with the first direction's dot product.
         Acc p0 = acc_zero(), p1 = acc_zero();
 #pragma unroll 1
@@ -411,7 +422,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
                 decide(ok, false, 0.0f);
         }
         __syncthreads();
-        while (s_run[tag & 1]) {
+        while (s_run) {
             // x += alpha d; r -= alpha A d; r.r, IMP:322-325.
             const float alpha = s_scal;
             Acc part = acc_zero();
@@ -441,7 +452,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
                 decide(ok, run, beta);
             }
             __syncthreads();
-            if (!s_run[tag & 1]) break;
+            if (!s_run) break;
             // d = r + beta d; d.(A d), IMP:320-321, 327.
             const float beta = s_scal;
             part = acc_zero();
@@ -462,7 +473,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
         if (!ok && C == 1) break;
         // The update (IMP:790-797) and the ellipsoid; the window's own part, and, for the other
         // CTAs and at the end, global memory.
-        const bool last = step + 1 == L.n_steps;
+        const bool last = step + 1 == n_steps;
         const bool prov = (ip.passes & OC_PASS_PROVOT) != 0;
 #pragma unroll
         for (int u = 0; u < VPT; ++u)

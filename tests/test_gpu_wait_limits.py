@@ -52,10 +52,6 @@ def test_whole_steps_in_one_launch(shapes, passes, block, polls, steps):
     check([grid(c, r, k, passes=passes) for k, (c, r) in enumerate(shapes)], steps, block, polls)
 
 
-def test_one_cta():
-    check([grid(15, 16, 1)], 3, 0, 1000)
-
-
 @pytest.mark.parametrize("polls", [50, 3000])
 @pytest.mark.parametrize("block", [0, 1])
 @pytest.mark.parametrize("shapes", [[(30, 30)], [(200, 190)], [(300, 280), (120, 90), (60, 60)],
