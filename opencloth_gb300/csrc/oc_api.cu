@@ -1166,6 +1166,7 @@ oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_
                 const int32_t n = (int32_t)std::min<int64_t>(cap - open_n, ip.nv - l);
                 PersistPiece pc{};
                 pc.inst = k;
+                pc.scale = sum_scale(ip.nv);
                 pc.head = l == 0;
                 pc.v = ip.v_off + l;
                 pc.n = n;
@@ -1269,6 +1270,7 @@ oc_status plan_coupled(oc_solver* s) {
             pc.v = ip.v_off + l;
             pc.n = (int32_t)std::min<int64_t>(each, ip.nv - l);
             pc.inst = k;
+            pc.scale = sum_scale(ip.nv);
             pc.idx = (int32_t)(pieces.size() - p0);
             pc.packet = P.n_packets;
             pieces.push_back(pc);

@@ -476,7 +476,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_bsr_resident(const BsrArgs a, c
     float p0 = r0, p1 = r1, p2 = r2;
     Acc d = acc_zero(), d1 = acc_zero(), d2 = acc_zero();
     float d3 = 0.0f, d4 = 0.0f;
-    // The total of the warps' pairs, in every lane (every eight lanes read all eight).
+    // The sums carry the factor 1 / kThreads, so that finite terms have a finite total (see
+    // sum_scale).  The total of the warps' pairs, in every lane (every eight lanes read all eight).
+    constexpr float kScale = 1.0f / kThreads;
+    const float tiny = sp.tiny * kScale;
     auto total = [&](const Acc* wacc) { return pair_norm(lanes_sum<4>(wacc[lane & 7])); };
     __syncthreads();  // init's reads of x are done
     // Three barriers an iteration: after the directions, the products (d2) and the update (d1);
@@ -510,8 +513,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_bsr_resident(const BsrArgs a, c
         }
         Acc pd = acc_zero(), pd2 = acc_zero();
         if (act) {
-            acc_add(pd, r0 * r0 + r1 * r1 + r2 * r2);
-            acc_add(pd2, n0 * q0 + n1 * q1 + n2 * q2);
+            acc_add(pd, (r0 * r0 + r1 * r1 + r2 * r2) * kScale);
+            acc_add(pd2, (n0 * q0 + n1 * q1 + n2 * q2) * kScale);
         }
         // d = r.r is the previous update's d1: the same terms in the same order.
         if (first) {
@@ -523,7 +526,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_bsr_resident(const BsrArgs a, c
         __syncthreads();
         d = first ? total(s_w0) : d1;
         d2 = total(s_w1);
-        d3 = quotient(d, pair_below(d2, sp.tiny) ? make_acc(sp.tiny, 0.0f) : d2);  // FEM:885-886
+        d3 = quotient(d, pair_below(d2, tiny) ? make_acc(tiny, 0.0f) : d2);  // FEM:885-886
         // k_bsr_update
         Acc pd1 = acc_zero();
         if (act) {
@@ -536,13 +539,13 @@ __global__ void __launch_bounds__(kThreads, 3) k_bsr_resident(const BsrArgs a, c
             p0 = n0;
             p1 = n1;
             p2 = n2;
-            acc_add(pd1, r0 * r0 + r1 * r1 + r2 * r2);
+            acc_add(pd1, (r0 * r0 + r1 * r1 + r2 * r2) * kScale);
         }
         pd1 = lanes_sum<16>(pd1);
         if (lane == 0) s_w2[w] = pd1;
         __syncthreads();
         d1 = total(s_w2);
-        d4 = quotient(d1, pair_below(d, sp.tiny) ? make_acc(sp.tiny, 0.0f) : d);  // FEM:908-909
+        d4 = quotient(d1, pair_below(d, tiny) ? make_acc(tiny, 0.0f) : d);  // FEM:908-909
     }
     if (valid) {
         if (act) {
@@ -555,9 +558,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_bsr_resident(const BsrArgs a, c
     }
     if (t == 0) {
         BsrState& st = a.state[k];
-        st.d = (double)d.s + (double)d.c;
-        st.d1 = (double)d1.s + (double)d1.c;
-        st.d2 = (double)d2.s + (double)d2.c;
+        st.d = ((double)d.s + (double)d.c) / kScale;
+        st.d1 = ((double)d1.s + (double)d1.c) / kScale;
+        st.d2 = ((double)d2.s + (double)d2.c) / kScale;
         st.d3 = d3;
         st.d4 = d4;
         st.iter = sp.imax;
@@ -594,7 +597,7 @@ struct BsrPiece {
     int64_t g0;
     int32_t idx, np;  // this CTA among its system's np CTAs
     int32_t packet;   // the system's first packet
-    int32_t pad_;
+    float scale;      // of the system's sums (sum_scale)
 };
 
 struct BsrPlan {
@@ -666,7 +669,7 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
     float d3 = 0.0f, d4 = 0.0f;
     if (pc.n > 0 && (int)blockIdx.x != P.withhold) {
         const BsrParams& sp = a.sys[pc.sys];
-        const float tiny = sp.tiny;
+        const float scale = pc.scale, tiny = sp.tiny * scale;  // as the sums
         const int rows = (pc.n + kBT - 1) / kBT;
         float x[kOwnRows][3], r[kOwnRows][3], p[kOwnRows][3], q[kOwnRows][3];
         bool own[kOwnRows];
@@ -701,7 +704,7 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
                     p[u][k] = r[u][k];
                     x[u][k] = a.x[k][g];
                 }
-                acc_add(part, r[u][0] * r[u][0] + r[u][1] * r[u][1] + r[u][2] * r[u][2]);
+                acc_add(part, (r[u][0] * r[u][0] + r[u][1] * r[u][1] + r[u][2] * r[u][2]) * scale);
             }
             if (in) {
                 a.r4[g] = make_float4(r[u][0], r[u][1], r[u][2], 0.0f);
@@ -714,7 +717,7 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
             float rr[3] = {0.0f, 0.0f, 0.0f};
             if (!a.fixed[g]) {
                 residual(g, rr);
-                acc_add(part, rr[0] * rr[0] + rr[1] * rr[1] + rr[2] * rr[2]);
+                acc_add(part, (rr[0] * rr[0] + rr[1] * rr[1] + rr[2] * rr[2]) * scale);
             }
             a.r4[g] = make_float4(rr[0], rr[1], rr[2], 0.0f);
             a.p4[g] = make_float4(rr[0], rr[1], rr[2], 0.0f);
@@ -735,7 +738,7 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
                     for (int k = 0; k < 3; ++k) p[u][k] = r[u][k] + p[u][k] * d4;
                 }
                 row_product(a, sp, pc.g0 + u * kBT + tid, first, d4, q[u][0], q[u][1], q[u][2]);
-                acc_add(part, p[u][0] * q[u][0] + p[u][1] * q[u][1] + p[u][2] * q[u][2]);
+                acc_add(part, (p[u][0] * q[u][0] + p[u][1] * q[u][1] + p[u][2] * q[u][2]) * scale);
             }
             for (int u = kOwnRows; u < rows; ++u) {
                 const int64_t g = pc.g0 + (int64_t)u * kBT + tid;
@@ -753,7 +756,7 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
                 a.q[0][g] = q0;
                 a.q[1][g] = q1;
                 a.q[2][g] = q2;
-                acc_add(part, n0 * q0 + n1 * q1 + n2 * q2);
+                acc_add(part, (n0 * q0 + n1 * q1 + n2 * q2) * scale);
             }
             bool ok = exchange(part, false, d2);
             settle(ok, w == 0 ? quotient(d, pair_below(d2, tiny) ? make_acc(tiny, 0.0f) : d2) : 0.0f);  // FEM:885-886
@@ -772,7 +775,7 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
                 }
                 a.r4[g] = make_float4(r[u][0], r[u][1], r[u][2], 0.0f);
                 a.p4[g] = make_float4(p[u][0], p[u][1], p[u][2], 0.0f);
-                acc_add(part, r[u][0] * r[u][0] + r[u][1] * r[u][1] + r[u][2] * r[u][2]);
+                acc_add(part, (r[u][0] * r[u][0] + r[u][1] * r[u][1] + r[u][2] * r[u][2]) * scale);
             }
             for (int u = kOwnRows; u < rows; ++u) {
                 const int64_t g = pc.g0 + (int64_t)u * kBT + tid;
@@ -789,7 +792,7 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
                 }
                 a.r4[g] = make_float4(rn[0], rn[1], rn[2], 0.0f);
                 a.p4[g] = make_float4(pn[0], pn[1], pn[2], 0.0f);
-                acc_add(part, rn[0] * rn[0] + rn[1] * rn[1] + rn[2] * rn[2]);
+                acc_add(part, (rn[0] * rn[0] + rn[1] * rn[1] + rn[2] * rn[2]) * scale);
             }
             ok = exchange(part, true, d1);
             settle(ok, w == 0 ? quotient(d1, pair_below(d, tiny) ? make_acc(tiny, 0.0f) : d) : 0.0f);  // FEM:908-909
@@ -805,9 +808,10 @@ __global__ void __launch_bounds__(kBT, 1) k_bsr_persist(const BsrArgs a, const B
                 }
             if (pc.idx == 0 && tid == 0) {
                 BsrState& st = a.state[pc.sys];
-                st.d = (double)d.s + (double)d.c;
-                st.d1 = (double)d1.s + (double)d1.c;
-                st.d2 = (double)d2.s + (double)d2.c;
+                const double unit = 1.0f / scale;  // (a power of two)
+                st.d = ((double)d.s + (double)d.c) * unit;
+                st.d1 = ((double)d1.s + (double)d1.c) * unit;
+                st.d2 = ((double)d2.s + (double)d2.c) * unit;
                 st.d3 = d3;
                 st.d4 = d4;
                 st.iter = sp.imax;
@@ -1036,6 +1040,7 @@ oc_status plan_bsr_persist(oc_bsr_solver* s, const std::vector<BsrParams>& sys) 
         for (int64_t r = 0; r < n; r += each) {
             BsrPiece pc{};
             pc.sys = k;
+            pc.scale = sum_scale(n);
             pc.g0 = sys[k].row0 + r;
             pc.n = (int32_t)std::min(each, n - r);
             pc.idx = (int32_t)(pieces.size() - p0);

@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kThreads) k_cpl_update(const StepArgs a) {
 constexpr int kCT = kCplThreads;
 
 struct CplScalars {  // a cloth's, written by thread 0
-    Acc dn, dq, thresh;  // delta_new, the last d.q, eps^2 delta0
+    Acc dn, dq, thresh;  // delta_new, the last d.q, eps^2 delta0, each times the piece's scale
     float alpha, beta;
     int it;
     uint32_t fl;
@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(kCT, 1) k_cpl_persist(const StepArgs a, const 
     const CplPiece pc = P.pieces[blockIdx.x];
     const int n = pc.n, S = P.smem_rows, in = min(n, S);
     const int64_t v = pc.v;
+    const float scale = pc.scale;
     const InstParams& ip = a.inst[pc.inst];
     InstState& is = a.state[pc.inst];
     const uint32_t base = *(volatile uint32_t*)&P.ctl->base;
@@ -350,9 +351,9 @@ __global__ void __launch_bounds__(kCT, 1) k_cpl_persist(const StepArgs a, const 
     float* const sP = sm + 12 * S;
     float* const sM = sm + 18 * S;
     if (tid == 0) {
-        sc.dn = pair_from(__ldcg(&is.delta_new));
+        sc.dn = pair_from(__ldcg(&is.delta_new) * scale);
         sc.dq = acc_zero();
-        sc.thresh = pair_from((double)ip.eps2 * __ldcg(&is.delta0));
+        sc.thresh = pair_from((double)ip.eps2 * __ldcg(&is.delta0) * scale);
         sc.alpha = sc.beta = 0.0f;
         sc.it = __ldcg(&is.iter);
         sc.fl = __ldcg(&is.flags);
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(kCT, 1) k_cpl_persist(const StepArgs a, const 
                 a.q[1][g] = q1;
                 a.q[2][g] = q2;
             }
-            acc_add(part, n0 * q0 + n1 * q1 + n2 * q2);
+            acc_add(part, (n0 * q0 + n1 * q1 + n2 * q2) * scale);
         }
         Acc total = acc_zero();
         ++tag;
@@ -484,7 +485,7 @@ __global__ void __launch_bounds__(kCT, 1) k_cpl_persist(const StepArgs a, const 
             matvec(Pi, r[0], r[1], r[2], z0, z1, z2);
             a.cpl_d[g] = make_float4(m[0], m[1], m[2], 0.0f);
             a.cpl_z[g] = make_float4(z0, z1, z2, 0.0f);
-            acc_add(part, r[0] * z0 + r[1] * z1 + r[2] * z2);
+            acc_add(part, (r[0] * z0 + r[1] * z1 + r[2] * z2) * scale);
         }
         ++tag;
         ok = pull_sum<kCT / 32>(part, P.packets + (size_t)(tag & 1) * P.n_packets + pc.packet, pc.idx, pc.np, tag, true,
@@ -514,8 +515,9 @@ __global__ void __launch_bounds__(kCT, 1) k_cpl_persist(const StepArgs a, const 
     if (tid == 0) {
         leave_tags(P.ctl, base, tag - base + 1);
         if (s_ok && pc.idx == 0) {
-            is.delta_new = (double)sc.dn.s + (double)sc.dn.c;
-            is.dq = (double)sc.dq.s + (double)sc.dq.c;
+            const double unit = 1.0f / scale;  // (a power of two)
+            is.delta_new = ((double)sc.dn.s + (double)sc.dn.c) * unit;
+            is.dq = ((double)sc.dq.s + (double)sc.dq.c) * unit;
             is.alpha = sc.alpha;
             is.beta = sc.beta;
             is.iter = sc.it;

@@ -154,34 +154,43 @@ __device__ __forceinline__ void leave_tags(PersistCtl* ctl, uint32_t base, uint3
     }
 }
 
-// a / b of two normalised pairs rounded to float; near the ends of the float range, where
-// pair_div's remainder would be lost, in FP64.
+// a / b of two normalised pairs rounded to float; in FP64 where pair_div's remainder would be lost:
+// the head's product reaches 47 bits below a (normal down to 2^-149), and the quotient must be normal.
 __device__ __forceinline__ float quotient(Acc a, Acc b) {
     const float ma = fabsf(a.s), mb = fabsf(b.s);
-    if (ma >= 0x1p-60f && ma <= 0x1p60f && mb >= 0x1p-60f && mb <= 0x1p60f) return pair_div(a, b);
+    if (ma >= 0x1p-90f && ma <= 0x1p90f && mb >= 0x1p-90f && mb <= 0x1p90f) {
+        const float q = pair_div(a, b), mq = fabsf(q);
+        if (mq >= 0x1p-100f && mq <= 0x1p100f) return q;
+    }
     return (float)(((double)a.s + (double)a.c) / ((double)b.s + (double)b.c));
 }
 
-// d = r + beta d (not in the first phase, IMP:327); the term of d.(A d).
+// The dot products' terms are FP32, and a solve whose terms are finite goes on even where their
+// total lies beyond FLT_MAX.  So each term is scaled by a power of two, at most one over the number of
+// vertices (sum_scale), and no sum of finite terms overflows; the scalars that come from the sums
+// (delta, threshold) carry the same factor, their quotients do not.  It is exact but for totals below
+// about 2^-101 / scale, whose pairs reach below the smallest float.
+
+// d = r + beta d (not in the first phase, IMP:327); the term of d.(A d) times scale.
 __device__ __forceinline__ void dir_vertex(const float (&A)[6], const float (&r)[3], float (&d)[3], bool first,
-                                           float beta, Acc& part) {
+                                           float beta, float scale, Acc& part) {
     if (!first) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) d[k] = r[k] + d[k] * beta;
     }
     float q0, q1, q2;
     matvec(A, d[0], d[1], d[2], q0, q1, q2);
-    acc_add(part, d[0] * q0 + d[1] * q1 + d[2] * q2);
+    acc_add(part, (d[0] * q0 + d[1] * q1 + d[2] * q2) * scale);
 }
 
-// r = r - alpha A d (IMP:323); the term of r.r.
+// r = r - alpha A d (IMP:323); the term of r.r times scale.
 __device__ __forceinline__ void res_vertex(const float (&A)[6], float (&r)[3], const float (&d)[3], float alpha,
-                                           Acc& part) {
+                                           float scale, Acc& part) {
     float q[3];
     matvec(A, d[0], d[1], d[2], q[0], q[1], q[2]);
 #pragma unroll
     for (int k = 0; k < 3; ++k) r[k] = r[k] - q[k] * alpha;
-    acc_add(part, r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
+    acc_add(part, (r[0] * r[0] + r[1] * r[1] + r[2] * r[2]) * scale);
 }
 
 }  // namespace

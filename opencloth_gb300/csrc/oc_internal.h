@@ -259,6 +259,13 @@ cudaError_t launch_test_cr_arith(unsigned long long* counts, uint64_t n_pairs, u
 // lies in one CTA's range of the concatenated streamed vertices; its slots are runs of up to
 // kPersistThreads of its vertices.
 constexpr int kPersistThreads = 256;
+// The factor of the sums over n vertices or rows that CTAs exchange as float pairs: the power of two
+// at most 1 / n (see dir_vertex).
+inline float sum_scale(int64_t n) {
+    float s = 1.0f;
+    for (; n > 1; n = (n + 1) / 2) s *= 0.5f;
+    return s;
+}
 constexpr int kPersistMaxCluster = 16;
 constexpr int kPersistPieceBytes = 336;  // shared memory of one piece's scalars
 struct PersistPiece {
@@ -275,6 +282,7 @@ struct PersistPiece {
     // packets (the cluster size x clusters of them).
     int32_t clusters, k, packet;
     int32_t full;          // 1: every CTA of those clusters has a piece of the cloth
+    float scale;           // of the cloth's sums (sum_scale)
 };
 struct PersistCtl {
     uint32_t base;  // tags up to base have been used by earlier launches
@@ -328,7 +336,7 @@ struct CplPiece {
     int32_t n, inst;
     int32_t idx, np;  // this CTA among its cloth's np CTAs
     int32_t packet;   // the cloth's first packet
-    int32_t pad_;
+    float scale;      // of the cloth's sums (sum_scale)
 };
 struct CplPlan {
     const CplPiece* pieces;  // one per CTA

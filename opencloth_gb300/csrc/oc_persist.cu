@@ -83,8 +83,8 @@ __device__ __forceinline__ bool clusters_as_planned(const PersistPlan& P) {
 // another CTA), and the scalars of its cloth.
 struct PieceState {
     ulonglong2 box[2][kWarps];
-    Acc dn, thresh;  // delta_new, eps^2 delta0
-    Acc dq;          // the last d.(A d)
+    Acc dn, thresh;  // delta_new, eps^2 delta0, each times the piece's scale
+    Acc dq;          // the last d.(A d), likewise
     double d0;
     float scal[2];   // beta or alpha of the phase of that parity
     float alpha, beta;
@@ -160,8 +160,8 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
 #pragma unroll
         for (int i = 0; i < kWarps; ++i) st[j].box[0][i] = st[j].box[1][i] = none;
         st[j].d0 = d0;
-        st[j].dn = pair_from(__ldcg(&is.delta_new));
-        st[j].thresh = pair_from((double)ip.eps2 * d0);
+        st[j].dn = pair_from(__ldcg(&is.delta_new) * pieces[j].scale);
+        st[j].thresh = pair_from((double)ip.eps2 * d0 * pieces[j].scale);
         st[j].dq = acc_zero();
         st[j].alpha = st[j].beta = 0.0f;
         st[j].it = __ldcg(&is.iter);
@@ -231,8 +231,8 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
                     fl |= OC_FLAG_NON_FINITE;
                     run = false;
                 }
-                st[j].dn = pair_from(total);
-                st[j].thresh = pair_from((double)ip.eps2 * total);
+                st[j].dn = pair_from(total * pieces[j].scale);
+                st[j].thresh = pair_from((double)ip.eps2 * total * pieces[j].scale);
                 st[j].d0 = total;
                 st[j].it = 0;
                 st[j].fl = fl;
@@ -261,15 +261,15 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
         for (int j = 0; j < np; ++j) {
             if (!st[j].run[cur]) continue;
             const int b = pieces[j].slot0, e = pieces[j].slot1, n = pieces[j].n;
-            const float scal = st[j].scal[cur];
+            const float scal = st[j].scal[cur], scale = pieces[j].scale;
             Acc part = acc_zero();
 #pragma unroll
             for (int u = 0; u < kRegSlots; ++u) {
                 if (u < b || u >= e) continue;  // a slot's lanes past its end hold zeros, whose terms are zeros
                 if (dir)
-                    dir_vertex(A[u], r[u], d[u], first, scal, part);
+                    dir_vertex(A[u], r[u], d[u], first, scal, scale, part);
                 else
-                    res_vertex(A[u], r[u], d[u], scal, part);
+                    res_vertex(A[u], r[u], d[u], scal, scale, part);
             }
 #pragma unroll 2
             for (int s = max(b, kRegSlots); s < min(e, s_end); ++s) {
@@ -284,13 +284,13 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
                     ds[k] = p[(9 + k) * kPT];
                 }
                 if (dir) {
-                    dir_vertex(As, rs, ds, first, scal, part);
+                    dir_vertex(As, rs, ds, first, scal, scale, part);
                     if (!first) {
 #pragma unroll
                         for (int k = 0; k < 3; ++k) p[(9 + k) * kPT] = ds[k];
                     }
                 } else {
-                    res_vertex(As, rs, ds, scal, part);
+                    res_vertex(As, rs, ds, scal, scale, part);
 #pragma unroll
                     for (int k = 0; k < 3; ++k) p[(6 + k) * kPT] = rs[k];
                 }
@@ -307,13 +307,13 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
                     ds[k] = a.d[k][g];
                 }
                 if (dir) {
-                    dir_vertex(As, rs, ds, first, scal, part);
+                    dir_vertex(As, rs, ds, first, scal, scale, part);
                     if (!first) {
 #pragma unroll
                         for (int k = 0; k < 3; ++k) a.d[k][g] = ds[k];
                     }
                 } else {
-                    res_vertex(As, rs, ds, scal, part);
+                    res_vertex(As, rs, ds, scal, scale, part);
 #pragma unroll
                     for (int k = 0; k < 3; ++k) a.r[k][g] = rs[k];
                 }
@@ -513,8 +513,9 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist(const StepArgs a, const P
             const PieceState& ps = st[j];
             InstState& is = a.state[pieces[j].inst];
             is.delta0 = ps.d0;
-            is.delta_new = (double)ps.dn.s + (double)ps.dn.c;
-            is.dq = (double)ps.dq.s + (double)ps.dq.c;
+            const double unit = 1.0f / pieces[j].scale;  // (a power of two)
+            is.delta_new = ((double)ps.dn.s + (double)ps.dn.c) * unit;
+            is.dq = ((double)ps.dq.s + (double)ps.dq.c) * unit;
             is.alpha = ps.alpha;
             is.beta = ps.beta;
             is.iter = ps.it;
@@ -553,6 +554,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
     const int n = pc.n, e = pc.slot1;
     const int64_t v = pc.v + tid;
     const bool upd = !a.cg_only;
+    const float scale = pc.scale;
 
     if (tid < 2) s_ok[tid] = 1;
     for (int i = tid; i < 2 * kMaxCluster * kWarps; i += kPT) (&s_box[0][0])[i] = empty_packet(base);
@@ -597,7 +599,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
                 V[u] = a.V[g];
             }
     }
-    // Warp 0's scalars (every lane): delta_new, the threshold, the last d.(A d).
+    // Warp 0's scalars (every lane): delta_new, the threshold, the last d.(A d), each times scale.
     Acc dn = acc_zero(), thresh = acc_zero(), dq = acc_zero();
     double d0 = 0.0;
     float alpha = 0.0f, beta = 0.0f;
@@ -610,7 +612,7 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
             const double total = strip_delta0<kWarps>(a, ip);
             if (w == 0) {
                 d0 = __shfl_sync(0xffffffffu, total, 0);
-                dn = pair_from(d0);
+                dn = pair_from(d0 * scale);
                 go = (0 < ip.imax) && (d0 > (double)ip.eps2 * d0);
                 if (!isfinite(d0)) {
                     fl |= OC_FLAG_NON_FINITE;
@@ -620,12 +622,12 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
         } else if (w == 0) {
             const InstState& is = a.state[pc.inst];
             d0 = __ldcg(&is.delta0);
-            dn = pair_from(__ldcg(&is.delta_new));
+            dn = pair_from(__ldcg(&is.delta_new) * scale);
             it = __ldcg(&is.iter);
             fl = __ldcg(&is.flags);
             go = __ldcg(&is.active) != 0;
         }
-        thresh = pair_from((double)ip.eps2 * d0);
+        thresh = pair_from((double)ip.eps2 * d0 * scale);
         imax = ip.imax;
     }
     if (tid == 0) {
@@ -659,10 +661,10 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
         if (dir) {
             const bool first = q == 0;
 #pragma unroll
-            for (int u = 0; u < KR; ++u) dir_vertex(A[u], r[u], d[u], first, scal, part);
+            for (int u = 0; u < KR; ++u) dir_vertex(A[u], r[u], d[u], first, scal, scale, part);
         } else {
 #pragma unroll
-            for (int u = 0; u < KR; ++u) res_vertex(A[u], r[u], d[u], scal, part);
+            for (int u = 0; u < KR; ++u) res_vertex(A[u], r[u], d[u], scal, scale, part);
         }
         if constexpr (!FULL) {
 #pragma unroll 2
@@ -678,13 +680,13 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
                     ds[k] = p[(9 + k) * kPT];
                 }
                 if (dir) {
-                    dir_vertex(As, rs, ds, q == 0, scal, part);
+                    dir_vertex(As, rs, ds, q == 0, scal, scale, part);
                     if (q > 0) {
 #pragma unroll
                         for (int k = 0; k < 3; ++k) p[(9 + k) * kPT] = ds[k];
                     }
                 } else {
-                    res_vertex(As, rs, ds, scal, part);
+                    res_vertex(As, rs, ds, scal, scale, part);
 #pragma unroll
                     for (int k = 0; k < 3; ++k) p[(6 + k) * kPT] = rs[k];
                 }
@@ -701,13 +703,13 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
                     ds[k] = a.d[k][g];
                 }
                 if (dir) {
-                    dir_vertex(As, rs, ds, q == 0, scal, part);
+                    dir_vertex(As, rs, ds, q == 0, scal, scale, part);
                     if (q > 0) {
 #pragma unroll
                         for (int k = 0; k < 3; ++k) a.d[k][g] = ds[k];
                     }
                 } else {
-                    res_vertex(As, rs, ds, scal, part);
+                    res_vertex(As, rs, ds, scal, scale, part);
 #pragma unroll
                     for (int k = 0; k < 3; ++k) a.r[k][g] = rs[k];
                 }
@@ -875,8 +877,9 @@ __global__ void __launch_bounds__(kPT, 1) k_cg_persist_one(const StepArgs a, con
         if (whole && pc.head && n > 0) {
             InstState& is = a.state[pc.inst];
             is.delta0 = d0;
-            is.delta_new = (double)dn.s + (double)dn.c;
-            is.dq = (double)dq.s + (double)dq.c;
+            const double unit = 1.0f / scale;  // (a power of two)
+            is.delta_new = ((double)dn.s + (double)dn.c) * unit;
+            is.dq = ((double)dq.s + (double)dq.c) * unit;
             is.alpha = alpha;
             is.beta = beta;
             is.iter = it;

@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
             const float alpha = s_scal;
             Acc part = acc_zero();
 #pragma unroll
-            for (int u = 0; u < VPT; ++u) res_vertex(A[u], r[u], d[u], alpha, part);
+            for (int u = 0; u < VPT; ++u) res_vertex(A[u], r[u], d[u], alpha, 1.0f, part);
             ++tag;
             send(part, 0);
 #pragma unroll
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
             const float beta = s_scal;
             part = acc_zero();
 #pragma unroll
-            for (int u = 0; u < VPT; ++u) dir_vertex(A[u], r[u], d[u], false, beta, part);
+            for (int u = 0; u < VPT; ++u) dir_vertex(A[u], r[u], d[u], false, beta, 1.0f, part);
             ++tag;
             send(part, 0);
             if (w == 0) {
