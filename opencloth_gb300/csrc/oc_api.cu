@@ -1123,6 +1123,13 @@ oc_status plan_sim(oc_solver* s) {
 // kPersistMaxCluster when those, which leave some SMs idle, hold every vertex on chip, else of
 // 2 (see oc_persist.cu for the exchanges' times).  Left without a grid when the device has no
 // cooperative launch or a CTA would hold too many pieces.
+//
+// CTAs of their own are uneven where a large cloth stands beside many small ones, which leave it few: the
+// launch takes as long as the largest, so they are taken while that is near the even share.  Measured, us a
+// step, without and with that limit: 1000 x 1000 with 151 of 130 x 130 18,900 / 663, with 125 964 / 559,
+// with 100 522 / 480; 90 of 130 x 130 (1.7 times the even share) 362 / 228; within it, 60 of them 150.
+bool own_ctas(int64_t chunk, int64_t even) { return 5 * chunk <= 7 * even || chunk <= even + kPersistThreads; }
+
 oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_t>& ids) {
     PersistPlan& P = *plan;
     P.grid = 0;
@@ -1137,17 +1144,21 @@ oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_
         cta_piece.assign(1, 0);
         P.cluster = cluster;
         P.n_packets = 0;
-        P.one = (int64_t)ids.size() <= most;
         int64_t want = std::min(most, (total + kPersistThreads - 1) / kPersistThreads);
         want = std::min(most, (want + cluster - 1) / cluster * cluster);
-        int64_t chunk = ((total + want - 1) / want + 31) / 32 * 32;
+        const int64_t even = ((total + want - 1) / want + 31) / 32 * 32;
+        int64_t chunk = even;
         auto ctas_of = [&](int32_t k) { return (s->inst_host[(size_t)k].nv + chunk - 1) / chunk; };
-        if (P.one)
+        P.one = (int64_t)ids.size() <= most;
+        if (P.one) {
             for (;; chunk += 32) {
                 int64_t n = 0;
                 for (int32_t k : ids) n += ctas_of(k);
                 if (n <= most) break;
             }
+            P.one = own_ctas(chunk, even);
+            if (!P.one) chunk = even;
+        }
         int32_t open_slots = 0, max_slots = 0;  // of the CTA being filled, of any
         int64_t open_n = 0;
         auto close = [&] {
@@ -1317,7 +1328,7 @@ bool may_join(const oc_solver* s) {
         for (const InstParams& ip : s->inst_host) n += (ip.nv + chunk - 1) / chunk;
         if (n <= most) break;
     }
-    return 5 * chunk <= 7 * even || chunk <= even + kPersistThreads;
+    return own_ctas(chunk, even);
 }
 
 // Whether the cloths small enough for the resident kernel stream too.  (a) Others of the handle do:
