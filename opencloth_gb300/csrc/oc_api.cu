@@ -113,6 +113,9 @@ struct oc_solver {
     PersistPlan aplan{};
     bool aplan_made = false;
     PersistPlan pplan{};  // the streamed REFERENCE cloths' pieces (grid 0: none, or not available)
+    bool arrive = false;  // their CG runs in k_cg_arrive, their state in memory
+    int arrive_per_sm = 0;
+    unsigned* d_words = nullptr;  // k_cg_arrive: one arrival count per cloth
     // k_assemble_finish runs when a strip-swept cloth is resident or the streamed CG is
     // not the persistent one; otherwise k_cg_persist forms their delta0 itself.
     bool strip_finish = true;
@@ -247,6 +250,16 @@ oc_status report_device_error(oc_solver* s, int h) {
                     "a wait between CTAs gave up (cloths whose solve had not ended were not updated)");
     }
     return OC_OK;
+}
+
+// The CG of the streamed REFERENCE cloths (a.blocks their table) in one cooperative launch.
+int arrive_grid(const oc_solver* s) { return std::min(s->arrive_per_sm * s->sm_count, std::max(1, s->n_streamed_blocks)); }
+
+cudaError_t persist_cg(oc_solver* s, const StepArgs& a) {
+    if (!s->arrive) return launch_cg_persist(a, s->pplan, s->stream);
+    const cudaError_t e = cudaMemsetAsync(s->d_words, 0, sizeof(unsigned) * (size_t)s->n_inst, s->stream);
+    if (e != cudaSuccess) return e;
+    return launch_cg_arrive(a, s->n_streamed_blocks, arrive_grid(s), s->d_words, s->d_perr, s->stream);
 }
 
 constexpr int kResidentDefaultVcta = 1024;  // vertices of a resident CTA
@@ -415,8 +428,8 @@ void account_step_bytes(const oc_solver* s, KernelTimer* t) {
         const double it = (double)st.iter;
         double dirs = it > 0 ? 36.0 * nv + 60.0 * nv * (it - 1.0) : 0.0;
         if (st.flags & OC_FLAG_BREAKDOWN) dirs += (it > 0 ? 60.0 : 36.0) * nv;
-        if (s->persist) {  // k_cg_persist: the same passes and the update in one launch
-            t->bytes[K_CG_PERSIST] += dirs + 84.0 * nv * it + 76.0 * nv;
+        if (s->persist) {  // the same passes and the update in one launch
+            t->bytes[s->arrive ? K_CG_ARRIVE : K_CG_PERSIST] += dirs + 84.0 * nv * it + 76.0 * nv;
             continue;
         }
         t->bytes[K_INTEGRATE] += 76.0 * nv;
@@ -547,11 +560,10 @@ oc_status step_host_driven(oc_solver* s, float dt, bool per_cloth, KernelTimer* 
         if ((st = launch_resident_all(s, a, t)) != OC_OK) return st;
         const int nb = s->n_streamed_blocks, nc = s->n_cpl_blocks;
         if (s->persist || s->cpl_persist) {  // (not both: k_cpl_persist wants every other cloth resident)
-            const KernelKind k = s->persist ? K_CG_PERSIST : K_CPL_PERSIST;
+            const KernelKind k = !s->persist ? K_CPL_PERSIST : s->arrive ? K_CG_ARRIVE : K_CG_PERSIST;
             if (t) OC_TRY(cudaEventRecord(t->ev[0], s->stream));
             sa.persist_d0 = 1;
-            OC_TRY(s->persist ? launch_cg_persist(sa, s->pplan, s->stream)
-                              : launch_cpl_persist(ca, s->cplan, s->stream));
+            OC_TRY(s->persist ? persist_cg(s, sa) : launch_cpl_persist(ca, s->cplan, s->stream));
             s->host_launches += 1;
             if (t) {
                 OC_TRY(cudaEventRecord(t->ev[1], s->stream));
@@ -721,12 +733,11 @@ oc_status build_graph(oc_solver* s, float dt) {
         pa.blocks = s->d_streamed_blocks;
         pa.use_cond = 0;
         pa.persist_d0 = 1;
-        cudaError_t le = persist ? launch_cg_persist(pa, s->pplan, s->stream)
-                                 : launch_cpl_persist(ca, s->cplan, s->stream);
+        cudaError_t le = persist ? persist_cg(s, pa) : launch_cpl_persist(ca, s->cplan, s->stream);
         cudaError_t ce = cudaStreamEndCapture(s->stream, &pg);
         if (le != cudaSuccess || ce != cudaSuccess) {
             if (pg) cudaGraphDestroy(pg);
-            return fail_cuda(s, le != cudaSuccess ? le : ce, persist ? "capture of k_cg_persist" : "capture of k_cpl_persist");
+            return fail_cuda(s, le != cudaSuccess ? le : ce, "capture of the CG's launch");
         }
         cudaError_t e = cudaGraphAddChildGraphNode(&n_pc, g, prev.data(), prev.size(), pg);
         cudaGraphDestroy(pg);
@@ -838,7 +849,7 @@ StepArgs gm_args(const oc_solver* s, float dt) {
 // The CG alone (no update) of every cloth, from the CG state set up in the planes and
 // the cloths' states: in one cooperative launch of k_cg_persist where plan_adjoint made one, else the
 // resident cloths on chip (k_resident unfused, one launch per bucket, beside) and the streamed ones in
-// k_cg_persist.
+// k_cg_persist or k_cg_arrive.
 oc_status solve_only(oc_solver* s, const StepArgs& a) {
     StepArgs pa = a;
     pa.cg_only = 1;
@@ -849,8 +860,9 @@ oc_status solve_only(oc_solver* s, const StepArgs& a) {
     }
     if (!s->buckets.empty())
         if (oc_status r = launch_resident_all(s, pa, nullptr)) return r;
-    if (s->pplan.grid > 0) {
-        OC_TRY(launch_cg_persist(pa, s->pplan, s->stream));
+    if (s->pplan.grid > 0 || s->arrive) {
+        pa.blocks = s->d_streamed_blocks;
+        OC_TRY(persist_cg(s, pa));
         s->host_launches += 1;
     }
     return OC_OK;
@@ -1129,6 +1141,20 @@ oc_status plan_sim(oc_solver* s) {
 // step, without and with that limit: 1000 x 1000 with 151 of 130 x 130 18,900 / 663, with 125 964 / 559,
 // with 100 522 / 480; 90 of 130 x 130 (1.7 times the even share) 362 / 228; within it, 60 of them 150.
 bool own_ctas(int64_t chunk, int64_t even) { return 5 * chunk <= 7 * even || chunk <= even + kPersistThreads; }
+
+// Whether k_cg_persist is the faster for a plan, and not k_cg_arrive, which streams the CG state with four
+// CTAs an SM: k_cg_persist holds 33 slots of a CTA (30 with several pieces) on chip, and its one CTA an SM
+// is slow with those that stay in the planes and with every piece.  Measured, us a step, k_cg_persist /
+// k_cg_arrive: one cloth of 1025 x 1025 (28 slots) 130 / 151, 1400 x 1400 (51) 281 / 287, 1500 x 1500 (58)
+// 337 / 332, 2000 x 2000 (103) 965 / 589; 130 of 130 x 130 (67, a CTA each) 410 / 389; with several pieces a
+// CTA, 90 of 130 x 130 (40) 229 / 279, 20 of 130 to 400 a side (40) 223 / 223, 110 of 130 x 130 (49) 385 / 320,
+// 300 of 130 x 130 (131) 1,107 / 768; 2,000 of 8 to 24 a side (19, 14 pieces) 202 / 200, 3,000 of them (28, 21
+// pieces) 340 / 267.
+constexpr int32_t kOnChipSlotsOne = 56, kOnChipSlots = 44;  // (the latter with the pieces)
+
+bool on_chip_enough(const PersistPlan& P) {
+    return P.grid > 0 && (P.one ? P.max_slots <= kOnChipSlotsOne : P.max_slots + P.max_pieces <= kOnChipSlots);
+}
 
 oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_t>& ids) {
     PersistPlan& P = *plan;
@@ -1469,13 +1495,21 @@ oc_status plan_execution(oc_solver* s) {
     std::vector<int32_t> streamed_ids;
     for (int32_t k = 0; k < s->n_inst; ++k)
         if (!s->resident[(size_t)k]) streamed_ids.push_back(k);
-    if (any_streamed && !any_coupled)
+    s->arrive = false;
+    if (any_streamed && !any_coupled) {
         if (oc_status r = plan_persist(s, &s->pplan, streamed_ids)) return r;
-    s->persist = cfg.persist && s->pplan.grid > 0;
+        s->arrive = !on_chip_enough(s->pplan) && s->coop && s->arrive_per_sm > 0 &&
+                    s->n_streamed_blocks <= (int64_t)arrive_max_entries_per_block() * arrive_grid(s);
+        if (s->arrive && !s->d_words) OC_TRY(dalloc(s, &s->d_words, (size_t)s->n_inst));
+        if (s->arrive)
+            if (oc_status r = alloc_error_word(s)) return r;
+    }
+    const bool one_launch = s->pplan.grid > 0 || s->arrive;
+    s->persist = cfg.persist && one_launch;
     if (any_coupled)
         if (oc_status r = plan_coupled(s)) return r;
     s->cpl_persist = cfg.persist && s->cplan.grid > 0;
-    s->adj_persist = s->adj_allowed && s->persist_smem_max > 0 && !any_coupled && (!any_streamed || s->pplan.grid > 0);
+    s->adj_persist = s->adj_allowed && s->persist_smem_max > 0 && !any_coupled && (!any_streamed || one_launch);
     if (oc_status r = plan_sim(s)) return r;
     s->strip_finish = false;
     for (int32_t k = 0; k < s->n_inst; ++k)
@@ -1757,7 +1791,8 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
         a.r[k] = planes + (9 + k) * stride;
         a.d[k] = planes + (12 + k) * stride;
     }
-    OC_CREATE_TRY(dalloc(s, &a.partials, P.blocks.size()));
+    OC_CREATE_TRY(dalloc(s, &a.partials, 2 * P.blocks.size()));
+    a.partials_b = a.partials + P.blocks.size();
     InstParams* inst = nullptr;
     OC_CREATE_TRY(upload(s, &inst, P.inst));
     a.inst = inst;
@@ -1841,6 +1876,7 @@ oc_status oc_create(const oc_cloth_desc* descs, int32_t n_instances, const oc_op
         s->coop = coop != 0;
         if (s->coop && s->executor != OC_EXEC_PLAIN && s->any_coupled) OC_CREATE_TRY(prepare_coupled(s->device, &s->cpl_rows_max));
         if (s->coop && s->executor != OC_EXEC_PLAIN) OC_CREATE_TRY(prepare_persist(s->device, &s->persist_smem_max, &s->persist_clusters, &s->persist_pairs));
+        s->arrive_per_sm = s->executor != OC_EXEC_PLAIN ? arrive_blocks_per_sm() : 0;
         if (s->executor != OC_EXEC_PLAIN) OC_CREATE_TRY(prepare_sim(s->device, &s->sim_smem_max));
         s->adj_allowed = !(pe && std::atoi(pe) == 0) && s->coop;
         s->h_blocks = P.blocks;
@@ -2358,7 +2394,7 @@ oc_status oc_profile_steps(oc_solver* s, float dt, int32_t n_steps, int32_t max_
     cudaEventDestroy(t.ev[1]);
     if (st != OC_OK) return st;
     const KernelKind kinds[] = {K_ASSEMBLE, K_ASSEMBLE_GRID, K_ASSEMBLE_KINDS, K_ASSEMBLE_STRIP, K_ASSEMBLE_FINISH, K_CG_DIR,
-                                K_CG_UPDATE, K_INTEGRATE, K_CG_PERSIST, K_RESIDENT, K_PROVOT,
+                                K_CG_UPDATE, K_INTEGRATE, K_CG_PERSIST, K_CG_ARRIVE, K_RESIDENT, K_PROVOT,
                                 K_CPL_ASSEMBLE, K_CPL_DIR, K_CPL_UPDATE, K_CPL_PERSIST};
     int32_t n = 0;
     for (KernelKind k : kinds) {
@@ -2368,7 +2404,7 @@ oc_status oc_profile_steps(oc_solver* s, float dt, int32_t n_steps, int32_t max_
         if ((k == K_ASSEMBLE_GRID || k == K_ASSEMBLE_KINDS) &&
             (s->n_grid_blocks == 0 || k != (s->executor == OC_EXEC_PLAIN ? K_ASSEMBLE_GRID : s->grid_kind)))
             continue;
-        if (k == K_CG_PERSIST && !s->persist) continue;
+        if ((k == K_CG_PERSIST || k == K_CG_ARRIVE) && (!s->persist || s->arrive != (k == K_CG_ARRIVE))) continue;
         if (k == K_CPL_PERSIST && !s->cpl_persist) continue;
         if ((k == K_CPL_DIR || k == K_CPL_UPDATE || k == K_INTEGRATE) && s->cpl_persist) continue;
         if ((k == K_CG_DIR || k == K_CG_UPDATE || k == K_INTEGRATE) && s->persist) continue;
@@ -2637,7 +2673,9 @@ oc_status plan_adjoint(oc_solver* s) {
     if (s->buckets.size() < 3 && (s->n_inst > 1 || s->inst_host[0].nv <= kResidentDefaultVcta)) return OC_OK;
     std::vector<int32_t> ids((size_t)s->n_inst);
     for (int32_t k = 0; k < s->n_inst; ++k) ids[(size_t)k] = k;
-    return plan_persist(s, &s->aplan, ids);
+    if (oc_status r = plan_persist(s, &s->aplan, ids)) return r;
+    if (!on_chip_enough(s->aplan)) s->aplan.grid = 0;
+    return OC_OK;
 }
 
 // Chooses the tape and its intervals, allocates it and runs the taped forward.

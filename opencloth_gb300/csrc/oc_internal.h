@@ -104,6 +104,7 @@ struct StepArgs {
     float* r[3];
     float* d[3];
     double* partials;        // one per streamed block
+    double* partials_b;      // a second set (k_cg_arrive's phases of odd parity)
     const InstParams* inst;
     InstState* state;
     const BlockInfo* blocks;
@@ -118,8 +119,8 @@ struct StepArgs {
     int32_t all_streamed;    // 1: every cloth's CG runs in the streamed loop (adjoint solves)
     int32_t cg_only;         // k_cg_persist: 1 = the CG alone, no update (adjoint solves)
     int32_t persist_d0;      // k_cg_persist: 1 = it forms its strip-swept cloths' delta0 (the step's launch)
-    // The waits of CTAs for one another's packets: polls before a wait gives up, and a block that
-    // sends none (-1: no such block; set only by oc_test_barrier_timeout).
+    // The waits of CTAs for one another's packets or arrivals: polls before a wait gives up, and a block
+    // that sends none (-1: no such block; set only by oc_test_barrier_timeout).
     uint32_t barrier_polls;
     int32_t withhold_block;
     // Kernel variants of this handle: the incidence-record gather of k_assemble (0 block
@@ -251,8 +252,16 @@ __host__ __device__ inline int stencil_class_1d(int32_t i, int32_t n) {
 enum KernelKind { K_ASSEMBLE = 0, K_CG_DIR = 1, K_CG_UPDATE = 2, K_INTEGRATE = 3, K_FORCES = 4, K_RESIDENT = 5,
                   K_PROVOT = 6, K_ELLIPSOID = 7, K_CPL_ASSEMBLE = 8, K_CPL_DIR = 9, K_CPL_UPDATE = 10,
                   K_ASSEMBLE_GRID = 11, K_CG_PERSIST = 12, K_ASSEMBLE_STRIP = 13, K_ASSEMBLE_FINISH = 14,
-                  K_CPL_PERSIST = 15, K_ASSEMBLE_KINDS = 16, K_COUNT = 17 };
+                  K_CPL_PERSIST = 15, K_ASSEMBLE_KINDS = 16, K_CG_ARRIVE = 17, K_COUNT = 18 };
 
+// The CG loop of the cloths of block table a.blocks[0, n_entries) in one cooperative launch of
+// `grid` blocks with the CG state in memory (k_cg_arrive, oc_kernels.cu), any number of cloths; a block
+// owns at most arrive_max_entries_per_block() entries.  words: one arrival count per cloth of the
+// handle, indexed by cloth, zeroed before each launch.  err: bit 0 set if a wait gave up.
+int arrive_max_entries_per_block();
+int arrive_blocks_per_sm();
+cudaError_t launch_cg_arrive(const StepArgs& a, int32_t n_entries, int grid, unsigned* words, int* err,
+                             cudaStream_t stream);
 cudaError_t launch_test_cr_arith(unsigned long long* counts, uint64_t n_pairs, uint64_t seed, cudaStream_t stream);
 // The persistent CG (k_cg_persist, oc_persist.cu): the whole CG loop and the update of the
 // streamed REFERENCE cloths in one cooperative launch.  A piece is the part of one cloth that

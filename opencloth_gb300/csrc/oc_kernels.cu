@@ -10,7 +10,9 @@
 //                the states in shared memory
 //   k_cg_dir     [d = r + beta d]; alpha = delta_new / d.(A d)    (IMP:320-321, 327)
 //   k_cg_update  x += alpha d; r -= alpha A d; delta_new = r.r     (IMP:322-326)
-//   (k_cg_persist, oc_persist.cu: the two passes above and the update in one launch)
+//   k_cg_arrive  the CG loop of any number of cloths and their update in one cooperative launch
+//                (the two passes above, per-cloth arrival counts); k_cg_persist (oc_persist.cu)
+//                where the CG state fits on chip
 //   k_integrate  V += dV dt; X += dt V; ground clamp               (IMP:790-797)
 //                [+ EllipsoidCollision, IMP:824-848]
 //   k_provot     ApplyProvotDynamicInverse as a per-vertex gather   (IMP:800-823)
@@ -32,6 +34,7 @@
 #include <cuda_runtime.h>
 
 #include "oc_device.cuh"
+#include "oc_exchange.cuh"
 #include "oc_internal.h"
 
 namespace oc {
@@ -727,6 +730,271 @@ __global__ void __launch_bounds__(kThreads) k_cg_update(const StepArgs a) {
     finish<K_CG_UPDATE>(a, bi.gblk, bi.inst, active, part);
 }
 
+// ---- the whole CG loop in one cooperative launch, the CG state in memory -----------------
+// k_cg_arrive runs every iteration of every cloth of its block table in one launch, all its
+// blocks co-resident (cooperative launch): what k_cg_persist (oc_persist.cu) does for cloths whose
+// state it holds on chip, for those that are too large for it (the rule and both sides' times:
+// on_chip_enough, oc_api.cu).  Block b
+// owns the table entries b, b + grid, b + 2 grid, ... and runs on them the same
+// per-block passes as k_cg_dir / k_cg_update, writing the same per-block partials.
+//
+// The cloths are independent, so there is no grid barrier: each cloth has its own word,
+// which counts the arrivals of its entries (it is never reset within the launch).  Phase
+// q of a cloth is the direction pass (q even) or the update pass (q odd) of iteration
+// q / 2.  Phase q - 1 of cloth c is complete once c's word reaches q nblk(c).  Then every
+// block that owns entries of c sums c's partials of phase q - 1 itself, in the
+// last-block epilogue's fixed order, and applies the epilogue's scalar rule to its own
+// copy of c's scalars in shared memory: all blocks compute the same totals and take the
+// same decisions, with no last block that has to publish them first.  The partials are
+// double buffered by phase parity: a block writes phase q + 1's only after phase q is
+// complete, that is after every block has read phase q - 1's.  The block owning c's first
+// entry writes c's state for the host.  Totals, scalars and decisions are those of the
+// two-kernel loop bit for bit.  Progress: a block waits at phase q only for cloths it
+// still runs, every owner of a running cloth makes its phase q - 1 arrival (one release
+// add per run of its consecutive entries of that cloth) before its phase-q wait, and all
+// blocks are co-resident.  A wait gives up after a.barrier_polls polls (the default,
+// 2^22 polls with a 32 ns back-off, is about half a second) or when another block has
+// given up: it sets bit 0 of *err and the block returns without its update.  The block
+// a.withhold_block (a testing aid; normally -1) returns before its first arrival, so the
+// waits on its cloths run out.
+
+constexpr int kPersistMaxOwn = kThreads;  // table entries one block owns (one waiting thread each)
+
+__device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned x) {
+    unsigned v;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "r"(x) : "memory");
+    return v;
+}
+
+// block_sum for blocks of at most 256 threads, with the same additions in the same order
+// (each warp's shuffle-down tree: lane l adds lane l + o for o = 16, 8, 4, 2, 1; then that
+// tree in warp 0 over the warps' sums), so the same bits.  The warps' trees run through
+// shared memory with the additions that reach the result packed into full warps: for 8
+// warps 4 + 2 + 1 + 1 + 1 FP64 warp instructions instead of 8 x 5, which matters when
+// every block of a grid forms the same total at once on GB300's slow FP64 pipe.
+__device__ double block_sum_packed(double v) {
+    __shared__ double buf[256];
+    const int t = threadIdx.x, nw = blockDim.x >> 5;
+    __syncthreads();  // warp 0 of a previous call may still read buf
+    buf[t] = v;
+    __syncthreads();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        // level o: in warp w, position l < o adds position l + o (reads never hit a write)
+        if (t < nw * o) {
+            const int i = (t / o) * 32 + t % o;
+            buf[i] = buf[i] + buf[i + o];
+        }
+        __syncthreads();
+    }
+    double r = 0.0;
+    if (t < 32) {
+        r = t < nw ? buf[t * 32] : 0.0;
+        r = warp_sum(r);
+    }
+    return r;
+}
+
+__global__ void __launch_bounds__(kThreads, 4) k_cg_arrive(const StepArgs a, int32_t n_entries, unsigned* words,
+                                                           int* err) {
+    __shared__ double s_part[kPersistMaxOwn];
+    __shared__ double s_dn[kPersistMaxOwn], s_d0[kPersistMaxOwn];  // delta_new, delta0
+    __shared__ float s_scal[kPersistMaxOwn];                        // beta or alpha for the next pass
+    __shared__ int s_it[kPersistMaxOwn];
+    __shared__ uint32_t s_fl[kPersistMaxOwn];
+    __shared__ unsigned char s_run[kPersistMaxOwn];  // 0 stopped, 1 runs, 2 runs its first direction pass
+    __shared__ unsigned char s_head[kPersistMaxOwn];  // first owned entry of a run of one cloth
+    __shared__ int s_any, s_ok;
+    const int own = ((int)n_entries - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    if (threadIdx.x == 0) s_ok = 1;
+    for (int j = threadIdx.x; j < own; j += blockDim.x) {
+        const int inst = a.blocks[blockIdx.x + j * gridDim.x].inst;
+        const InstState& st = a.state[inst];
+        s_head[j] = (j == 0 || a.blocks[blockIdx.x + (j - 1) * gridDim.x].inst != inst) ? 1 : 0;
+        s_run[j] = __ldcg(&st.active) ? 2 : 0;
+        s_dn[j] = __ldcg(&st.delta_new);
+        s_d0[j] = __ldcg(&st.delta0);
+        s_it[j] = __ldcg(&st.iter);
+        s_fl[j] = __ldcg(&st.flags);
+        s_scal[j] = 0.0f;
+    }
+    __syncthreads();
+    if (a.persist_d0) {
+        // The strip-swept cloths' delta0 and the decision to iterate, formed here as
+        // k_assemble_finish forms them (the step then launches that kernel only for the
+        // strip-swept cloths this launch does not run).
+        for (int j = 0; j < own; ++j) {
+            if (!s_head[j]) continue;
+            const BlockInfo bj = a.blocks[blockIdx.x + j * gridDim.x];
+            const InstParams& ip = a.inst[bj.inst];
+            if (!ip.strip) continue;
+            const double total = strip_delta0<kThreads / 32>(a, ip);
+            if (threadIdx.x == 0) {
+                uint32_t fl = 0u;
+                bool run = (0 < ip.imax) && (total > (double)ip.eps2 * total);
+                if (!isfinite(total)) {
+                    fl |= OC_FLAG_NON_FINITE;
+                    run = false;
+                }
+                for (int k = j; k < own && (k == j || !s_head[k]); ++k) {
+                    s_run[k] = run ? 2 : 0;
+                    s_dn[k] = total;
+                    s_d0[k] = total;
+                    s_it[k] = 0;
+                    s_fl[k] = fl;
+                    s_scal[k] = 0.0f;
+                }
+                if (bj.gblk == ip.blk0) {
+                    InstState& st = a.state[bj.inst];
+                    st.ticket = 0;
+                    st.delta0 = total;
+                    st.delta_new = total;
+                    st.dq = 0.0;
+                    st.alpha = 0.0f;
+                    st.beta = 0.0f;
+                    st.iter = 0;
+                    st.flags = fl;
+                    st.active = run ? 1 : 0;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    for (unsigned q = 0;; ++q) {
+        const bool dir = (q & 1u) == 0u;
+        if (q > 0) {
+            // Phase q - 1 of every running cloth: wait for its arrivals (one thread per run).
+            for (int j = threadIdx.x; j < own; j += blockDim.x) {
+                if (!s_run[j] || !s_head[j]) continue;
+                const BlockInfo bi = a.blocks[blockIdx.x + j * gridDim.x];
+                const unsigned need = q * (unsigned)a.inst[bi.inst].nblk;
+                unsigned spins = 0;
+                while ((int)(load_acquire(words + bi.inst) - need) < 0) {
+                    if (++spins > a.barrier_polls || ((spins & 63u) == 0 && load_relaxed(err) != 0)) {
+                        atomicOr(err, 1);
+                        s_ok = 0;
+                        break;
+                    }
+                    __nanosleep(32);
+                }
+            }
+            __syncthreads();
+            if (!s_ok) break;
+            // Totals and rule of phase q - 1, per run of one cloth, in every block.
+            const double* prev = (q & 1u) ? a.partials : a.partials_b;
+            for (int j = 0; j < own; ++j) {
+                if (!s_run[j] || !s_head[j]) continue;
+                const int inst = a.blocks[blockIdx.x + j * gridDim.x].inst;
+                const InstParams& ip = a.inst[inst];
+                double acc = 0.0;
+#pragma unroll 8
+                for (int k = threadIdx.x; k < ip.nblk; k += blockDim.x) acc += __ldcg(prev + ip.blk0 + k);
+                const double total = block_sum_packed(acc);  // block_sum's bits (kThreads = 256)
+                if (threadIdx.x == 0) {
+                    uint32_t fl = s_fl[j];
+                    int it = s_it[j];
+                    double dn = s_dn[j];
+                    float scal = 0.0f;
+                    bool run = true;
+                    if (!dir) {  // phase q - 1 was a direction pass: d.(A d) -> alpha
+                        if (!(total > 0.0) || !isfinite(total)) {
+                            fl |= isfinite(total) ? OC_FLAG_BREAKDOWN : OC_FLAG_NON_FINITE;
+                            run = false;
+                        } else {
+                            scal = (float)(dn / total);
+                        }
+                    } else {  // an update pass: r.r -> beta, the stop test
+                        it += 1;
+                        scal = (float)(total / dn);
+                        dn = total;
+                        const bool more = it < ip.imax && total > (double)ip.eps2 * s_d0[j];
+                        if (!isfinite(total)) fl |= OC_FLAG_NON_FINITE;
+                        if (!more || !isfinite(total)) {
+                            if (isfinite(total) && total > (double)ip.eps2 * s_d0[j]) fl |= OC_FLAG_NOT_CONVERGED;
+                            run = false;
+                        }
+                    }
+                    // The run's entries share the cloth's copy.
+                    for (int k = j; k < own && (k == j || !s_head[k]); ++k) {
+                        s_fl[k] = fl;
+                        s_it[k] = it;
+                        s_dn[k] = dn;
+                        s_scal[k] = scal;
+                        s_run[k] = run ? 1 : 0;
+                    }
+                    if (a.blocks[blockIdx.x + j * gridDim.x].gblk == ip.blk0) {  // the cloth's first entry
+                        InstState& st = a.state[inst];
+                        if (!dir) {
+                            st.dq = total;
+                            if (run) st.alpha = scal;
+                        } else {
+                            st.delta_new = dn;
+                            st.beta = scal;
+                            st.iter = it;
+                        }
+                        st.flags = fl;
+                        if (!run) st.active = 0;
+                        st.ticket = 0;
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        if (threadIdx.x == 0) {
+            int any = 0;
+            for (int j = 0; j < own; ++j) any |= s_run[j];
+            s_any = any;
+        }
+        __syncthreads();
+        if (!s_any) break;
+        // The passes of the owned entries that run.
+        for (int j = 0; j < own; ++j) {
+            if (!s_run[j]) continue;
+            const BlockInfo bi = a.blocks[blockIdx.x + j * gridDim.x];
+            const double bsum = block_sum_acc(dir ? cg_dir_block(a, bi, s_run[j] == 2, s_scal[j])
+                                                  : cg_update_block(a, bi, s_scal[j]));
+            if (threadIdx.x == 0) s_part[j] = bsum;
+        }
+        __syncthreads();
+        if ((int)blockIdx.x == a.withhold_block) {
+            s_ok = 0;
+            break;
+        }
+        // Arrivals: the partials of phase q into the buffer of its parity, then one release
+        // add per run of one cloth.
+        double* cur = (q & 1u) ? a.partials_b : a.partials;
+        for (int j = threadIdx.x; j < own; j += blockDim.x) {
+            if (!s_run[j] || !s_head[j]) continue;
+            const int inst = a.blocks[blockIdx.x + j * gridDim.x].inst;
+            unsigned n = 0;
+            for (int k = j; k < own; ++k) {
+                const BlockInfo bk = a.blocks[blockIdx.x + k * gridDim.x];
+                if (bk.inst != inst) break;
+                cur[bk.gblk] = s_part[k];
+                ++n;
+            }
+            atom_add_acq_rel(words + inst, n);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int j = 0; j < own; ++j)
+                if (s_run[j] == 2) s_run[j] = 1;
+        __syncthreads();
+    }
+    if (s_ok && !a.cg_only) {
+        for (int32_t e = blockIdx.x; e < n_entries; e += gridDim.x) {
+            const BlockInfo bi = a.blocks[e];
+            update_range(a, a.inst[bi.inst], bi.v_begin, bi.v_end);
+        }
+    }
+}
+
 // ---- the replay tape ---------------------------------------------------------------
 // Given the step's solution dV, the update (IMP:790-797) is elementwise: the forward
 // keeps dV of every step and a cloth's (X, V) every `every` steps, and the reverse pass
@@ -1111,6 +1379,7 @@ const char* kernel_name(KernelKind k) {
         case K_ASSEMBLE_GRID: return "k_assemble_grid";
         case K_ASSEMBLE_KINDS: return "k_assemble_kinds";
         case K_CG_PERSIST: return "k_cg_persist";
+        case K_CG_ARRIVE: return "k_cg_arrive";
         case K_ASSEMBLE_STRIP: return "k_assemble_strip";
         case K_ASSEMBLE_FINISH: return "k_assemble_finish";
         case K_CPL_DIR: return "k_cpl_dir";
@@ -1211,6 +1480,29 @@ cudaError_t launch_kernel(KernelKind k, const StepArgs& a, int nblocks, cudaStre
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
+}
+
+int arrive_max_entries_per_block() { return kPersistMaxOwn; }
+
+int arrive_blocks_per_sm() {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_cg_arrive, kThreads, 0) != cudaSuccess) return 0;
+    return n;
+}
+
+cudaError_t launch_cg_arrive(const StepArgs& a, int32_t n_entries, int grid, unsigned* words, int* err,
+                             cudaStream_t stream) {
+    if (grid <= 0 || (int64_t)n_entries > (int64_t)kPersistMaxOwn * grid) return cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)kThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_cg_arrive, a, n_entries, words, err);
 }
 
 cudaError_t launch_snapshot(const float4* X, const float4* V, float4* dX, float4* dV, const float* x, float* dx,
