@@ -1270,20 +1270,28 @@ oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_
 }
 
 // k_cpl_persist's plan: every COUPLED cloth on CTAs of its own, in proportion to its vertices and
-// with at least kCplMinRows each, where there are no more such cloths than SMs.  Streamed
+// with at least kCplMinRows each, where there are no more such cloths than SMs and the largest piece is
+// small enough: the launch takes as long as that, the loop of launches as the even share and its gaps.
+// Measured, us a step of four iterations, one launch / loop (largest piece, even share): one cloth of 500 x 500
+// (1,644) 123 / 189, 1025 x 1025 (6,912) 567 / 623, 1300 x 1300 (11,118) 937 / 914, 2000 x 2000 2,208 / 1,987;
+// 500 x 500 with 80 of 30 x 30 (3,472, 2,118) 252 / 274, with 100 (4,808, 2,237) 305 / 284, with 110 (5,952,
+// 2,296) 354 / 288; 200 x 200 with 140 (3,333, 1,092) 190 / 209, with 145 (5,714, 1,122) 251 / 214, with 151
+// 1,238 / 196; 100 of 100 x 75 (7,500, 4,934) 604 / 526.  Streamed
 // REFERENCE cloths beside them keep the WHILE loop of both (two cooperative launches of one CTA
 // per SM would run one behind the other).
 constexpr int64_t kCplMinRows = 256;
+bool cpl_pieces_small(int64_t piece, int64_t even) { return piece <= 7000 && 2 * piece <= 3 * even + 3400; }
 
 oc_status plan_coupled(oc_solver* s) {
     CplPlan& P = s->cplan;
     P.grid = 0;
     if (!s->coop || s->cpl_rows_max <= 0) return OC_OK;
-    int64_t total = 0;
+    int64_t total = 0, largest = 0;
     int32_t cloths = 0;
     for (const InstParams& ip : s->inst_host)
         if (ip.coupled) {
             total += ip.nv;
+            largest = std::max<int64_t>(largest, ip.nv);
             ++cloths;
         }
     if (cloths == 0 || cloths > s->sm_count || s->n_streamed_blocks > 0) return OC_OK;
@@ -1294,6 +1302,7 @@ oc_status plan_coupled(oc_solver* s) {
             if (ip.coupled) n += (ip.nv + chunk - 1) / chunk;
         if (n <= s->sm_count) break;
     }
+    if (!cpl_pieces_small(std::min(chunk, largest), (total + s->sm_count - 1) / s->sm_count)) return OC_OK;
     std::vector<CplPiece> pieces;
     P.n_packets = 0;
     int64_t most = 0;

@@ -6,7 +6,7 @@ import time
 import numpy as np
 import pytest
 
-from opencloth_gb300 import ClothDesc, ClothSolver, grid_cloth
+from opencloth_gb300 import JAC_COUPLED, ClothDesc, ClothSolver, grid_cloth
 
 pytestmark = pytest.mark.gpu
 DT = 1.0 / 60.0
@@ -48,3 +48,8 @@ def check_cloths(shapes, **kw):
 @pytest.mark.parametrize("large,count", [(700, 151), (700, 120), (300, 150), (400, 60)])
 def test_reference(large, count):
     check_cloths([(large, large)] + [(130, 130)] * count, cg_max_iter=200)
+
+
+@pytest.mark.parametrize("large,count", [(500, 150), (500, 60), (200, 151), (200, 120)])
+def test_coupled(large, count):
+    check_cloths([(large, large)] + [(30, 30)] * count, cg_max_iter=10, jacobian_mode=JAC_COUPLED)
