@@ -1011,8 +1011,14 @@ cudaError_t launch_bsr_persist(const oc_bsr_solver* s) {
 
 // k_bsr_persist's plan: every streamed system on CTAs of its own, in proportion to its rows and
 // with at least kBsrMinRows each (a CTA of few rows has idle warps, but its rows' chains of
-// dependent loads run side by side), where there are no more systems than SMs.
+// dependent loads run side by side), where there are no more systems than SMs and the largest piece is
+// small enough: the launch takes as long as that, the loop of launches as the even share and its gaps.
+// Measured, us a solve of 20 iterations, one launch / loop (largest piece, even share, rows): one system of
+// 216,000 rows (1,426) 566 / 899, of 1.89 M (12,442) 5,112 / 5,533; one of 40,625 with 130 of 833 rows (1,847, 980)
+// 441 / 854, with 140 (3,386, 1,035) 737 / 891, with 146 (6,771, 1,067) 1,220 / 880, with 151 6,458 / 860; one of 5,577
+// with 149 (1,859, 853) 370 / 834, with 151 (5,577, 864) 895 / 860; 14 of 40,625 with 86 (10,157, 4,213) 2,469 / 1,976.
 constexpr int64_t kBsrMinRows = 256;
+bool bsr_pieces_small(int64_t piece, int64_t even) { return 5 * piece <= 9 * even + 10000; }
 constexpr uint32_t kBsrPolls = 1u << 22;  // about a second
 
 oc_status plan_bsr_persist(oc_bsr_solver* s, const std::vector<BsrParams>& sys) {
@@ -1029,6 +1035,9 @@ oc_status plan_bsr_persist(oc_bsr_solver* s, const std::vector<BsrParams>& sys) 
         for (int32_t k : ids) n += (sys[k].n_rows + chunk - 1) / chunk;
         if (n <= sms) break;
     }
+    int64_t largest = 0;
+    for (int32_t k : ids) largest = std::max<int64_t>(largest, sys[k].n_rows);
+    if (!bsr_pieces_small(std::min(chunk, largest), (s->st_rows + sms - 1) / sms)) return OC_OK;
     std::vector<BsrPiece> pieces;
     int32_t packets = 0;
     s->persist_bytes = 0.0;

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from opencloth_gb300 import JAC_COUPLED, ClothDesc, ClothSolver, grid_cloth
+from opencloth_gb300.fem import BsrSolver, fem_system
 
 pytestmark = pytest.mark.gpu
 DT = 1.0 / 60.0
@@ -53,3 +54,20 @@ def test_reference(large, count):
 @pytest.mark.parametrize("large,count", [(500, 150), (500, 60), (200, 151), (200, 120)])
 def test_coupled(large, count):
     check_cloths([(large, large)] + [(30, 30)] * count, cg_max_iter=10, jacobian_mode=JAC_COUPLED)
+
+
+@pytest.mark.parametrize("count", [151, 120])
+def test_fem(count):
+    """(Without a graph the loop is driven from the host: the time is held against the large system's alone.)"""
+    large, small = fem_system(64, 24, 24), fem_system(16, 6, 6)
+
+    def solver(systems, **kw):
+        s = BsrSolver(systems, executor=1, **kw)
+        s.set_system(*(np.concatenate([g[k] for g in systems]) for k in ("blocks", "b", "V")))
+        s.solve()
+        return s
+
+    with solver([large] + [small] * count) as s, solver([large] + [small] * count, use_graph=False) as t, solver([large]) as u:
+        assert all(np.array_equal(a, b) for a, b in zip(s.solution(), t.solution()))
+        ts, tu = (best(x.solve, x.synchronize) for x in (s, u))
+    assert ts < 6 * tu, (ts, tu)
