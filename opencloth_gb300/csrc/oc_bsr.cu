@@ -344,10 +344,15 @@ __global__ void __launch_bounds__(kThreads) k_bsr_update(const BsrArgs a) {
 // record the neighbours gather; x passes through it during init); the blocks of the free rows
 // without padding, as two float4 planes and one of {component 8, 16 x local column} (a resident
 // system has at most 256 rows), with 32 more entries that a slot's idle lanes may read; and each
-// warp's offset of each slot (`stride` of them per warp, a multiple of kResSlots).
-__host__ __device__ constexpr int64_t resident_entries(int64_t nnzb) { return (nnzb + 32 + 7) / 8 * 8; }
-__host__ __device__ constexpr size_t resident_smem_bytes(int threads, int64_t nnzb, int stride) {
-    return 16 * (size_t)threads + 40 * (size_t)resident_entries(nnzb) + 4 * (size_t)(threads / 32) * stride;
+// warp's offset of each slot (`stride` of them per warp, a multiple of kResSlots).  PACKED, in a launch of
+// their own for systems that would not fit otherwise: component 8 and an 8-bit column in planes of their
+// own, 37 bytes a block, and no spare entries (idle lanes read entry 0).
+__host__ __device__ constexpr int64_t resident_entries(int64_t nnzb, bool packed) {
+    return packed ? (nnzb + 15) / 16 * 16 : (nnzb + 32 + 7) / 8 * 8;
+}
+__host__ __device__ constexpr size_t resident_smem_bytes(int threads, int64_t nnzb, int stride, bool packed) {
+    return 16 * (size_t)threads + (packed ? 37 : 40) * (size_t)resident_entries(nnzb, packed) +
+           4 * (size_t)(threads / 32) * stride;
 }
 constexpr int kResSlots = 4;    // slots of a row multiplied together in the resident loop
 constexpr int kResMaxDeg = 64;  // blocks of a resident system's longest row (bounds the offset table)
@@ -380,18 +385,21 @@ __device__ __forceinline__ bool pair_below(Acc v, float tiny) {
 // demo's 176 rows, 20 iterations: 238 -> 181 us (the pack is 8 to 11 us of each CTA's 60, an
 // iteration 5,500 cycles with three CTAs an SM and 4,000 alone).  Rows in the caller's order, whose
 // gathers have half the wavefronts, need nearly twice the slots (109 against 56) and took 243.
-__global__ void __launch_bounds__(kThreads, 3) k_bsr_resident(const BsrArgs a, const int32_t* ids, int64_t nnzb_max,
+template <bool PACKED>
+__global__ void __launch_bounds__(kThreads, PACKED ? 1 : 3) k_bsr_resident(const BsrArgs a, const int32_t* ids, int64_t nnzb_max,
                                                            const uint32_t* map, int stride) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_wcount[kThreads / 32];
     __shared__ Acc s_w0[8], s_w1[8], s_w2[8];
     static_assert(kThreads / 32 <= 8, "the totals take at most 8 warps");
-    const int64_t entries = resident_entries(nnzb_max);
+    const int64_t entries = resident_entries(nnzb_max, PACKED);
     float4* s_n4 = reinterpret_cast<float4*>(smem);
     float4* s_b0 = s_n4 + blockDim.x;
     float4* s_b1 = s_b0 + entries;
     float2* s_b2 = reinterpret_cast<float2*>(s_b1 + entries);
-    int* s_pre = reinterpret_cast<int*>(s_b2 + entries);
+    float* s_b8 = reinterpret_cast<float*>(s_b1 + entries);         // PACKED, in the place of s_b2
+    uint8_t* s_col = reinterpret_cast<uint8_t*>(s_b8 + entries);
+    int* s_pre = PACKED ? reinterpret_cast<int*>(s_col + entries) : reinterpret_cast<int*>(s_b2 + entries);
     constexpr unsigned kFull = 0xffffffffu;
 
     const int k = ids[blockIdx.x];
@@ -424,7 +432,12 @@ __global__ void __launch_bounds__(kThreads, 3) k_bsr_resident(const BsrArgs a, c
             const float* m = a.cblk + 9 * (size_t)e;
             s_b0[pos] = make_float4(m[0], m[1], m[2], m[3]);
             s_b1[pos] = make_float4(m[4], m[5], m[6], m[7]);
-            s_b2[pos] = make_float2(m[8], __int_as_float((int)(mp >> 16) * 16));
+            if constexpr (PACKED) {
+                s_b8[pos] = m[8];
+                s_col[pos] = (uint8_t)(mp >> 16);
+            } else {
+                s_b2[pos] = make_float2(m[8], __int_as_float((int)(mp >> 16) * 16));
+            }
         }
     }
     __syncthreads();
@@ -447,8 +460,11 @@ __global__ void __launch_bounds__(kThreads, 3) k_bsr_resident(const BsrArgs a, c
         const int pos[kResSlots] = {off.x + lane, off.y + lane, off.z + lane, off.w + lane};
 #pragma unroll
         for (int u = 0; u < kResSlots; ++u) {
-            const float4 b0 = s_b0[pos[u]], b1 = s_b1[pos[u]];
-            const float2 b2 = s_b2[pos[u]];
+            const int p = PACKED && j + u >= n ? 0 : pos[u];
+            const float4 b0 = s_b0[p], b1 = s_b1[p];
+            float2 b2;
+            if constexpr (PACKED) b2 = make_float2(s_b8[p], __int_as_float(s_col[p] * 16));
+            else b2 = s_b2[p];
             const int at = j + u < n ? __float_as_int(b2.y) : 0;
             const float4 nc = *reinterpret_cast<const float4*>(n4 + at);
             const float m[9] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w, b2.x};
@@ -926,13 +942,16 @@ struct oc_bsr_solver {
     unsigned long long* h_loop = nullptr;
     SpmvFn spmv = nullptr;
     // Systems solved by k_bsr_resident (one CTA each) and its launch shape.
-    int32_t n_res = 0;
-    int32_t* d_res_ids = nullptr;
-    int32_t res_threads = 0;
-    int64_t res_nnzb_max = 0;  // blocks in the free rows of the largest resident system
-    int32_t res_stride = 0;    // blocks of the longest row of a resident system
+    // [1]: those that fit only PACKED.
+    struct ResidentGroup {
+        std::vector<int32_t> ids;
+        int32_t* d_ids = nullptr;
+        int32_t threads = 0;
+        int64_t nnzb_max = 0;  // blocks in the free rows of the largest system
+        int32_t stride = 0;    // blocks of the longest row, rounded up
+        size_t smem = 0;
+    } res[2];
     uint32_t* d_res_map = nullptr;
-    size_t res_smem = 0;
     BsrPlan plan{};     // k_bsr_persist over the streamed systems (grid 0: the WHILE loop)
     int64_t st_rows = 0, st_nnzb = 0, res_rows = 0, res_nnzb = 0;  // streamed / resident sizes
     std::string err;
@@ -991,9 +1010,17 @@ void launch(void (*k)(BsrArgs), const BsrArgs& a, int n, cudaStream_t stream) {
     if (n > 0) k<<<n, kThreads, 0, stream>>>(a);
 }
 
+typedef void (*ResidentFn)(BsrArgs, const int32_t*, int64_t, const uint32_t*, int);
+ResidentFn resident_fn(bool packed) { return packed ? k_bsr_resident<true> : k_bsr_resident<false>; }
+
+int resident_launches(const oc_bsr_solver* s) { return !s->res[0].ids.empty() + !s->res[1].ids.empty(); }
+
 void launch_resident(const oc_bsr_solver* s, const BsrArgs& a) {
-    k_bsr_resident<<<s->n_res, s->res_threads, s->res_smem, s->stream>>>(a, s->d_res_ids, s->res_nnzb_max,
-                                                                        s->d_res_map, s->res_stride);
+    for (int i = 0; i < 2; ++i) {
+        const auto& g = s->res[i];
+        if (!g.ids.empty())
+            resident_fn(i)<<<(int)g.ids.size(), g.threads, g.smem, s->stream>>>(a, g.d_ids, g.nnzb_max, s->d_res_map, g.stride);
+    }
 }
 
 cudaError_t launch_bsr_persist(const oc_bsr_solver* s) {
@@ -1104,17 +1131,15 @@ oc_status bsr_build_graph(oc_bsr_solver* s) {
         return p;
     };
     cudaGraphNode_t n_reset, n_init, n_loop, n_spmv, n_upd, n_res;
-    if (s->n_res > 0) {  // independent of the streamed systems' nodes
-        const int32_t* ids = s->d_res_ids;
-        int64_t nnzb_max = s->res_nnzb_max;
-        const uint32_t* map = s->d_res_map;
-        int stride = s->res_stride;
-        void* rparams[] = {&a, &ids, &nnzb_max, &map, &stride};
+    for (int i = 0; i < 2; ++i) {  // independent of the streamed systems' nodes
+        auto& r = s->res[i];
+        if (r.ids.empty()) continue;
+        void* rparams[] = {&a, &r.d_ids, &r.nnzb_max, &s->d_res_map, &r.stride};
         cudaKernelNodeParams p{};
-        p.func = (void*)k_bsr_resident;
-        p.gridDim = dim3((unsigned)s->n_res);
-        p.blockDim = dim3((unsigned)s->res_threads);
-        p.sharedMemBytes = (unsigned)s->res_smem;
+        p.func = (void*)resident_fn(i);
+        p.gridDim = dim3((unsigned)r.ids.size());
+        p.blockDim = dim3((unsigned)r.threads);
+        p.sharedMemBytes = (unsigned)r.smem;
         p.kernelParams = rparams;
         BSR_TRY(cudaGraphAddKernelNode(&n_res, g, nullptr, 0, &p));
     }
@@ -1225,7 +1250,6 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
     std::vector<BlockInfo> blocks;
     std::vector<int64_t> slice_ptr;
     std::vector<int32_t> width;
-    std::vector<int32_t> res_ids;
     int smem_optin = 0;
     BSR_CREATE_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
     // Room for the kernel's static shared memory (block sums and the two broadcast scalars).
@@ -1255,8 +1279,10 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
         // A system of one block of rows whose blocks fit in shared memory runs resident.
         int32_t maxdeg = 0;
         for (int32_t r = 0; r < d.n_rows; ++r) maxdeg = std::max(maxdeg, degree(r));
-        const bool fits = d.n_rows <= kThreads && maxdeg <= kResMaxDeg &&
-                          resident_smem_bytes(kThreads, d.nnzb, kResMaxDeg) <= smem_cap && d.nnzb < 0xffff;
+        // (By the packed bytes alone: smem_cap leaves 1,024 for the rounding to 16 entries, the offsets
+        // of the slots past kResMaxDeg and the kernel's static shared memory.)
+        const size_t need = resident_smem_bytes(kThreads, 0, kResMaxDeg, true) + (37 * (size_t)d.nnzb + 15) / 16 * 16;
+        const bool fits = d.n_rows <= kThreads && maxdeg <= kResMaxDeg && need <= smem_cap;
         if (o.executor == OC_EXEC_RESIDENT && !fits) {
             bsr_fail(s, OC_ERR_UNSUPPORTED, who_of(k) + "too large for the resident executor");
             return bail(OC_ERR_UNSUPPORTED);
@@ -1288,12 +1314,13 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
         if (resident) {
             sp.blk0 = 0;
             sp.nblk = 0;
-            res_ids.push_back(k);
             int64_t kept = 0;
             for (int32_t r = 0; r < d.n_rows; ++r) kept += weight[r];
-            s->res_nnzb_max = std::max(s->res_nnzb_max, kept);
-            s->res_stride = std::max(s->res_stride, (maxdeg / kResSlots + 1) * kResSlots);
-            s->res_threads = std::max(s->res_threads, (d.n_rows + 31) / 32 * 32);
+            auto& g = s->res[resident_smem_bytes(kThreads, kept, kResMaxDeg, false) > smem_cap];
+            g.ids.push_back(k);
+            g.nnzb_max = std::max(g.nnzb_max, kept);
+            g.stride = std::max(g.stride, (maxdeg / kResSlots + 1) * kResSlots);
+            g.threads = std::max(g.threads, (d.n_rows + 31) / 32 * 32);
             s->res_rows += d.n_rows;
             s->res_nnzb += d.nnzb;
             continue;
@@ -1396,14 +1423,19 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
     BSR_CREATE_TRY(cudaMemset(a.grid_ticket, 0, sizeof(uint32_t)));
     BSR_CREATE_TRY(cudaMemset(a.loop_count, 0, sizeof(unsigned long long)));
     BSR_CREATE_TRY(cudaMallocHost(&s->h_loop, sizeof(unsigned long long)));
-    s->n_res = (int32_t)res_ids.size();
-    if (s->n_res > 0) {
-        BSR_CREATE_TRY(bsr_upload(s, &s->d_res_ids, res_ids));
-        s->res_smem = resident_smem_bytes(s->res_threads, s->res_nnzb_max, s->res_stride);
+    if (resident_launches(s) > 0) {
+        for (int i = 0; i < 2; ++i) {
+            auto& g = s->res[i];
+            if (g.ids.empty()) continue;
+            BSR_CREATE_TRY(bsr_upload(s, &g.d_ids, g.ids));
+            g.smem = resident_smem_bytes(g.threads, g.nnzb_max, g.stride, i == 1);
+            BSR_CREATE_TRY(cudaFuncSetAttribute(resident_fn(i), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+        }
         // Where each block of a free row goes, warp by warp and slot by slot in lane order, and its
         // internal local column.
         std::vector<uint32_t> map((size_t)std::max<int64_t>(nnzb, 1), 0xffffu);
-        for (int32_t k : res_ids) {
+        for (int32_t k = 0; k < n_systems; ++k) {
+            if (sys[k].nblk > 0) continue;
             const oc_bsr_desc& d = descs[k];
             const int64_t r0 = s->row_off[k], e0 = s->nnz_off[k];
             uint32_t pos = 0;  // the warp's first entry
@@ -1427,8 +1459,6 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
             }
         }
         BSR_CREATE_TRY(bsr_upload(s, &s->d_res_map, map));
-        BSR_CREATE_TRY(cudaFuncSetAttribute(k_bsr_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)s->res_smem));
     }
     if (oc_status st = plan_bsr_persist(s, sys)) return bail(st);
     BSR_CREATE_TRY(cudaDeviceSynchronize());
@@ -1505,12 +1535,10 @@ oc_status oc_bsr_solve(oc_bsr_solver* s) {
     if (!bsr_valid(s)) return OC_ERR_INVALID_ARGUMENT;
     BSR_TRY(cudaSetDevice(s->device));
     if (s->use_graph && s->plan.grid > 0) {
-        if (s->n_res > 0) {
-            launch_resident(s, s->args);
-            BSR_TRY(cudaGetLastError());
-        }
+        launch_resident(s, s->args);
+        BSR_TRY(cudaGetLastError());
         BSR_TRY(launch_bsr_persist(s));
-        s->launches += 1 + (s->n_res > 0 ? 1 : 0);
+        s->launches += 1 + resident_launches(s);
         return OC_OK;
     }
     if (s->use_graph) {
@@ -1519,16 +1547,14 @@ oc_status oc_bsr_solve(oc_bsr_solver* s) {
             if (st != OC_OK) return st;
         }
         BSR_TRY(cudaGraphLaunch(s->exec, s->stream));
-        s->launches += (s->n_blocks > 0 ? 1 : 0) + (s->n_res > 0 ? 1 : 0);
+        s->launches += (s->n_blocks > 0 ? 1 : 0) + resident_launches(s);
         return OC_OK;
     }
     BsrArgs a = s->args;
     a.use_cond = 0;
-    if (s->n_res > 0) {
-        launch_resident(s, a);
-        BSR_TRY(cudaGetLastError());
-        s->launches += 1;
-    }
+    launch_resident(s, a);
+    BSR_TRY(cudaGetLastError());
+    s->launches += resident_launches(s);
     if (s->n_blocks == 0) return OC_OK;
     BSR_TRY(cudaMemsetAsync(a.unfinished, 0, sizeof(int32_t), s->stream));
     launch(k_bsr_init, a, s->n_blocks, s->stream);
@@ -1603,7 +1629,7 @@ oc_status oc_bsr_profile(oc_bsr_solver* s, int32_t n_solves, int32_t max_kernels
         return x;
     };
     for (int32_t i = 0; i < n_solves && e == cudaSuccess; ++i) {
-        if (s->n_res > 0) e = timed(4);
+        if (resident_launches(s) > 0) e = timed(4);
         if (s->n_blocks == 0) continue;
         if (e == cudaSuccess) e = cudaMemsetAsync(a.unfinished, 0, sizeof(int32_t), s->stream);
         if (e == cudaSuccess) e = timed(0);
