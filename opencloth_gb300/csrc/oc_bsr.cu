@@ -1429,7 +1429,11 @@ oc_status oc_bsr_create(const oc_bsr_desc* descs, int32_t n_systems, const oc_op
             if (g.ids.empty()) continue;
             BSR_CREATE_TRY(bsr_upload(s, &g.d_ids, g.ids));
             g.smem = resident_smem_bytes(g.threads, g.nnzb_max, g.stride, i == 1);
-            BSR_CREATE_TRY(cudaFuncSetAttribute(resident_fn(i), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+            // (The most that a launch may have, and not this handle's: the limit is the kernel's in every handle.)
+            cudaFuncAttributes fa;
+            BSR_CREATE_TRY(cudaFuncGetAttributes(&fa, resident_fn(i)));
+            BSR_CREATE_TRY(cudaFuncSetAttribute(resident_fn(i), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                smem_optin - (int)fa.sharedSizeBytes));
         }
         // Where each block of a free row goes, warp by warp and slot by slot in lane order, and its
         // internal local column.

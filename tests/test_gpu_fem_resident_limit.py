@@ -41,3 +41,15 @@ def test_refused():
     with pytest.raises(OcError) as e:
         BsrSolver([system(6089)], executor=2)
     assert e.value.status == 7
+
+
+@pytest.mark.parametrize("nnzb", [5000, 6000])
+def test_a_smaller_handle_made_later(nnzb):
+    """Its shared memory is no limit for the larger handle's solves."""
+    large, small = system(nnzb), system(1400, n=100, longest=20)
+    want = solve([large], 1)
+    with BsrSolver([large], executor=2) as s:
+        with BsrSolver([small], executor=2):
+            s.set_system(large["blocks"], large["b"], large["V"])
+            s.solve()
+            assert all(np.array_equal(a, b) for a, b in zip(s.solution(), want))
