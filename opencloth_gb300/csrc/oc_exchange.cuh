@@ -154,14 +154,11 @@ __device__ __forceinline__ void leave_tags(PersistCtl* ctl, uint32_t base, uint3
     }
 }
 
-// a / b of two normalised pairs rounded to float; in FP64 where pair_div's remainder would be lost:
-// the head's product reaches 47 bits below a (normal down to 2^-149), and the quotient must be normal.
+// a / b of two normalised pairs rounded to float; in FP64 where pair_div's remainder or the quotient
+// would leave the float range.  The interval lies low because the sums are scaled down (sum_scale).
 __device__ __forceinline__ float quotient(Acc a, Acc b) {
     const float ma = fabsf(a.s), mb = fabsf(b.s);
-    if (ma >= 0x1p-90f && ma <= 0x1p90f && mb >= 0x1p-90f && mb <= 0x1p90f) {
-        const float q = pair_div(a, b), mq = fabsf(q);
-        if (mq >= 0x1p-100f && mq <= 0x1p100f) return q;
-    }
+    if (ma >= 0x1p-80f && ma <= 0x1p40f && mb >= 0x1p-80f && mb <= 0x1p40f) return pair_div(a, b);
     return (float)(((double)a.s + (double)a.c) / ((double)b.s + (double)b.c));
 }
 

@@ -60,7 +60,7 @@ __device__ __forceinline__ bool cluster_sum(Acc part, int C, int rank, SumBuffer
     total = lanes_sum<W / 2>(b.warps[cur][lane & (W - 1)]);
     if (C > 1) {
         ulonglong2* const box = b.box[cur];
-        if (lane < C && (int)blockIdx.x != a.withhold_block) put_cluster(box + rank, lane, total, tag);
+        if (lane < C) put_cluster(box + rank, lane, total, tag);
         Acc v = acc_zero();
         ok = poll<1>(lane < C ? 1u : 0u, a, err, [&](int) { return get_cluster(box + lane, tag, v); });
         total = lanes_sum<kResidentMaxCluster / 2>(v);
@@ -110,12 +110,13 @@ __global__ void __launch_bounds__(T, resident_min_blocks<T>()) k_resident(const 
 #pragma unroll
     for (int u = 0; u < kResidentVpt; ++u) own[u] = (int)threadIdx.x + u * T < n_local;
 
+    const bool withheld = (int)blockIdx.x == a.withhold_block;  // (a testing aid) it leaves before the loop's first sum
     uint32_t tag = 0;
     Acc part, total = acc_zero();
     if (threadIdx.x == 0) {
         s_delta0 = 0.0;
         s_flags = 0u;
-        s_ok = 1;
+        s_ok = withheld ? 0 : 1;
     }
     if (C > 1) {
         if (threadIdx.x < 2 * kResidentMaxCluster) (&sums.box[0][0])[threadIdx.x] = make_ulonglong2(0, 0);
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(T, resident_min_blocks<T>()) k_resident(const 
                 run = false;
             }
             if (!ok) give_up();
-            s_go = run && ok ? 1 : 0;
+            s_go = run && ok && !withheld ? 1 : 0;
         }
     } else {
         // The CG state k_assemble left in the planes: A -> shared memory, x, r, d ->
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(T, resident_min_blocks<T>()) k_resident(const 
             const InstState& st0 = a.state[inst];
             s_delta0 = st0.delta0;
             s_flags = st0.flags;
-            s_go = st0.active != 0 ? 1 : 0;
+            s_go = st0.active != 0 && !withheld ? 1 : 0;
         }
         if (C > 1) cluster_wait();
     }
