@@ -1149,11 +1149,15 @@ bool own_ctas(int64_t chunk, int64_t even) { return 5 * chunk <= 7 * even || chu
 // 337 / 332, 2000 x 2000 (103) 965 / 589; 130 of 130 x 130 (67, a CTA each) 410 / 389; with several pieces a
 // CTA, 90 of 130 x 130 (40) 229 / 279, 20 of 130 to 400 a side (40) 223 / 223, 110 of 130 x 130 (49) 385 / 320,
 // 300 of 130 x 130 (131) 1,107 / 768; 2,000 of 8 to 24 a side (19, 14 pieces) 202 / 200, 3,000 of them (28, 21
-// pieces) 340 / 267.
+// pieces) 340 / 267.  k_cg_arrive takes as long as the even share, so CTAs of their own that spill count
+// only while they are even: 44 cloths of 129 to 500 a side (54 slots, even 42) 327 / 312.
 constexpr int32_t kOnChipSlotsOne = 56, kOnChipSlots = 44;  // (the latter with the pieces)
+constexpr int32_t kOnChipOnly = 34, kOnChipUneven = 2;
 
 bool on_chip_enough(const PersistPlan& P) {
-    return P.grid > 0 && (P.one ? P.max_slots <= kOnChipSlotsOne : P.max_slots + P.max_pieces <= kOnChipSlots);
+    if (P.grid == 0) return false;
+    if (!P.one) return P.max_slots + P.max_pieces <= kOnChipSlots;
+    return P.max_slots <= kOnChipOnly || (P.max_slots <= kOnChipSlotsOne && P.max_slots <= P.even_slots + kOnChipUneven);
 }
 
 oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_t>& ids) {
@@ -1173,6 +1177,7 @@ oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_
         int64_t want = std::min(most, (total + kPersistThreads - 1) / kPersistThreads);
         want = std::min(most, (want + cluster - 1) / cluster * cluster);
         const int64_t even = ((total + want - 1) / want + 31) / 32 * 32;
+        P.even_slots = (int32_t)((even + kPersistThreads - 1) / kPersistThreads);
         int64_t chunk = even;
         auto ctas_of = [&](int32_t k) { return (s->inst_host[(size_t)k].nv + chunk - 1) / chunk; };
         P.one = (int64_t)ids.size() <= most;

@@ -308,6 +308,7 @@ struct PersistPlan {
     int32_t n_packets;         // of one set
     int32_t one;               // 1: pieces[b] is CTA b's only piece (n = 0: none)
     int32_t max_pieces, max_slots;  // of one CTA
+    int32_t even_slots;        // of a CTA if all had the same
     int32_t smem_slots;        // slots of a CTA held in shared memory
     int32_t x_slots;           // slots of a CTA whose x is in shared memory
     int32_t on_chip;           // 1: no slot left in the planes
