@@ -59,6 +59,7 @@ struct oc_solver {
     };
     std::vector<SimGroup> sim;
     int sim_smem_max = 0;
+    bool sim_one = true;  // a call of one step goes there too (the passes may change without a new plan)
     // OC_RESIDENT_FUSED=1: resident cloths assemble inside the resident kernel (no
     // k_assemble pass over them).  Off by default: on 4096 cloths of 64 to 16,384 vertices
     // the fused step measured 4.97 ms against 4.37 ms for the separate passes (the
@@ -1056,7 +1057,23 @@ oc_status alloc_error_word(oc_solver* s) {
 // 12 for 4 of them, and 14 on 512-vertex ones): then a step is bound by latencies, which k_sim shortens; with more cloths it is
 // bound by instructions, and the assembly's and the resident CG's own launches keep more warps in
 // flight.
+//
+// A call of one step of a large general mesh with Provot's pass goes to the separate launches: its loads of
+// neighbours outside the window follow one another, twice a step, and a launch of one step has the
+// state to fetch and to store besides.  Measured, us a step, k_sim / launches: 120 x 120, springs in random
+// order, 43.4 / 36.9, five of them 47.1 / 39.4, seven of 128 x 128 with both passes 50.8 / 48.4, five of 60 to 128
+// a side 49.8 / 41.4; 90 x 90 (8,100 vertices) 30.6 / 37.1.  Eight steps a call, 38.8 / 36.9, 40.8 / 40.0, 44.8 / 49.1:
+// left to k_sim.
+constexpr int32_t kSimProvotMesh = 8192;
+
+bool sim_takes_one(const oc_solver* s) {
+    for (const InstParams& ip : s->inst_host)
+        if (ip.grid_cols <= 0 && (ip.passes & OC_PASS_PROVOT) && ip.nv > kSimProvotMesh) return false;
+    return true;
+}
+
 oc_status plan_sim(oc_solver* s) {
+    s->sim_one = sim_takes_one(s);
     for (auto& g : s->sim) dfree(s, &g.d_ids);
     s->sim.clear();
     if (s->sim_smem_max <= 0 || s->resident_fused || s->any_coupled) return OC_OK;
@@ -2182,13 +2199,16 @@ oc_status oc_step(oc_solver* s, float dt, int32_t n_steps) {
         // One step of several launches goes as a graph: the launches and the events that fork and join
         // them are more host time than the step (12 cloths of 16 to 96 a side, 10 launches).
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (n_steps == 1 && s->sim.size() > 1) OC_TRY(cudaStreamIsCapturing(s->stream, &cap));
-        if (n_steps != 1 || s->sim.size() == 1 || cap != cudaStreamCaptureStatusNone) return step_sim(s, dt, n_steps);
-        if (!s->exec || s->graph_dt != dt)
-            if (oc_status st = build_sim_graph(s, dt)) return st;
-        OC_TRY(cudaGraphLaunch(s->exec, s->stream));
-        s->host_launches += (int64_t)s->sim.size();
-        return OC_OK;
+        if (n_steps == 1 && (s->sim.size() > 1 || !s->sim_one)) OC_TRY(cudaStreamIsCapturing(s->stream, &cap));
+        if (n_steps != 1 || (s->sim_one && s->sim.size() == 1) || cap != cudaStreamCaptureStatusNone)
+            return step_sim(s, dt, n_steps);
+        if (s->sim_one) {
+            if (!s->exec || s->graph_dt != dt)
+                if (oc_status st = build_sim_graph(s, dt)) return st;
+            OC_TRY(cudaGraphLaunch(s->exec, s->stream));
+            s->host_launches += (int64_t)s->sim.size();
+            return OC_OK;
+        }
     }
     if (!s->exec || s->graph_dt != dt) {
         oc_status st = build_graph(s, dt);
@@ -2228,6 +2248,7 @@ oc_status oc_set_passes(oc_solver* s, int32_t instance, int32_t passes) {
         s->any_passes = s->any_passes || ip.passes != 0;
         s->any_provot = s->any_provot || (ip.passes & OC_PASS_PROVOT);
     }
+    s->sim_one = sim_takes_one(s);
     if (s->exec) {  // the graph's node set depends on the passes
         cudaGraphExecDestroy(s->exec);
         s->exec = nullptr;
