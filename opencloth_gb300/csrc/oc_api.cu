@@ -1028,10 +1028,12 @@ void drop_graphs(oc_solver* s) {
     }
 }
 
-// Streams beside the handle's own for `want` concurrent launches (at most 8).
+// Streams beside the handle's own for `want` concurrent launches.
+constexpr size_t kMaxAux = 8;
+
 oc_status ensure_aux(oc_solver* s, size_t want) {
     if (!s->fork_ev) OC_TRY(cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming));
-    while (s->aux.size() < std::min<size_t>(want, 8)) {
+    while (s->aux.size() < std::min<size_t>(want, kMaxAux)) {
         cudaStream_t x = nullptr;
         cudaEvent_t e = nullptr;
         OC_TRY(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
@@ -1063,17 +1065,19 @@ oc_status alloc_error_word(oc_solver* s) {
 // state to fetch and to store besides.  Measured, us a step, k_sim / launches: 120 x 120, springs in random
 // order, 43.4 / 36.9, five of them 47.1 / 39.4, seven of 128 x 128 with both passes 50.8 / 48.4, five of 60 to 128
 // a side 49.8 / 41.4; 90 x 90 (8,100 vertices) 30.6 / 37.1.  Eight steps a call, 38.8 / 36.9, 40.8 / 40.0, 44.8 / 49.1:
-// left to k_sim.
+// left to k_sim.  And where the launch shapes are more than the streams, so that some run one behind the
+// other: 15 cloths of 20 to 60 a side (9 shapes) 33.9 / 26.8, with Provot's pass 44.4 / 36.3; with 8 shapes 27.8 /
+// 26.8 and 33.5 / 34.9.
 constexpr int32_t kSimProvotMesh = 8192;
 
 bool sim_takes_one(const oc_solver* s) {
+    if (s->sim.size() > kMaxAux) return false;
     for (const InstParams& ip : s->inst_host)
         if (ip.grid_cols <= 0 && (ip.passes & OC_PASS_PROVOT) && ip.nv > kSimProvotMesh) return false;
     return true;
 }
 
 oc_status plan_sim(oc_solver* s) {
-    s->sim_one = sim_takes_one(s);
     for (auto& g : s->sim) dfree(s, &g.d_ids);
     s->sim.clear();
     if (s->sim_smem_max <= 0 || s->resident_fused || s->any_coupled) return OC_OK;
@@ -1141,6 +1145,7 @@ oc_status plan_sim(oc_solver* s) {
         g.launch.inst_ids = g.d_ids;
         s->sim.push_back(g);
     }
+    s->sim_one = sim_takes_one(s);
     return ensure_aux(s, s->sim.size());
 }
 

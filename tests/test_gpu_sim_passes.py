@@ -29,3 +29,18 @@ def test_mixed_calls(n, others):
             out.append((*s.get_state(), s.stats()[0], s.stats()[2]))
     assert all(same_bits(a, b) for a, b in zip(out[0][:3], out[1][:3]))
     assert np.array_equal(out[0][3], out[1][3]) and np.array_equal(out[0][4], out[1][4])
+
+
+def test_more_shapes_than_streams():
+    """Ten launch shapes: calls of one step take the separate launches, longer ones k_sim."""
+    parts = [grid(16 * k + 5, 16, k) for k in range(1, 11)]
+    X, V = np.concatenate([p[1] for p in parts]), np.concatenate([p[2] for p in parts])
+    out = []
+    for executor in ("auto", "streamed"):
+        with ClothSolver([p[0] for p in parts], executor=executor) as s:
+            s.set_state(X, V)
+            for k in (1, 3, 1, 1, 2):
+                s.step(DT, k)
+            out.append((*s.get_state(), s.stats()[0], s.stats()[2]))
+    assert all(same_bits(a, b) for a, b in zip(out[0][:3], out[1][:3]))
+    assert np.array_equal(out[0][3], out[1][3]) and np.array_equal(out[0][4], out[1][4])
