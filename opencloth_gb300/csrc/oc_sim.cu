@@ -309,29 +309,27 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
     // The cluster's barrier inside a step: true when no CTA's wait has given up.  One whose has takes the
     // barrier like the others, having told them first, and all of them leave behind the same barrier: a
     // CTA that left alone would be missing at the others' next barrier, and their packets would go to
-    // shared memory that is no longer its own.  Two flags, as a CTA may be one barrier ahead of
-    // another that has not read its flag yet, but not two.
-    unsigned met = 0;
-    auto together = [&]() -> bool {
-        int* const gone = &s_gone[met++ & 1];
+    // shared memory that is no longer its own.  Two flags, by the parity of these barriers, as a CTA may be
+    // one barrier ahead of another that has not read its flag yet, but not two.
+    auto together = [&](int parity) -> bool {
+        int* const gone = &s_gone[parity];
         if (!s_ok && tid < C) flag_cluster(gone, tid);
         cluster_arrive();
         cluster_wait();
         return *(volatile int*)gone == 0;
     };
-    bool all_ok = true;
+    const int n_steps = L.n_steps;
+    int step = 0;
 
     __syncthreads();
     if (C > 1) cluster_wait();
-    int32_t n_steps = L.n_steps;
     if ((int)blockIdx.x == a.withhold_block) {  // (a testing aid) sends no packets, meets the others at their first barrier
         if (tid == 0) s_ok = 0;
         __syncthreads();
-        if (C > 1 && (n_steps > 1 || (ip.passes & OC_PASS_PROVOT))) together();
-        all_ok = false;
-        n_steps = 0;
+        if (C > 1 && (n_steps > 1 || (ip.passes & OC_PASS_PROVOT))) together(0);
+        step = n_steps;
     }
-    for (int32_t step = 0; step < n_steps; ++step) {
+    for (; step < n_steps; ++step) {
         // The assembly of the CTA's vertices, with the first direction's dot product.
         Acc p0 = acc_zero(), p1 = acc_zero();
 #pragma unroll 1
@@ -468,16 +466,14 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
             __syncthreads();
         }
         // A wait that gave up: no update; the CTAs of a cluster go on to their next barrier.
-        const bool ok = s_ok != 0;
-        all_ok = ok;
-        if (!ok && C == 1) break;
+        if (C == 1 && !s_ok) break;
         // The update (IMP:790-797) and the ellipsoid; the window's own part, and, for the other
         // CTAs and at the end, global memory.
         const bool last = step + 1 == n_steps;
         const bool prov = (ip.passes & OC_PASS_PROVOT) != 0;
 #pragma unroll
         for (int u = 0; u < VPT; ++u)
-            if (own[u] && ok) {
+            if (own[u] && s_ok) {
                 const int j = tid + u * kST, i = lb + j - wlo;
                 float4 X = wX[i], V = wV[i];
                 update_vertex(ip, a.dt, x[u][0], x[u][1], x[u][2], X, V);
@@ -495,8 +491,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
             }
         if (prov) {
             if (C > 1) {
-                all_ok = together();
-                if (!all_ok) break;
+                if (!together(0)) break;
                 for (int i = wlo + tid; i < whi; i += kST)
                     if (i < lb || i >= lb + n) wX[i - wlo] = __ldcg(a.X + vo + i);
             }
@@ -514,8 +509,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
         }
         if (!last) {
             if (C > 1) {  // the neighbouring CTAs' new state into the halo
-                all_ok = together();
-                if (!all_ok) break;
+                if (!together(prov ? 1 : step & 1)) break;
                 for (int i = wlo + tid; i < whi; i += kST)
                     if (i < lb || i >= lb + n) {
                         if (!prov) wX[i - wlo] = __ldcg(a.X + vo + i);
@@ -525,7 +519,7 @@ __global__ void __launch_bounds__(kST, 1) k_sim(const StepArgs a, const SimLaunc
             __syncthreads();
         }
     }
-    if (rank == 0 && tid == 0 && all_ok) {
+    if (rank == 0 && tid == 0 && s_ok && step == n_steps) {
         InstState& st = a.state[inst];
         st.delta0 = (double)dn0.s + (double)dn0.c;
         st.delta_new = (double)dn.s + (double)dn.c;
