@@ -1173,12 +1173,19 @@ bool own_ctas(int64_t chunk, int64_t even) { return 5 * chunk <= 7 * even || chu
 // 300 of 130 x 130 (131) 1,107 / 768; 2,000 of 8 to 24 a side (19, 14 pieces) 202 / 200, 3,000 of them (28, 21
 // pieces) 340 / 267.  k_cg_arrive takes as long as the even share, so CTAs of their own that spill count
 // only while they are even: 44 cloths of 129 to 500 a side (54 slots, even 42) 327 / 312.
+// Beside resident launches, which run at the same time as k_cg_arrive but before k_cg_persist, whose CTAs
+// want whole SMs: six of 300 to 600 a side (37) with 300 of 20 to 60 283 / 325, 1250 x 1250 (41) with 35 of
+// them 288 / 272, 1450 x 1450 (55) with 35 401 / 373.  All cloths joined in one
+// k_cg_persist against those two: 20 of 60 to 128 a side with 12 of 200 to 500 (44, even 39) 262 / 272, 50 with
+// four of 500 to 600 (47, even 42) 293 / 277, 35 of 20 to 60 with 12 of 200 to 500 (59, even 44) 357 / 279.
 constexpr int32_t kOnChipSlotsOne = 56, kOnChipSlots = 44;  // (the latter with the pieces)
-constexpr int32_t kOnChipOnly = 34, kOnChipUneven = 2;
+constexpr int32_t kOnChipOnly = 34, kOnChipUneven = 2, kOnChipBeside = 38;
+enum class Beside { none, resident, joined };
 
-bool on_chip_enough(const PersistPlan& P) {
-    if (P.grid == 0) return false;
+bool on_chip_enough(const PersistPlan& P, Beside b) {
+    if (P.grid == 0 || (b == Beside::resident && P.max_slots > kOnChipBeside)) return false;
     if (!P.one) return P.max_slots + P.max_pieces <= kOnChipSlots;
+    if (b == Beside::joined && P.max_slots <= kOnChipSlots) return true;
     return P.max_slots <= kOnChipOnly || (P.max_slots <= kOnChipSlotsOne && P.max_slots <= P.even_slots + kOnChipUneven);
 }
 
@@ -1433,7 +1440,7 @@ oc_status all_stream(oc_solver* s, bool* join) {
 // cloths grouped by launch shape into buckets, the assembly tables (record gather,
 // stencil, strip sweep), the update table, and the persistent CG of the streamed cloths.
 // Run at create and again by oc_set_launch_config (an earlier plan's tables are freed).
-oc_status plan_execution(oc_solver* s) {
+oc_status plan_execution(oc_solver* s, bool may_stream_all = true) {
     const oc_launch_config& cfg = s->cfg;
     StepArgs& a = s->args;
     a.gather_variant = cfg.gather_variant;
@@ -1441,7 +1448,8 @@ oc_status plan_execution(oc_solver* s) {
     s->resident_fused = cfg.resident_fused != 0;
     const int max_res = cfg.resident_max_vertices;
     bool join = false;
-    if (oc_status r = all_stream(s, &join)) return r;
+    if (may_stream_all)
+        if (oc_status r = all_stream(s, &join)) return r;
     s->resident.assign((size_t)s->n_inst, 0);
     for (oc_solver::Bucket& b : s->buckets) dfree(s, &b.d_ids);
     s->buckets.clear();
@@ -1534,8 +1542,11 @@ oc_status plan_execution(oc_solver* s) {
     s->arrive = false;
     if (any_streamed && !any_coupled) {
         if (oc_status r = plan_persist(s, &s->pplan, streamed_ids)) return r;
-        s->arrive = !on_chip_enough(s->pplan) && s->coop && s->arrive_per_sm > 0 &&
+        const Beside b = join ? Beside::joined : s->buckets.empty() ? Beside::none : Beside::resident;
+        s->arrive = !on_chip_enough(s->pplan, b) && s->coop && s->arrive_per_sm > 0 &&
                     s->n_streamed_blocks <= (int64_t)arrive_max_entries_per_block() * arrive_grid(s);
+        // Small cloths join the others on chip or not at all: in k_cg_arrive they cost more than beside it.
+        if (s->arrive && join) return plan_execution(s, false);
         if (s->arrive && !s->d_words) OC_TRY(dalloc(s, &s->d_words, (size_t)s->n_inst));
         if (s->arrive)
             if (oc_status r = alloc_error_word(s)) return r;
@@ -2714,7 +2725,7 @@ oc_status plan_adjoint(oc_solver* s) {
     std::vector<int32_t> ids((size_t)s->n_inst);
     for (int32_t k = 0; k < s->n_inst; ++k) ids[(size_t)k] = k;
     if (oc_status r = plan_persist(s, &s->aplan, ids)) return r;
-    if (!on_chip_enough(s->aplan)) s->aplan.grid = 0;
+    if (!on_chip_enough(s->aplan, Beside::joined)) s->aplan.grid = 0;
     return OC_OK;
 }
 

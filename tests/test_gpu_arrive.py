@@ -89,3 +89,14 @@ def test_a_wait_that_runs_out_is_reported():
         s.step(DT, 2)
         t.step(DT, 2)
         assert all(same_bits(a, b) for a, b in zip(s.get_state(), t.get_state()))
+
+
+@pytest.mark.parametrize("large,small", [([(1250, 1240)], 35), ([(1500, 1400)], 20), ([(500, 400)] * 6, 10), ([(500, 400)] * 5, 100)])
+def test_beside_small_cloths(large, small):
+    """Cloths for both kernels with small ones that join them or run resident beside them."""
+    ps = [cloth(c, r, k) for k, (c, r) in enumerate(large + [(20 + 7 * k % 40, 21 + 5 * k % 37) for k in range(small)])]
+    descs, X, V = [p[0] for p in ps], np.concatenate([p[1] for p in ps]), np.concatenate([p[2] for p in ps])
+    a, sa = run(descs, X, V, 3, True)
+    b, sb = run(descs, X, V, 3, False)
+    assert all(same_bits(x, y) for x, y in zip(a, b))
+    assert np.array_equal(sa[0], sb[0]) and np.array_equal(sa[2], sb[2])
