@@ -1310,11 +1310,11 @@ oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_
 // (1,644) 123 / 189, 1025 x 1025 (6,912) 567 / 623, 1300 x 1300 (11,118) 937 / 914, 2000 x 2000 2,208 / 1,987;
 // 500 x 500 with 80 of 30 x 30 (3,472, 2,118) 252 / 274, with 100 (4,808, 2,237) 305 / 284, with 110 (5,952,
 // 2,296) 354 / 288; 200 x 200 with 140 (3,333, 1,092) 190 / 209, with 145 (5,714, 1,122) 251 / 214, with 151
-// 1,238 / 196; 100 of 100 x 75 (7,500, 4,934) 604 / 526.  Streamed
+// 1,238 / 196; 100 of 100 x 75 (7,500, 4,934) 604 / 526; 37 of 157 x 181 (7,136, 6,917) 498 / 570 for the solve.  Streamed
 // REFERENCE cloths beside them keep the WHILE loop of both (two cooperative launches of one CTA
 // per SM would run one behind the other).
 constexpr int64_t kCplMinRows = 256;
-bool cpl_pieces_small(int64_t piece, int64_t even) { return piece <= 7000 && 2 * piece <= 3 * even + 3400; }
+bool cpl_pieces_small(int64_t piece, int64_t even) { return piece <= 9000 && 2 * piece <= 3 * even + 3400; }
 
 oc_status plan_coupled(oc_solver* s) {
     CplPlan& P = s->cplan;
