@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <array>
+#include <limits>
 #include <map>
 #include <set>
 #include <tuple>
@@ -59,7 +60,7 @@ struct oc_solver {
     };
     std::vector<SimGroup> sim;
     int sim_smem_max = 0;
-    bool sim_one = true;  // a call of one step goes there too (the passes may change without a new plan)
+    int32_t sim_from = 1;  // calls of this many steps at least go there (the passes may change without a new plan)
     // OC_RESIDENT_FUSED=1: resident cloths assemble inside the resident kernel (no
     // k_assemble pass over them).  Off by default: on 4096 cloths of 64 to 16,384 vertices
     // the fused step measured 4.97 ms against 4.37 ms for the separate passes (the
@@ -1060,21 +1061,22 @@ oc_status alloc_error_word(oc_solver* s) {
 // bound by instructions, and the assembly's and the resident CG's own launches keep more warps in
 // flight.
 //
-// A call of one step of a large general mesh with Provot's pass goes to the separate launches: its loads of
-// neighbours outside the window follow one another, twice a step, and a launch of one step has the
-// state to fetch and to store besides.  Measured, us a step, k_sim / launches: 120 x 120, springs in random
-// order, 43.4 / 36.9, five of them 47.1 / 39.4, seven of 128 x 128 with both passes 50.8 / 48.4, five of 60 to 128
-// a side 49.8 / 41.4; 90 x 90 (8,100 vertices) 30.6 / 37.1.  Eight steps a call, 38.8 / 36.9, 40.8 / 40.0, 44.8 / 49.1:
-// left to k_sim.  And where the launch shapes are more than the streams, so that some run one behind the
-// other: 15 cloths of 20 to 60 a side (9 shapes) 33.9 / 26.8, with Provot's pass 44.4 / 36.3; with 8 shapes 27.8 /
-// 26.8 and 33.5 / 34.9.
-constexpr int32_t kSimProvotMesh = 8192;
+// Large general meshes with Provot's pass go to the separate launches: their loads of neighbours outside
+// the window follow one another, twice a step.  Measured, us a step, one and eight steps a call, k_sim /
+// launches: 120 x 120, springs in random order, 43.4 and 38.8 / 36.9; five of 60 to 128 a side (36,000 vertices)
+// 49.8 and 44.8 / 41.4; 90 x 90 (8,100) 30.6 and 25.6 / 37.1.  With more of
+// them only calls of one step, where k_sim has the state to fetch and to store besides: five of 120 x 120
+// (70,000) with both passes 48.8 and 42.7 / 45.1, seven of 128 x 128 50.8 and 44.8 / 48.9.
+// So do calls of one step where the launch shapes are more than the streams, so that some run one behind
+// the other: 15 cloths of 20 to 60 a side (9 shapes) 33.9 / 26.8, with Provot's pass 44.4 / 36.3; with 8 shapes
+// 27.8 / 26.8 and 33.5 / 34.9.
+constexpr int32_t kSimProvotMesh = 8192, kSimProvotTotal = 60000;
 
-bool sim_takes_one(const oc_solver* s) {
-    if (s->sim.size() > kMaxAux) return false;
+int32_t sim_from_steps(const oc_solver* s) {  // the calls that k_sim takes: of this many steps at least
     for (const InstParams& ip : s->inst_host)
-        if (ip.grid_cols <= 0 && (ip.passes & OC_PASS_PROVOT) && ip.nv > kSimProvotMesh) return false;
-    return true;
+        if (ip.grid_cols <= 0 && (ip.passes & OC_PASS_PROVOT) && ip.nv > kSimProvotMesh)
+            return s->nv <= kSimProvotTotal ? std::numeric_limits<int32_t>::max() : 2;
+    return s->sim.size() > kMaxAux ? 2 : 1;
 }
 
 oc_status plan_sim(oc_solver* s) {
@@ -1145,7 +1147,7 @@ oc_status plan_sim(oc_solver* s) {
         g.launch.inst_ids = g.d_ids;
         s->sim.push_back(g);
     }
-    s->sim_one = sim_takes_one(s);
+    s->sim_from = sim_from_steps(s);
     return ensure_aux(s, s->sim.size());
 }
 
@@ -2215,10 +2217,10 @@ oc_status oc_step(oc_solver* s, float dt, int32_t n_steps) {
         // One step of several launches goes as a graph: the launches and the events that fork and join
         // them are more host time than the step (12 cloths of 16 to 96 a side, 10 launches).
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (n_steps == 1 && (s->sim.size() > 1 || !s->sim_one)) OC_TRY(cudaStreamIsCapturing(s->stream, &cap));
-        if (n_steps != 1 || (s->sim_one && s->sim.size() == 1) || cap != cudaStreamCaptureStatusNone)
-            return step_sim(s, dt, n_steps);
-        if (s->sim_one) {
+        const bool here = n_steps >= s->sim_from || n_steps == 0, single = n_steps == 1 && s->sim.size() > 1;
+        if (single || !here) OC_TRY(cudaStreamIsCapturing(s->stream, &cap));
+        if ((here && !single) || cap != cudaStreamCaptureStatusNone) return step_sim(s, dt, n_steps);
+        if (here) {
             if (!s->exec || s->graph_dt != dt)
                 if (oc_status st = build_sim_graph(s, dt)) return st;
             OC_TRY(cudaGraphLaunch(s->exec, s->stream));
@@ -2264,7 +2266,7 @@ oc_status oc_set_passes(oc_solver* s, int32_t instance, int32_t passes) {
         s->any_passes = s->any_passes || ip.passes != 0;
         s->any_provot = s->any_provot || (ip.passes & OC_PASS_PROVOT);
     }
-    s->sim_one = sim_takes_one(s);
+    s->sim_from = sim_from_steps(s);
     if (s->exec) {  // the graph's node set depends on the passes
         cudaGraphExecDestroy(s->exec);
         s->exec = nullptr;

@@ -9,10 +9,11 @@ from test_gpu_sim import DT, grid, mesh, same_bits
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("others", [False, True])
+@pytest.mark.parametrize("others", ["none", "some", "many"])
 @pytest.mark.parametrize("n", [8000, 9001, 16384])
 def test_mixed_calls(n, others):
-    parts = [mesh(n, n)] + ([grid(40, 30, 3), mesh(500, 4)] if others else [])
+    """(With "many", beyond 60,000 vertices, calls of several steps stay in k_sim.)"""
+    parts = [mesh(n, n)] + {"none": [], "some": [grid(40, 30, 3), mesh(500, 4)], "many": [grid(128, 127, k) for k in range(5)]}[others]
     X, V = np.concatenate([p[1] for p in parts]), np.concatenate([p[2] for p in parts])
     out = []
     for executor in ("auto", "streamed"):
