@@ -1174,20 +1174,23 @@ bool own_ctas(int64_t chunk, int64_t even) { return 5 * chunk <= 7 * even || chu
 // CTA, 90 of 130 x 130 (40) 229 / 279, 20 of 130 to 400 a side (40) 223 / 223, 110 of 130 x 130 (49) 385 / 320,
 // 300 of 130 x 130 (131) 1,107 / 768; 2,000 of 8 to 24 a side (19, 14 pieces) 202 / 200, 3,000 of them (28, 21
 // pieces) 340 / 267.  k_cg_arrive takes as long as the even share, so CTAs of their own that spill count
-// only while they are even: 44 cloths of 129 to 500 a side (54 slots, even 42) 327 / 312.
+// only while few or even: 58 cloths of 129 to 200 a side (47, even 39) 279 / 296, 44 of 129 to 500 (55, even
+// 42) 327 / 312.
 // Beside resident launches, which run at the same time as k_cg_arrive but before k_cg_persist, whose CTAs
-// want whole SMs: six of 300 to 600 a side (37) with 300 of 20 to 60 283 / 325, 1250 x 1250 (41) with 35 of
+// want whole SMs (if they are long enough to count: 182 of 3 to 20 a side with 11 of 200 to 500 (46) 326 / 338):
+// six of 300 to 600 a side (37) with 300 of 20 to 60 283 / 325, 1250 x 1250 (41) with 35 of
 // them 288 / 272, 1450 x 1450 (55) with 35 401 / 373.  All cloths joined in one
 // k_cg_persist against those two: 20 of 60 to 128 a side with 12 of 200 to 500 (44, even 39) 262 / 272, 50 with
 // four of 500 to 600 (47, even 42) 293 / 277, 35 of 20 to 60 with 12 of 200 to 500 (59, even 44) 357 / 279.
 constexpr int32_t kOnChipSlotsOne = 56, kOnChipSlots = 44;  // (the latter with the pieces)
-constexpr int32_t kOnChipOnly = 34, kOnChipUneven = 2, kOnChipBeside = 38;
+constexpr int32_t kOnChipOnly = 47, kOnChipUneven = 2, kOnChipBeside = 38;
+constexpr int64_t kBesideVertices = 40000;
 enum class Beside { none, resident, joined };
 
 bool on_chip_enough(const PersistPlan& P, Beside b) {
     if (P.grid == 0 || (b == Beside::resident && P.max_slots > kOnChipBeside)) return false;
     if (!P.one) return P.max_slots + P.max_pieces <= kOnChipSlots;
-    if (b == Beside::joined && P.max_slots <= kOnChipSlots) return true;
+    if (b == Beside::joined) return P.max_slots <= kOnChipSlots;
     return P.max_slots <= kOnChipOnly || (P.max_slots <= kOnChipSlotsOne && P.max_slots <= P.even_slots + kOnChipUneven);
 }
 
@@ -1544,7 +1547,10 @@ oc_status plan_execution(oc_solver* s, bool may_stream_all = true) {
     s->arrive = false;
     if (any_streamed && !any_coupled) {
         if (oc_status r = plan_persist(s, &s->pplan, streamed_ids)) return r;
-        const Beside b = join ? Beside::joined : s->buckets.empty() ? Beside::none : Beside::resident;
+        int64_t resident = 0;
+        for (int32_t k = 0; k < s->n_inst; ++k)
+            if (s->resident[(size_t)k]) resident += s->inst_host[(size_t)k].nv;
+        const Beside b = join ? Beside::joined : resident <= kBesideVertices ? Beside::none : Beside::resident;
         s->arrive = !on_chip_enough(s->pplan, b) && s->coop && s->arrive_per_sm > 0 &&
                     s->n_streamed_blocks <= (int64_t)arrive_max_entries_per_block() * arrive_grid(s);
         // Small cloths join the others on chip or not at all: in k_cg_arrive they cost more than beside it.
