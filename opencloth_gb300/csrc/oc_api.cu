@@ -1069,14 +1069,17 @@ oc_status alloc_error_word(oc_solver* s) {
 // (70,000) with both passes 48.8 and 42.7 / 45.1, seven of 128 x 128 50.8 and 44.8 / 48.9.
 // So do calls of one step where the launch shapes are more than the streams, so that some run one behind
 // the other: 15 cloths of 20 to 60 a side (9 shapes) 33.9 / 26.8, with Provot's pass 44.4 / 36.3; with 8 shapes
-// 27.8 / 26.8 and 33.5 / 34.9.
-constexpr int32_t kSimProvotMesh = 8192, kSimProvotTotal = 60000;
+// 27.8 / 26.8 and 33.5 / 34.9.  And where a thread has two vertices: one of 100 x 100 26.8 / 24.7, with Provot's
+// pass 36.5 / 31.2, three of 120 x 120 28.8 / 26.9, but six of 128 x 128 28.8 / 30.9.
+constexpr int32_t kSimProvotMesh = 8192, kSimOneTotal = 60000;
 
 int32_t sim_from_steps(const oc_solver* s) {  // the calls that k_sim takes: of this many steps at least
     for (const InstParams& ip : s->inst_host)
         if (ip.grid_cols <= 0 && (ip.passes & OC_PASS_PROVOT) && ip.nv > kSimProvotMesh)
-            return s->nv <= kSimProvotTotal ? std::numeric_limits<int32_t>::max() : 2;
-    return s->sim.size() > kMaxAux ? 2 : 1;
+            return s->nv <= kSimOneTotal ? std::numeric_limits<int32_t>::max() : 2;
+    bool two = s->sim.size() > kMaxAux;
+    for (const auto& g : s->sim) two = two || (g.launch.vpt > 1 && s->nv <= kSimOneTotal);
+    return two ? 2 : 1;
 }
 
 oc_status plan_sim(oc_solver* s) {

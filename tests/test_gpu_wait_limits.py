@@ -45,7 +45,7 @@ def check(parts, steps, block, polls, **kw):
 @pytest.mark.parametrize("polls", [50, 3000])
 @pytest.mark.parametrize("block", [0, 1])
 @pytest.mark.parametrize("passes", [0, PASS_PROVOT])
-@pytest.mark.parametrize("shapes", [[(30, 30)], [(60, 60)] * 3, [(120, 100)] * 5, [(30, 20), (100, 90), (60, 60)]],
+@pytest.mark.parametrize("shapes", [[(30, 30)], [(60, 60)] * 3, [(120, 101)] * 5, [(30, 20), (90, 90), (60, 60)]],
                          ids=["two CTAs", "clusters", "of sixteen", "groups"])
 def test_whole_steps_in_one_launch(shapes, passes, block, polls, steps):
     """k_sim: CTAs that give up at different exchanges leave their cluster together."""
