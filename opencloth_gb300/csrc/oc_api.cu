@@ -115,6 +115,9 @@ struct oc_solver {
     PersistPlan aplan{};
     bool aplan_made = false;
     PersistPlan pplan{};  // the streamed REFERENCE cloths' pieces (grid 0: none, or not available)
+    // Per cloth, the vertices whose A, r and d, and whose x, pplan (or cplan: all of the CG state) leaves in
+    // the planes, for account_step_bytes.
+    std::vector<int64_t> in_planes, x_in_planes;
     bool arrive = false;  // their CG runs in k_cg_arrive, their state in memory
     int arrive_per_sm = 0;
     unsigned* d_words = nullptr;  // k_cg_arrive: one arrival count per cloth
@@ -402,8 +405,15 @@ void account_step_bytes(const oc_solver* s, KernelTimer* t) {
             const double it = (double)st.iter;
             double dirs = it > 0 ? 37.0 * nv + 53.0 * nv * (it - 1.0) + 48.0 * ns * it : 0.0;
             if (st.flags & OC_FLAG_BREAKDOWN) dirs += (it > 0 ? 53.0 : 37.0) * nv + 48.0 * ns;
-            if (s->cpl_persist) {  // k_cpl_persist: the same passes and the update in one launch
-                t->bytes[K_CPL_PERSIST] += dirs + (it > 0 ? 132.0 * nv + 148.0 * nv * (it - 1.0) : 0.0) + 76.0 * nv;
+            if (s->cpl_persist) {
+                // k_cpl_persist: x, r, P^-1 and m' in (52 B) and, with the update, x out and X, V in and out
+                // (76 B) once; a direction pass reads z (and d) and the blocks, an update writes z and d.
+                // A vertex whose state is in the planes: m' and q in the first, z, d, x, r, q and P^-1 in the
+                // second instead.
+                const double pl = (double)s->in_planes[(size_t)k];
+                const double passes = it + (st.flags & OC_FLAG_BREAKDOWN ? 1.0 : 0.0);
+                t->bytes[K_CPL_PERSIST] += 128.0 * nv - 40.0 * pl + passes * (25.0 * nv + 48.0 * ns + 16.0 * pl) +
+                                           16.0 * nv * std::max(0.0, passes - 1.0) + it * (32.0 * nv + 116.0 * pl);
                 continue;
             }
             t->bytes[K_CPL_DIR] += dirs;
@@ -430,8 +440,17 @@ void account_step_bytes(const oc_solver* s, KernelTimer* t) {
         const double it = (double)st.iter;
         double dirs = it > 0 ? 36.0 * nv + 60.0 * nv * (it - 1.0) : 0.0;
         if (st.flags & OC_FLAG_BREAKDOWN) dirs += (it > 0 ? 60.0 : 36.0) * nv;
-        if (s->persist) {  // the same passes and the update in one launch
-            t->bytes[s->arrive ? K_CG_ARRIVE : K_CG_PERSIST] += dirs + 84.0 * nv * it + 76.0 * nv;
+        if (s->persist && !s->arrive) {
+            // k_cg_persist: the CG state and X, V in, x, X and V out once, as k_resident; what it leaves in the
+            // planes, A, r and d in and d or r out in every pass, x in and out in every update, instead.
+            const double pl = (double)s->in_planes[(size_t)k], xp = (double)s->x_in_planes[(size_t)k];
+            const double passes = it + (st.flags & OC_FLAG_BREAKDOWN ? 1.0 : 0.0);
+            t->bytes[K_CG_PERSIST] += 136.0 * nv - 48.0 * pl - 12.0 * xp + pl * (60.0 * passes - (passes > 0 ? 12.0 : 0.0)) +
+                                      it * (72.0 * pl + 24.0 * xp);
+            continue;
+        }
+        if (s->persist) {  // k_cg_arrive: the two kernels' passes and the update in one launch
+            t->bytes[K_CG_ARRIVE] += dirs + 84.0 * nv * it + 76.0 * nv;
             continue;
         }
         t->bytes[K_INTEGRATE] += 76.0 * nv;
@@ -1292,6 +1311,17 @@ oc_status plan_persist(oc_solver* s, PersistPlan* plan, const std::vector<int32_
         cut(2 * s->persist_pairs >= all ? 2 : 1, all);
     }
     if (P.smem > (size_t)s->persist_smem_max) return OC_OK;
+    if (plan == &s->pplan) {
+        s->in_planes.assign((size_t)s->n_inst, 0);
+        s->x_in_planes.assign((size_t)s->n_inst, 0);
+        for (const PersistPiece& pc : pieces) {
+            auto beyond = [&](int32_t slots) {
+                return (int64_t)std::max(0, pc.n - std::max(0, slots - pc.slot0) * kPersistThreads);
+            };
+            s->in_planes[(size_t)pc.inst] += beyond(P.chip_slots);
+            s->x_in_planes[(size_t)pc.inst] += beyond(P.chip_x);
+        }
+    }
     auto put = [&](auto** p, const auto& v) {
         auto* q = const_cast<std::remove_const_t<std::remove_pointer_t<std::remove_reference_t<decltype(*p)>>>*>(*p);
         const cudaError_t e = reupload(s, &q, v);
@@ -1368,6 +1398,8 @@ oc_status plan_coupled(oc_solver* s) {
         most = std::max(most, each);
     }
     P.smem_rows = (int32_t)std::min<int64_t>(most, s->cpl_rows_max);
+    s->in_planes.assign((size_t)s->n_inst, 0);
+    for (const CplPiece& pc : pieces) s->in_planes[(size_t)pc.inst] += std::max(0, pc.n - P.smem_rows);
     CplPiece* d = const_cast<CplPiece*>(P.pieces);
     OC_TRY(reupload(s, &d, pieces));
     P.pieces = d;

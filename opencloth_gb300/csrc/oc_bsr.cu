@@ -1070,7 +1070,9 @@ oc_status plan_bsr_persist(oc_bsr_solver* s, const std::vector<BsrParams>& sys) 
     s->persist_bytes = 0.0;
     for (int32_t k : ids) {
         const double rows = (double)sys[k].n_rows, blocks = (double)(s->nnz_off[k + 1] - s->nnz_off[k]);
-        s->persist_bytes += 40.0 * blocks + 61.0 * rows + sys[k].imax * (40.0 * blocks + 162.0 * rows);
+        // Once: the blocks, b, x, and r and p out (61 B a row), x out.  An iteration: the blocks, a row's
+        // counts and its r and p out (45 B); of a row beyond a thread's own, r, p and q in and out and x.
+        s->persist_bytes += 40.0 * blocks + 73.0 * rows + sys[k].imax * (40.0 * blocks + 45.0 * rows);
         const int64_t n = sys[k].n_rows, c = (n + chunk - 1) / chunk, each = ((n + c - 1) / c + 31) / 32 * 32;
         const size_t p0 = pieces.size();
         for (int64_t r = 0; r < n; r += each) {
@@ -1081,6 +1083,7 @@ oc_status plan_bsr_persist(oc_bsr_solver* s, const std::vector<BsrParams>& sys) 
             pc.n = (int32_t)std::min(each, n - r);
             pc.idx = (int32_t)(pieces.size() - p0);
             pc.packet = packets;
+            s->persist_bytes += sys[k].imax * 112.0 * std::max(0, pc.n - kOwnRows * kBT);
             pieces.push_back(pc);
         }
         for (size_t i = p0; i < pieces.size(); ++i) pieces[i].np = (int32_t)(pieces.size() - p0);

@@ -312,6 +312,7 @@ struct PersistPlan {
     int32_t smem_slots;        // slots of a CTA held in shared memory
     int32_t x_slots;           // slots of a CTA whose x is in shared memory
     int32_t on_chip;           // 1: no slot left in the planes
+    int32_t chip_slots, chip_x;  // slots whose A, r and d, and whose x, stay on chip through the loop
     size_t smem;               // dynamic shared memory
 };
 __host__ __device__ constexpr size_t persist_state_bytes(int max_pieces) {

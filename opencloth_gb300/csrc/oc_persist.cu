@@ -952,6 +952,7 @@ void persist_layout(PersistPlan* plan, int max_smem) {
     P.smem_slots = P.x_slots = 0;
     P.smem = fixed;
     P.on_chip = 1;
+    P.chip_slots = P.chip_x = P.max_slots;
     if (P.one && P.max_slots <= kFullSlots) return;
     P.smem_slots = std::max(0, P.max_slots - (P.one ? kOneRegSlots : kRegSlots));
     if (fixed >= room) P.smem_slots = 0;
@@ -960,6 +961,8 @@ void persist_layout(PersistPlan* plan, int max_smem) {
     if (P.smem < room) P.x_slots = (int32_t)std::min<size_t>((size_t)P.max_slots, (room - P.smem) / xs);
     P.smem += P.x_slots * xs;
     P.on_chip = P.x_slots == P.max_slots && P.smem <= room;
+    P.chip_slots = (P.one ? kOneRegSlots : kRegSlots) + P.smem_slots;
+    P.chip_x = P.x_slots;
 }
 
 cudaError_t prepare_persist(int device, int* max_smem, int* max_clusters, int* max_pairs) {
