@@ -404,12 +404,12 @@ class ClothSolver:
         return A9, b
 
     def profile(self, dt: float, n_steps: int) -> dict:
-        names = C.create_string_buffer(32 * 8)
-        ms = np.zeros(8, np.float64)
-        launches = np.zeros(8, np.int64)
-        byts = np.zeros(8, np.float64)
+        names = C.create_string_buffer(32 * 24)
+        ms = np.zeros(24, np.float64)
+        launches = np.zeros(24, np.int64)
+        byts = np.zeros(24, np.float64)
         n = C.c_int32()
-        self._call(self._lib.oc_profile_steps(self._h, float(dt), int(n_steps), 8, names, ptr(ms), ptr(launches),
+        self._call(self._lib.oc_profile_steps(self._h, float(dt), int(n_steps), 24, names, ptr(ms), ptr(launches),
                                               ptr(byts), C.byref(n)))
         raw = names.raw
         out = {}
