@@ -2756,7 +2756,7 @@ oc_status taped_forward(oc_solver* s, float dt) {
 
 // The plan of solve_only's one launch: where it can run every cloth (may_join) and the resident
 // launches are several (three or more) or one cluster's.  Measured, us of four steps forward and
-// back, start's resident launches and the one launch: 24 cloths of 16 to 96 a side 789 / 725, 18 of 16
+// back, the resident launches and the one launch: 24 cloths of 16 to 96 a side 789 / 725, 18 of 16
 // to 128 907 / 856; in the displacement mode, where every solve goes this way, one 64 x 64 cloth 585 /
 // 565, but 24 of them (one launch either way) 904 / 935 and 8 of them 646 / 674.
 oc_status plan_adjoint(oc_solver* s) {
