@@ -336,7 +336,7 @@ oc_status oc_tune_cache_lookup(const char* path, const char* key, oc_launch_conf
 oc_status oc_tune_cache_store(const char* path, const char* key, const oc_launch_config* cfg, double ms_per_step);
 
 /* ---- testing aid: the bounded waits ------------------------------------------------- */
-/* The CTAs of a CG launch (k_cg_persist, k_cpl_persist, k_sim, k_resident) wait for one another's partial sums.
+/* The CTAs of a CG launch (k_cg_persist, k_cg_arrive, k_cpl_persist, k_sim, k_resident) wait for one another's partial sums.
  * Each wait gives up after a bounded number of polls, or when another wait of the handle has given
  * up; the step then fails with OC_ERR_DEVICE_TIMEOUT at the next oc_synchronize / oc_get_state /
  * oc_get_stats, after which the handle steps on.  A cloth whose solve had not ended on any of its CTAs
